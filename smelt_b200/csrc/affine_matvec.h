@@ -38,8 +38,8 @@ struct AffineArgs {
     AffineSeg seg[3];
     int ks, nsplit;        // filled by the launcher
     int sm_count;          // SMs of the device (0 = assume 148)
-    // Tensor-memory QMM only: where CTAs that split a row tile's K leave their fp32 sums
-    // (part_scratch_bytes bytes) and count their arrivals (one int per row tile, 4096 of them,
+    // Tensor-core product only: where CTAs that share a tile leave their fp32 sums
+    // (part_scratch_bytes bytes) and count their arrivals (one int per tile, 4096 of them,
     // all zero between launches).  Launches that use them must not overlap on the device.
     float* part_scratch;
     size_t part_scratch_bytes;
@@ -50,10 +50,10 @@ struct AffineArgs {
 
 cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int group);
 cudaError_t launch_affine_stream(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
-// Tensor-memory QMM for batches of seventeen rows and more (affine_qmm.cu).
-cudaError_t launch_affine_qmm(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
-// Wide-batch form (more than 64 rows of x): accumulates all of K in tensor memory (affine_qmm_wide.cu).
-cudaError_t launch_affine_qmm_wide(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
+// Tensor-core product for seventeen rows of x and more (affine_wide.cu).
+cudaError_t launch_affine_wide(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
+// Whether the streaming kernel takes the launch (its first pass, of up to sixteen rows).
+bool affine_stream_takes(int mode, const AffineArgs& args, int group);
 cudaError_t launch_affine_imma(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
 
 }  // namespace smelt

@@ -379,36 +379,49 @@ cudaError_t launch_stream_mode(const Launch& l, const AffineArgs& a, bool* handl
 
 }  // namespace
 
+// Passes over the weights that the launch takes, 0 where the kernel does not take it.
+static int stream_passes(int mode, const AffineArgs& a, int group) {
+    if (group != kGroup || a.batch > 16 || a.cols % kStageCols != 0) return 0;
+    const int nw = (mode == kAffineGateUp || mode == kAffineDual) ? 2 : 1;
+    if (a.nseg > 1) {
+        for (int i = 0; i < a.nseg; ++i) {
+            if ((reinterpret_cast<uintptr_t>(a.seg[i].w) | reinterpret_cast<uintptr_t>(a.seg[i].s) | reinterpret_cast<uintptr_t>(a.seg[i].b)) & 15u) return 0;
+            if (i + 1 < a.nseg && a.seg[i].rows % kTileRows != 0) return 0;
+        }
+    } else {
+        for (int s = 0; s < nw; ++s)
+            if ((reinterpret_cast<uintptr_t>(a.w[s]) | reinterpret_cast<uintptr_t>(a.s[s]) | reinterpret_cast<uintptr_t>(a.b[s])) & 15u) return 0;
+    }
+    if (a.norm_w && (reinterpret_cast<uintptr_t>(a.norm_w) & 15u)) return 0;
+    if (reinterpret_cast<uintptr_t>(a.x) & 15u) return 0;
+    // Rows of the batch that fit in shared memory beside the shallowest ring go in one pass;
+    // a larger batch (or very wide activations) takes up to four passes over the same weights,
+    // which the later passes find in L2 for the matrices of a decoder layer.
+    int bmax = a.batch < 8 ? a.batch : 8;
+    while (bmax > 0 && stream_layout(nw, 3, a.cols, bmax, 8).total > 226u * 1024u) --bmax;
+    if (bmax == 0) return 0;
+    const int passes = (a.batch + bmax - 1) / bmax;
+    if (passes > 4) return 0;
+    // Eight rows or fewer that need two passes: the general kernel's K split over a cluster is as fast.
+    if (passes > 1 && a.batch <= 8 && !a.norm_w && a.nseg <= 1) return 0;
+    return passes;
+}
+
+bool affine_stream_takes(int mode, const AffineArgs& args, int group) {
+    AffineArgs a = args;
+    if (a.batch > 16) a.batch = 16;
+    return (a.nseg <= 1 || (mode == kAffinePlain && a.nseg <= 3)) && stream_passes(mode, a, group) > 0;
+}
+
 // Launches the streaming kernel when the shape is eligible (group 64, batch <= 16, cols a
 // multiple of 1024, 16-byte aligned operands; up to eight batch rows per pass, fewer when the
 // activations would not stay resident);
 // *handled tells the caller whether it did.
 cudaError_t launch_affine_stream(const Launch& l, int mode, const AffineArgs& a, int group, bool* handled) {
     *handled = false;
-    if (group != kGroup || a.batch > 16 || a.cols % kStageCols != 0) return cudaSuccess;
-    const int nw = (mode == kAffineGateUp || mode == kAffineDual) ? 2 : 1;
-    if (a.nseg > 1) {
-        if (nw != 1 || a.nseg > 3 || mode != kAffinePlain) return cudaErrorInvalidValue;
-        for (int i = 0; i < a.nseg; ++i) {
-            if ((reinterpret_cast<uintptr_t>(a.seg[i].w) | reinterpret_cast<uintptr_t>(a.seg[i].s) | reinterpret_cast<uintptr_t>(a.seg[i].b)) & 15u) return cudaSuccess;
-            if (i + 1 < a.nseg && a.seg[i].rows % kTileRows != 0) return cudaSuccess;
-        }
-    } else {
-        for (int s = 0; s < nw; ++s)
-            if ((reinterpret_cast<uintptr_t>(a.w[s]) | reinterpret_cast<uintptr_t>(a.s[s]) | reinterpret_cast<uintptr_t>(a.b[s])) & 15u) return cudaSuccess;
-    }
-    if (a.norm_w && (reinterpret_cast<uintptr_t>(a.norm_w) & 15u)) return cudaSuccess;
-    if (reinterpret_cast<uintptr_t>(a.x) & 15u) return cudaSuccess;
-    // Rows of the batch that fit in shared memory beside the shallowest ring go in one pass;
-    // a larger batch (or very wide activations) takes up to four passes over the same weights,
-    // which the later passes find in L2 for the matrices of a decoder layer.
-    int bmax = a.batch < 8 ? a.batch : 8;
-    while (bmax > 0 && stream_layout(nw, 3, a.cols, bmax, 8).total > 226u * 1024u) --bmax;
-    if (bmax == 0) return cudaSuccess;
-    const int passes = (a.batch + bmax - 1) / bmax;
-    if (passes > 4) return cudaSuccess;
-    // Eight rows or fewer that need two passes: the general kernel's K split over a cluster is as fast.
-    if (passes > 1 && a.batch <= 8 && !a.norm_w && a.nseg <= 1) return cudaSuccess;
+    if (a.nseg > 1 && (mode != kAffinePlain || a.nseg > 3) && group == kGroup && a.batch <= 16 && a.cols % kStageCols == 0) return cudaErrorInvalidValue;
+    const int passes = stream_passes(mode, a, group);
+    if (passes == 0) return cudaSuccess;
     const int per_pass = (a.batch + passes - 1) / passes;
     for (int b0 = 0; b0 < a.batch; b0 += per_pass) {
         AffineArgs p = a;

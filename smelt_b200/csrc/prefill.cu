@@ -9,7 +9,7 @@
 // causally to keys [seqStart, startPos + t], seqStart from the sliding window, softmax in fp32,
 // fp16 out [T, qHeads, headDim].  The matmuls of the chunk are the batched affine kernels
 // (agent_affine_qmm_fixed_batched_full, Resources/Shaders/agent_affine_qmm.h:107-316), which
-// from seventeen rows on run on the tensor-memory QMM (affine_qmm.cu).
+// from seventeen rows on run on the tensor-core product (affine_wide.cu).
 //
 // attn_prefill_kernel: one CTA per (eight consecutive query positions, KV head); warp w owns
 // position 8 * block + w with all query heads that share the KV head, on the decode kernel's

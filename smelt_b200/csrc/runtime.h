@@ -144,7 +144,7 @@ struct smelt_cuda_ctx {
     void* attn_scratch = nullptr;
     size_t attn_scratch_bytes = 0;
     float* rope_table = nullptr;   // cos | sin of the current position (256 floats), written once per interpretation
-    float* qmm_scratch = nullptr;  // tensor-memory QMM: fp32 sums of CTAs that split a row tile's K (affine_qmm.cu)
+    float* qmm_scratch = nullptr;  // tensor-core product: fp32 sums of CTAs that share a tile (affine_wide.cu)
     size_t qmm_scratch_bytes = 0;
     void* prefill_scratch = nullptr;  // activations of one prompt chunk (prefill.cu), grown on demand
     size_t prefill_scratch_bytes = 0;

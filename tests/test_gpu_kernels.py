@@ -173,6 +173,32 @@ def test_affine_qmm_modes(ctx, oracle, rows, cols, batch):
         buf.free()
 
 
+# the same product where its tiles, stages and shares of a tile end: one group, part of a stage, rows and columns that no tile
+# divides, tiles of one CTA and of several, each width of the accumulator
+@pytest.mark.parametrize("batch", [17, 64, 65, 130, 257])
+@pytest.mark.parametrize("rows,cols", [(8, 64), (72, 192), (264, 576), (1000, 1984), (2056, 320)])
+def test_affine_wide_edges(ctx, oracle, rows, cols, batch):
+    a, b = (synth.affine_u4(34, n, rows, cols, 64) for n in ("wa", "wb"))
+    x, res = synth.activations(34, "wx", batch, cols), synth.activations(34, "wres", batch, rows)
+    d = dev(ctx, *a, *b, x, res)
+    y0, y1 = ctx.alloc(batch * rows * 2 + 64).fill(0xFF), ctx.alloc(batch * rows * 2 + 64).fill(0xFF)
+    ref_a, ref_b = (oracle.affine_matvec(*m, x, rows, cols, 64) for m in (a, b))
+    ctx.call("affine_dual_matvec", *d[:7], y0, y1, rows, cols, 64, batch)
+    assert rel_err(y0.download(np.float16, (batch, rows)), ref_a) < REL_TOL and rel_err(y1.download(np.float16, (batch, rows)), ref_b) < REL_TOL
+    ctx.call("affine_matvec_add", *d[:3], d[6], d[7], y0, rows, cols, 64, batch)
+    assert add_rel_err(y0.download(np.float16, (batch, rows)), oracle.affine_matvec_add(*a, x, res, rows, cols, 64), ref_a) < REL_TOL
+    ctx.call("affine_gate_up_swiglu", *d[:7], y1, rows, cols, 64, batch)
+    assert rel_err(y1.download(np.float16, (batch, rows)), oracle.affine_gate_up_swiglu(*a, *b, x, rows, cols, 64, round_gate_up=False)) < REL_TOL
+    first = y1.download(np.uint16, (batch, rows))
+    ctx.call("affine_gate_up_swiglu", *d[:7], y1, rows, cols, 64, batch)
+    assert np.array_equal(y1.download(np.uint16, (batch, rows)), first)  # run-to-run determinism
+    for y in (y0, y1):
+        assert np.all(y.download(np.uint8, (64,), offset=batch * rows * 2) == 0xFF)
+    assert ctx.device_error() == 0
+    for buf in d + [y0, y1]:
+        buf.free()
+
+
 # batch 1 and 2 run on the integer-MMA kernel: every mode, row / K tails, long K, few chunks per warp
 IMMA_SHAPES = [(4096, 4096, 1), (4096, 12288, 1), (100, 128, 2), (48, 256, 1), (1000, 2048, 2), (6144, 4096, 2), (16, 8192, 1)]
 
