@@ -39,6 +39,7 @@ enum DenseMode : int {
     kDenseAddF32 = 1,      // y0 fp32, added to
     kDenseStoreAct = 2,    // y0 and y1 in the activations' type
     kDenseStoreMixed = 3,  // y0 fp32, y1 in the activations' type
+    kDenseStoreF16 = 5,    // W and X in fp16: y0 fp16, clamped to its finite range
     kDenseStoreGlu = 4,    // rows are (gate, up) pairs: y0[row / 2] = clamped_glu, in the activations' type
 };
 // Applied to the rows from `split` on; in kDenseStoreF32 kDenseDecay applies to all rows.

@@ -12,6 +12,8 @@
 // the launch in front.  With experts, a unit is a row tile of one expert's matrix and up to BN rows
 // of the activations that chose it, both taken from a table that an earlier launch has written.
 //
+// fp16 weights and activations go the same way (kDenseStoreF16: the LM head of several sequences).
+//
 // Every wait is bounded: on expiry the CTA raises bit 11 of the device error word, its roles stop,
 // copies and MMAs in flight are waited for (bounded too) and the tensor memory is freed.
 //
@@ -178,7 +180,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBlockRows >> 4) << 24);  // f32 += bf16 x bf16, K-major both
+            constexpr uint32_t kType = MODE == kDenseStoreF16 ? 0u : (1u << 7) | (1u << 10);  // fp16 or bf16, both operands
+            constexpr uint32_t idesc = (1u << 4) | kType | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBlockRows >> 4) << 24);  // fp32 sums, K-major both
             uint32_t it = 0, done = 0;
             bool alive = true;
             for (int u = blockIdx.x; u < units && alive; u += gridDim.x, ++done) {
@@ -284,7 +287,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
 #pragma unroll
                             for (int j = 0; j < kChunk; ++j) v[j] += b;
                         }
-                        if (MODE == kDenseAddF32) {
+                        if (MODE == kDenseStoreF16) {
+                            __half* y = static_cast<__half*>(a.out.y0) + (size_t)(m0 + c0) * a.out.ld0 + row;
+#pragma unroll
+                            for (int j = 0; j < kChunk; ++j)
+                                if (c0 + j < cnt) y[(size_t)j * a.out.ld0] = __float2half_rn(fminf(fmaxf(v[j], -65504.f), 65504.f));
+                        } else if (MODE == kDenseAddF32) {
                             float* y = static_cast<float*>(a.out.y0) + (size_t)(m0 + c0) * a.out.ld0 + row;
 #pragma unroll
                             for (int j = 0; j < kChunk; ++j)
@@ -361,6 +369,7 @@ cudaError_t launch_bf16_t(const Launch& l, int mode, const DenseGemmArgs& a, con
     switch (mode) {
         case kDenseStoreF32: return a.out.act == kDenseDecay ? go(gemm_bf16_kernel<BN, kDenseStoreF32, kDenseDecay, false>) : go(gemm_bf16_kernel<BN, kDenseStoreF32, kDenseXielu, false>);
         case kDenseAddF32: return go(gemm_bf16_kernel<BN, kDenseAddF32, kDenseXielu, false>);
+        case kDenseStoreF16: return go(gemm_bf16_kernel<BN, kDenseStoreF16, kDenseXielu, false>);
         case kDenseStoreAct:
             switch (a.out.act) {
                 case kDenseXielu: return go(gemm_bf16_kernel<BN, kDenseStoreAct, kDenseXielu, false>);
@@ -510,7 +519,7 @@ cudaError_t launch_f32(const Launch& l, int mode, const DenseGemmArgs& a) {
 
 cudaError_t launch_dense_gemm(const Launch& l, DenseType type, int mode, const DenseGemmArgs& a) {
     if (a.rows <= 0 || a.cols <= 0 || a.cols % 64 || a.m <= 0 || (mode != kDenseStoreAct && mode != kDenseStoreMixed && a.out.split != a.rows)) return cudaErrorInvalidValue;
-    if ((a.group_rows && (a.group_rows % kBlockRows || a.x_group < a.m || a.groups <= 0)) || (a.table && (a.experts <= 0 || a.max_entries <= 0 || a.group_rows)) || (mode == kDenseStoreGlu && (!a.table || a.rows % kBlockRows)) || (mode == kDenseAddF32 && a.out.bias))
+    if ((a.group_rows && (a.group_rows % kBlockRows || a.x_group < a.m || a.groups <= 0)) || (a.table && (a.experts <= 0 || a.max_entries <= 0 || a.group_rows)) || (mode == kDenseStoreGlu && (!a.table || a.rows % kBlockRows)) || (mode == kDenseAddF32 && a.out.bias) || (mode == kDenseStoreF16 && (type == kDenseF32 || a.table || a.out.bias)))
         return cudaErrorInvalidValue;
     if ((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.x)) & 15u) return cudaErrorInvalidValue;
     return type == kDenseF32 ? launch_f32(l, mode, a) : launch_bf16(l, mode, a);

@@ -2,6 +2,7 @@
 // RoPE, KV-cache append, argmax, the on-device u4 dequant probe and the dense fp16 matvec
 // used as LM head.  Each kernel cites the reference kernel whose arithmetic and rounding
 // points it keeps.
+#include "dense.h"
 #include "glue.h"
 #include "rope.cuh"
 
@@ -477,6 +478,19 @@ cudaError_t launch_argmax_reduce(const Launch& l, const uint64_t* partials, int3
 cudaError_t launch_fp16_matvec(const Launch& l, const __half* w, const __half* x, __half* y, int rows, int cols,
                                int batch, int sm_count) {
     if (cols % 8 != 0 || batch <= 0) return cudaErrorInvalidValue;
+    if (std::min(batch, 8) * (size_t)cols * 2 > 200 * 1024) return cudaErrorInvalidValue;
+    // Several rows: one row of weights for all of them on the tensor cores, at HBM speed, where a warp per row spends its time
+    // on two conversions and eight FMAs per weight and row of x, once per eight rows (151936 x 4096, us: 8 rows 885 -> 228,
+    // 32 rows 3535 -> 256).  The kernel has no guard of its own.
+    if (batch > 1 && cols % 64 == 0 && !l.guard_lt && !l.guard_ge && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0) {
+        DenseGemmArgs a = {};
+        a.w = reinterpret_cast<const bf16*>(w);  // two bytes an element either way
+        a.x = x;
+        a.rows = rows; a.cols = cols; a.m = batch;
+        a.out.y0 = y; a.out.ld0 = rows; a.out.split = rows;
+        a.sm_count = sm_count;
+        return launch_dense_gemm(l, kDenseBf16, kDenseStoreF16, a);
+    }
     for (int b0 = 0; b0 < batch; b0 += 8) {
         const int nb = batch - b0 < 8 ? batch - b0 : 8;
         const size_t smem = (size_t)nb * cols * 2;

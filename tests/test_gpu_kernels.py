@@ -422,6 +422,22 @@ def test_fp16_matvec(ctx, oracle, rows, cols, batch):
     assert rel_err(got, oracle.fp16_matvec(w, x, rows, cols)) < REL_TOL
 
 
+# several rows run on the tensor cores: fewer rows than a tile, tails of both, each tile width, two tiles of x; 72 columns do not
+@pytest.mark.parametrize("rows,cols,batch", [(1, 64, 2), (130, 192, 17), (4100, 1024, 33), (257, 64, 300), (136, 72, 5)])
+def test_fp16_matvec_several_rows(ctx, oracle, rows, cols, batch):
+    w, x = synth.normal_f16(6, "head", (rows, cols), 0.02), synth.activations(6, "x", batch, cols)
+    w[0, :] = 60000.0  # the first output leaves the finite range where its activations' sum is large enough
+    x[0, :] = 1.0
+    dw, dx = dev(ctx, w, x)
+    y = ctx.alloc(batch * rows * 2 + 64).fill(0xFF)
+    ctx.call("fp16_matvec", dw, dx, y, rows, cols, batch)
+    got, want = y.download(np.float16, (batch, rows)), oracle.fp16_matvec(w, x, rows, cols)
+    assert got[0, 0] == np.float16(65504)
+    if rows > 1:
+        assert rel_err(got[:, 1:], want[:, 1:]) < REL_TOL
+    assert np.all(y.download(np.uint8, (64,), offset=batch * rows * 2) == 0xFF)
+
+
 def test_fp16_matvec_clamps(ctx):
     w = np.full((8, 64), 60000.0, np.float16)
     x = np.ones(64, np.float16)
