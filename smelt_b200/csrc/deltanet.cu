@@ -12,6 +12,8 @@
 // (32 KB per head at D = 128): one warp per (head, output row) with the row's Dk values in
 // registers, lane l holding dk = l * D/32 ..., exactly the reference's partition, so that the two
 // warp sums run over the same operands in the same order.
+#include <algorithm>
+
 #include <string>
 
 #include "common.cuh"
@@ -141,14 +143,21 @@ __global__ void __launch_bounds__(256) deltanet_recurrence_decode_kernel(__half*
 // products with fp16 weights are exact in fp32, which makes the fused multiply-adds of the
 // c6144_k4 specialisation and the per-token rounding of the checkpoint variant equal to the
 // generic kernel; one body serves the three names.  history (may be null) [T + 1, C, K].
+//
+// A CTA owns 32 channels (its lanes) and cuts the chunk into one stretch of positions per warp.  The outputs replace the
+// inputs, so every warp takes the inputs in front of its stretch before any warp writes; inside a stretch eight positions are
+// loaded at a time.  The chain it replaces walked all positions with one load in flight: 136 us at 300 positions of 8192
+// channels, 17 us here.
+constexpr int kConvWarps = 32, kConvAhead = 8;
 template <int K>
-__global__ void __launch_bounds__(128) conv1d_update_silu_prefill_kernel(__half* state, __half* qkv, const __half* weight, int seq_len,
-                                                                         int channels, int kernel_size, __half* history, DevDyn dyn) {
+__global__ void __launch_bounds__(kConvWarps * 32) conv1d_update_silu_prefill_kernel(__half* state, __half* qkv, const __half* weight, int seq_len,
+                                                                                     int channels, int kernel_size, __half* history, DevDyn dyn) {
     pdl_trigger();
     pdl_wait();
     if (dyn_skip(dyn)) return;
-    const int ch = blockIdx.x * blockDim.x + threadIdx.x;
-    if (ch >= channels) return;
+    const int ch = blockIdx.x * 32 + (threadIdx.x & 31), warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int len = (seq_len + warps - 1) / warps, p0 = min(seq_len, warp * len), p1 = min(seq_len, p0 + len);
+    const bool in = ch < channels;
     const int ks = K > 0 ? K : kernel_size;
     __half* st = state + (size_t)ch * ks;
     const size_t hs = (size_t)channels * ks;
@@ -156,35 +165,45 @@ __global__ void __launch_bounds__(128) conv1d_update_silu_prefill_kernel(__half*
     float w[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-        if (k < ks) {
-            cached[k] = st[k];
+        if (k < ks && in) {
+            const int pos = p0 - ks + k;  // the taps as position p0 finds them
+            cached[k] = pos < 0 ? st[ks + pos] : qkv[(size_t)pos * channels + ch];
             w[k] = __half2float(weight[(size_t)ch * ks + k]);
-            if (history) history[(size_t)ch * ks + k] = cached[k];
+            if (history && warp == 0) history[(size_t)ch * ks + k] = cached[k];
         }
-    __half x = seq_len > 0 ? qkv[ch] : __ushort_as_half(0);
-    for (int pos = 0; pos < seq_len; ++pos) {
-        const __half next = pos + 1 < seq_len ? qkv[(size_t)(pos + 1) * channels + ch] : __ushort_as_half(0);
+    __syncthreads();
+    if (!in) return;
+    for (int base = p0; base < p1; base += kConvAhead) {
+        __half x[kConvAhead];
 #pragma unroll
-        for (int k = 0; k < 7; ++k)
-            if (k + 1 < ks) cached[k] = cached[k + 1];
+        for (int j = 0; j < kConvAhead; ++j) x[j] = base + j < p1 ? qkv[(size_t)(base + j) * channels + ch] : __ushort_as_half(0);
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k == ks - 1) cached[k] = x;
-        float acc = 0.0f;
+        for (int j = 0; j < kConvAhead; ++j) {
+            const int pos = base + j;
+            if (pos >= p1) break;
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < ks) acc = __fadd_rn(acc, __fmul_rn(__half2float(cached[k]), w[k]));
-        qkv[(size_t)pos * channels + ch] = silu_staged_half(__float2half_rn(acc));
-        if (history) {
+            for (int k = 0; k < 7; ++k)
+                if (k + 1 < ks) cached[k] = cached[k + 1];
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-                if (k < ks) history[(size_t)(pos + 1) * hs + (size_t)ch * ks + k] = cached[k];
-        }
-        x = next;
-    }
+                if (k == ks - 1) cached[k] = x[j];
+            float acc = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
-        if (k < ks) st[k] = cached[k];
+            for (int k = 0; k < 8; ++k)
+                if (k < ks) acc = __fadd_rn(acc, __fmul_rn(__half2float(cached[k]), w[k]));
+            qkv[(size_t)pos * channels + ch] = silu_staged_half(__float2half_rn(acc));
+            if (history) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (k < ks) history[(size_t)(pos + 1) * hs + (size_t)ch * ks + k] = cached[k];
+            }
+        }
+    }
+    if (p1 == seq_len && p0 < p1) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k < ks) st[k] = cached[k];
+    }
 }
 
 // Prompt chunk of the recurrence (prefill_recurrence.metal:290-775).  The loop over positions
@@ -480,7 +499,8 @@ cudaError_t launch_conv1d_update_silu_prefill(const Launch& l, __half* state, __
     if (channels <= 0 || kernel_size <= 0 || kernel_size > 8 || seq_len < 0) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    cfg_launch(l, cfg, attr, dim3((channels + 127) / 128), dim3(128));
+    const int warps = std::max(1, std::min(kConvWarps, (seq_len + kConvAhead - 1) / kConvAhead));
+    cfg_launch(l, cfg, attr, dim3((channels + 31) / 32), dim3(warps * 32));
     if (kernel_size == 4) {
         prefer_max_shared(conv1d_update_silu_prefill_kernel<4>);
         return cudaLaunchKernelEx(&cfg, conv1d_update_silu_prefill_kernel<4>, state, qkv, weight, seq_len, channels, kernel_size, history, dev_dyn(l));

@@ -369,6 +369,13 @@ def test_oracle_conv1d_prefill_is_the_iterated_update(oracle):
     assert np.array_equal(st.view(np.uint16), cur.view(np.uint16))
 
 
+# stretches of positions: shorter than the taps, one warp's and several', a ragged last one, channels that fill no warp
+@pytest.mark.gpu
+@pytest.mark.parametrize("channels,ksize,seq_len", [(96, 4, 300), (40, 8, 41), (33, 2, 257), (40, 8, 9)])
+def test_conv1d_prefill_stretches(ctx, oracle, channels, ksize, seq_len):
+    test_conv1d_update_silu_prefill(ctx, oracle, channels, ksize, seq_len, True)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("channels,ksize,seq_len,history", [(6144, 4, 65, False), (6144, 4, 3, True), (1000, 4, 64, False), (512, 3, 17, True), (64, 8, 1, False), (64, 8, 0, False)])
 def test_conv1d_update_silu_prefill(ctx, oracle, channels, ksize, seq_len, history):
