@@ -109,10 +109,10 @@ __device__ __forceinline__ void tile_scores(const unsigned char* ku, const uint3
 }
 
 // Its first half with the online softmax of the tile's columns.
-// valid_a / valid_b: this thread's keys g and g + 8 of the tile take part.  Leaves P^T as fp16
+// valid: whether this thread's key g takes part in columns 2t and 2t + 1, then the same for its key g + 8.  Leaves P^T as fp16
 // high and low parts in B-operand layout (pb0, pb1, pl0, pl1) and rescales m_run, l_run, o.
 template <int D, int NH>
-__device__ __forceinline__ void tile_scores_softmax(const unsigned char* ku, const uint32_t (&qf)[NH][D / 8], bool valid_a, bool valid_b,
+__device__ __forceinline__ void tile_scores_softmax(const unsigned char* ku, const uint32_t (&qf)[NH][D / 8], const bool (&valid)[NH][4],
                                                     float scale2, float (&m_run)[NH][2], float (&l_run)[NH][2], float (&o)[NH][D / 16][4],
                                                     uint32_t (&pb0)[NH], uint32_t (&pb1)[NH], uint32_t (&pl0)[NH], uint32_t (&pl1)[NH]) {
     constexpr int MT = D / 16;
@@ -122,8 +122,8 @@ __device__ __forceinline__ void tile_scores_softmax(const unsigned char* ku, con
     // ── online softmax per query head (columns 2t, 2t+1 of the tile) ──
 #pragma unroll
     for (int nh = 0; nh < NH; ++nh) {
-        float v0 = valid_a ? s[nh][0] * scale2 : kNegBig, v1 = valid_a ? s[nh][1] * scale2 : kNegBig;
-        float v2 = valid_b ? s[nh][2] * scale2 : kNegBig, v3 = valid_b ? s[nh][3] * scale2 : kNegBig;
+        float v0 = valid[nh][0] ? s[nh][0] * scale2 : kNegBig, v1 = valid[nh][1] ? s[nh][1] * scale2 : kNegBig;
+        float v2 = valid[nh][2] ? s[nh][2] * scale2 : kNegBig, v3 = valid[nh][3] ? s[nh][3] * scale2 : kNegBig;
         float mx0 = fmaxf(v0, v2), mx1 = fmaxf(v1, v3);
 #pragma unroll
         for (int off = 4; off < 32; off <<= 1) {
@@ -134,8 +134,8 @@ __device__ __forceinline__ void tile_scores_softmax(const unsigned char* ku, con
         const float c0 = exp2f(m_run[nh][0] - mn0), c1 = exp2f(m_run[nh][1] - mn1);
         m_run[nh][0] = mn0; m_run[nh][1] = mn1;
         // p = hi + lo with both halves fp16: the tensor pipe sees 22 significant bits of p
-        const float p0 = valid_a ? exp2f(v0 - mn0) : 0.f, p1 = valid_a ? exp2f(v1 - mn1) : 0.f;
-        const float p2 = valid_b ? exp2f(v2 - mn0) : 0.f, p3 = valid_b ? exp2f(v3 - mn1) : 0.f;
+        const float p0 = valid[nh][0] ? exp2f(v0 - mn0) : 0.f, p1 = valid[nh][1] ? exp2f(v1 - mn1) : 0.f;
+        const float p2 = valid[nh][2] ? exp2f(v2 - mn0) : 0.f, p3 = valid[nh][3] ? exp2f(v3 - mn1) : 0.f;
         const __half2 pa = __floats2half2_rn(p0, p1), pb = __floats2half2_rn(p2, p3);
         const float2 paf = __half22float2(pa), pbf = __half22float2(pb);
         const __half2 pa_lo = __floats2half2_rn(p0 - paf.x, p1 - paf.y), pb_lo = __floats2half2_rn(p2 - pbf.x, p3 - pbf.y);
@@ -409,7 +409,10 @@ __device__ __forceinline__ void attn_decode_body(const AttnDev& p, float* smem_f
         const unsigned char* ku = ring + (size_t)(unit % NU) * CH * 512;
 
         uint32_t pb0[NH], pb1[NH], pl0[NH], pl1[NH];
-        tile_scores_softmax<D, NH>(ku, qf, valid_a, valid_b, scale2, m_run, l_run, o, pb0, pb1, pl0, pl1);
+        bool valid[NH][4];
+#pragma unroll
+        for (int nh = 0; nh < NH; ++nh) { valid[nh][0] = valid[nh][1] = valid_a; valid[nh][2] = valid[nh][3] = valid_b; }
+        tile_scores_softmax<D, NH>(ku, qf, valid, scale2, m_run, l_run, o, pb0, pb1, pl0, pl1);
 
         // ── O^T += V^T · P^T ──
         issue_unit(unit + NU);

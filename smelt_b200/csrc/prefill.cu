@@ -11,13 +11,14 @@
 // (agent_affine_qmm_fixed_batched_full, Resources/Shaders/agent_affine_qmm.h:107-316), which
 // from seventeen rows on run on the tensor-core product (affine_wide.cu).
 //
-// attn_prefill_kernel: one CTA per (eight consecutive query positions, KV head); warp w owns
-// position 8 * block + w with all query heads that share the KV head, on the decode kernel's
-// tile arithmetic (attention.cuh: S^T = K.Q^T and O^T = V^T.P^T on mma.sync, P as fp16 high +
-// low parts).  The CTA walks the 16-key tiles up to its last position's causal limit; a tile's
-// K and V halves are copied once per CTA with cp.async into one of two buffers, in the
-// piece-per-lane layout the tile functions read, and every warp masks the keys beyond its own
-// position.  No split over keys and no merge: a prompt chunk has positions enough to fill the GPU.
+// attn_prefill_kernel: one CTA per (run of query positions, KV head) on the decode kernel's tile arithmetic (attention.cuh:
+// S^T = K.Q^T and O^T = V^T.P^T on mma.sync, P as fp16 high + low parts).  A tile has eight columns: the query heads that
+// share the KV head, at as many positions as fit, so four heads take two positions a warp.  The CTA walks the 16-key
+// tiles up to its last position's causal limit, KS of them at a time, each for a set of warps of its own; a tile's
+// K and V halves are copied once per CTA with cp.async into one of two buffers, in the piece-per-lane layout the tile
+// functions read, and every column masks the keys beyond its own position.  The key sets' states are merged through
+// shared memory in order.  Against one position a warp and one key set (32 query and 8 KV heads of 128, us): 512 positions
+// from 0 71.1 -> 49.9, 77 positions from 1300 87.6 -> 55.6.
 //
 // smelt_cuda_prefill drives a plain attention decoder (the descriptor smelt_cuda_build_decoder
 // takes, one sequence, one GPU) chunk by chunk and leaves the KV caches and the argmax of the
@@ -36,34 +37,61 @@ namespace {
 
 using namespace attn;
 
-__global__ void __launch_bounds__(128) rope_kv_prefill_kernel(__half* q, __half* k, const __half* v, const __half* cos_t,
-                                                              const __half* sin_t, __half* k_cache, __half* v_cache, int head_dim,
-                                                              int rope_dim, int q_heads, int kv_heads, uint32_t start_pos,
-                                                              uint32_t capacity, int layout, float base_log2, int math_mode,
-                                                              size_t table_stride) {
+// One CTA per position.  The angles are evaluated once per pair (in double where they are analytic), before the wait for the
+// launch in front if no table holds them; then the threads take (head, pair) items, four loads in flight each.  With a
+// thread per pair that walked the heads the kernel waited for one load after the other: 27.4 us at 512 positions of 32 + 8
+// heads of 128, 11.4 us here.
+constexpr int kRopeThreads = 256;
+__global__ void __launch_bounds__(kRopeThreads) rope_kv_prefill_kernel(__half* q, __half* k, const __half* v, const __half* cos_t,
+                                                                       const __half* sin_t, __half* k_cache, __half* v_cache, int head_dim,
+                                                                       int rope_dim, int q_heads, int kv_heads, uint32_t start_pos,
+                                                                       uint32_t capacity, int layout, float base_log2, int math_mode,
+                                                                       size_t table_stride) {
+    extern __shared__ float4 trig[];  // {cos, sin} of a pair's first and second element
     pdl_trigger();
-    pdl_wait();
+    if (cos_t) pdl_wait();
     const uint32_t t = blockIdx.x, pos = start_pos + t;
     if (pos >= capacity) return;  // the host validates; never write outside the cache
     const int half_rope = rope_dim / 2;
     if (cos_t) { cos_t += (size_t)pos * table_stride; sin_t += (size_t)pos * table_stride; }
-    __half* qrow = q + (size_t)t * q_heads * head_dim;
-    __half* krow = k + (size_t)t * kv_heads * head_dim;
-    for (int pair = threadIdx.x; pair < half_rope; pair += blockDim.x) {
+    for (int pair = threadIdx.x; pair < half_rope; pair += kRopeThreads) {
         int d0, d1, c0i, c1i;
         rope_indices(layout, pair, half_rope, head_dim, d0, d1, c0i, c1i);
-        float c0, s0, c1, s1;  // once per (position, pair), shared by every head
-        rope_trig(pair, half_rope, pos, base_log2, math_mode, cos_t, sin_t, c0i, c1i, c0, s0, c1, s1);
-        for (int h = 0; h < q_heads + kv_heads; ++h) {
+        float4 c;
+        rope_trig(pair, half_rope, pos, base_log2, math_mode, cos_t, sin_t, c0i, c1i, c.x, c.y, c.z, c.w);
+        trig[pair] = c;
+    }
+    if (!cos_t) pdl_wait();
+    __syncthreads();
+    __half* qrow = q + (size_t)t * q_heads * head_dim;
+    __half* krow = k + (size_t)t * kv_heads * head_dim;
+    const int items = (q_heads + kv_heads) * half_rope;
+    for (int base = threadIdx.x; base < items; base += 4 * kRopeThreads) {
+        __half *a[4], *b[4];
+        float x0[4], x1[4];
+        int pair[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = base + j * kRopeThreads, h = min(i, items - 1) / half_rope;
+            pair[j] = min(i, items - 1) - h * half_rope;
+            int d0, d1, c0i, c1i;
+            rope_indices(layout, pair[j], half_rope, head_dim, d0, d1, c0i, c1i);
             __half* row = h < q_heads ? qrow + (size_t)h * head_dim : krow + (size_t)(h - q_heads) * head_dim;
-            const float x0 = __half2float(row[d0]), x1 = __half2float(row[d1]);
-            row[d0] = __float2half_rn(__fsub_rn(__fmul_rn(x0, c0), __fmul_rn(x1, s0)));
-            row[d1] = __float2half_rn(__fadd_rn(__fmul_rn(x1, c1), __fmul_rn(x0, s1)));
+            a[j] = row + d0;
+            b[j] = row + d1;
+            if (i < items) { x0[j] = __half2float(*a[j]); x1[j] = __half2float(*b[j]); }
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (base + j * kRopeThreads >= items) break;
+            const float4 c = trig[pair[j]];
+            *a[j] = __float2half_rn(__fsub_rn(__fmul_rn(x0[j], c.x), __fmul_rn(x1[j], c.y)));
+            *b[j] = __float2half_rn(__fadd_rn(__fmul_rn(x1[j], c.z), __fmul_rn(x0[j], c.w)));
         }
     }
     __syncthreads();  // the rotated keys are complete before they are copied
     const __half* vrow = v + (size_t)t * kv_heads * head_dim;
-    for (int i = threadIdx.x; i < kv_heads * head_dim / 2; i += blockDim.x) {
+    for (int i = threadIdx.x; i < kv_heads * head_dim / 2; i += kRopeThreads) {
         const int h = (2 * i) / head_dim, d = (2 * i) % head_dim;
         const size_t dst = ((size_t)h * capacity + pos) * head_dim + d;
         *reinterpret_cast<__half2*>(k_cache + dst) = *reinterpret_cast<const __half2*>(krow + 2 * i);
@@ -71,51 +99,74 @@ __global__ void __launch_bounds__(128) rope_kv_prefill_kernel(__half* q, __half*
     }
 }
 
-template <int D, int NH>
+constexpr uint32_t kAttnFill = 148;  // SMs
+
+template <int D, int NH, int KS>
+__host__ __device__ constexpr size_t prefill_attn_smem() {  // two buffers of KS tiles' K and V halves, and later the key parts' sums
+    const size_t tiles = (size_t)2 * KS * 2 * (D / 16) * 512, sums = KS > 1 ? (size_t)(kAttnWarps - kAttnWarps / KS) * 32 * NH * (D / 4 + 4) * sizeof(float) : 0;
+    return tiles > sums ? tiles : sums;
+}
+
+template <int D, int NH, int KS>
 __global__ void __launch_bounds__(kAttnThreads) attn_prefill_kernel(const __half* __restrict__ q, const __half* __restrict__ k_cache,
                                                                     const __half* __restrict__ v_cache, __half* __restrict__ out, int n_q,
                                                                     int n_kv, uint32_t n_pos, uint32_t start_pos, uint32_t capacity,
-                                                                    float scale, uint32_t window) {
-    constexpr int MT = D / 16, KJ = D / 32, CH = D / 16;
+                                                                    float scale, uint32_t window, uint32_t per_warp) {
+    constexpr int MT = D / 16, KJ = D / 32, CH = D / 16, PG = kAttnWarps / KS;  // PG warps beside one another in positions, KS in keys
     constexpr int kUnit = CH * 512;  // bytes of a tile's K half (and of its V half)
-    __shared__ __align__(16) unsigned char tiles[2][2][kUnit];  // [buffer][K | V]
+    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned char* tiles = smem;  // [buffer][key part][K | V]
     pdl_trigger();
     pdl_wait();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int pg = warp % PG, part = warp / PG;
     const int kvh = blockIdx.y, ratio = n_q / n_kv;
-    const uint32_t p_first = blockIdx.x * kAttnWarps, p = p_first + warp;
+    // this warp's positions: p .. p + per_warp - 1; column c of its tile is head c % ratio at position p + c / ratio
+    const uint32_t p_first = blockIdx.x * (PG * per_warp), p = p_first + pg * per_warp;
     const bool active = p < n_pos;
-    const uint32_t p_last = min(n_pos, p_first + kAttnWarps) - 1u;
-    // this warp's keys: [w_lo, w_hi); the CTA's tiles: from the first position's window start to the last position's limit
-    const uint32_t w_hi = start_pos + p + 1u, w_lo = (window > 0 && window < w_hi) ? w_hi - window : 0u;
+    const uint32_t p_last = min(n_pos, p_first + PG * per_warp) - 1u;
+    uint32_t lo[NH][2], hi[NH][2];  // keys [lo, hi) of this thread's columns 2t, 2t + 1
+#pragma unroll
+    for (int nh = 0; nh < NH; ++nh)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const uint32_t off = (uint32_t)(nh * 8 + 2 * t + c) / (uint32_t)ratio;
+            const bool in = off < per_warp && p + off < n_pos;
+            hi[nh][c] = in ? start_pos + p + off + 1u : 0u;
+            lo[nh][c] = window > 0 && window < hi[nh][c] ? hi[nh][c] - window : 0u;
+        }
+    const uint32_t w_hi = start_pos + min(p + per_warp, n_pos), w_lo = window > 0 && window < start_pos + p + 1u ? start_pos + p + 1u - window : 0u;
+    // the CTA's tiles: from the first position's window start to the last position's limit
     const uint32_t c_hi = start_pos + p_last + 1u, first_hi = start_pos + p_first + 1u;
     const uint32_t c_lo = ((window > 0 && window < first_hi) ? first_hi - window : 0u) & ~15u;
     const __half* Kb = k_cache + (size_t)kvh * capacity * D;
     const __half* Vb = v_cache + (size_t)kvh * capacity * D;
 
-    auto issue_tile = [&](uint32_t kt, int buf) {
+    auto issue_tiles = [&](uint32_t kt, int buf) {
         const uint32_t last = c_hi - 1u;
-        for (int i = tid; i < CH * 32; i += kAttnThreads) {
-            const int c = i >> 5, ln = i & 31, gg = ln >> 2, tt = ln & 3;
+        for (int j = tid; j < KS * CH * 32; j += kAttnThreads) {
+            const int z = j / (CH * 32), i = j % (CH * 32), c = i >> 5, ln = i & 31, gg = ln >> 2, tt = ln & 3;
+            const uint32_t k0 = kt + 16u * z;
+            unsigned char* dst = tiles + ((buf * KS + z) * 2) * kUnit + i * 16;
             // K piece c of lane ln: row gg (+8 for odd c), halves [32 (c / 2) + 8 tt, +8)
-            const uint32_t krow = min(kt + gg + 8u * (c & 1), last);
-            cp_async16(&tiles[buf][0][i * 16], Kb + (size_t)krow * D + 32 * (c >> 1) + 8 * tt);
+            const uint32_t krow = min(k0 + gg + 8u * (c & 1), last);
+            cp_async16(dst, Kb + (size_t)krow * D + 32 * (c >> 1) + 8 * tt);
             // V piece c = 4 cc + kk of lane ln: row 2 tt + (kk & 1) + 8 (kk / 2), halves [64 cc + 8 gg, +8)
             const int kk = c & 3;
-            const uint32_t vrow = min(kt + 2u * tt + (kk & 1) + 8u * (kk >> 1), last);
-            cp_async16(&tiles[buf][1][i * 16], Vb + (size_t)vrow * D + 64 * (c >> 2) + 8 * gg);
+            const uint32_t vrow = min(k0 + 2u * tt + (kk & 1) + 8u * (kk >> 1), last);
+            cp_async16(dst + kUnit, Vb + (size_t)vrow * D + 64 * (c >> 2) + 8 * gg);
         }
         cp_async_commit();
     };
-    issue_tile(c_lo, 0);
+    issue_tiles(c_lo, 0);
 
-    // Q^T fragments of this warp's position: thread (g,t) keeps head g's dims [32j + 8t, +8)
+    // Q^T fragments: thread (g,t) keeps column g's dims [32j + 8t, +8)
     uint32_t qf[NH][D / 8];
 #pragma unroll
     for (int nh = 0; nh < NH; ++nh) {
-        const int hl = nh * 8 + g;
-        if (active && hl < ratio) {
-            const __half* qh = q + ((size_t)p * n_q + (size_t)kvh * ratio + hl) * D;
+        const uint32_t off = (uint32_t)(nh * 8 + g) / (uint32_t)ratio, hl = (uint32_t)(nh * 8 + g) % (uint32_t)ratio;
+        if (off < per_warp && p + off < n_pos) {
+            const __half* qh = q + ((size_t)(p + off) * n_q + (size_t)kvh * ratio + hl) * D;
 #pragma unroll
             for (int j = 0; j < KJ; ++j) {
                 const uint4 v = *reinterpret_cast<const uint4*>(qh + 32 * j + 8 * t);
@@ -137,22 +188,30 @@ __global__ void __launch_bounds__(kAttnThreads) attn_prefill_kernel(const __half
     }
 
     int buf = 0;
-    for (uint32_t kt = c_lo; kt < c_hi; kt += 16, buf ^= 1) {
-        if (kt + 16 < c_hi) issue_tile(kt + 16, buf ^ 1);
+    for (uint32_t kt = c_lo; kt < c_hi; kt += 16 * KS, buf ^= 1) {
+        if (kt + 16 * KS < c_hi) issue_tiles(kt + 16 * KS, buf ^ 1);
         else cp_async_commit();  // the group count stays uniform
         cp_async_wait<1>();
-        __syncthreads();  // every thread's pieces of this tile have landed
-        if (active && kt < w_hi && kt + 16 > w_lo) {
-            const uint32_t ka = kt + g, kb = kt + g + 8;
-            const bool valid_a = ka < w_hi && ka >= w_lo, valid_b = kb < w_hi && kb >= w_lo;
+        __syncthreads();  // every thread's pieces of these tiles have landed
+        const uint32_t k0 = kt + 16 * part;
+        if (active && k0 < w_hi && k0 + 16 > w_lo) {
+            const uint32_t ka = k0 + g, kb = k0 + g + 8;
+            bool valid[NH][4];
+#pragma unroll
+            for (int nh = 0; nh < NH; ++nh)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    valid[nh][c] = ka < hi[nh][c] && ka >= lo[nh][c];
+                    valid[nh][2 + c] = kb < hi[nh][c] && kb >= lo[nh][c];
+                }
+            const unsigned char* tile = tiles + ((buf * KS + part) * 2) * kUnit + lane * 16;
             uint32_t pb0[NH], pb1[NH], pl0[NH], pl1[NH];
-            tile_scores_softmax<D, NH>(&tiles[buf][0][lane * 16], qf, valid_a, valid_b, scale2, m_run, l_run, o, pb0, pb1, pl0, pl1);
-            tile_weighted_sum<D, NH>(&tiles[buf][1][lane * 16], o, pb0, pb1, pl0, pl1);
+            tile_scores_softmax<D, NH>(tile, qf, valid, scale2, m_run, l_run, o, pb0, pb1, pl0, pl1);
+            tile_weighted_sum<D, NH>(tile + kUnit, o, pb0, pb1, pl0, pl1);
         }
         __syncthreads();  // the buffer may be refilled
     }
     cp_async_wait<0>();
-    if (!active) return;
     // per-thread partial denominators cover keys g, g + 8 only: finish the sum over g
 #pragma unroll
     for (int nh = 0; nh < NH; ++nh)
@@ -161,27 +220,74 @@ __global__ void __launch_bounds__(kAttnThreads) attn_prefill_kernel(const __half
             l_run[nh][0] += __shfl_xor_sync(0xffffffffu, l_run[nh][0], off);
             l_run[nh][1] += __shfl_xor_sync(0xffffffffu, l_run[nh][1], off);
         }
+    if (KS > 1) {  // the key parts' states, merged in order by the first part's warps; value v of lane `lane` of a warp at [v][lane]
+        constexpr int kVals = NH * (MT * 4 + 4);
+        float* sums = reinterpret_cast<float*>(smem);
+        __syncthreads();  // every copy has landed and every tile has been read
+        if (part > 0) {
+            float* s = sums + (size_t)(warp - PG) * kVals * 32 + lane;
+#pragma unroll
+            for (int nh = 0; nh < NH; ++nh) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c) { s[(nh * (MT * 4 + 4) + c) * 32] = m_run[nh][c]; s[(nh * (MT * 4 + 4) + 2 + c) * 32] = l_run[nh][c]; }
+#pragma unroll
+                for (int i = 0; i < MT; ++i)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) s[(nh * (MT * 4 + 4) + 4 + i * 4 + c) * 32] = o[nh][i][c];
+            }
+        }
+        __syncthreads();
+        if (part > 0) return;
+        for (int z = 1; z < KS; ++z) {
+            const float* s = sums + (size_t)((z - 1) * PG + pg) * kVals * 32 + lane;
+#pragma unroll
+            for (int nh = 0; nh < NH; ++nh) {
+                float mine[2], theirs[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const float m = s[(nh * (MT * 4 + 4) + c) * 32], top = fmaxf(m_run[nh][c], m);
+                    mine[c] = exp2f(m_run[nh][c] - top);
+                    theirs[c] = exp2f(m - top);
+                    m_run[nh][c] = top;
+                    l_run[nh][c] = l_run[nh][c] * mine[c] + s[(nh * (MT * 4 + 4) + 2 + c) * 32] * theirs[c];
+                }
+#pragma unroll
+                for (int i = 0; i < MT; ++i)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) o[nh][i][c] = o[nh][i][c] * mine[c & 1] + s[(nh * (MT * 4 + 4) + 4 + i * 4 + c) * 32] * theirs[c & 1];
+            }
+        }
+    }
+    if (!active) return;
 #pragma unroll
     for (int nh = 0; nh < NH; ++nh)
 #pragma unroll
-        for (int i = 0; i < MT; ++i)
+        for (int c = 0; c < 2; ++c) {
+            const uint32_t off = (uint32_t)(nh * 8 + 2 * t + c) / (uint32_t)ratio, head = (uint32_t)(nh * 8 + 2 * t + c) % (uint32_t)ratio;
+            if (off >= per_warp || p + off >= n_pos) continue;
+            __half* row = out + ((size_t)(p + off) * n_q + (size_t)kvh * ratio + head) * D;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int head = nh * 8 + 2 * t + (c & 1);
-                if (head >= ratio) continue;
-                const int j = 2 * i + (c >> 1);
-                const int dim = 64 * (j >> 3) + 8 * g + (j & 7);
-                out[((size_t)p * n_q + (size_t)kvh * ratio + head) * D + dim] = __float2half_rn(o[nh][i][c] / l_run[nh][c & 1]);
-            }
+            for (int i = 0; i < MT; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int j = 2 * i + h;
+                    row[64 * (j >> 3) + 8 * g + (j & 7)] = __float2half_rn(o[nh][i][2 * h + c] / l_run[nh][c]);
+                }
+        }
 }
 
-template <int D, int NH>
-cudaError_t launch_prefill_attention_t(const Launch& l, const __half* q, const __half* kc, const __half* vc, __half* out, int n_q, int n_kv,
-                                       uint32_t n_pos, uint32_t start_pos, uint32_t capacity, float scale, uint32_t window) {
-    auto kern = attn_prefill_kernel<D, NH>;
+template <int D, int NH, int KS>
+cudaError_t launch_prefill_attention_ks(const Launch& l, const __half* q, const __half* kc, const __half* vc, __half* out, int n_q, int n_kv,
+                                        uint32_t n_pos, uint32_t start_pos, uint32_t capacity, float scale, uint32_t window, uint32_t per_warp) {
+    auto kern = attn_prefill_kernel<D, NH, KS>;
+    constexpr size_t smem = prefill_attn_smem<D, NH, KS>();
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const uint32_t step = kAttnWarps / KS * per_warp;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((n_pos + kAttnWarps - 1) / kAttnWarps, n_kv);
+    cfg.gridDim = dim3((n_pos + step - 1) / step, n_kv);
     cfg.blockDim = dim3(kAttnThreads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = l.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -189,7 +295,18 @@ cudaError_t launch_prefill_attention_t(const Launch& l, const __half* q, const _
     cfg.attrs = attr;
     cfg.numAttrs = l.pdl ? 1 : 0;
     prefer_max_shared(kern);
-    return cudaLaunchKernelEx(&cfg, kern, q, kc, vc, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window);
+    return cudaLaunchKernelEx(&cfg, kern, q, kc, vc, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, per_warp);
+}
+
+// Key parts: as few as give every SM a CTA (a CTA walks its keys tile by tile, about 1 us each, whatever its positions).
+template <int D, int NH>
+cudaError_t launch_prefill_attention_t(const Launch& l, const __half* q, const __half* kc, const __half* vc, __half* out, int n_q, int n_kv,
+                                       uint32_t n_pos, uint32_t start_pos, uint32_t capacity, float scale, uint32_t window) {
+    const uint32_t per_warp = std::max(1, 8 * NH / (n_q / n_kv));
+    auto ctas = [&](uint32_t ks) { const uint32_t step = kAttnWarps / ks * per_warp; return (n_pos + step - 1) / step * (uint32_t)n_kv; };
+    if (ctas(1) >= kAttnFill) return launch_prefill_attention_ks<D, NH, 1>(l, q, kc, vc, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, per_warp);
+    if (ctas(2) >= kAttnFill) return launch_prefill_attention_ks<D, NH, 2>(l, q, kc, vc, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, per_warp);
+    return launch_prefill_attention_ks<D, NH, 4>(l, q, kc, vc, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, per_warp);
 }
 
 Launch lch(smelt_cuda_ctx* ctx) {  // chunk launches chain with programmatic dependent launch, as a decode table's do
@@ -210,7 +327,12 @@ cudaError_t launch_rope_kv_prefill(const Launch& l, __half* q, __half* k, const 
         return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_pos);
-    cfg.blockDim = dim3(128);
+    cfg.blockDim = dim3(kRopeThreads);
+    cfg.dynamicSmemBytes = (size_t)rope_dim / 2 * sizeof(float4);
+    if (cfg.dynamicSmemBytes > 48 * 1024) {  // more than 6144 rotated dimensions
+        const cudaError_t e = cudaFuncSetAttribute(rope_kv_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+        if (e != cudaSuccess) return e;
+    }
     cfg.stream = l.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -79,6 +79,24 @@ def test_attention_prefill_matches_the_oracle_per_position(ctx, oracle, n_q, n_k
         b.free()
 
 
+# one, two and four key sets; heads that do not fill the tile's columns (a ratio of 3 takes two positions a warp, 5 and 12 one), a ragged last run
+@pytest.mark.parametrize("n_q,n_kv,d", [(24, 8, 128), (5, 1, 64), (12, 1, 128), (8, 8, 64), (64, 16, 64)])
+@pytest.mark.parametrize("n_pos,start,window", [(1, 0, 0), (3, 700, 0), (149, 5, 0), (149, 70, 33)])
+def test_attention_prefill_key_sets(ctx, oracle, n_q, n_kv, d, n_pos, start, window):
+    cap = start + n_pos
+    k, v = (synth.kv_cache(34, n, 1, n_kv, cap, d)[0] for n in "kv")
+    q = synth.activations(34, "q", n_pos, n_q, d)
+    bufs = [ctx.to_device(a) for a in (q, k, v)] + [ctx.alloc(n_pos * n_q * d * 2 + 64).fill(0xFF)]
+    ctx.call("attention_prefill", *bufs, n_q, n_kv, d, n_pos, start, cap, C.c_float(1 / np.sqrt(d)), window)
+    got = bufs[3].download(np.float16, (n_pos, n_q, d))
+    for t in {*range(0, n_pos, 11), n_pos - 1}:
+        ref = oracle.attention_decode(q[t], k, v, n_q, n_kv, d, cap, start + t + 1, sliding_window=window)
+        assert rel_err(got[t], ref) < REL_TOL and inf_err(got[t], ref) < INF_TOL, f"position {start + t}"
+    assert np.all(bufs[3].download(np.uint8, (64,), offset=n_pos * n_q * d * 2) == 0xFF)
+    for b in bufs:
+        b.free()
+
+
 def rms_err(got, ref) -> float:
     g, r = got.astype(np.float32), ref.astype(np.float32)
     return float(np.max(np.abs(g - r)) / np.sqrt(np.mean(r * r)))
