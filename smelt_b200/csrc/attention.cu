@@ -172,11 +172,15 @@ cudaError_t launch_attention_decode(const Launch& l, const AttnArgs& a) {
     // Short contexts are latency bound: up to 4096 keys, eight splits of a KV head run as one
     // thread-block cluster and merge through distributed shared memory, with no partials in
     // global memory (measured against one tile per warp and the ticket merge: 11.2 against
-    // 13.9 us at 4096 keys, batch 1).  Always eight: the key ranges are cut from the live
-    // length, so with a fixed split count the summation order, and with it every output bit,
-    // is the same whatever capacity the cache was given or has grown to.
+    // 13.9 us at 4096 keys, batch 1).  The key ranges are cut from the live length, so with a split
+    // count that no capacity changes the summation order, and with it every output bit, is the
+    // same whatever capacity the cache was given or has grown to.
     const bool cluster = n_max <= 4096 && by_len >= 2 && !a.mlx_partials;
-    if (cluster) nsplits = 8;
+    // As many sequences and KV heads as fill the GPU by themselves take fewer splits, by their number alone, so that the CTAs stay
+    // one wave: of a handful of tiles per CTA most is launch and merge (32 query and 8 KV heads of 128, us with 8 | 4 | 2 | 1
+    // splits: 8 sequences of 1023 keys 16.5 | 12.4 | 16.2 | 17.6, 16 of 300 23.0 | 12.7 | 9.8 | 11.3, 32 of 300 44.6 | 24.7 |
+    // 18.5 | 12.3, 32 of 4000 132 | 115 | 107 | 110; 4 sequences of 1023 9.0 | 11.5 | 13.2 | 16.2).
+    if (cluster) for (nsplits = 8; nsplits > 1 && (long)nsplits * base > slots;) nsplits /= 2;
     AttnDev p;
     p.a = a;
     p.nsplits = nsplits;

@@ -1,5 +1,5 @@
 // Inline-PTX wrappers for the fifth-generation tensor core path (tcgen05.mma with accumulators in
-// tensor memory) and the mbarrier waits around it, shared by the QMM kernels.
+// tensor memory) and the mbarrier waits around it, shared by the kernels that use it.
 #pragma once
 #include "common.cuh"
 

@@ -594,6 +594,12 @@ def test_attention_other_head_shapes(ctx, oracle, n_q, n_kv, d, ctx_len, batch):
     _attention_case(ctx, oracle, n_q, n_kv, d, ctx_len, batch)
 
 
+# KV heads times sequences from which the key ranges of a short context become fewer: eight, four, two and one of them
+@pytest.mark.parametrize("batch,ctx_len", [(4, 150), (5, 150), (9, 700), (18, 150), (19, 700), (38, 200)])
+def test_attention_many_sequences(ctx, oracle, batch, ctx_len):
+    _attention_case(ctx, oracle, 16, 8, 128, ctx_len, batch)
+
+
 @pytest.mark.parametrize("n_q,n_kv,d,position,batch,layout", [(32, 8, 128, 0, 1, 1), (32, 8, 128, 530, 1, 1), (16, 4, 128, 4095, 2, 1),
                                                               (8, 2, 256, 777, 1, 0), (16, 1, 64, 129, 3, 1), (4, 1, 128, 600, 1, 1), (8, 2, 128, 5000, 1, 1)])
 def test_rope_attention_decode_is_the_four_kernels(ctx, oracle, n_q, n_kv, d, position, batch, layout):
