@@ -31,7 +31,7 @@ bool encode(CUtensorMap* map, CUtensorMapDataType type, int width, const void* b
 
 bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps* maps, Line* line, int* grid) {
     if (group != kLineGroup || a.cols % kLineGroup != 0 || a.norm_w) return false;
-    if (a.nseg > 1 && !affine_stream_takes(mode, a, group)) return false;
+    if (a.nseg > 1 && affine_stream_passes(mode, a, group) == 0) return false;
     const bool paired = mode == kAffineGateUp || mode == kAffineDual, segs = a.nseg > 1;
     const int sm = a.sm_count > 0 ? a.sm_count : 148;
     if (reinterpret_cast<uintptr_t>(a.x) & 15u) return false;

@@ -445,15 +445,24 @@ cudaError_t launch_group(const Launch& l, const AffineArgs& a, int group) {
     }
 }
 
-// Rows of x from which the tensor-core product takes a launch: at 12 rows its expansion of the weights takes as long as two
-// passes of eight rows (gate/up 12288 x 4096: 43.6 against 45.6 us, 4096 x 4096: 13.5 against 13.6), at 32 it is ahead by a third.
-constexpr int kWideRows = 17;
+// Whether the tensor-core product (affine_wide.cu) takes a launch first.  Its expansion of the weights costs the same for any
+// number of rows, so the streaming kernel stays ahead as long as it reads the weights once, and with a pair of matrices up to
+// sixteen rows.  From 17 rows on (gate/up 12288 x 4096, us, passes against it: 16 rows 46.8 : 50.4, 32 rows 77.8 : 52.2), and
+// where several passes, or the general kernel, stage 64 K values of x: + residual 4096 x 12288, 6 rows 17.9 : 27.8 (one pass),
+// 8 rows 29.4 : 27.8, 16 rows 51.4 : 28.0; 5120 x 17408, 6 rows 56.9 : 42.6, 16 rows 116 : 42.9; 4096 x 4096, 12 rows (49 K)
+// 13.5 : 13.5, 16 rows 15.6 : 13.5; gate/up 3000 x 6976 (no streaming) 8 rows (56 K) 31.9 : 38.6, 12 rows 54.8 : 38.5.
+bool wide_first(int mode, const AffineArgs& a, int group) {
+    if (a.batch >= 17) return true;
+    if (a.norm_w || a.nseg > 1 || (size_t)a.batch * a.cols < 65536) return false;
+    const int passes = affine_stream_passes(mode, a, group);
+    return passes == 0 ? a.batch > 2 : passes > 1 && mode != kAffineGateUp && mode != kAffineDual;
+}
 
 }  // namespace
 
 cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int group) {
     if (args.rows <= 0 || args.cols <= 0 || args.batch <= 0 || args.cols % group != 0) return cudaErrorInvalidValue;
-    if (args.batch >= kWideRows) {  // tcgen05: the weights are expanded once per 256 rows of x
+    if (wide_first(mode, args, group)) {  // tcgen05: the weights are expanded once per 256 rows of x
         bool handled = false;
         cudaError_t e = launch_affine_wide(l, mode, args, group, &handled);
         if (handled || e != cudaSuccess) return e;

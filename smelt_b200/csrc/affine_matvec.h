@@ -52,8 +52,8 @@ cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int
 cudaError_t launch_affine_stream(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
 // Tensor-core product for seventeen rows of x and more (affine_wide.cu).
 cudaError_t launch_affine_wide(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
-// Whether the streaming kernel takes the launch (its first pass, of up to sixteen rows).
-bool affine_stream_takes(int mode, const AffineArgs& args, int group);
+// Passes of the streaming kernel over the weights for up to sixteen rows of x, 0 where it does not take the launch.
+int affine_stream_passes(int mode, const AffineArgs& args, int group);
 cudaError_t launch_affine_imma(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
 
 }  // namespace smelt

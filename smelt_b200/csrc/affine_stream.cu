@@ -407,10 +407,10 @@ static int stream_passes(int mode, const AffineArgs& a, int group) {
     return passes;
 }
 
-bool affine_stream_takes(int mode, const AffineArgs& args, int group) {
+int affine_stream_passes(int mode, const AffineArgs& args, int group) {
     AffineArgs a = args;
     if (a.batch > 16) a.batch = 16;
-    return (a.nseg <= 1 || (mode == kAffinePlain && a.nseg <= 3)) && stream_passes(mode, a, group) > 0;
+    return a.nseg <= 1 || (mode == kAffinePlain && a.nseg <= 3) ? stream_passes(mode, a, group) : 0;
 }
 
 // Launches the streaming kernel when the shape is eligible (group 64, batch <= 16, cols a
