@@ -449,11 +449,11 @@ cudaError_t launch_group(const Launch& l, const AffineArgs& a, int group) {
 // number of rows, so the streaming kernel stays ahead as long as it reads the weights once, and with a pair of matrices up to
 // sixteen rows.  From 17 rows on (gate/up 12288 x 4096, us, passes against it: 16 rows 46.8 : 50.4, 32 rows 77.8 : 52.2), and
 // where several passes, or the general kernel, stage 64 K values of x: + residual 4096 x 12288, 6 rows 17.9 : 27.8 (one pass),
-// 8 rows 29.4 : 27.8, 16 rows 51.4 : 28.0; 5120 x 17408, 6 rows 56.9 : 42.6, 16 rows 116 : 42.9; 4096 x 4096, 12 rows (49 K)
+// 8 rows (96 K, the least that up to eight rows have to pass) 29.4 : 27.8 but a whole step of 8 sequences 3.62 : 3.75 ms, 16 rows 51.4 : 28.0; 5120 x 17408, 6 rows 56.9 : 42.6, 16 rows 116 : 42.9; 4096 x 4096, 12 rows (49 K)
 // 13.5 : 13.5, 16 rows 15.6 : 13.5; gate/up 3000 x 6976 (no streaming) 8 rows (56 K) 31.9 : 38.6, 12 rows 54.8 : 38.5.
 bool wide_first(int mode, const AffineArgs& a, int group) {
     if (a.batch >= 17) return true;
-    if (a.norm_w || a.nseg > 1 || (size_t)a.batch * a.cols < 65536) return false;
+    if (a.norm_w || a.nseg > 1 || (size_t)a.batch * a.cols < (a.batch <= 8 ? 98305u : 65536u)) return false;
     const int passes = affine_stream_passes(mode, a, group);
     return passes == 0 ? a.batch > 2 : passes > 1 && mode != kAffineGateUp && mode != kAffineDual;
 }
