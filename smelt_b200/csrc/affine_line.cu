@@ -38,7 +38,8 @@ bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps*
     *line = {};
     line->groups = a.cols / kLineGroup;
     const int wanted = (a.batch + max_cols - 1) / max_cols;
-    line->tile_cols = ((a.batch + wanted - 1) / wanted + 15) & ~15;
+    line->tile_cols = (a.batch + wanted - 1) / wanted;
+    line->tile_cols = line->tile_cols <= 128 ? (line->tile_cols + 15) & ~15 : (line->tile_cols + 31) & ~31;  // above 128 two MMAs share them
     line->col_tiles = (a.batch + line->tile_cols - 1) / line->tile_cols;
     line->first1 = line->first2 = INT_MAX;
     for (int s = 0; s < (paired ? 2 : segs ? a.nseg : 1); ++s) {
@@ -54,8 +55,9 @@ bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps*
     if (paired) line->row_tiles = (a.rows + 63) / 64;
     const long tiles = (long)line->row_tiles * line->col_tiles, units = tiles * line->groups;
     if (units >= 1l << 30 || !encode(&maps->x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.x, a.batch, a.cols, line->tile_cols)) return false;
-    const size_t sums = (size_t)sm * 2 * line->tile_cols * kLineRows * sizeof(float);  // of shared tiles
-    const bool split = a.part_scratch && a.part_counters && tiles <= 4096 && sums <= a.part_scratch_bytes;
+    const size_t sums = (size_t)sm * 2 * line->tile_cols * kLineRows * sizeof(float);  // two tiles of every CTA
+    if (!a.part_scratch || !a.part_counters || sums > a.part_scratch_bytes) return false;
+    const bool split = tiles <= 4096;  // a counter each
     line->quantum = !split ? line->groups : line->groups % kStageGroups == 0 ? kStageGroups : 1;
     // At most about four CTAs to a tile: each more costs the last one as much time as it saves the others
     // (K | V 1024 x 4096 x 2, 64 rows of x: 30.4 us over 148 CTAs, 17.3 us over 64).

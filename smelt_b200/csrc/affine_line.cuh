@@ -153,31 +153,10 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
 // Scales and biases of a stage on their way to shared memory, by a warp of its own: a thread that fetched its own row's
 // beside its other work waited for them.  A lane takes rows `row + 32 i` of the tile; store(stage, i, group of the stage,
 // {scale, bias}) is called after wait(stage), done(stage) behind it.
-template <int MODE, int ROWS, typename Wait, typename Store, typename Done>
+template <int MODE, typename Wait, typename Store, typename Done>
 __device__ __forceinline__ void feed_scales(const AffineArgs& a, const Line& p, int u0, int u1, int row, Wait wait, Store store, Done done) {
-    struct At {
-        int u, g;
-        Part t;
-        const __half *s[ROWS], *b[ROWS];
-        bool ok[ROWS];
-    } at;
+    constexpr int kRows = 4;
     const bool vec = (p.quantum & 3) == 0 && (p.groups & 3) == 0;  // every stage begins at a multiple of four groups
-    auto enter = [&](int u) {
-        at.u = u;
-        at.t = part_at(p, u, u1, a.batch);
-        at.g = at.t.g0;
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) {
-            const LineRow o = line_row<MODE>(a, p, at.t.row_tile, row + 32 * i);
-            at.s[i] = o.s; at.b[i] = o.b; at.ok[i] = o.row < o.rows;
-            if (at.ok[i])
-                for (int g = at.t.g0; g < at.t.g1; g += 16) {
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(at.s[i] + g));
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(at.b[i] + g));
-                }
-        }
-    };
-    uint2 sc[ROWS], bi[ROWS];
     auto four = [&](const __half* q, int n) {
         if (vec && (reinterpret_cast<uintptr_t>(q) & 7u) == 0) return __ldg(reinterpret_cast<const uint2*>(q));
         uint32_t h[4];
@@ -185,38 +164,39 @@ __device__ __forceinline__ void feed_scales(const AffineArgs& a, const Line& p, 
         for (int j = 0; j < 4; ++j) h[j] = j < n ? (uint32_t)__half_as_ushort(__ldg(q + j)) : 0u;
         return make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
     };
-    auto load = [&] {
-        const int n = min(kStageGroups, at.t.g1 - at.g);
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) {
-            sc[i] = at.ok[i] ? four(at.s[i] + at.g, n) : make_uint2(0, 0);
-            bi[i] = at.ok[i] ? four(at.b[i] + at.g, n) : make_uint2(0, 0);
+    uint32_t stage = 0;
+    for (int u = u0; u < u1;) {
+        const Part t = part_at(p, u, u1, a.batch);
+#pragma unroll 1
+        for (int i = 0; i < kRows; ++i) {
+            const LineRow o = line_row<MODE>(a, p, t.row_tile, row + 32 * i);
+            if (o.row < o.rows)
+                for (int g = t.g0; g < t.g1; g += 16) {
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(o.s + g));
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(o.b + g));
+                }
         }
-    };
-    enter(u0);
-    load();
-    for (uint32_t stage = 0;; ++stage) {
-        uint2 s[ROWS], b[ROWS];
+        for (int g = t.g0; g < t.g1; g += kStageGroups, ++stage) {
+            const int n = min(kStageGroups, t.g1 - g);
+            uint2 s[kRows], b[kRows];
 #pragma unroll
-        for (int i = 0; i < ROWS; ++i) { s[i] = sc[i]; b[i] = bi[i]; }
-        at.g += kStageGroups;
-        bool more = true;
-        if (at.g >= at.t.g1) {
-            const int u = at.u + at.t.g1 - at.t.g0;
-            more = u < u1;
-            if (more) enter(u);
+            for (int i = 0; i < kRows; ++i) {
+                const LineRow o = line_row<MODE>(a, p, t.row_tile, row + 32 * i);
+                const bool ok = o.row < o.rows;
+                s[i] = ok ? four(o.s + g, n) : make_uint2(0, 0);
+                b[i] = ok ? four(o.b + g, n) : make_uint2(0, 0);
+            }
+            if (!wait(stage)) return;
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                const uint32_t sw[2] = {s[i].x, s[i].y}, bw[2] = {b[i].x, b[i].y};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) store(stage, i, j, __byte_perm(sw[j >> 1], bw[j >> 1], (j & 1) ? 0x7632 : 0x5410));
+            }
+            __syncwarp();
+            done(stage);
         }
-        if (more) load();  // the next stage's, while this one's are stored
-        if (!wait(stage)) return;
-#pragma unroll
-        for (int i = 0; i < ROWS; ++i) {
-            const uint32_t sw[2] = {s[i].x, s[i].y}, bw[2] = {b[i].x, b[i].y};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) store(stage, i, j, __byte_perm(sw[j >> 1], bw[j >> 1], (j & 1) ? 0x7632 : 0x5410));
-        }
-        __syncwarp();
-        done(stage);
-        if (!more) return;
+        u += t.g1 - t.g0;
     }
 }
 

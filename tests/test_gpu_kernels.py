@@ -202,6 +202,35 @@ def test_affine_wide_edges(ctx, oracle, rows, cols, batch):
         buf.free()
 
 
+# The tensor core truncates the sums it adds to, so no accumulator may hold more than a few of them: of fp32 sums of K products that
+# are rounded to nearest (relative error about 4e-7 here), 4e-7 / 2^-11 = 0.1 % lie on the other side of a rounding boundary of
+# fp16 than the exact product; four times that is allowed.
+@pytest.mark.parametrize("rows,cols,batch", [(1024, 4096, 32), (200, 12288, 64), (136, 12288, 9), (264, 4096, 130), (128, 1984, 300), (512, 12288, 300)])
+def test_affine_wide_rounds_like_exact_sums(ctx, rows, cols, batch):
+    w, s, b = synth.affine_u4(35, "rw", rows, cols, 64)
+    x = synth.activations(35, "rx", batch, cols)
+    d = dev(ctx, w, s, b, x)
+    y = ctx.alloc(batch * rows * 2)
+    ctx.call("affine_matvec", *d, y, rows, cols, 64, batch)
+    q = np.stack([w & 15, w >> 4], -1).reshape(rows, cols // 64, 64).astype(np.float64)
+    want = x.astype(np.float64) @ (q * s.astype(np.float64)[..., None] + b.astype(np.float64)[..., None]).reshape(rows, cols).T
+    assert np.mean(y.download(np.float16, (batch, rows)) != want.astype(np.float16)) < 4e-3
+
+
+# weights beyond fp16's range, of which the nibble, the scale and the bias are not: they were never rounded to fp16
+@pytest.mark.parametrize("rows,cols,batch", [(72, 1984, 17), (136, 12288, 9), (128, 4096, 64), (264, 576, 130), (200, 512, 300)])
+def test_affine_wide_large_weights(ctx, oracle, rows, cols, batch):
+    w, s, b = synth.affine_u4(36, "lw", rows, cols, 64)
+    s[:, ::2], b[:, ::2] = 9000.0, -30000.0
+    s[:, 1::3], b[:, 1::3] = 6e-8, 0.0  # a subnormal scale, alone in its group and beside a large one
+    x = (synth.activations(36, "lx", batch, cols).astype(np.float32) * 2e-4).astype(np.float16)
+    d = dev(ctx, w, s, b, x)
+    y = ctx.alloc(batch * rows * 2)
+    ctx.call("affine_matvec", *d, y, rows, cols, 64, batch)
+    got, want = y.download(np.float16, (batch, rows)), oracle.affine_matvec(w, s, b, x, rows, cols, 64)
+    assert np.all(np.isfinite(want)) and rel_err(got, want) < REL_TOL
+
+
 # batch 1 and 2 run on the integer-MMA kernel: every mode, row / K tails, long K, few chunks per warp
 IMMA_SHAPES = [(4096, 4096, 1), (4096, 12288, 1), (100, 128, 2), (48, 256, 1), (1000, 2048, 2), (6144, 4096, 2), (16, 8192, 1)]
 
