@@ -116,8 +116,8 @@ __device__ __forceinline__ void registers_up() { asm volatile("setmaxnreg.inc.sy
 template <int REGS>
 __device__ __forceinline__ void registers_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
 
-// silu(gate) * up in fp32; the quotient within two units in the last place, far below the fp16 result's
-__device__ __forceinline__ __half swiglu_f32(float gate, float up) { return __float2half_rn(__fdividef(gate, 1.0f + expf(-gate)) * up); }
+// silu(gate) * up in fp32
+__device__ __forceinline__ __half swiglu_f32(float gate, float up) { return __float2half_rn(gate / (1.0f + expf(-gate)) * up); }
 
 template <int MODE, int N>
 __global__ void __launch_bounds__(kThreads, 1) affine_wide_kernel(const __grid_constant__ LineMaps maps, const AffineArgs a, const Line line) {
