@@ -12,7 +12,10 @@
 // the launch in front.  With experts, a unit is a row tile of one expert's matrix and up to BN rows
 // of the activations that chose it, both taken from a table that an earlier launch has written.
 //
-// fp16 weights and activations go the same way (kDenseStoreF16: the LM head of several sequences).
+// fp16 weights and activations go the same way (kDenseStoreF16: the LM head of several sequences), with every 64 columns'
+// sums taken out of tensor memory and added in fp32 registers: the tensor core truncates each sum it adds to, and over all of K
+// that moved 1.7 % of the logits of 4096 columns to another fp16 value than the correctly rounded one; so 0.1 % are, as many as
+// of the fused multiply-adds that one sequence takes.
 //
 // Every wait is bounded: on expiry the CTA raises bit 11 of the device error word, its roles stop,
 // copies and MMAs in flight are waited for (bounded too) and the tensor memory is freed.
@@ -96,6 +99,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
     constexpr int kStages = gemm_stages(BN);
     constexpr uint32_t kStageBytes = gemm_stage_bytes(BN), kTmemCols = 2 * BN < 32 ? 32 : 2 * BN;
     constexpr int kChunk = BN < 32 ? BN : 32;
+    constexpr bool kSums = MODE == kDenseStoreF16;  // an accumulator holds one column block
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2];
@@ -186,20 +190,25 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
             bool alive = true;
             for (int u = blockIdx.x; u < units && alive; u += gridDim.x, ++done) {
                 const Unit t = unit_at(u);
-                const uint32_t buf = done & 1, use = done >> 1;
-                if (use > 0 && !(alive = wait_alive(&acc_empty[buf], (use - 1) & 1, dead))) break;
+                uint32_t buf = done & 1, use = done >> 1;
+                if (!kSums && use > 0 && !(alive = wait_alive(&acc_empty[buf], (use - 1) & 1, dead))) break;
                 tc_fence_after();
                 for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
                     const uint32_t s = it % kStages;
+                    if (kSums) {
+                        buf = it & 1; use = it >> 1;
+                        if (use > 0 && !(alive = wait_alive(&acc_empty[buf], (use - 1) & 1, dead))) break;
+                    }
                     if (!(alive = wait_alive(&full[s], (it / kStages) & 1, dead))) break;
                     tc_fence_after();
                     const uint32_t w = smem_u32(smem + s * kStageBytes), x = w + kATile;
 #pragma unroll
                     for (int k = 0; k < kBlockCols / 16; ++k)
-                        umma_f16(tmem + buf * BN, smem_desc_sw128(w + k * 32), smem_desc_sw128(x + k * 32), idesc, (kb != t.kb0 || k != 0) ? 1u : 0u);
+                        umma_f16(tmem + buf * BN, smem_desc_sw128(w + k * 32), smem_desc_sw128(x + k * 32), idesc, ((!kSums && kb != t.kb0) || k != 0) ? 1u : 0u);
                     umma_commit(&empty[s]);
+                    if (kSums) umma_commit(&acc_full[buf]);
                 }
-                if (alive) umma_commit(&acc_full[buf]);
+                if (!kSums && alive) umma_commit(&acc_full[buf]);
             }
             // MMAs in flight read shared memory and write tensor memory: wait for the last stage they were given
             if (it > 0) mbar_poll_bounded(&empty[(it - 1) % kStages], ((it - 1) / kStages) & 1);
@@ -209,11 +218,37 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
         const int quad = warp & 3, et = tid - 64;
         const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
         uint32_t done = 0;
+        float sums[kSums ? BN : 1];
         for (int u = blockIdx.x; u < units; u += gridDim.x, ++done) {
             const Unit t = unit_at(u);
             const int m0 = t.m0, tile = t.tile;
             const uint32_t buf = done & 1;
-            bool alive = wait_alive(&acc_full[buf], (done >> 1) & 1, dead);
+            bool alive = true;
+            if constexpr (kSums) {
+#pragma unroll
+                for (int j = 0; j < BN; ++j) sums[j] = 0.f;
+                for (int kb = t.kb0; kb < t.kb1; ++kb, ++done) {
+                    const uint32_t b = done & 1;
+                    if (!(alive = __all_sync(0xffffffffu, wait_alive(&acc_full[b], (done >> 1) & 1, dead)))) break;
+                    tc_fence_after();
+#pragma unroll
+                    for (int c0 = 0; c0 < BN; c0 += 16) {
+                        uint32_t v[16];
+                        tmem_ld16(lane_base + b * BN + c0, v);
+                        tmem_wait_ld16(v);
+                        if (c0 + 16 >= BN) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&acc_empty[b]);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) sums[c0 + j] += __uint_as_float(v[j]);
+                    }
+                }
+                --done;
+            } else {
+                alive = wait_alive(&acc_full[buf], (done >> 1) & 1, dead);
+            }
             if (plan.ksplit > 1) {  // the four warps meet below: they go on together or not at all
                 if (!alive) *dead = 1u;
                 asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory");
@@ -227,11 +262,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
             bool finish = true;
             if (plan.ksplit > 1) {
                 float* mine = a.part_scratch + (size_t)u * (BN * kBlockRows);
-                for (int c0 = 0; c0 < cnt; c0 += kChunk) {
+#pragma unroll(kSums ? BN / kChunk : 1)
+                for (int c0 = 0; c0 < (kSums ? BN : cnt); c0 += kChunk) {
+                    if (kSums && c0 >= cnt) continue;
                     uint32_t v[kChunk / 8][8];
+                    if constexpr (kSums) {
 #pragma unroll
-                    for (int j = 0; j < kChunk / 8; ++j) tmem_ld8(lane_base + buf * BN + c0 + 8 * j, v[j]);
-                    tmem_wait_ld();
+                        for (int j = 0; j < kChunk; ++j) v[j / 8][j % 8] = __float_as_uint(sums[c0 + j]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < kChunk / 8; ++j) tmem_ld8(lane_base + buf * BN + c0 + 8 * j, v[j]);
+                        tmem_wait_ld();
+                    }
 #pragma unroll
                     for (int j = 0; j < kChunk; ++j) __stcg(mine + (size_t)(c0 + j) * kBlockRows + r, __uint_as_float(v[j / 8][j % 8]));
                 }
@@ -247,7 +289,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
             }
             if (finish) {
                 const float* parts = a.part_scratch + (size_t)tile * plan.ksplit * (BN * kBlockRows) + r;
-                for (int c0 = 0; c0 < cnt; c0 += kChunk) {  // positions, kChunk at a time: their loads are in flight together
+#pragma unroll(kSums ? BN / kChunk : 1)
+                for (int c0 = 0; c0 < (kSums ? BN : cnt); c0 += kChunk) {  // positions, kChunk at a time: their loads are in flight together
+                    if (kSums && c0 >= cnt) continue;
                     float v[kChunk];
                     float old[MODE == kDenseAddF32 ? kChunk : 1];
                     if (MODE == kDenseAddF32 && row < a.rows) {  // in flight beside the sums
@@ -262,6 +306,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
                         for (int z = 1; z < plan.ksplit; ++z)
 #pragma unroll
                             for (int j = 0; j < kChunk; ++j) v[j] += __ldcg(parts + (size_t)z * (BN * kBlockRows) + (size_t)(c0 + j) * kBlockRows);
+                    } else if constexpr (kSums) {
+#pragma unroll
+                        for (int j = 0; j < kChunk; ++j) v[j] = sums[c0 + j];
                     } else {
                         uint32_t w[kChunk / 8][8];
 #pragma unroll
@@ -316,9 +363,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
                     __syncwarp();  // the next tensor-memory load needs the whole warp
                 }
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            if (!kSums) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[buf]);
+            }
         }
     }
     if (tid == 0 && a.err && *dead) atomicOr(a.err, 0x800u);
@@ -369,7 +418,9 @@ cudaError_t launch_bf16_t(const Launch& l, int mode, const DenseGemmArgs& a, con
     switch (mode) {
         case kDenseStoreF32: return a.out.act == kDenseDecay ? go(gemm_bf16_kernel<BN, kDenseStoreF32, kDenseDecay, false>) : go(gemm_bf16_kernel<BN, kDenseStoreF32, kDenseXielu, false>);
         case kDenseAddF32: return go(gemm_bf16_kernel<BN, kDenseAddF32, kDenseXielu, false>);
-        case kDenseStoreF16: return go(gemm_bf16_kernel<BN, kDenseStoreF16, kDenseXielu, false>);
+        case kDenseStoreF16:
+            if constexpr (BN <= 128) return go(gemm_bf16_kernel<BN, kDenseStoreF16, kDenseXielu, false>);
+            return cudaErrorInvalidValue;
         case kDenseStoreAct:
             switch (a.out.act) {
                 case kDenseXielu: return go(gemm_bf16_kernel<BN, kDenseStoreAct, kDenseXielu, false>);
@@ -390,13 +441,13 @@ cudaError_t launch_bf16_t(const Launch& l, int mode, const DenseGemmArgs& a, con
 // Tile width and column split with the shortest estimated time: waves of units, a unit being its
 // column blocks at the slower of the tensor core (2 BN cycles a block) and the operand fill, plus
 // its epilogue.
-int plan_gemm(const DenseGemmArgs& a, GemmPlan* best) {
+int plan_gemm(const DenseGemmArgs& a, int max_bn, GemmPlan* best) {
     const int sm = a.sm_count > 0 ? a.sm_count : 148, kblocks = a.cols / kBlockCols, row_tiles = (a.rows + kBlockRows - 1) / kBlockRows;
     double best_cost = 0;
     int best_bn = 0;
     for (int bn : {16, 32, 64, 128, 256}) {
         const int token_tiles = (a.m + bn - 1) / bn;
-        if (token_tiles > 1 && bn < 64) continue;
+        if ((token_tiles > 1 && bn < 64) || bn > max_bn) continue;
         const long tiles = (long)row_tiles * token_tiles;
         for (int ks = 1; ks <= 16; ++ks) {
             if (ks > 1 && (tiles * ks > sm || ks * 4 > kblocks || tiles > 4096 || !a.part_scratch || !a.part_counters ||
@@ -422,7 +473,7 @@ cudaError_t launch_bf16(const Launch& l, int mode, const DenseGemmArgs& a) {
         plan = GemmPlan{row_tiles, 1, 1, row_tiles * a.max_entries};
         return a.tile == 32 ? launch_bf16_t<32>(l, mode, a, plan) : a.tile == 64 ? launch_bf16_t<64>(l, mode, a, plan) : a.tile == 128 ? launch_bf16_t<128>(l, mode, a, plan) : cudaErrorInvalidValue;
     }
-    switch (plan_gemm(a, &plan)) {
+    switch (plan_gemm(a, mode == kDenseStoreF16 ? 128 : 256, &plan)) {  // there a thread holds a tile's sums of its row
         case 16: return launch_bf16_t<16>(l, mode, a, plan);
         case 32: return launch_bf16_t<32>(l, mode, a, plan);
         case 64: return launch_bf16_t<64>(l, mode, a, plan);

@@ -1174,8 +1174,10 @@ smelt_status run_record(Interp& in, const smelt_dispatch_record& rec_in) {
             const int rows = (int)rec.grid[0], batch = batch_of(rec);
             if (rows <= 0 || cols == 0 || cols % 8) return fail(ctx, SMELT_ERR_BAD_ARGUMENT, "fp16_matvec: cols must be a positive multiple of 8");
             NEED_BYTES(0, (size_t)rows * cols * 2); NEED_BYTES(1, (size_t)batch * cols * 2); NEED_BYTES(2, (size_t)batch * rows * 2);
-            in.launches += (batch + 7) / 8;
-            return check_cuda(ctx, launch_fp16_matvec(l, (const __half*)r.buf[0].ptr, (const __half*)r.buf[1].ptr, (__half*)r.buf[2].ptr, rows, (int)cols, batch, ctx->sm_count), "fp16_matvec");
+            int launches = 0;
+            const cudaError_t e = launch_fp16_matvec(l, (const __half*)r.buf[0].ptr, (const __half*)r.buf[1].ptr, (__half*)r.buf[2].ptr, rows, (int)cols, batch, ctx->sm_count, shared_tiles(ctx), &launches);
+            in.launches += launches;
+            return check_cuda(ctx, e, "fp16_matvec");
         }
         case PK_EMBEDDING_GATHER: {
             // lut_matvec.metal:951-956: 0 table, 1 token id, 2 out, 3 hidden.

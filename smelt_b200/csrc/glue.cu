@@ -476,25 +476,31 @@ cudaError_t launch_argmax_reduce(const Launch& l, const uint64_t* partials, int3
 }
 
 cudaError_t launch_fp16_matvec(const Launch& l, const __half* w, const __half* x, __half* y, int rows, int cols,
-                               int batch, int sm_count) {
+                               int batch, int sm_count, const SharedTiles& shared, int* launches) {
+    if (launches) *launches = 1;
     if (cols % 8 != 0 || batch <= 0) return cudaErrorInvalidValue;
     if (std::min(batch, 8) * (size_t)cols * 2 > 200 * 1024) return cudaErrorInvalidValue;
-    // Several rows: one row of weights for all of them on the tensor cores, at HBM speed, where a warp per row spends its time
-    // on two conversions and eight FMAs per weight and row of x, once per eight rows (151936 x 4096, us: 8 rows 885 -> 228,
-    // 32 rows 3535 -> 256).  The kernel has no guard of its own.
-    if (batch > 1 && cols % 64 == 0 && !l.guard_lt && !l.guard_ge && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0) {
+    // Several rows: one row of weights for all of them on the tensor cores, where a warp per row spends its time on two conversions
+    // and eight FMAs per weight and row of x, once per eight rows (us: 151936 x 4096, 2 rows 391 -> 304, 8 rows 880 -> 305, 32 rows
+    // 3520 -> 308; 32768 x 2048, 2 rows 54.6 -> 37.9; 4096 x 4096, 2 rows 15.2 -> 13.5, 8 rows 39.0 -> 13.5; 128 x 4096, columns split
+    // over 16 CTAs, 2 rows 7.4 -> 7.8, 3 rows 8.7 -> 7.8, 8 rows 13.9 -> 7.8; 8 x 2048, 4 rows 5.6 -> 6.8, 8 rows 7.7 -> 6.8). A single
+    // tile of 128 rows of weights is worth it from 12288 activations on.  The kernel has no guard of its own.
+    const bool worth = rows > 128 || (long)batch * cols >= 12288;
+    if (batch > 1 && worth && cols % 64 == 0 && !l.guard_lt && !l.guard_ge && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0) {
         DenseGemmArgs a = {};
         a.w = reinterpret_cast<const bf16*>(w);  // two bytes an element either way
         a.x = x;
         a.rows = rows; a.cols = cols; a.m = batch;
         a.out.y0 = y; a.out.ld0 = rows; a.out.split = rows;
         a.sm_count = sm_count;
+        a.err = shared.err;
+        a.part_scratch = shared.scratch; a.part_scratch_bytes = shared.scratch_bytes; a.part_counters = shared.counters;
         return launch_dense_gemm(l, kDenseBf16, kDenseStoreF16, a);
     }
+    if (launches) *launches = (batch + 7) / 8;
     for (int b0 = 0; b0 < batch; b0 += 8) {
         const int nb = batch - b0 < 8 ? batch - b0 : 8;
         const size_t smem = (size_t)nb * cols * 2;
-        if (smem > 200 * 1024) return cudaErrorInvalidValue;
         // As many CTAs as can be resident at once (eight of 256 threads per SM), no fewer: a smaller
         // grid launched programmatically behind a kernel that still holds most SMs piles up to
         // eight CTAs on each of the few SMs that are free and leaves the others without work.

@@ -61,7 +61,15 @@ cudaError_t launch_dn_readout(const Launch& l, int mode, const __half* state, co
 cudaError_t launch_dn_compute_delta(const Launch& l, const __half* value, const float* kv_mem, const __half* beta, float* delta, int head_dim, int heads);
 cudaError_t launch_dn_fused_decode(const Launch& l, __half* state, const __half* qkv, const __half* b_proj, const __half* a_proj, const __half* a_log, const __half* dt_bias, __half* out, __half* conv_state, const __half* conv_weight, const __half* z_proj, const __half* norm_weight, int head_dim, float head_scale, int qkv_dim, int conv_k, int heads, float rms_eps, int tgs);
 cudaError_t launch_dn_fused_prefill(const Launch& l, __half* state, __half* conv_state, __half* qkv, const __half* conv_weight, const __half* a_log, const __half* dt_bias, const __half* b_buf, const __half* a_buf, __half* out, int head_dim, int heads, int seq_len, int qkv_dim, int conv_k, float head_scale, float l2_eps, int tgs);
-cudaError_t launch_fp16_matvec(const Launch& l, const __half* w, const __half* x, __half* y, int rows, int cols, int batch, int sm_count);
+// A context's error word and the scratch of products whose CTAs share tiles.
+struct SharedTiles {
+    uint32_t* err;
+    float* scratch;
+    size_t scratch_bytes;
+    int* counters;
+};
+// launches: how many it took (may be null).
+cudaError_t launch_fp16_matvec(const Launch& l, const __half* w, const __half* x, __half* y, int rows, int cols, int batch, int sm_count, const SharedTiles& shared, int* launches);
 
 // attention.cu — split-K flash-decode.  scratch holds fp32 partials; see attention_scratch_bytes.
 struct AttnArgs {

@@ -506,7 +506,7 @@ smelt_status smelt_cuda_prefill(smelt_cuda_ctx* ctx, const smelt_decoder_desc* d
             __half* logits = (__half*)ctx->slots[kLogits].ptr;
             const int achunk = 2048, parts = (V + achunk - 1) / achunk;
             PF(launch_rms_norm_1pw(l, last, (const __half*)(W + d->final_norm), xn, H, d->eps, 1), "prefill: final norm");
-            PF(launch_fp16_matvec(l, (const __half*)(W + d->lm_head), xn, logits, V, H, 1, ctx->sm_count), "prefill: LM head");
+            PF(launch_fp16_matvec(l, (const __half*)(W + d->lm_head), xn, logits, V, H, 1, ctx->sm_count, shared_tiles(ctx), nullptr), "prefill: LM head");
             PF(launch_argmax_partials(l, logits, (uint64_t*)ctx->slots[kArgmaxScratch].ptr, V, achunk, 1), "prefill: argmax partials");
             PF(launch_argmax_reduce(l, (const uint64_t*)ctx->slots[kArgmaxScratch].ptr, (int32_t*)ctx->slots[kArgmax].ptr, parts, 1, 1), "prefill: argmax");
         }

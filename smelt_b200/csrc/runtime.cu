@@ -484,7 +484,7 @@ smelt_status smelt_cuda_fp16_matvec(smelt_cuda_ctx* ctx, const void* w, const vo
     CTX_OR_FAIL();
     if (!w || !x || !y || rows <= 0 || cols <= 0 || cols % 8 || batch <= 0 || !aligned16(w) || !aligned16(x))
         return fail(ctx, SMELT_ERR_BAD_ARGUMENT, "fp16 matvec: cols must be a multiple of 8 and pointers 16-byte aligned");
-    return check_cuda(ctx, launch_fp16_matvec(typed_launch(ctx), (const __half*)w, (const __half*)x, (__half*)y, rows, cols, batch, ctx->sm_count), "fp16 matvec");
+    return check_cuda(ctx, launch_fp16_matvec(typed_launch(ctx), (const __half*)w, (const __half*)x, (__half*)y, rows, cols, batch, ctx->sm_count, shared_tiles(ctx), nullptr), "fp16 matvec");
 }
 
 static smelt_status signed_common(smelt_cuda_ctx* ctx, int mode, int format, const void* c0, const void* s0,

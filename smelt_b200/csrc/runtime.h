@@ -6,6 +6,7 @@
 
 #include "../../include/smelt_cuda.h"
 #include "common.cuh"
+#include "glue.h"
 
 namespace smelt {
 
@@ -183,6 +184,7 @@ constexpr int kSlotCount = 1024;
 constexpr int kLogitRowsSlot = 36;  // row list of smelt_cuda_enqueue_prefill_rows
 constexpr int kGraphBurst = 8;  // tokens per launch of the multi-token decode graph
 void destroy_decode_graphs(smelt_cuda_ctx* ctx);  // the single-token and the multi-token graph
+inline SharedTiles shared_tiles(const smelt_cuda_ctx* ctx) { return {ctx->err_dev, ctx->qmm_scratch, ctx->qmm_scratch_bytes, ctx->qmm_counters}; }
 smelt_status fail(smelt_cuda_ctx* ctx, smelt_status code, const std::string& msg);
 smelt_status check_cuda(smelt_cuda_ctx* ctx, cudaError_t e, const char* what);
 smelt_status tp_all_reduce_f16(smelt_cuda_ctx* ctx, void* data, size_t count, cudaStream_t stream);

@@ -470,6 +470,17 @@ def test_fp16_matvec_several_rows(ctx, oracle, rows, cols, batch):
     assert np.all(y.download(np.uint8, (64,), offset=batch * rows * 2) == 0xFF)
 
 
+# as test_affine_wide_rounds_like_exact_sums, at the LM head's K and a longer one, split over CTAs and not
+@pytest.mark.parametrize("rows,cols,batch", [(5000, 4096, 2), (1000, 4096, 40), (260, 12288, 8), (20000, 2048, 33)])
+def test_fp16_matvec_several_rows_round_like_exact_sums(ctx, rows, cols, batch):
+    w, x = synth.normal_f16(7, "head", (rows, cols), 0.02), synth.activations(7, "x", batch, cols)
+    dw, dx = dev(ctx, w, x)
+    y = ctx.alloc(batch * rows * 2)
+    ctx.call("fp16_matvec", dw, dx, y, rows, cols, batch)
+    want = (x.astype(np.float64) @ w.T.astype(np.float64)).astype(np.float16)
+    assert np.mean(y.download(np.float16, (batch, rows)) != want) < 4e-3
+
+
 def test_fp16_matvec_clamps(ctx):
     w = np.full((8, 64), 60000.0, np.float16)
     x = np.ones(64, np.float16)
