@@ -630,8 +630,10 @@ SMELT_CUDA_API smelt_status smelt_cuda_affine_dual_matvec(smelt_cuda_ctx* ctx, c
  * affine_multi_matvec: rms_norm_1pw (norms.metal:9-67; skipped when norm_w_dev is NULL)
  * followed by up to three affine_matvec launches that share x (for example the Q, K and V
  * projections) in one kernel.  Needs group 64, cols a multiple of 1024, every tensor but the
- * last with rows a multiple of 16.  More than eight batch rows run as several passes over the
- * weights. */
+ * last with rows a multiple of 16.  Nine to sixteen batch rows, and more with a norm, run as several
+ * passes over the weights.  Up to sixteen rows the results are those of the separate launches bit for
+ * bit, except for three to eight rows of which x does not fit into shared memory (eight rows of 12288
+ * columns), where these take another kernel; with more rows sums may be cut elsewhere along K. */
 typedef struct {
     const void* w_dev;
     const void* scales_dev;

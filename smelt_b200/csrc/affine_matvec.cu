@@ -446,16 +446,23 @@ cudaError_t launch_group(const Launch& l, const AffineArgs& a, int group) {
 }
 
 // Whether the tensor-core product (affine_wide.cu) takes a launch first.  Its expansion of the weights costs the same for any
-// number of rows, so the streaming kernel stays ahead as long as it reads the weights once, and with a pair of matrices up to
-// sixteen rows.  From 17 rows on (gate/up 12288 x 4096, us, passes against it: 16 rows 46.8 : 50.4, 32 rows 77.8 : 52.2), and
-// where several passes, or the general kernel, stage 64 K values of x: + residual 4096 x 12288, 6 rows 17.9 : 27.8 (one pass),
-// 8 rows (96 K, the least that up to eight rows have to pass) 29.4 : 27.8 but a whole step of 8 sequences 3.62 : 3.75 ms, 16 rows 51.4 : 28.0; 5120 x 17408, 6 rows 56.9 : 42.6, 16 rows 116 : 42.9; 4096 x 4096, 12 rows (49 K)
-// 13.5 : 13.5, 16 rows 15.6 : 13.5; gate/up 3000 x 6976 (no streaming) 8 rows (56 K) 31.9 : 38.6, 12 rows 54.8 : 38.5.
+// number of rows, about as much as two passes of the streaming kernel with all its activations to stage.
+//   * 17 rows and more: always (gate/up 12288 x 4096, 16 rows on the streaming kernel 46.8 us, 17 rows here 57.3, 32 rows 57.7,
+//     where the streaming kernel would take four passes).
+//   * 9 to 16 rows with a residual, where the streaming kernel takes several passes over 128 K activations and more (us, passes
+//     against it): 4096 x 12288, 9 rows (108 K) 32.7 : 34.4, 12 rows (144 K) 35.5 : 34.3, 16 rows 51.4 : 34.5; 5120 x 17408, 9 rows
+//     (153 K) 56.6 : 52.2, 16 rows 108 : 52.3.
+//   * 9 to 16 rows that the streaming kernel does not take, from 64 K activations on: gate/up 3000 x 6976, 9 rows (61 K) 49.4 on
+//     the general kernel, 12 rows (82 K) 54.8 : 38.6, 16 rows 61.5 : 38.4.
+//   * Plain products that the streaming kernel takes stay there up to 16 rows: one launch over several tensors
+//     (affine_multi_matvec) runs on it, and gives the bits of a launch for each.
+//   * Up to eight rows never: the general kernel splits K over a cluster, and few rows of weights make no tile worth the
+//     expansion (512 x 17408, 6 rows 8.1 : 38.2).
 bool wide_first(int mode, const AffineArgs& a, int group) {
     if (a.batch >= 17) return true;
-    if (a.norm_w || a.nseg > 1 || (size_t)a.batch * a.cols < (a.batch <= 8 ? 98305u : 65536u)) return false;
+    if (a.batch <= 8 || a.norm_w || a.nseg > 1) return false;
     const int passes = affine_stream_passes(mode, a, group);
-    return passes == 0 ? a.batch > 2 : passes > 1 && mode != kAffineGateUp && mode != kAffineDual;
+    return passes == 0 ? (size_t)a.batch * a.cols >= 65536u : passes > 1 && mode == kAffineAdd && (size_t)a.batch * a.cols >= 131072u;
 }
 
 }  // namespace

@@ -50,7 +50,7 @@ struct AffineArgs {
 
 cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int group);
 cudaError_t launch_affine_stream(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
-// Tensor-core product for seventeen rows of x and more (affine_wide.cu).
+// Tensor-core product for many rows of x (affine_wide.cu; from how many: wide_first in affine_matvec.cu).
 cudaError_t launch_affine_wide(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
 // Passes of the streaming kernel over the weights for up to sixteen rows of x, 0 where it does not take the launch.
 int affine_stream_passes(int mode, const AffineArgs& args, int group);

@@ -359,7 +359,9 @@ def _multi(ctx, tensors, x, norm_w, eps, cols, batch):
 
 @pytest.mark.parametrize("rows,cols,batch,norm", [((4096, 1024, 1024), 4096, 1, True), ((256, 64, 72), 1024, 3, True),
                                                   ((512, 128, 128), 2048, 8, False), ((48, 16, 5), 1024, 1, True),
-                                                  ((256, 64, 40), 4096, 11, True), ((512, 128, 128), 4096, 1, True)])
+                                                  ((256, 64, 40), 4096, 11, True), ((512, 128, 128), 4096, 1, True),
+                                                  # from 65,536 activations on, where a separate product with a residual goes to the tensor cores
+                                                  ((256, 64, 40), 4096, 16, True), ((256, 64, 40), 4096, 16, False), ((64, 40), 8192, 9, False)])
 def test_affine_multi_matvec(ctx, oracle, rows, cols, batch, norm):
     eps = 1e-6
     tensors = [(*synth.affine_u4(21, f"t{i}", r, cols, 64), r) for i, r in enumerate(rows)]
@@ -374,6 +376,18 @@ def test_affine_multi_matvec(ctx, oracle, rows, cols, batch, norm):
         ctx.call("affine_matvec", *dev(ctx, w, s, b), dxn, y, r, cols, 64, batch)
         sep = y.download(np.float16, (batch, r))
         assert np.array_equal(g.view(np.uint16), sep.view(np.uint16)), "one launch per tensor must give the same bits"
+
+
+# many rows: one line of work over all tensors, whose stretches cut a tensor's tiles elsewhere than its own launch does
+@pytest.mark.parametrize("rows,cols,batch", [((208, 40), 1024, 17), ((272, 144, 130), 2048, 65), ((16, 16, 8), 4096, 257)])
+def test_affine_multi_matvec_many_rows(ctx, oracle, rows, cols, batch):
+    tensors = [(*synth.affine_u4(24, f"t{i}", r, cols, 64), r) for i, r in enumerate(rows)]
+    x = synth.activations(24, "x", batch, cols)
+    st, got = _multi(ctx, tensors, x, None, 1e-6, cols, batch)
+    assert st == 0, ctx.last_error()
+    for (w, s, b, r), g in zip(tensors, got):
+        ref = oracle.affine_matvec(w, s, b, x, r, cols, 64)
+        assert rel_err(g, ref) < REL_TOL and inf_err(g, ref) < INF_TOL
 
 
 def test_affine_multi_matvec_rejects_ineligible_shapes(ctx):
