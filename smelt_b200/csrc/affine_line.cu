@@ -27,6 +27,25 @@ bool encode(CUtensorMap* map, CUtensorMapDataType type, int width, const void* b
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// How many CTAs take the line: either a whole number for each tile, or all SMs, whose stretches then begin and end anywhere.
+// Estimated in us.  A group takes a CTA 0.53 us with 32 rows of x, 0.57 with 128 and 0.96 with 256; the CTA that finishes a tile
+// needs 0.011 us per column and CTA whose sums it adds, and with stretches anywhere it may finish two, of one CTA more each.
+// Measured (us, by CTAs of a tile; 148: all SMs): 1024 x 12288, 32 rows: 4 30.7, 8 19.4, 16 15.6, 148 19.2; 256 rows: 4 63.3,
+// 8 51.6, 16 60.2, 148 72.3; 4096 x 4096, 32 rows: 2 22.6, 4 15.5, 148 18.0; 256 rows: 4 36.2, 148 47.7; K | V 1024 x 4096 x 2,
+// 32 rows: 4 13.8, 8 11.2, 148 14.7; 512 rows: 4 35.8, 148 47.5; 4096 x 12288, 32 rows: 4 33.7, 148 34.4; gate/up 6144 x 2048,
+// 32 rows: 1 22.6, 148 22.3.
+long ctas_for(const Line& p, int sm) {
+    const long tiles = (long)p.row_tiles * p.col_tiles, quanta = p.groups / p.quantum;
+    const double group = p.tile_cols <= 128 ? 0.52 + 0.0004 * p.tile_cols : 0.96, sum = 0.011 * p.tile_cols;
+    long best = sm;
+    double least = (double)tiles * p.groups / sm * group + 2.0 * sum * ((double)sm / tiles + 1.0);
+    for (long k = 1; k <= quanta && tiles * k <= sm; ++k) {
+        const double cost = (double)((quanta + k - 1) / k * p.quantum) * group + (k > 1 ? sum * k : 0.0);
+        if (cost < least) { least = cost; best = tiles * k; }
+    }
+    return std::min(best, tiles * quanta);
+}
+
 }  // namespace
 
 bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps* maps, Line* line, int* grid) {
@@ -59,9 +78,7 @@ bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps*
     if (!a.part_scratch || !a.part_counters || sums > a.part_scratch_bytes) return false;
     const bool split = tiles <= 4096;  // a counter each
     line->quantum = !split ? line->groups : line->groups % kStageGroups == 0 ? kStageGroups : 1;
-    // At most about four CTAs to a tile: each more costs the last one as much time as it saves the others
-    // (K | V 1024 x 4096 x 2, 64 rows of x: 30.4 us over 148 CTAs, 17.3 us over 64).
-    *grid = (int)std::max(1l, split ? std::min({(long)sm, 4 * tiles, units / kStageGroups}) : std::min((long)sm, tiles));
+    *grid = (int)(split ? ctas_for(*line, sm) : std::min((long)sm, tiles));
     return true;
 }
 
