@@ -29,6 +29,8 @@
 // the work twice, and the ends of tiles, which it waits for.  Against the form that expanded through shared memory and drained
 // or staged by the same threads (us; gate/up 12288 x 4096 x 2 | 4096 x 12288 | 4096 x 4096): 32 rows 77.8 -> 57.7 | 43.9 ->
 // 33.7 | 17.0 -> 15.5; 128 rows 190 -> 74.3 | 78.4 -> 41.2 | 34.4 -> 22.4; 512 rows 347 -> 226 | 164 -> 105 | 77.8 -> 52.4.
+// A launch in front may take longer than a wait may (its waits on a peer are as long): every role waits for it before the first
+// wait that depends on the activations, and only what needs none of them goes ahead.
 // Every wait is bounded: on expiry the CTA sets bit 10 of the error word, its roles stop, copies and MMAs in flight are
 // waited for (bounded too) and the tensor memory is freed.
 #include "affine_line.cuh"
@@ -169,6 +171,7 @@ __global__ void __launch_bounds__(kThreads, 1) affine_wide_kernel(const __grid_c
                 const Part t = part_at(line, u, u1, a.batch);
                 for (int g = t.g0; g < t.g1; g += kStageGroups, ++it) {
                     const uint32_t s = it % C::kRawStages, use = it / C::kRawStages;
+                    if (it == C::kRawStages) pdl_wait();
                     if (use > 0 && !(alive = wait_alive(&raw_empty[s], (use - 1) & 1, dead))) break;
                     mbar_arrive_expect_tx(&raw_full[s], kRawBytes);
                     request_weights<MODE>(maps, line, t.row_tile, g, raw + s * kRawBytes, &raw_full[s]);
@@ -203,6 +206,7 @@ __global__ void __launch_bounds__(kThreads, 1) affine_wide_kernel(const __grid_c
         // ── issue ──
         const uint32_t idesc = (1u << 4) | ((uint32_t)(mma_cols >> 3) << 17) | ((uint32_t)(kLineRows >> 4) << 24);  // f32 += f16 x f16, K-major both
         const uint32_t x_base = smem_u32(x_tiles);
+        pdl_wait();
         uint32_t turn = 0, unit = 0;
         bool alive = true;
         for (int u = u0; u < u1 && alive;) {
@@ -236,7 +240,10 @@ __global__ void __launch_bounds__(kThreads, 1) affine_wide_kernel(const __grid_c
     } else if (warp == 3) {
         // ── scales and biases ──
         feed_scales<MODE>(a, line, u0, u1, lane,
-            [&](uint32_t it) { return it < C::kRawStages || wait_warp(&raw_empty[it % C::kRawStages], (it / C::kRawStages - 1) & 1, dead); },
+            [&](uint32_t it) {
+                if (it == C::kRawStages) pdl_wait();
+                return it < C::kRawStages || wait_warp(&raw_empty[it % C::kRawStages], (it / C::kRawStages - 1) & 1, dead);
+            },
             [&](uint32_t it, int i, int j, uint32_t sb) { scales[it % C::kRawStages][j][lane + 32 * i] = sb; },
             [&](uint32_t it) { if (lane == 0) mbar_arrive(&scale_full[it % C::kRawStages]); });
     }
@@ -398,6 +405,7 @@ __global__ void __launch_bounds__(kThreads, 1) affine_wide_kernel(const __grid_c
                 for (int k = 0; 2 * k < n; ++k, ++turn) {
                     const uint32_t as = turn % kASlots;
                     if ((int)as != set) continue;
+                    if (turn >= kASlots && turn < 2 * kASlots) pdl_wait();
                     if (turn >= kASlots && !turn_done(turn - kASlots, wait_warp)) { alive = false; break; }
                     tc_fence_after();
                     const int last = min(n - 1, 2 * k + 1);

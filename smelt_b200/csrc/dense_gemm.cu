@@ -184,6 +184,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
         }
     } else if (warp == 1) {
         if (lane == 0) {
+            if (!EXPERTS) pdl_wait();  // a launch in front may take longer than a wait may
             constexpr uint32_t kType = MODE == kDenseStoreF16 ? 0u : (1u << 7) | (1u << 10);  // fp16 or bf16, both operands
             constexpr uint32_t idesc = (1u << 4) | kType | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBlockRows >> 4) << 24);  // fp32 sums, K-major both
             uint32_t it = 0, done = 0;

@@ -141,6 +141,12 @@ void* smelt_cuda_stream(smelt_cuda_ctx* ctx) { return ctx ? (void*)ctx->stream :
 
 int smelt_cuda_sm_count(const smelt_cuda_ctx* ctx) { return ctx ? ctx->sm_count : 0; }
 
+// A kernel that gave up may have left arrivals at shared tiles behind, which the next product would count as its own.
+static cudaError_t clear_after_timeout(smelt_cuda_ctx* ctx) {
+    const cudaError_t e = cudaMemset(ctx->qmm_counters, 0, 4096 * sizeof(int));
+    return e == cudaSuccess ? cudaMemset(ctx->err_dev, 0, sizeof(uint32_t)) : e;
+}
+
 smelt_status smelt_cuda_device_error(smelt_cuda_ctx* ctx, uint32_t* out_flags) {
     CTX_OR_FAIL();
     if (!out_flags) return fail(ctx, SMELT_ERR_BAD_ARGUMENT, "out_flags is null");
@@ -149,7 +155,7 @@ smelt_status smelt_cuda_device_error(smelt_cuda_ctx* ctx, uint32_t* out_flags) {
     s = check_cuda(ctx, cudaMemcpy(out_flags, ctx->err_dev, 4, cudaMemcpyDeviceToHost), "read error word");
     if (s) return s;
     if (*out_flags) {
-        cudaMemset(ctx->err_dev, 0, 4);
+        clear_after_timeout(ctx);
         return fail(ctx, SMELT_ERR_DEVICE_TIMEOUT, "a kernel's bounded wait gave up (flags " + std::to_string(*out_flags) + ")");
     }
     return SMELT_OK;
@@ -158,7 +164,7 @@ smelt_status smelt_cuda_device_error(smelt_cuda_ctx* ctx, uint32_t* out_flags) {
 smelt_status smelt_cuda_clear_device_error(smelt_cuda_ctx* ctx) {
     CTX_OR_FAIL();
     smelt_status s = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
-    if (!s) s = check_cuda(ctx, cudaMemset(ctx->err_dev, 0, sizeof(uint32_t)), "clear error word");
+    if (!s) s = check_cuda(ctx, clear_after_timeout(ctx), "clear error word");
     return s;
 }
 

@@ -209,3 +209,38 @@ def test_exchange_wait_gives_up_and_reports():
         assert np.array_equal(y.download(np.float16, (1, n)), want)
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("product", ["affine_matvec", "fp16_matvec"])
+def test_product_behind_a_launch_longer_than_its_waits(oracle, product):
+    """Launched programmatically behind a reduction that polls for its absent peer for more than a second, a product neither
+    reports a timeout of its own nor computes anything wrong, and neither does the next one."""
+    rows, cols, batch = 1000, 4096, 32
+    c = capi.Context(0)
+    try:
+        c.call("tp_exchange_open_loopback", 2)
+        part, res, out = (c.to_device(synth.activations(12, n, 1, 4096)) for n in "pro")
+        x = synth.activations(14, "x", batch, cols)
+        if product == "affine_matvec":
+            w = synth.affine_u4(14, "w", rows, cols, 64)
+            ref, tail = oracle.affine_matvec(*w, x, rows, cols, 64), (rows, cols, 64, batch)
+        else:
+            w = (synth.normal_f16(14, "w", (rows, cols), 0.02),)
+            ref, tail = oracle.fp16_matvec(*w, x, rows, cols), (rows, cols, batch)
+        args = (*(c.to_device(a) for a in (*w, x)), c.alloc(batch * rows * 2).fill(0xFF))
+        c.call("capture_begin")
+        c.call("tp_reduce_add", part, res, out, C.c_size_t(4096))
+        c.call(product, *args, *tail)
+        c.call("capture_end")
+        ms = C.c_float(0)
+        c._check(c.lib.smelt_cuda_capture_replay(c.h, 0, 1, C.byref(ms)))
+        with pytest.raises(capi.SmeltError) as caught:
+            c.device_error()
+        assert str(caught.value).endswith("(flags 256)")  # the reduction's
+        assert ms.value > 1000
+        assert rel_err(args[-1].download(np.float16, (batch, rows)), ref) < 2e-3
+        args[-1].fill(0xFF)
+        c.call(product, *args, *tail)
+        assert rel_err(args[-1].download(np.float16, (batch, rows)), ref) < 2e-3 and c.device_error() == 0
+    finally:
+        c.close()
