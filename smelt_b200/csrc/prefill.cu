@@ -41,52 +41,55 @@ using namespace attn;
 // launch in front if no table holds them; then the threads take (head, pair) items, four loads in flight each.  With a
 // thread per pair that walked the heads the kernel waited for one load after the other: 27.4 us at 512 positions of 32 + 8
 // heads of 128, 11.4 us here.
-constexpr int kRopeThreads = 256;
+constexpr int kRopeThreads = 256, kRopePairs = 1024;  // pairs whose angles are held at a time
 __global__ void __launch_bounds__(kRopeThreads) rope_kv_prefill_kernel(__half* q, __half* k, const __half* v, const __half* cos_t,
                                                                        const __half* sin_t, __half* k_cache, __half* v_cache, int head_dim,
                                                                        int rope_dim, int q_heads, int kv_heads, uint32_t start_pos,
                                                                        uint32_t capacity, int layout, float base_log2, int math_mode,
                                                                        size_t table_stride) {
-    extern __shared__ float4 trig[];  // {cos, sin} of a pair's first and second element
+    __shared__ float4 trig[kRopePairs];  // {cos, sin} of a pair's first and second element
     pdl_trigger();
     if (cos_t) pdl_wait();
     const uint32_t t = blockIdx.x, pos = start_pos + t;
     if (pos >= capacity) return;  // the host validates; never write outside the cache
     const int half_rope = rope_dim / 2;
     if (cos_t) { cos_t += (size_t)pos * table_stride; sin_t += (size_t)pos * table_stride; }
-    for (int pair = threadIdx.x; pair < half_rope; pair += kRopeThreads) {
-        int d0, d1, c0i, c1i;
-        rope_indices(layout, pair, half_rope, head_dim, d0, d1, c0i, c1i);
-        float4 c;
-        rope_trig(pair, half_rope, pos, base_log2, math_mode, cos_t, sin_t, c0i, c1i, c.x, c.y, c.z, c.w);
-        trig[pair] = c;
-    }
-    if (!cos_t) pdl_wait();
-    __syncthreads();
     __half* qrow = q + (size_t)t * q_heads * head_dim;
     __half* krow = k + (size_t)t * kv_heads * head_dim;
-    const int items = (q_heads + kv_heads) * half_rope;
-    for (int base = threadIdx.x; base < items; base += 4 * kRopeThreads) {
-        __half *a[4], *b[4];
-        float x0[4], x1[4];
-        int pair[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int i = base + j * kRopeThreads, h = min(i, items - 1) / half_rope;
-            pair[j] = min(i, items - 1) - h * half_rope;
+    for (int first = 0; first < half_rope; first += kRopePairs) {
+        const int pairs = min(kRopePairs, half_rope - first), items = (q_heads + kv_heads) * pairs;
+        if (first > 0) __syncthreads();
+        for (int i = threadIdx.x; i < pairs; i += kRopeThreads) {
             int d0, d1, c0i, c1i;
-            rope_indices(layout, pair[j], half_rope, head_dim, d0, d1, c0i, c1i);
-            __half* row = h < q_heads ? qrow + (size_t)h * head_dim : krow + (size_t)(h - q_heads) * head_dim;
-            a[j] = row + d0;
-            b[j] = row + d1;
-            if (i < items) { x0[j] = __half2float(*a[j]); x1[j] = __half2float(*b[j]); }
+            rope_indices(layout, first + i, half_rope, head_dim, d0, d1, c0i, c1i);
+            float4 c;
+            rope_trig(first + i, half_rope, pos, base_log2, math_mode, cos_t, sin_t, c0i, c1i, c.x, c.y, c.z, c.w);
+            trig[i] = c;
         }
+        if (!cos_t && first == 0) pdl_wait();
+        __syncthreads();
+        for (int base = threadIdx.x; base < items; base += 4 * kRopeThreads) {
+            __half *a[4], *b[4];
+            float x0[4], x1[4];
+            int pair[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (base + j * kRopeThreads >= items) break;
-            const float4 c = trig[pair[j]];
-            *a[j] = __float2half_rn(__fsub_rn(__fmul_rn(x0[j], c.x), __fmul_rn(x1[j], c.y)));
-            *b[j] = __float2half_rn(__fadd_rn(__fmul_rn(x1[j], c.z), __fmul_rn(x0[j], c.w)));
+            for (int j = 0; j < 4; ++j) {
+                const int i = base + j * kRopeThreads, h = min(i, items - 1) / pairs;
+                pair[j] = min(i, items - 1) - h * pairs;
+                int d0, d1, c0i, c1i;
+                rope_indices(layout, first + pair[j], half_rope, head_dim, d0, d1, c0i, c1i);
+                __half* row = h < q_heads ? qrow + (size_t)h * head_dim : krow + (size_t)(h - q_heads) * head_dim;
+                a[j] = row + d0;
+                b[j] = row + d1;
+                if (i < items) { x0[j] = __half2float(*a[j]); x1[j] = __half2float(*b[j]); }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (base + j * kRopeThreads >= items) break;
+                const float4 c = trig[pair[j]];
+                *a[j] = __float2half_rn(__fsub_rn(__fmul_rn(x0[j], c.x), __fmul_rn(x1[j], c.y)));
+                *b[j] = __float2half_rn(__fadd_rn(__fmul_rn(x1[j], c.z), __fmul_rn(x0[j], c.w)));
+            }
         }
     }
     __syncthreads();  // the rotated keys are complete before they are copied
@@ -328,11 +331,6 @@ cudaError_t launch_rope_kv_prefill(const Launch& l, __half* q, __half* k, const 
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_pos);
     cfg.blockDim = dim3(kRopeThreads);
-    cfg.dynamicSmemBytes = (size_t)rope_dim / 2 * sizeof(float4);
-    if (cfg.dynamicSmemBytes > 48 * 1024) {  // more than 6144 rotated dimensions
-        const cudaError_t e = cudaFuncSetAttribute(rope_kv_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
-        if (e != cudaSuccess) return e;
-    }
     cfg.stream = l.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

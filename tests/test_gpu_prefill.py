@@ -60,6 +60,21 @@ def test_rope_kv_prefill_is_the_per_position_kernels(ctx, oracle, layout, rope_d
     assert st == capi.OUT_OF_RANGE
 
 
+# more pairs than a CTA holds the angles of, and more than its shared memory could
+@pytest.mark.parametrize("layout,d", [(0, 2050), (1, 60000)])
+def test_rope_kv_prefill_wide_heads(ctx, oracle, layout, d):
+    n_pos, cap, base_log2 = 2, 5, float(np.log2(10000.0))
+    q, k, v = (synth.activations(37, n, n_pos, 1, d) for n in "qkv")
+    bufs = [ctx.to_device(a) for a in (q, k, v)] + [ctx.alloc(cap * d * 2).fill(0) for _ in range(2)]
+    ctx.call("rope_kv_prefill", *bufs[:3], None, None, *bufs[3:], d, d, 1, 1, n_pos, 1, cap, layout, C.c_float(base_log2), 1)
+    got_q, got_k = bufs[0].download(np.uint16, (n_pos, d)), bufs[3].download(np.uint16, (cap, d))
+    for t in range(n_pos):
+        assert np.array_equal(got_q[t], oracle.apply_rope(q[t], d, d, 1, layout, 1 + t, base_log2, 1, None, None).reshape(d).view(np.uint16))
+        assert np.array_equal(got_k[1 + t], oracle.apply_rope(k[t], d, d, 1, layout, 1 + t, base_log2, 1, None, None).reshape(d).view(np.uint16))
+    for b in bufs:
+        b.free()
+
+
 @pytest.mark.parametrize("n_q,n_kv,d", [(16, 4, 128), (8, 2, 256), (8, 8, 64), (16, 1, 64), (32, 8, 128)])
 @pytest.mark.parametrize("n_pos,start,window", [(37, 0, 0), (64, 200, 0), (5, 1000, 0), (40, 90, 48)])
 def test_attention_prefill_matches_the_oracle_per_position(ctx, oracle, n_q, n_kv, d, n_pos, start, window):
