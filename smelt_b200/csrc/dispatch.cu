@@ -1471,7 +1471,7 @@ smelt_status run_record(Interp& in, const smelt_dispatch_record& rec_in) {
             NEED_BYTES(0, (size_t)t * hq * d * 2); NEED_BYTES(3, (size_t)t * hq * d * 2); NEED_BYTES(1, (size_t)hkv * cap * d * 2); NEED_BYTES(2, (size_t)hkv * cap * d * 2);
             in.launches += 1;
             return check_cuda(ctx, launch_attention_prefill(l, (const __half*)r.buf[0].ptr, (const __half*)r.buf[1].ptr, (const __half*)r.buf[2].ptr, (__half*)r.buf[3].ptr, hq, (int)hkv, (int)d,
-                                                            t, start, cap, as_f32(scale_bits), window), p.name.c_str());
+                                                            t, start, cap, as_f32(scale_bits), window, ctx->sm_count), p.name.c_str());
         }
         case PK_EMBEDDING_GATHER_BATCHED: {
             // lut_matvec.metal:1121-1134: 0 table, 1 token ids [B], 2 out [B, hidden], 3 hidden, 4 batchSize.

@@ -40,7 +40,7 @@ cudaError_t launch_elementwise(const Launch& l, int op, const __half* a, const _
 cudaError_t launch_row_norm(const Launch& l, const __half* x, const __half* pre, const __half* w, const __half* residual, const __half* scalar, __half* y, float* scale_out, int rows, int dim, float eps, int topology, int tgs, int value, int scale, int group_rows = 0, int group_stride = 0);
 // prompt-chunk RoPE + KV write and causal attention (prefill.cu)
 cudaError_t launch_rope_kv_prefill(const Launch& l, __half* q, __half* k, const __half* v, const __half* cos_t, const __half* sin_t, __half* k_cache, __half* v_cache, int head_dim, int rope_dim, int q_heads, int kv_heads, uint32_t n_pos, uint32_t start_pos, uint32_t capacity, int layout, float base_log2, int math_mode, size_t table_stride);
-cudaError_t launch_attention_prefill(const Launch& l, const __half* q, const __half* k_cache, const __half* v_cache, __half* out, int n_q, int n_kv, int head_dim, uint32_t n_pos, uint32_t start_pos, uint32_t capacity, float scale, uint32_t window);
+cudaError_t launch_attention_prefill(const Launch& l, const __half* q, const __half* k_cache, const __half* v_cache, __half* out, int n_q, int n_kv, int head_dim, uint32_t n_pos, uint32_t start_pos, uint32_t capacity, float scale, uint32_t window, int sm_count);
 cudaError_t launch_gate_split(const Launch& l, const __half* in, __half* query, __half* gate, int heads, int head_dim);
 cudaError_t launch_head_norm(const Launch& l, int mode, const __half* x, const __half* w, __half* y, int heads, int head_dim, float eps, int tgs);
 cudaError_t launch_signed_embedding_gather(const Launch& l, int format, const uint8_t* codes, const __half* scales, const int32_t* token_ids, __half* out, int hidden, int batch);

@@ -102,8 +102,6 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kv_prefill_kernel(__half* q
     }
 }
 
-constexpr uint32_t kAttnFill = 148;  // SMs
-
 template <int D, int NH, int KS>
 __host__ __device__ constexpr size_t prefill_attn_smem() {  // two buffers of KS tiles' K and V halves, and later the key parts' sums
     const size_t tiles = (size_t)2 * KS * 2 * (D / 16) * 512, sums = KS > 1 ? (size_t)(kAttnWarps - kAttnWarps / KS) * 32 * NH * (D / 4 + 4) * sizeof(float) : 0;
@@ -304,11 +302,11 @@ cudaError_t launch_prefill_attention_ks(const Launch& l, const __half* q, const 
 // Key parts: as few as give every SM a CTA (a CTA walks its keys tile by tile, about 1 us each, whatever its positions).
 template <int D, int NH>
 cudaError_t launch_prefill_attention_t(const Launch& l, const __half* q, const __half* kc, const __half* vc, __half* out, int n_q, int n_kv,
-                                       uint32_t n_pos, uint32_t start_pos, uint32_t capacity, float scale, uint32_t window) {
+                                       uint32_t n_pos, uint32_t start_pos, uint32_t capacity, float scale, uint32_t window, uint32_t sm_count) {
     const uint32_t per_warp = std::max(1, 8 * NH / (n_q / n_kv));
     auto ctas = [&](uint32_t ks) { const uint32_t step = kAttnWarps / ks * per_warp; return (n_pos + step - 1) / step * (uint32_t)n_kv; };
-    if (ctas(1) >= kAttnFill) return launch_prefill_attention_ks<D, NH, 1>(l, q, kc, vc, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, per_warp);
-    if (ctas(2) >= kAttnFill) return launch_prefill_attention_ks<D, NH, 2>(l, q, kc, vc, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, per_warp);
+    if (ctas(1) >= sm_count) return launch_prefill_attention_ks<D, NH, 1>(l, q, kc, vc, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, per_warp);
+    if (ctas(2) >= sm_count) return launch_prefill_attention_ks<D, NH, 2>(l, q, kc, vc, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, per_warp);
     return launch_prefill_attention_ks<D, NH, 4>(l, q, kc, vc, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, per_warp);
 }
 
@@ -344,14 +342,14 @@ cudaError_t launch_rope_kv_prefill(const Launch& l, __half* q, __half* k, const 
 
 cudaError_t launch_attention_prefill(const Launch& l, const __half* q, const __half* k_cache, const __half* v_cache, __half* out, int n_q,
                                      int n_kv, int head_dim, uint32_t n_pos, uint32_t start_pos, uint32_t capacity, float scale,
-                                     uint32_t window) {
+                                     uint32_t window, int sm_count) {
     if (n_pos == 0) return cudaSuccess;
     if (n_q <= 0 || n_kv <= 0 || n_q % n_kv || n_q / n_kv > 16 || (uint64_t)start_pos + n_pos > capacity) return cudaErrorInvalidValue;
     const int nh = n_q / n_kv > 8 ? 2 : 1;
 #define SMELT_PREFILL_CASE(DD)                                                                                                           \
     case DD:                                                                                                                             \
-        return nh == 1 ? launch_prefill_attention_t<DD, 1>(l, q, k_cache, v_cache, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window) \
-                       : launch_prefill_attention_t<DD, 2>(l, q, k_cache, v_cache, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window);
+        return nh == 1 ? launch_prefill_attention_t<DD, 1>(l, q, k_cache, v_cache, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, sm_count) \
+                       : launch_prefill_attention_t<DD, 2>(l, q, k_cache, v_cache, out, n_q, n_kv, n_pos, start_pos, capacity, scale, window, sm_count);
     switch (head_dim) {
         SMELT_PREFILL_CASE(64)
         SMELT_PREFILL_CASE(128)
@@ -401,7 +399,7 @@ smelt_status smelt_cuda_attention_prefill(smelt_cuda_ctx* ctx, const void* q, co
     l.stream = ctx->stream;
     l.pdl = ctx->capturing && ctx->pdl;
     return check_cuda(ctx, launch_attention_prefill(l, (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, (__half*)out, n_q, n_kv,
-                                                    head_dim, n_pos, start_pos, capacity, scale, sliding_window),
+                                                    head_dim, n_pos, start_pos, capacity, scale, sliding_window, ctx->sm_count),
                       "attention prefill");
 }
 
@@ -492,7 +490,7 @@ smelt_status smelt_cuda_prefill(smelt_cuda_ctx* ctx, const smelt_decoder_desc* d
             PF(affine(kAffinePlain, w.q, nullptr, xn, qb, nullptr, nullptr, qd, H, n), "prefill: Q projection");
             PF(affine(kAffineDual, w.k, &w.v, xn, kb, vb, nullptr, kvd, H, n), "prefill: K | V projection");
             PF(launch_rope_kv_prefill(l, qb, kb, vb, nullptr, nullptr, kc, vc, D, D, d->n_q, d->n_kv, (uint32_t)n, p0, cap, 1, log2_theta, 1, 0), "prefill: rope + kv write");
-            PF(launch_attention_prefill(l, qb, kc, vc, ab, d->n_q, d->n_kv, D, (uint32_t)n, p0, cap, scale, 0), "prefill: attention");
+            PF(launch_attention_prefill(l, qb, kc, vc, ab, d->n_q, d->n_kv, D, (uint32_t)n, p0, cap, scale, 0, ctx->sm_count), "prefill: attention");
             PF(affine(kAffineAdd, w.o, nullptr, ab, x1, nullptr, x0, H, qd, n), "prefill: O projection + residual");
             PF(launch_rms_norm_1pw(l, x1, (const __half*)(W + w.post_norm), xn, H, d->eps, n), "prefill: post norm");
             PF(affine(kAffineGateUp, w.gate, &w.up, xn, hb, nullptr, nullptr, I, H, n), "prefill: gate / up + SwiGLU");
