@@ -807,7 +807,7 @@ SMELT_CUDA_API smelt_status smelt_cuda_attention_prefill(smelt_cuda_ctx* ctx, co
                                                          uint32_t sliding_window);
 /* Prompt tokens [start_pos, start_pos + n_tokens) of one sequence through the decoder that
  * smelt_cuda_build_decoder was given (same descriptor and layer references, batch 1, one GPU),
- * `chunk` positions at a time (0 = 512): batched projections (tensor-memory QMM from 17 rows),
+ * `chunk` positions at a time (0 = 512): batched projections (the tensor-core product from 17 rows),
  * rope_kv_prefill, attention_prefill; LM head and argmax for the last position only.  Leaves
  * the KV caches filled, the last logits in the logits slot and *out_token (optional) = the
  * argmax after the last prompt token, so decoding continues with smelt_cuda_graph_seed /

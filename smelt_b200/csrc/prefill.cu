@@ -9,7 +9,7 @@
 // causally to keys [seqStart, startPos + t], seqStart from the sliding window, softmax in fp32,
 // fp16 out [T, qHeads, headDim].  The matmuls of the chunk are the batched affine kernels
 // (agent_affine_qmm_fixed_batched_full, Resources/Shaders/agent_affine_qmm.h:107-316), which
-// from seventeen rows on run on the tensor-core product (affine_wide.cu).
+// from seventeen rows on (nine with a long K) run on the tensor-core product (affine_wide.cu).
 //
 // attn_prefill_kernel: one CTA per (run of query positions, KV head) on the decode kernel's tile arithmetic (attention.cuh:
 // S^T = K.Q^T and O^T = V^T.P^T on mma.sync, P as fp16 high + low parts).  A tile has eight columns: the query heads that
