@@ -18,15 +18,6 @@ EncodeTiled encode_tiled() {
     return fn;
 }
 
-// A row-major matrix read in boxes of box_rows rows x 128 bytes, 128-byte swizzle; beyond its edges: zeros.
-bool encode(CUtensorMap* map, CUtensorMapDataType type, int width, const void* base, long rows, long cols, int box_rows) {
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)(cols * width)};
-    const cuuint32_t box[2] = {(cuuint32_t)(128 / width), (cuuint32_t)box_rows}, step[2] = {1, 1};
-    const EncodeTiled fn = encode_tiled();
-    return fn && fn(map, type, 2, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // How many CTAs take the line: either a whole number for each tile, or all SMs, whose stretches then begin and end anywhere.
 // Estimated in us.  A group takes a CTA 0.53 us with 32 rows of x, 0.57 with 128 and 0.96 with 256; the CTA that finishes a tile
 // needs 0.011 us per column and CTA whose sums it adds, and with stretches anywhere it may finish two, of one CTA more each.
@@ -48,6 +39,14 @@ long ctas_for(const Line& p, int sm) {
 
 }  // namespace
 
+bool encode_rows(CUtensorMap* map, CUtensorMapDataType type, int width, const void* base, long rows, long cols, int box_rows) {
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)(cols * width)};
+    const cuuint32_t box[2] = {(cuuint32_t)(128 / width), (cuuint32_t)box_rows}, step[2] = {1, 1};
+    const EncodeTiled fn = encode_tiled();
+    return fn && fn(map, type, 2, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps* maps, Line* line, int* grid) {
     if (group != kLineGroup || a.cols % kLineGroup != 0 || a.norm_w) return false;
     if (a.nseg > 1 && affine_stream_passes(mode, a, group) == 0) return false;
@@ -64,7 +63,7 @@ bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps*
     for (int s = 0; s < (paired ? 2 : segs ? a.nseg : 1); ++s) {
         const uint8_t* w = segs ? a.seg[s].w : a.w[s];
         const int rows = segs ? a.seg[s].rows : a.rows;
-        if ((reinterpret_cast<uintptr_t>(w) & 15u) || !encode(&maps->w[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w, rows, a.cols / 2, paired ? 64 : kLineRows)) return false;
+        if ((reinterpret_cast<uintptr_t>(w) & 15u) || !encode_rows(&maps->w[s], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w, rows, a.cols / 2, paired ? 64 : kLineRows)) return false;
         if (!paired) {
             if (s == 1) line->first1 = line->row_tiles;
             if (s == 2) line->first2 = line->row_tiles;
@@ -73,7 +72,7 @@ bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps*
     }
     if (paired) line->row_tiles = (a.rows + 63) / 64;
     const long tiles = (long)line->row_tiles * line->col_tiles, units = tiles * line->groups;
-    if (units >= 1l << 30 || !encode(&maps->x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.x, a.batch, a.cols, line->tile_cols)) return false;
+    if (units >= 1l << 30 || !encode_rows(&maps->x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.x, a.batch, a.cols, line->tile_cols)) return false;
     const size_t sums = (size_t)sm * 2 * line->tile_cols * kLineRows * sizeof(float);  // two tiles of every CTA
     if (!a.part_scratch || !a.part_counters || sums > a.part_scratch_bytes) return false;
     const bool split = tiles <= 4096;  // a counter each

@@ -76,40 +76,18 @@ __device__ __forceinline__ LineRow line_row(const AffineArgs& a, const Line& p, 
     return o;
 }
 
-__device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y),
-                 "r"(smem_u32(bar))
-                 : "memory");
-}
 // Packed weights of one stage: groups g .. g + 3 of the tile's rows.
 template <int MODE>
 __device__ __forceinline__ void request_weights(const LineMaps& maps, const Line& p, int row_tile, int g, uint8_t* dst, uint64_t* bar) {
     if (MODE == kAffineGateUp || MODE == kAffineDual) {
-        tma_2d(dst, &maps.w[0], g * (kLineGroup / 2), row_tile * 64, bar);
-        tma_2d(dst + kRawBytes / 2, &maps.w[1], g * (kLineGroup / 2), row_tile * 64, bar);
+        tma_load_2d(dst, &maps.w[0], g * (kLineGroup / 2), row_tile * 64, bar);
+        tma_load_2d(dst + kRawBytes / 2, &maps.w[1], g * (kLineGroup / 2), row_tile * 64, bar);
     } else {
         const int seg = (row_tile >= p.first1) + (row_tile >= p.first2);
-        tma_2d(dst, &maps.w[seg], g * (kLineGroup / 2), (row_tile - (seg == 0 ? 0 : seg == 1 ? p.first1 : p.first2)) * kLineRows, bar);
+        tma_load_2d(dst, &maps.w[seg], g * (kLineGroup / 2), (row_tile - (seg == 0 ? 0 : seg == 1 ? p.first1 : p.first2)) * kLineRows, bar);
     }
 }
 
-// Waits for a phase; gives up after about a second, or as soon as another role has.
-__device__ __forceinline__ bool wait_alive(uint64_t* bar, uint32_t parity, volatile uint32_t* dead) {
-    for (uint32_t i = 0; i < (1u << 20); ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
-            : "memory");
-        if (ok) return true;
-        if (*dead) return false;
-    }
-    *dead = 1u;
-    return false;
-}
 __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* dead) { return __all_sync(0xffffffffu, wait_alive(bar, parity, dead)); }
 // Whether a phase has completed, without waiting: several are asked at once and only what is missing is waited for.
 __device__ __forceinline__ bool peek(uint64_t* bar, uint32_t parity) {

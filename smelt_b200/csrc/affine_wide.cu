@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kThreads, 1) affine_wide_kernel(const __grid_c
                     if (it >= C::kXStages && !(alive = turn_done(it - C::kXStages, wait_alive))) break;
                     const int n = min(2, t.g1 - g);
                     mbar_arrive_expect_tx(&x_full[s], bytes * n);
-                    for (int i = 0; i < n; ++i) tma_2d(x_tiles + (2 * s + i) * C::kXBytes, &maps.x, (g + i) * kLineGroup, t.col0, &x_full[s]);
+                    for (int i = 0; i < n; ++i) tma_load_2d(x_tiles + (2 * s + i) * C::kXBytes, &maps.x, (g + i) * kLineGroup, t.col0, &x_full[s]);
                 }
                 u += t.g1 - t.g0;
             }

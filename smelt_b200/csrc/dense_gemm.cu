@@ -1,6 +1,6 @@
 // Matrix products of a prompt chunk: Y[m, rows] = X[m, cols] . W[rows, cols]^T, bf16 weights.
 //
-// gemm_bf16_kernel (bf16 activations): tcgen05.  The weight rows are the MMA's M (128 per tile),
+// gemm_16bit_kernel (bf16 activations): tcgen05.  The weight rows are the MMA's M (128 per tile),
 // the chunk's positions its N (16 .. 256 per tile), so a tile's output is transposed on the way out:
 // tensor-memory lane r is weight row r, and a warp stores 32 adjacent rows of one position at a
 // time.  Warp 0 brings both operands with TMA (64 columns = one 128-byte swizzled row per stage,
@@ -21,8 +21,6 @@
 // copies and MMAs in flight are waited for (bounded too) and the tensor memory is freed.
 //
 // gemm_f32_kernel: fp32 activations and arithmetic on the CUDA cores (the fp32 table).
-#include <cuda.h>
-
 #include <algorithm>
 
 #include "dense.h"
@@ -47,30 +45,6 @@ __host__ __device__ constexpr int gemm_stages(int bn) { return bn == 256 ? 4 : b
 __host__ __device__ constexpr uint32_t gemm_stage_bytes(int bn) { return kATile + (uint32_t)bn * kBlockCols * 2; }
 __host__ __device__ constexpr uint32_t gemm_smem(int bn) { return gemm_stages(bn) * gemm_stage_bytes(bn) + 1024; }
 
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y),
-                 "r"(smem_u32(bar))
-                 : "memory");
-}
-
-// Waits for a phase; gives up after about a second, or as soon as another role has.
-__device__ __forceinline__ bool wait_alive(uint64_t* bar, uint32_t parity, volatile uint32_t* dead) {
-    for (uint32_t i = 0; i < (1u << 20); ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
-            : "memory");
-        if (ok) return true;
-        if (*dead) return false;
-    }
-    *dead = 1u;
-    return false;
-}
-
 struct GemmPlan {
     int row_tiles, token_tiles, ksplit, units;
 };
@@ -94,7 +68,7 @@ __device__ __forceinline__ void activate(float (&v)[N], const DenseOut& o) {
 
 // ACT: what the rows past the split go through; kDenseStoreF32: kDenseDecay, or anything else for nothing.
 template <int BN, int MODE, int ACT, bool EXPERTS>
-__global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const DenseGemmArgs a,
+__global__ void __launch_bounds__(kGemmThreads, 1) gemm_16bit_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const DenseGemmArgs a,
                                                                     const GemmPlan plan) {
     constexpr int kStages = gemm_stages(BN);
     constexpr uint32_t kStageBytes = gemm_stage_bytes(BN), kTmemCols = 2 * BN < 32 ? 32 : 2 * BN;
@@ -380,59 +354,39 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_bf16_kernel(const __grid
     }
 }
 
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_tiled() {
-    static const EncodeTiled fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult found;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) p = nullptr;
-        return reinterpret_cast<EncodeTiled>(p);
-    }();
-    return fn;
-}
-
-// A row-major [rows, cols] bf16 matrix read in boxes of box_rows x 64 columns, 128-byte swizzle.
-bool encode_rows(CUtensorMap* map, const void* base, int rows, int cols, int box_rows) {
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)cols * 2};
-    const cuuint32_t box[2] = {kBlockCols, (cuuint32_t)box_rows}, step[2] = {1, 1};
-    const EncodeTiled fn = encode_tiled();
-    return fn && fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 template <int BN>
 cudaError_t launch_bf16_t(const Launch& l, int mode, const DenseGemmArgs& a, const GemmPlan& plan) {
     CUtensorMap mw, mx;
     const int groups = a.group_rows ? a.groups : 1;
-    if (!encode_rows(&mw, a.w, a.table ? a.rows * a.experts : a.rows, a.cols, kBlockRows) || !encode_rows(&mx, a.x, a.m + (groups - 1) * a.x_group, a.cols, BN)) return cudaErrorInvalidValue;
+    const CUtensorMapDataType type = mode == kDenseStoreF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    if (!encode_rows(&mw, type, 2, a.w, a.table ? a.rows * a.experts : a.rows, a.cols, kBlockRows) || !encode_rows(&mx, type, 2, a.x, a.m + (groups - 1) * a.x_group, a.cols, BN))
+        return cudaErrorInvalidValue;
     const dim3 grid(std::min(plan.units, a.sm_count > 0 ? a.sm_count : 148)), block(kGemmThreads);
     auto go = [&](auto kernel) { return launch_chained(l, kernel, grid, block, gemm_smem(BN), mw, mx, a, plan); };
     if (a.table) {
         if constexpr (BN >= 32 && BN <= 128) {
-            if (mode == kDenseStoreF32) return go(gemm_bf16_kernel<BN, kDenseStoreF32, kDenseXielu, true>);
-            if (mode == kDenseStoreGlu) return go(gemm_bf16_kernel<BN, kDenseStoreGlu, kDenseXielu, true>);
+            if (mode == kDenseStoreF32) return go(gemm_16bit_kernel<BN, kDenseStoreF32, kDenseXielu, true>);
+            if (mode == kDenseStoreGlu) return go(gemm_16bit_kernel<BN, kDenseStoreGlu, kDenseXielu, true>);
         }
         return cudaErrorInvalidValue;
     }
     switch (mode) {
-        case kDenseStoreF32: return a.out.act == kDenseDecay ? go(gemm_bf16_kernel<BN, kDenseStoreF32, kDenseDecay, false>) : go(gemm_bf16_kernel<BN, kDenseStoreF32, kDenseXielu, false>);
-        case kDenseAddF32: return go(gemm_bf16_kernel<BN, kDenseAddF32, kDenseXielu, false>);
+        case kDenseStoreF32: return a.out.act == kDenseDecay ? go(gemm_16bit_kernel<BN, kDenseStoreF32, kDenseDecay, false>) : go(gemm_16bit_kernel<BN, kDenseStoreF32, kDenseXielu, false>);
+        case kDenseAddF32: return go(gemm_16bit_kernel<BN, kDenseAddF32, kDenseXielu, false>);
         case kDenseStoreF16:
-            if constexpr (BN <= 128) return go(gemm_bf16_kernel<BN, kDenseStoreF16, kDenseXielu, false>);
+            if constexpr (BN <= 128) return go(gemm_16bit_kernel<BN, kDenseStoreF16, kDenseXielu, false>);
             return cudaErrorInvalidValue;
         case kDenseStoreAct:
             switch (a.out.act) {
-                case kDenseXielu: return go(gemm_bf16_kernel<BN, kDenseStoreAct, kDenseXielu, false>);
-                case kDenseRelu2: return go(gemm_bf16_kernel<BN, kDenseStoreAct, kDenseRelu2, false>);
-                case kDenseTanh: return go(gemm_bf16_kernel<BN, kDenseStoreAct, kDenseTanh, false>);
+                case kDenseXielu: return go(gemm_16bit_kernel<BN, kDenseStoreAct, kDenseXielu, false>);
+                case kDenseRelu2: return go(gemm_16bit_kernel<BN, kDenseStoreAct, kDenseRelu2, false>);
+                case kDenseTanh: return go(gemm_16bit_kernel<BN, kDenseStoreAct, kDenseTanh, false>);
                 default: return cudaErrorInvalidValue;
             }
         case kDenseStoreMixed:
             switch (a.out.act) {
-                case kDenseRelu2: return go(gemm_bf16_kernel<BN, kDenseStoreMixed, kDenseRelu2, false>);
-                case kDenseTanh: return go(gemm_bf16_kernel<BN, kDenseStoreMixed, kDenseTanh, false>);
+                case kDenseRelu2: return go(gemm_16bit_kernel<BN, kDenseStoreMixed, kDenseRelu2, false>);
+                case kDenseTanh: return go(gemm_16bit_kernel<BN, kDenseStoreMixed, kDenseTanh, false>);
                 default: return cudaErrorInvalidValue;
             }
         default: return cudaErrorInvalidValue;

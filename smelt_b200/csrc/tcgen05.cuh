@@ -1,6 +1,8 @@
 // Inline-PTX wrappers for the fifth-generation tensor core path (tcgen05.mma with accumulators in
 // tensor memory) and the mbarrier waits around it, shared by the kernels that use it.
 #pragma once
+#include <cuda.h>
+
 #include "common.cuh"
 
 namespace smelt {
@@ -24,6 +26,29 @@ __device__ __forceinline__ bool mbar_poll_bounded(uint64_t* bar, uint32_t parity
         if (ok) return true;
     }
     return false;
+}
+// Waits for a phase; gives up after about a second, or as soon as another role has.
+__device__ __forceinline__ bool wait_alive(uint64_t* bar, uint32_t parity, volatile uint32_t* dead) {
+    for (uint32_t i = 0; i < (1u << 20); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
+            : "memory");
+        if (ok) return true;
+        if (*dead) return false;
+    }
+    *dead = 1u;
+    return false;
+}
+// A box of a 2-D tensor map, x the inner coordinate (a multiple of 16 bytes).
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y),
+                 "r"(smem_u32(bar))
+                 : "memory");
 }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -74,5 +99,9 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t base, uint32_t cols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// A row-major matrix of `width`-byte elements read in boxes of box_rows rows x 128 bytes, 128-byte swizzle; beyond its edges: zeros
+// (affine_line.cu).
+bool encode_rows(CUtensorMap* map, CUtensorMapDataType type, int width, const void* base, long rows, long cols, int box_rows);
 
 }  // namespace smelt
