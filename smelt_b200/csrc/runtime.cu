@@ -143,8 +143,8 @@ int smelt_cuda_sm_count(const smelt_cuda_ctx* ctx) { return ctx ? ctx->sm_count 
 
 // A kernel that gave up may have left arrivals at shared tiles behind, which the next product would count as its own.
 static cudaError_t clear_after_timeout(smelt_cuda_ctx* ctx) {
-    const cudaError_t e = cudaMemset(ctx->qmm_counters, 0, 4096 * sizeof(int));
-    return e == cudaSuccess ? cudaMemset(ctx->err_dev, 0, sizeof(uint32_t)) : e;
+    const cudaError_t e = cudaMemsetAsync(ctx->qmm_counters, 0, 4096 * sizeof(int), ctx->stream);  // ahead of the next launch
+    return e == cudaSuccess ? cudaMemsetAsync(ctx->err_dev, 0, sizeof(uint32_t), ctx->stream) : e;
 }
 
 smelt_status smelt_cuda_device_error(smelt_cuda_ctx* ctx, uint32_t* out_flags) {
