@@ -20,7 +20,8 @@ EncodeTiled encode_tiled() {
 
 // How many CTAs take the line: either a whole number for each tile, or all SMs, whose stretches then begin and end anywhere.
 // Estimated in us.  A group takes a CTA 0.53 us with 32 rows of x, 0.57 with 128 and 0.96 with 256; the CTA that finishes a tile
-// needs 0.011 us per column and CTA whose sums it adds, and with stretches anywhere it may finish two, of one CTA more each.
+// needs 0.011 us per column and CTA whose sums it adds, and with stretches anywhere it may finish two, of one CTA more each
+// (weighed with 1.5: at 512 rows 4096 x 12288 takes 110.8 by whole numbers and 104.6 by stretches, 6144 x 2048 49.2 and 46.4).
 // Measured (us, by CTAs of a tile; 148: all SMs): 1024 x 12288, 32 rows: 4 30.7, 8 19.4, 16 15.6, 148 19.2; 256 rows: 4 63.3,
 // 8 51.6, 16 60.2, 148 72.3; 4096 x 4096, 32 rows: 2 22.6, 4 15.5, 148 18.0; 256 rows: 4 36.2, 148 47.7; K | V 1024 x 4096 x 2,
 // 32 rows: 4 13.8, 8 11.2, 148 14.7; 512 rows: 4 35.8, 148 47.5; 4096 x 12288, 32 rows: 4 33.7, 148 34.4; gate/up 6144 x 2048,
@@ -29,7 +30,7 @@ long ctas_for(const Line& p, int sm) {
     const long tiles = (long)p.row_tiles * p.col_tiles, quanta = p.groups / p.quantum;
     const double group = p.tile_cols <= 128 ? 0.52 + 0.0004 * p.tile_cols : 0.96, sum = 0.011 * p.tile_cols;
     long best = sm;
-    double least = (double)tiles * p.groups / sm * group + 2.0 * sum * ((double)sm / tiles + 1.0);
+    double least = (double)tiles * p.groups / sm * group + 1.5 * sum * ((double)sm / tiles + 1.0);
     for (long k = 1; k <= quanta && tiles * k <= sm; ++k) {
         const double cost = (double)((quanta + k - 1) / k * p.quantum) * group + (k > 1 ? sum * k : 0.0);
         if (cost < least) { least = cost; best = tiles * k; }

@@ -449,20 +449,22 @@ cudaError_t launch_group(const Launch& l, const AffineArgs& a, int group) {
 // number of rows, about as much as two passes of the streaming kernel with all its activations to stage.
 //   * 17 rows and more: always (gate/up 12288 x 4096, 16 rows on the streaming kernel 46.8 us, 17 rows here 57.3, 32 rows 57.7,
 //     where the streaming kernel would take four passes).
-//   * 9 to 16 rows with a residual, where the streaming kernel takes several passes over 128 K activations and more (us, passes
-//     against it): 4096 x 12288, 9 rows (108 K) 32.7 : 34.4, 12 rows (144 K) 35.5 : 34.3, 16 rows 51.4 : 34.5; 5120 x 17408, 9 rows
-//     (153 K) 56.6 : 52.2, 16 rows 108 : 52.3.
+//   * 9 to 16 rows with a residual, where the streaming kernel takes several passes over 64 K activations and more (us, passes
+//     against it): 4096 x 4096, 12 rows (48 K) 14.6 : 15.1, 16 rows 16.7 : 15.1; 2048 x 6144, 16 rows (96 K) 17.0 : 12.9; 4096 x 12288,
+//     9 rows (108 K) 32.7 : 32.9, 16 rows 51.5 : 32.9; 1024 x 12288, 9 rows 20.8 : 13.5; 5120 x 17408, 9 rows 60.2 : 50.2, 16 rows
+//     117 : 50.3.
 //   * 9 to 16 rows that the streaming kernel does not take, from 64 K activations on: gate/up 3000 x 6976, 9 rows (61 K) 49.4 on
-//     the general kernel, 12 rows (82 K) 54.8 : 38.6, 16 rows 61.5 : 38.4.
+//     the general kernel, 12 rows (82 K) 54.9 : 38.6; 4096 x 6976, 10 rows (68 K) 27.2 : 29.8, 12 rows
+//     54.1 : 29.8.
 //   * Plain products that the streaming kernel takes stay there up to 16 rows: one launch over several tensors
 //     (affine_multi_matvec) runs on it, and gives the bits of a launch for each.
 //   * Up to eight rows never: the general kernel splits K over a cluster, and few rows of weights make no tile worth the
-//     expansion (512 x 17408, 6 rows 8.1 : 38.2).
+//     expansion (1024 x 12288, 8 rows 9.4 : 13.4; 5120 x 17408, 8 rows 62.3 : 50.2).
 bool wide_first(int mode, const AffineArgs& a, int group) {
     if (a.batch >= 17) return true;
     if (a.batch <= 8 || a.norm_w || a.nseg > 1) return false;
     const int passes = affine_stream_passes(mode, a, group);
-    return passes == 0 ? (size_t)a.batch * a.cols >= 65536u : passes > 1 && mode == kAffineAdd && (size_t)a.batch * a.cols >= 131072u;
+    return passes == 0 ? (size_t)a.batch * a.cols >= 65536u : passes > 1 && mode == kAffineAdd && (size_t)a.batch * a.cols >= 65536u;
 }
 
 }  // namespace
