@@ -19,23 +19,22 @@ EncodeTiled encode_tiled() {
 }
 
 // How many CTAs take the line: either a whole number for each tile, or all SMs, whose stretches then begin and end anywhere.
-// Estimated in us.  A group takes a CTA 0.53 us with 32 rows of x, 0.57 with 128 and 0.96 with 256; the CTA that finishes a tile
-// needs 0.011 us per column and CTA whose sums it adds, and with stretches anywhere it may finish two, of one CTA more each
-// (weighed with 1.5: at 512 rows 4096 x 12288 takes 110.8 by whole numbers and 104.6 by stretches, 6144 x 2048 49.2 and 46.4).
-// Measured (us, by CTAs of a tile; 148: all SMs): 1024 x 12288, 32 rows: 4 30.7, 8 19.4, 16 15.6, 148 19.2; 256 rows: 4 63.3,
-// 8 51.6, 16 60.2, 148 72.3; 4096 x 4096, 32 rows: 2 22.6, 4 15.5, 148 18.0; 256 rows: 4 36.2, 148 47.7; K | V 1024 x 4096 x 2,
-// 32 rows: 4 13.8, 8 11.2, 148 14.7; 512 rows: 4 35.8, 148 47.5; 4096 x 12288, 32 rows: 4 33.7, 148 34.4; gate/up 6144 x 2048,
-// 32 rows: 1 22.6, 148 22.3.
-long ctas_for(const Line& p, int sm) {
-    const long tiles = (long)p.row_tiles * p.col_tiles, quanta = p.groups / p.quantum;
-    const double group = p.tile_cols <= 128 ? 0.52 + 0.0004 * p.tile_cols : 0.96, sum = 0.011 * p.tile_cols;
-    long best = sm;
-    double least = (double)tiles * p.groups / sm * group + 1.5 * sum * ((double)sm / tiles + 1.0);
-    for (long k = 1; k <= quanta && tiles * k <= sm; ++k) {
-        const double cost = (double)((quanta + k - 1) / k * p.quantum) * group + (k > 1 ? sum * k : 0.0);
-        if (cost < least) { least = cost; best = tiles * k; }
+// Estimated in us.  A stage takes a CTA 0.99 us with 32 rows of x, 1.8 with 64 and 1.7 with 128 (whose group sums are made in front);
+// a tile of k CTAs needs 1 us and 0.57, 0.85 or 2.0 for each of them more; stretches that begin anywhere 3 us and 1.3 times as much for
+// each of the CTAs that may share a tile.  Measured (us, by CTAs of a tile; 148: all SMs): 1024 x 12288, 32 rows: 4 17.3, 8 13.8, 16 15.0,
+// 148 18.5; 128 rows: 4 34.0, 6 29.9, 8 31.4, 16 43.7, 148 49.1; 4096 x 4096, 32 rows: 2 13.1, 4 10.8, 148 12.5; 128 rows: 4 23.3,
+// 148 27.7; 4096 x 12288, 64 rows: 4 31.1, 148 32.1; gate/up 6144 x 2048, 32 rows: 1 12.1, 148 14.5; 512 rows: 148 63.8 (three waves
+// of whole tiles would be 3 x 16).
+int ctas_for(const Line& p, int sm, int* per_tile) {
+    const long tiles = (long)p.row_tiles * p.col_tiles;
+    const double stage = p.tile_cols <= 32 ? 0.99 : p.tile_cols <= 64 ? 1.8 : 1.7, sum = p.tile_cols <= 32 ? 0.57 : p.tile_cols <= 64 ? 0.85 : 2.0;
+    *per_tile = 0;
+    double least = (double)tiles * p.stages / sm * stage + 3.0 + 1.3 * sum * ((double)sm / tiles + 1.0);
+    for (int k = 1; k <= p.stages && tiles * k <= sm; ++k) {
+        const double cost = (double)((p.stages + k - 1) / k) * stage + (k > 1 ? 1.0 + sum * k : 0.0);
+        if (cost < least) { least = cost; *per_tile = k; }
     }
-    return std::min(best, tiles * quanta);
+    return (int)(*per_tile ? tiles * *per_tile : std::min((long)sm, tiles * p.stages));
 }
 
 }  // namespace
@@ -48,7 +47,7 @@ bool encode_rows(CUtensorMap* map, CUtensorMapDataType type, int width, const vo
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps* maps, Line* line, int* grid) {
+bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, int own_cols, LineMaps* maps, Line* line, GroupSums* group_sums, int* grid) {
     if (group != kLineGroup || a.cols % kLineGroup != 0 || a.norm_w) return false;
     if (a.nseg > 1 && affine_stream_passes(mode, a, group) == 0) return false;
     const bool paired = mode == kAffineGateUp || mode == kAffineDual, segs = a.nseg > 1;
@@ -56,6 +55,7 @@ bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps*
     if (reinterpret_cast<uintptr_t>(a.x) & 15u) return false;
     *line = {};
     line->groups = a.cols / kLineGroup;
+    line->stages = (line->groups + kStageGroups - 1) / kStageGroups;
     const int wanted = (a.batch + max_cols - 1) / max_cols;
     line->tile_cols = (a.batch + wanted - 1) / wanted;
     line->tile_cols = line->tile_cols <= 128 ? (line->tile_cols + 15) & ~15 : (line->tile_cols + 31) & ~31;  // above 128 two MMAs share them
@@ -72,13 +72,20 @@ bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps*
         }
     }
     if (paired) line->row_tiles = (a.rows + 63) / 64;
-    const long tiles = (long)line->row_tiles * line->col_tiles, units = tiles * line->groups;
-    if (units >= 1l << 30 || !encode_rows(&maps->x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.x, a.batch, a.cols, line->tile_cols)) return false;
-    const size_t sums = (size_t)sm * 2 * line->tile_cols * kLineRows * sizeof(float);  // two tiles of every CTA
-    if (!a.part_scratch || !a.part_counters || sums > a.part_scratch_bytes) return false;
+    const long tiles = (long)line->row_tiles * line->col_tiles, units = tiles * line->stages;
+    if (units >= 1l << 28 || !encode_rows(&maps->x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.x, a.batch, a.cols, line->tile_cols)) return false;
+    const size_t shared = (size_t)sm * 2 * line->tile_cols * kLineRows;  // two tiles of every CTA
+    *group_sums = {nullptr, line->tile_cols > own_cols ? (size_t)a.batch * line->stages * 2 * kStageGroups : 0};
+    if (!a.part_scratch || !a.part_counters || (shared + group_sums->floats) * sizeof(float) > a.part_scratch_bytes) return false;
+    if (group_sums->floats) {
+        group_sums->at = a.part_scratch + shared;
+        if (!encode_rows(&maps->sums, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, group_sums->at, a.batch, (long)line->stages * 2 * kStageGroups, line->tile_cols)) return false;
+    }
     const bool split = tiles <= 4096;  // a counter each
-    line->quantum = !split ? line->groups : line->groups % kStageGroups == 0 ? kStageGroups : 1;
-    *grid = (int)(split ? ctas_for(*line, sm) : std::min((long)sm, tiles));
+    line->quantum = split ? 1 : line->stages;
+    *grid = split ? ctas_for(*line, sm, &line->per_tile) : (int)std::min((long)sm, tiles);
+    line->share = (int)(units / line->quantum / *grid);
+    line->extra = (int)(units / line->quantum % *grid);
     return true;
 }
 

@@ -15,38 +15,53 @@ constexpr int kLineRows = 128, kLineGroup = 64, kStageGroups = 4;     // weight 
 constexpr int kRawBytes = kLineRows * kStageGroups * kLineGroup / 2;  // packed weights of a stage: 16 KB
 
 struct LineMaps {
-    CUtensorMap w[3], x;
+    CUtensorMap w[3], x, sums;  // sums: what group_sums_kernel wrote, where the tile is wide
 };
 
-// The work is the line of all (tile, group) units, tile after tile; a tile is 128 weight rows (64 of each matrix
-// in the paired forms) and up to tile_cols rows of x.  Every CTA takes an equal stretch of the line, whatever the
-// matrix' shape, so no SM waits for a last wave (192 tiles of gate/up 12288 x 4096 over 148 SMs would take two
-// waves, the second one third full).  A tile that lies in the stretches of several CTAs is put together from
-// fp32 sums in scratch, in column order, by the last of them to finish: results do not depend on timing.
+// The work is the line of all (tile, stage) units, tile after tile; a tile is 128 weight rows (64 of each matrix
+// in the paired forms) and up to tile_cols rows of x, a stage four groups (a row's last one may have fewer).  Every CTA takes
+// an equal stretch of the line, whatever the matrix' shape, so no SM waits for a last wave (192 tiles of gate/up 12288 x 4096
+// over 148 SMs would take two waves, the second one third full).  A tile that lies in the stretches of several CTAs is put
+// together from fp32 sums in scratch, in column order, by the last of them to finish: results do not depend on timing.
 struct Line {
-    int row_tiles, col_tiles, tile_cols, groups;
+    int row_tiles, col_tiles, tile_cols, groups, stages;
     int first1, first2;  // first row tile of the second and third tensor
-    int quantum;         // groups that are never split: a stage's where the row is whole stages, a tile's where there is no scratch
+    int per_tile;        // CTAs of every tile; 0: equal stretches of the whole line
+    int quantum;         // stretches: stages that are never split, one, or a tile's where there is no counter for it
+    int share, extra;    // CTAs before `extra` take share + 1 quanta, the others share
 };
 
-__host__ __device__ inline int line_at(const Line& p, int c, int n) {  // where CTA c of n begins
-    return (int)((long)c * (p.row_tiles * p.col_tiles * p.groups / p.quantum) / n) * p.quantum;
+__device__ __forceinline__ int line_at(const Line& p, int c) {  // where CTA c begins, in stages
+    return p.per_tile ? c / p.per_tile * p.stages + c % p.per_tile * p.stages / p.per_tile : (c * p.share + min(c, p.extra)) * p.quantum;
 }
 
 // One tile's part of a stretch.
 struct Part {
-    int tile, g0, g1, row_tile, col0, live;  // groups [g0, g1); first row of x and how many
+    int tile, s0, s1, row_tile, col_tile, col0, live;  // stages [s0, s1); first row of x and how many
 };
+__device__ __forceinline__ void part_rows(const Line& p, Part& t, int batch) {
+    t.col0 = t.col_tile * p.tile_cols;
+    t.live = min(p.tile_cols, batch - t.col0);
+}
 __device__ __forceinline__ Part part_at(const Line& p, int u, int end, int batch) {
     Part t;
-    t.tile = u / p.groups;
-    t.g0 = u - t.tile * p.groups;
-    t.g1 = min(p.groups, t.g0 + (end - u));
+    t.tile = u / p.stages;
+    t.s0 = u - t.tile * p.stages;
+    t.s1 = min(p.stages, t.s0 + (end - u));
     t.row_tile = t.tile / p.col_tiles;
-    t.col0 = (t.tile - t.row_tile * p.col_tiles) * p.tile_cols;
-    t.live = min(p.tile_cols, batch - t.col0);
+    t.col_tile = t.tile - t.row_tile * p.col_tiles;
+    part_rows(p, t, batch);
     return t;
 }
+// The next tile's part, from stage u of the line on (roles walk the line with this: a division each would be code in front of every loop).
+__device__ __forceinline__ void next_part(const Line& p, Part& t, int u, int end, int batch) {
+    ++t.tile;
+    t.s0 = 0;
+    t.s1 = min(p.stages, end - u);
+    if (++t.col_tile == p.col_tiles) { t.col_tile = 0; ++t.row_tile; }
+    part_rows(p, t, batch);
+}
+__device__ __forceinline__ int stage_groups(const Line& p, int stage) { return min(kStageGroups, p.groups - stage * kStageGroups); }
 
 // Where row r of a tile lies: matrix row, its scales and biases, its output.
 struct LineRow {
@@ -76,28 +91,62 @@ __device__ __forceinline__ LineRow line_row(const AffineArgs& a, const Line& p, 
     return o;
 }
 
-// Packed weights of one stage: groups g .. g + 3 of the tile's rows.
+// Packed weights of one stage of the tile's rows.
 template <int MODE>
-__device__ __forceinline__ void request_weights(const LineMaps& maps, const Line& p, int row_tile, int g, uint8_t* dst, uint64_t* bar) {
+__device__ __forceinline__ void request_weights(const LineMaps& maps, const Line& p, int row_tile, int stage, uint32_t dst, uint32_t bar) {
     if (MODE == kAffineGateUp || MODE == kAffineDual) {
-        tma_load_2d(dst, &maps.w[0], g * (kLineGroup / 2), row_tile * 64, bar);
-        tma_load_2d(dst + kRawBytes / 2, &maps.w[1], g * (kLineGroup / 2), row_tile * 64, bar);
+        tma_load_2d_at(dst, &maps.w[0], stage * 128, row_tile * 64, bar);
+        tma_load_2d_at(dst + kRawBytes / 2, &maps.w[1], stage * 128, row_tile * 64, bar);
     } else {
         const int seg = (row_tile >= p.first1) + (row_tile >= p.first2);
-        tma_load_2d(dst, &maps.w[seg], g * (kLineGroup / 2), (row_tile - (seg == 0 ? 0 : seg == 1 ? p.first1 : p.first2)) * kLineRows, bar);
+        tma_load_2d_at(dst, &maps.w[seg], stage * 128, (row_tile - (seg == 0 ? 0 : seg == 1 ? p.first1 : p.first2)) * kLineRows, bar);
     }
 }
 
-__device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* dead) { return __all_sync(0xffffffffu, wait_alive(bar, parity, dead)); }
+// The same by a whole warp, all of it or none: bar and dead are addresses of shared memory.
+__device__ __forceinline__ uint32_t lds_word(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, uint32_t dead) {
+    if (__all_sync(0xffffffffu, mbar_tries(bar, parity))) return true;
+    const uint64_t begin = now_ns();
+#pragma unroll 1
+    for (;;) {
+        if (__all_sync(0xffffffffu, mbar_tries(bar, parity))) return true;
+        const bool late = now_ns() - begin >= kWaitNs;
+        if (late) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
+        if (__any_sync(0xffffffffu, late || lds_word(dead) != 0u)) return false;
+    }
+}
+// By one thread.
+__device__ __forceinline__ bool wait_one(uint32_t bar, uint32_t parity, uint32_t dead) {
+    if (mbar_tries(bar, parity)) return true;
+    const uint64_t begin = now_ns();
+#pragma unroll 1
+    for (;;) {
+        if (mbar_tries(bar, parity)) return true;
+        if (lds_word(dead) != 0u) return false;
+        if (now_ns() - begin >= kWaitNs) break;
+    }
+    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
+    return false;
+}
+// A value that is the same in all lanes, where the compiler can see it: what follows from it stays in uniform registers.
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ Part uniform(const Part& t) {
+    return {uniform(t.tile), uniform(t.s0), uniform(t.s1), uniform(t.row_tile), uniform(t.col_tile), uniform(t.col0), uniform(t.live)};
+}
 // Whether a phase has completed, without waiting: several are asked at once and only what is missing is waited for.
-__device__ __forceinline__ bool peek(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool peek(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     return ok != 0;
 }
@@ -112,15 +161,17 @@ __device__ __forceinline__ float2 unpack2(uint64_t v) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
     return f;
 }
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
+// acc += a * b, in the accumulator's own registers
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
 }
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
     uint4 v;
@@ -128,54 +179,47 @@ __device__ __forceinline__ uint4 lds128(uint32_t a) {
     return v;
 }
 
-// Scales and biases of a stage on their way to shared memory, by a warp of its own: a thread that fetched its own row's
-// beside its other work waited for them.  A lane takes rows `row + 32 i` of the tile; store(stage, i, group of the stage,
-// {scale, bias}) is called after wait(stage), done(stage) behind it.
-template <int MODE, typename Wait, typename Store, typename Done>
-__device__ __forceinline__ void feed_scales(const AffineArgs& a, const Line& p, int u0, int u1, int row, Wait wait, Store store, Done done) {
+// Scales and biases of a stage on their way to shared memory, by a warp that has little else to do, as many stages ahead as there are
+// slots: a lane takes rows `row + 32 i` of the tile; dst(stage, i, which) is where the four values of such a row go, after
+// wait(stage, part, stage of the part).  Every lane arrives at full(stage) when its copies have.
+template <int MODE, typename Wait, typename Dst, typename Full>
+__device__ __forceinline__ void feed_scales(const AffineArgs& a, const Line& p, Part t, int u0, int u1, int row, Wait wait, Dst dst, Full full) {
     constexpr int kRows = 4;
-    const bool vec = (p.quantum & 3) == 0 && (p.groups & 3) == 0;  // every stage begins at a multiple of four groups
-    auto four = [&](const __half* q, int n) {
-        if (vec && (reinterpret_cast<uintptr_t>(q) & 7u) == 0) return __ldg(reinterpret_cast<const uint2*>(q));
-        uint32_t h[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) h[j] = j < n ? (uint32_t)__half_as_ushort(__ldg(q + j)) : 0u;
-        return make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
-    };
-    uint32_t stage = 0;
-    for (int u = u0; u < u1;) {
-        const Part t = part_at(p, u, u1, a.batch);
+    uint32_t it = 0;
 #pragma unroll 1
-        for (int i = 0; i < kRows; ++i) {
-            const LineRow o = line_row<MODE>(a, p, t.row_tile, row + 32 * i);
-            if (o.row < o.rows)
-                for (int g = t.g0; g < t.g1; g += 16) {
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(o.s + g));
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(o.b + g));
+    for (int u = u0; u < u1; next_part(p, t, u, u1, a.batch)) {
+        // Rows 64 apart may lie in two matrices; those 32 apart are in one.
+        const LineRow o0 = line_row<MODE>(a, p, t.row_tile, row), o1 = line_row<MODE>(a, p, t.row_tile, row + 64);
+        const __half* from[4] = {o0.s, o0.b, o1.s, o1.b};
+        const int live[2] = {o0.rows - o0.row, o1.rows - o1.row}, step = 32 * p.groups;
+        bool async = (p.groups & 3) == 0;  // eight bytes at a time
+#pragma unroll
+        for (int i = 0; i < 4; ++i) async = async && (reinterpret_cast<uintptr_t>(from[i]) & 7u) == 0;
+#pragma unroll 1
+        for (int st = t.s0; st < t.s1; ++st, ++it) {
+            if (!wait(it, t, st)) { cp_async_wait<0>(); return; }
+            const int g = st * kStageGroups, n = stage_groups(p, st);
+#pragma unroll
+            for (int i = 0; i < 2 * kRows; ++i) {
+                const uint32_t to = dst(it, i >> 1, i & 1);
+                const __half* q = from[(i >> 2) * 2 + (i & 1)] + (i >> 1 & 1) * step + g;
+                const bool ok = live[i >> 2] > (i >> 1 & 1) * 32;
+                if (async) {
+                    if (ok) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(q) : "memory");
+                } else {
+                    uint32_t h[4] = {0, 0, 0, 0};
+                    if (ok)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) h[j] = j < n ? (uint32_t)__half_as_ushort(__ldg(q + j)) : 0u;
+                    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(to), "r"(h[0] | h[1] << 16), "r"(h[2] | h[3] << 16) : "memory");
                 }
-        }
-        for (int g = t.g0; g < t.g1; g += kStageGroups, ++stage) {
-            const int n = min(kStageGroups, t.g1 - g);
-            uint2 s[kRows], b[kRows];
-#pragma unroll
-            for (int i = 0; i < kRows; ++i) {
-                const LineRow o = line_row<MODE>(a, p, t.row_tile, row + 32 * i);
-                const bool ok = o.row < o.rows;
-                s[i] = ok ? four(o.s + g, n) : make_uint2(0, 0);
-                b[i] = ok ? four(o.b + g, n) : make_uint2(0, 0);
             }
-            if (!wait(stage)) return;
-#pragma unroll
-            for (int i = 0; i < kRows; ++i) {
-                const uint32_t sw[2] = {s[i].x, s[i].y}, bw[2] = {b[i].x, b[i].y};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) store(stage, i, j, __byte_perm(sw[j >> 1], bw[j >> 1], (j & 1) ? 0x7632 : 0x5410));
-            }
-            __syncwarp();
-            done(stage);
+            if (async) asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full(it)) : "memory");
+            else arrive_at(full(it));
         }
-        u += t.g1 - t.g0;
+        u += t.s1 - t.s0;
     }
+    cp_async_wait<0>();
 }
 
 // A tile that several CTAs share: CTA first holds its first group, CTA last its last; a CTA has at most two such tiles, its
@@ -184,17 +228,30 @@ struct Sharers {
     int first, last, first_slot;
     __device__ __forceinline__ int slot(int cta) const { return cta == first ? first_slot : 2 * cta; }
 };
-__device__ __forceinline__ Sharers sharers(const Line& p, int tile, int n) {
-    const int total = p.row_tiles * p.col_tiles * p.groups / p.quantum, tile_q = p.groups / p.quantum, start = tile * tile_q;
+__device__ __forceinline__ Sharers sharers(const Line& p, int tile) {
     Sharers s;
-    s.first = (int)(((start + 1l) * n - 1) / total);
-    s.last = (int)(((long)(start + tile_q) * n - 1) / total);
-    s.first_slot = 2 * s.first + (line_at(p, s.first, n) < tile * p.groups ? 1 : 0);
+    if (p.per_tile) {
+        s.first = tile * p.per_tile;
+        s.last = s.first + p.per_tile - 1;
+    } else {
+        const int start = tile * p.stages, end = start + p.stages - 1, longer = p.extra * (p.share + 1);
+        s.first = start < longer ? start / (p.share + 1) : p.extra + (start - longer) / p.share;
+        s.last = end < longer ? end / (p.share + 1) : p.extra + (end - longer) / p.share;
+    }
+    s.first_slot = 2 * s.first + (line_at(p, s.first) < tile * p.stages ? 1 : 0);
     return s;
 }
 
+constexpr int kSumWindow = 4;  // stages whose group sums of x lie in one 128-byte row of the tile that the biases multiply
+// Sums of x by group as two tf32 values each, behind the shared tiles in scratch: per row of x and stage {hi of four groups, lo of four groups}.
+struct GroupSums {
+    float* at;  // null: the product sums for itself
+    size_t floats;
+};
+
 // Whether the product takes the launch (group 64, 16-byte aligned weights and activations, no folded norm; several
-// tensors where the streaming kernel takes them), and if so its maps and its line, in tiles of up to max_cols rows of x.
-bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, LineMaps* maps, Line* line, int* grid);
+// tensors where the streaming kernel takes them), and if so its maps and its line, in tiles of up to max_cols rows of x; tiles of more
+// than own_cols have their group sums made in front.
+bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, int own_cols, LineMaps* maps, Line* line, GroupSums* sums, int* grid);
 
 }  // namespace smelt

@@ -479,13 +479,7 @@ cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int
     // Batches beyond 16 rows are processed in passes of 16 (weights re-streamed per pass).
     if (args.batch > 16) {
         for (int b0 = 0; b0 < args.batch; b0 += 16) {
-            AffineArgs s = args;
-            s.batch = args.batch - b0 < 16 ? args.batch - b0 : 16;
-            s.x = args.x + (size_t)b0 * args.cols;
-            s.y = args.y + (size_t)b0 * args.rows;
-            if (args.y2) s.y2 = args.y2 + (size_t)b0 * args.rows;
-            if (args.residual) s.residual = args.residual + (size_t)b0 * args.rows;
-            for (int i = 0; i < args.nseg && i < 3; ++i) s.seg[i].y = args.seg[i].y + (size_t)b0 * args.seg[i].rows;
+            const AffineArgs s = affine_rows(args, b0, args.batch - b0 < 16 ? args.batch - b0 : 16);
             cudaError_t e = launch_affine(l, mode, s, group);
             if (e != cudaSuccess) return e;
         }

@@ -48,6 +48,18 @@ struct AffineArgs {
     DevDyn dyn;            // filled by the launcher
 };
 
+// The launch for rows [r0, r0 + n) of x.
+inline AffineArgs affine_rows(const AffineArgs& a, int r0, int n) {
+    AffineArgs s = a;
+    s.batch = n;
+    s.x = a.x + (size_t)r0 * a.cols;
+    if (a.y) s.y = a.y + (size_t)r0 * a.rows;
+    if (a.y2) s.y2 = a.y2 + (size_t)r0 * a.rows;
+    if (a.residual) s.residual = a.residual + (size_t)r0 * a.rows;
+    for (int i = 0; i < a.nseg && i < 3; ++i) s.seg[i].y = a.seg[i].y + (size_t)r0 * a.seg[i].rows;
+    return s;
+}
+
 cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int group);
 cudaError_t launch_affine_stream(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
 // Tensor-core product for many rows of x (affine_wide.cu; from how many: wide_first in affine_matvec.cu).

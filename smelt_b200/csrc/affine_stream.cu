@@ -424,13 +424,7 @@ cudaError_t launch_affine_stream(const Launch& l, int mode, const AffineArgs& a,
     if (passes == 0) return cudaSuccess;
     const int per_pass = (a.batch + passes - 1) / passes;
     for (int b0 = 0; b0 < a.batch; b0 += per_pass) {
-        AffineArgs p = a;
-        p.batch = a.batch - b0 < per_pass ? a.batch - b0 : per_pass;
-        p.x = a.x + (size_t)b0 * a.cols;
-        if (a.y) p.y = a.y + (size_t)b0 * a.rows;
-        if (a.y2) p.y2 = a.y2 + (size_t)b0 * a.rows;
-        if (a.residual) p.residual = a.residual + (size_t)b0 * a.rows;
-        for (int i = 0; i < a.nseg && i < 3; ++i) p.seg[i].y = a.seg[i].y + (size_t)b0 * a.seg[i].rows;
+        const AffineArgs p = affine_rows(a, b0, a.batch - b0 < per_pass ? a.batch - b0 : per_pass);
         cudaError_t e;
         switch (mode) {
             case kAffinePlain: e = launch_stream_mode<kAffinePlain>(l, p, handled); break;

@@ -2,33 +2,36 @@
 // Y[M, R] = X[M, K] . W[R, K]^T with W affine u4, group 64, on the fifth-generation tensor cores.
 //
 // Replaces agent_affine_qmm_fixed_batched_full and its fused gate/up form (Resources/Shaders/agent_affine_qmm.h:107-316,
-// :360-742; wrappers Resources/Shaders/lut_matvec.metal:6519-6545, :6615-6635).  The tensor core multiplies the
-// dequantised weight w = scale * q + bias, evaluated in fp32 with one FMA, as TWO fp16 operands: hi = half(w) and
-// lo = half(w - hi).  The weights of a row in two groups are first brought near the top of fp16's range by a power of two of
-// their own, so that hi + lo carries 22 significant bits of the largest of them whatever the scales are, and no weight is too
-// large; the sums are multiplied by its inverse.
+// :360-742; wrappers Resources/Shaders/lut_matvec.metal:6519-6545, :6615-6635), in their factored form: per group
+// y += scale * sum(q x) + bias * sum(x).  The tensor core multiplies the nibbles (exact in fp16) by x, one accumulator a group;
+// epilogue warps multiply what they drain by the scale and add it to fp32 registers.  The nibbles are centred (q - 8) and the bias is
+// bias + 8 scale, so that neither sum is much larger than the result.  The tensor core truncates what it adds to, here four
+// K = 16 products at a time.  Share of fp16 results that are not the correctly rounded ones, against two fp16 operands per
+// dequantised weight summed over two groups (before -> now): 4096 x 4096, 32 rows 0.12 -> 0.09 %, 512 rows 0.12 -> 0.08; gate and
+// up 12288 x 4096, 32 rows 0.20 -> 0.19, 512 rows 0.21 -> 0.15.
 //
-// The tensor core truncates every sum it adds to.  Over all of K in one accumulator that made 0.5 to 7 % of the fp16 results
-// another value than the correctly rounded one, and all of them a little small; so an accumulator holds the products of two
-// groups, the small ones first, and its contents are added in fp32 registers: 0.1 to 0.2 % of the results differ, as many as of
-// the matvec family's (4096 x 4096, 32 rows: 0.12 %, exact nibbles with scale and bias applied group by group 0.12 %, all of K
-// 0.53 %; 4096 x 12288: 0.12, 0.14, 1.4 %; gate and up 12288 x 4096: 0.20, 0.21, 2.6 %).
+// bias * sum(x).  Tiles of up to 64 rows of x: four warps sum x from shared memory, the epilogue adds the products in fp32.  More
+// rows: the sums are made once in front (group_sums_kernel), as two tf32 values each, and the biases of up to sixteen groups
+// multiply them on the tensor core as one more turn; where bias + 8 scale is not exact in tf32 the group's nibbles stay as they are
+// and its bias, which is an fp16, is the operand.
 //
-// Mapping.  One CTA an SM takes an equal stretch of the launch's line of work (affine_line.cuh); a tile is 128 weight
-// rows, the MMA's M, by up to 256 rows of x, its N.  The roles, each on warps of its own, each a ring ahead of the next:
-//   * weights: TMA, 128 rows x 256 columns of packed nibbles a stage, requested before the wait for the launch in front;
-//   * activations: TMA, two 64-column groups a stage, 128-byte swizzled: the MMA's B operand as it is;
-//   * scales and biases, one warp;
-//   * expansion: a thread owns a weight row and turns its 64 nibbles of a group into hi and lo, in pairs, straight into
-//     tensor memory, from where the MMA takes its A operand.  (An A tile in shared memory is written once and read once per
-//     256 rows of x, which with the B tile's two reads and its write is more than the SM's 128 bytes a clock.)
-//   * issue: sixteen K = 16 MMAs a turn of two groups, in a loop of four (unrolled, its code was fetched from beyond the
-//     instruction cache every turn: 89 clocks an MMA, of 16 with 32 rows of x and 64 with 128 that it takes alone);
-//   * sums and epilogue: plain, + residual, SwiGLU of gate and up, dual.
-// What bounds it: up to 128 rows the expansion, about 370 instructions per row and group; with 256 the tensor pipe, which does
-// the work twice, and the ends of tiles, which it waits for.  Against the form that expanded through shared memory and drained
-// or staged by the same threads (us; gate/up 12288 x 4096 x 2 | 4096 x 12288 | 4096 x 4096): 32 rows 77.8 -> 57.7 | 43.9 ->
-// 33.7 | 17.0 -> 15.5; 128 rows 190 -> 74.3 | 78.4 -> 41.2 | 34.4 -> 22.4; 512 rows 347 -> 226 | 164 -> 105 | 77.8 -> 52.4.
+// Mapping.  One CTA an SM takes a stretch of the launch's line of work (affine_line.cuh); a tile is 128 weight
+// rows, the MMA's M, by up to 128 rows of x, its N.  The roles, each on warps of its own, each a ring ahead of the next:
+//   * weights, TMA, 128 rows x 256 columns of packed nibbles a stage, and their scales and biases, cp.async: requested before the
+//     wait for the launch in front;
+//   * activations: TMA, 128-byte swizzled: the MMA's B operand as it is;
+//   * expansion: a thread owns a weight row and turns its nibbles of a group into fp16 pairs straight in tensor memory, from where
+//     the MMA takes its A operand: 11 instructions for eight nibbles;
+//   * issue: two warps take turns;
+//   * sums and epilogue, eight warps: plain, + residual, SwiGLU of gate and up, dual.  A turn is 128 columns of tensor memory: four
+//     groups of 32 rows of x, two of 64, one of 128.
+// What bounds it: instruction issue (0.6 an SM quarter and clock).  What cost most on the way here: code beyond the 32 KB that the
+// instruction cache holds (wait loops unrolled by the compiler: 122 KB), spilled registers (the shared memory leaves no first-level
+// cache: a reload is an L2 round trip), waits with a time hint (a timed loop each), shared addresses made anew at every use, packed
+// FMAs (a move each).
+// us, graph replay over distinct weights, before -> now (gate/up 12288 x 4096 x 2 | 4096 x 12288 | 4096 x 4096): 32 rows
+// 58.4 -> 31.3 | 34.4 -> 19.6 | 15.5 -> 10.8; 64 rows 63.9 -> 50.2 | 40.0 -> 31.0 | 18.3 -> 15.2; 128 rows 74.6 -> 57.1 |
+// 43.5 -> 42.0 | 22.4 -> 23.3; 512 rows 227 -> 184 | 113 -> 91 | 51.5 -> 36.0.
 // A launch in front may take longer than a wait may (its waits on a peer are as long): every role waits for it before the first
 // wait that depends on the activations, and only what needs none of them goes ahead.
 // Every wait is bounded: on expiry the CTA sets bit 10 of the error word, its roles stop, copies and MMAs in flight are
@@ -39,40 +42,90 @@ namespace smelt {
 
 namespace {
 
-constexpr int kThreads = 640, kEpilogueWarp = 4, kEpilogueWarps = 8, kExpandWarp = 12, kExpandWarps = 8;
+constexpr int kEpilogueWarp = 4, kEpilogueWarps = 8, kExpandWarp = 12, kExpandWarps = 8, kSumWarp = 20, kSumWarps = 4;
 constexpr int kEpilogueThreads = kEpilogueWarps * 32;
-constexpr int kASlots = 2;     // hi | lo of two groups: 128 columns of tensor memory each
 constexpr int kDone = 16;      // barriers that units' completion goes through, one after the other: no role is that far behind another
-constexpr int kPowers = 16;    // turns whose powers of two are kept: two in the A slots, up to eight in accumulators
+constexpr int kOwnCols = 64;   // up to so many rows of x a tile's CTAs make the group sums themselves
+constexpr float kNibble = 512.f;  // the tensor core gets nibbles as 2^-9 of their value
+
+// A position in a ring of barriers and the parity of its present use.
+template <int N>
+struct Ring {
+    uint32_t i = 0, phase = 0;
+    __device__ __forceinline__ void next(uint32_t steps = 1) {
+        if ((i += steps) >= N) { i -= N; phase ^= 1u; }
+    }
+};
 
 template <int N>
 struct WideCfg {
-    static constexpr int kHalves = N == 256 ? 2 : 1, kMma = N / kHalves;  // an MMA takes up to 128 rows of x, so that one half is drained while the other is multiplied
-    static constexpr int kSlots = 256 / kMma;                             // accumulators
-    static constexpr int kSums = N / 2;                                   // of a thread: two sets of epilogue warps share the columns
-    static constexpr int kXBytes = N * kLineGroup * 2, kXStages = N == 256 ? 2 : 4, kRawStages = N <= 64 ? 6 : 4;  // a stage of x is two groups
-    static constexpr uint32_t kSmem = kRawStages * kRawBytes + kXStages * 2 * kXBytes + 1024;
-    static_assert(kSmem + 30 * 1024 <= 227u * 1024u, "shared memory");
-    static_assert(kPowers >= kASlots + kSlots / kHalves, "powers");
+    static constexpr bool kOwn = N <= kOwnCols;
+    static constexpr int kThreads = kOwn ? 768 : 640;
+    // Registers of the roles in front, the epilogue, and the others; together no more than the launch's.
+    static constexpr int kFront = 48, kDrain = N == 128 ? 160 : 128, kBehind = 56;
+    static constexpr int kTurn = N <= 32 ? 4 : N <= 64 ? 2 : 1;           // groups of a turn: multiplied into accumulators side by side
+    static constexpr int kSlots = kOwn ? 2 : 3;                           // of accumulators: 128 columns of tensor memory each
+    static constexpr int kASlots = kOwn ? 256 / (32 * kTurn) : 4, kACol = kSlots * 128;
+    static constexpr int kXBytes = N * kLineGroup * 2, kXStages = N == 128 ? 5 : 4, kRawStages = N == 128 ? 4 : 6;  // a stage of x is a turn's
+    static constexpr int kScaleStages = kOwn ? 8 : 12;
+    static constexpr int kWindow = kOwn ? 0 : N * 128;                    // group sums of kSumWindow stages
+    static constexpr int kOwnSlots = kOwn ? 4 : 1;                        // turns whose own group sums are kept
+    static constexpr uint32_t kSmem = kRawStages * kRawBytes + kXStages * kTurn * kXBytes + kWindow + 1024;
+    static_assert(kSmem + 28 * 1024 <= 227u * 1024u, "shared memory");
+    static_assert(kACol + kASlots * kTurn * 32 <= 512 && kTurn * N <= 128, "tensor memory");
+    static_assert(kScaleStages >= 2 * kSumWindow, "the biases of a window wait for it");
+    // Barriers, by the address of the first one of a kind.
+    static constexpr int kRawFull = 0, kRawEmpty = kRawFull + kRawStages, kScaleFull = kRawEmpty + kRawStages, kScaleEmpty = kScaleFull + kScaleStages, kXFull = kScaleEmpty + kScaleStages,
+                         kXEmpty = kXFull + kXStages, kAFull = kXEmpty + kXStages, kTurnDone = kAFull + kASlots, kAccEmpty = kTurnDone + kDone, kSumFull = kAccEmpty + kSlots,
+                         kSumEmpty = kSumFull + kOwnSlots, kWindowFull = kSumEmpty + kOwnSlots, kWindowEmpty = kWindowFull + 1, kBarriers = kWindowEmpty + 1;
+    static_assert(128 * kFront + kEpilogueThreads * kDrain + (kThreads - 128 - kEpilogueThreads) * kBehind <= kThreads * (65536 / kThreads / 8 * 8), "registers");
 };
 
-// D[128 x N] (+)= A[128 x 64] . B[N x 64]^T, A from tensor memory (lane = row, two fp16 a column), as four MMAs of 16 columns: eight
+template <int N>
+struct WideShared {
+    using C = WideCfg<N>;
+    uint64_t bars[C::kBarriers];
+    uint2 scales[C::kScaleStages][2][kLineRows];                                    // four scales and four biases of a row
+    alignas(16) float own_sums[C::kOwnSlots][C::kOwn ? C::kTurn : 1][C::kOwn ? N : 4];  // of x by group
+    uint32_t x_turns[C::kXStages];                                                  // the turn that reads a stage of x
+    uint32_t tmem, dead, ticket, go;
+    int u0, u1;
+    Part first;
+};
+
+// D[128 x N] = A[128 x 64] . B[N x 64]^T, A from tensor memory (lane = row, two fp16 a column), as four MMAs of 16 columns: eight
 // columns of tensor memory, 32 bytes in the descriptor's address field.  A whole warp calls it, one lane issues: the operands stay in
 // the uniform registers that the instruction reads.
-__device__ __forceinline__ void umma_f16_group(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_f16_group(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc) {
     asm volatile(
         "{\n\t.reg .pred p, q, t;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\t"
         "elect.sync _|q, 0xffffffff;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "setp.eq.b32 t, 0, 0;\n\t"
+        "setp.ne.b32 p, 0, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
         "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
         "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n\t}"
+        ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc)
+        : "memory");
+}
+// D (+)= A[128 x 8] . B[N x 8]^T in tf32, likewise.
+__device__ __forceinline__ void umma_tf32_step(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(d), "r"(a), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+// The lane that issued, too (elect.sync chooses the same one every time).
+__device__ __forceinline__ void commit_elected(uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t t, const uint32_t (&v)[16]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(t), "r"(v[0]), "r"(v[1]), "r"(v[2]),
@@ -83,35 +136,35 @@ __device__ __forceinline__ void tmem_st8(uint32_t t, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(t), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
+// What a group's sum of x is multiplied by when its nibbles go to the tensor core as q - 8: bias + 8 scale, where a tf32 operand holds that
+// exactly (the bias of a row's group whose weights have both signs); else the bias, and the nibbles stay as they are.
+__device__ __forceinline__ float tf32_bias(float s, float b, bool* centred) {
+    const float t = fmaf(8.f, s, b);
+    *centred = (__float_as_uint(t) & 0x1FFFu) == 0u && t - 8.f * s == b;
+    return *centred ? t : b;
 }
-// Eight nibbles -> four pairs of adjacent columns, hi and lo; s2, b2: scale and bias, twice.
-__device__ __forceinline__ void expand_hi_lo(uint32_t word, uint64_t s2, uint64_t b2, uint32_t* hi, uint32_t* lo) {
-    const uint64_t minus = pack2(-8388608.f, -8388608.f), neg = pack2(-1.f, -1.f);
+// Eight nibbles -> four pairs of adjacent columns: a byte that holds a nibble is an fp16 of 2^-24 of its value, brought to 2^-9 of it (and
+// centred) by one packed FMA.  (The tensor core takes the subnormals exactly too, but aligns their products by an exponent that is up to ten
+// bits too high: four times as many results were misrounded.)
+__device__ __forceinline__ void expand_nibbles(uint32_t word, uint32_t minus, uint32_t* pair) {
     const uint32_t even = word & 0x0F0F0F0Fu, odd = (word >> 4) & 0x0F0F0F0Fu;
+    // 8 and C: the sign of such a byte, zero
+    asm("prmt.b32 %0, %4, %5, 0xC480;\n\tprmt.b32 %1, %4, %5, 0xD591;\n\tprmt.b32 %2, %4, %5, 0xE6A2;\n\tprmt.b32 %3, %4, %5, 0xF7B3;"
+        : "=&r"(pair[0]), "=&r"(pair[1]), "=&r"(pair[2]), "=&r"(pair[3])
+        : "r"(even), "r"(odd));
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-        const uint32_t sel = 0x7440u + b;  // the byte under the exponent of 2^23
-        const uint64_t q = add2(pack2(__uint_as_float(__byte_perm(even, 0x4B000000u, sel)), __uint_as_float(__byte_perm(odd, 0x4B000000u, sel))), minus);
-        const uint64_t w = fma2(q, s2, b2);
-        const float2 wf = unpack2(w);
-        const __half2 h = __floats2half2_rn(wf.x, wf.y);
-        const float2 hf = __half22float2(h);
-        const float2 rest = unpack2(fma2(pack2(hf.x, hf.y), neg, w));
-        hi[b] = h2_as_u32(h);
-        lo[b] = h2_as_u32(__floats2half2_rn(rest.x, rest.y));
-    }
+    for (int b = 0; b < 4; ++b) asm("fma.rn.f16x2 %0, %0, %1, %2;" : "+r"(pair[b]) : "r"(0x78007800u), "r"(minus));  // 2^15
 }
-
-// Exponent field of the largest weight that {scale, bias} can give: |w| <= max(|bias|, |15 scale + bias|) < 2^(top - 126).
-__device__ __forceinline__ uint32_t top_of(float2 f) {
-    return max(__float_as_uint(fmaxf(fabsf(f.y), fabsf(fmaf(15.f, f.x, f.y)))) >> 23, 64u);
+__device__ __forceinline__ float lds_half(uint32_t a) {
+    uint16_t h;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(a));
+    return __half2float(__ushort_as_half(h));
 }
-__device__ __forceinline__ float power_up(uint32_t top) { return __uint_as_float((268u - top) << 23); }    // 2^14 / 2^(top - 127)
-__device__ __forceinline__ float power_down(uint32_t top) { return __uint_as_float((top - 14u) << 23); }  // its inverse
+__device__ __forceinline__ float tf32_of(float v) {
+    uint32_t u;
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(v));
+    return __uint_as_float(u);
+}
 
 template <int REGS>
 __device__ __forceinline__ void registers_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS)); }
@@ -121,214 +174,343 @@ __device__ __forceinline__ void registers_down() { asm volatile("setmaxnreg.dec.
 // silu(gate) * up in fp32
 __device__ __forceinline__ __half swiglu_f32(float gate, float up) { return __float2half_rn(gate / (1.0f + expf(-gate)) * up); }
 
+// Sums of x by group for tiles of many rows, as hi + lo of eleven bits each (what a tf32 operand holds): a warp takes four groups of a row.
+__global__ void __launch_bounds__(256) group_sums_kernel(const __half* __restrict__ x, float* __restrict__ out, int batch, int cols, int stages) {
+    pdl_trigger();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, row = blockIdx.x;
+    for (int st = blockIdx.y * 8 + (threadIdx.x >> 5); st < stages; st += gridDim.y * 8) {
+        const int c = st * (kStageGroups * kLineGroup) + lane * 8;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (c < cols) v = *reinterpret_cast<const uint4*>(x + (size_t)row * cols + c);
+        const float2 f0 = __half22float2(u32_as_h2(v.x)), f1 = __half22float2(u32_as_h2(v.y)), f2 = __half22float2(u32_as_h2(v.z)), f3 = __half22float2(u32_as_h2(v.w));
+        float sum = ((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y));
+#pragma unroll
+        for (int o = 1; o < 8; o *= 2) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        sum = __shfl_sync(0xffffffffu, sum, (lane & 3) * 8);
+        const float hi = tf32_of(sum);
+        if (lane < 8) out[((size_t)row * stages + st) * 8 + lane] = lane < 4 ? hi : tf32_of(sum - hi);
+    }
+}
+
 template <int MODE, int N>
-__global__ void __launch_bounds__(kThreads, 1) affine_wide_kernel(const __grid_constant__ LineMaps maps, const AffineArgs a, const Line line) {
+__global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(const __grid_constant__ LineMaps maps, const AffineArgs a, const Line line) {
     using C = WideCfg<N>;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t* raw = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t* x_tiles = raw + C::kRawStages * kRawBytes;
-    __shared__ uint64_t raw_full[C::kRawStages], raw_empty[C::kRawStages], scale_full[C::kRawStages], x_full[C::kXStages], a_full[kASlots], done[kDone], acc_empty[C::kSlots];
-    __shared__ uint32_t scales[C::kRawStages][kStageGroups][kLineRows];  // {scale, bias}
-    __shared__ float powers[kPowers][kLineRows];                         // what the products of two groups are to be multiplied by
-    __shared__ uint32_t s_tmem, s_dead, s_ticket, s_go;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __shared__ WideShared<N> sh;
+    const uint32_t raw = kept((smem_u32(smem_raw) + 1023u) & ~1023u), shared = kept(smem_u32(&sh));
+    const uint32_t x_tiles = raw + C::kRawStages * kRawBytes, window = x_tiles + C::kXStages * C::kTurn * C::kXBytes;
+    const uint32_t scales = shared + (uint32_t)offsetof(WideShared<N>, scales), own_sums = shared + (uint32_t)offsetof(WideShared<N>, own_sums), dead = shared + (uint32_t)offsetof(WideShared<N>, dead);
+    auto bar = [&](int kind, uint32_t i = 0) { return shared + 8u * (kind + i); };
+    const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
 
     pdl_trigger();
     if (tid == 0) {
-        for (int i = 0; i < C::kRawStages; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], kExpandWarps); mbar_init(&scale_full[i], 1); }
-        for (int i = 0; i < C::kXStages; ++i) mbar_init(&x_full[i], 1);
-        for (int i = 0; i < kASlots; ++i) mbar_init(&a_full[i], 4);
-        for (int i = 0; i < kDone; ++i) mbar_init(&done[i], 2);
-        for (int i = 0; i < C::kSlots; ++i) mbar_init(&acc_empty[i], kEpilogueWarps);
-        s_dead = 0u;
+        auto init = [&](int kind, int n, int count) {
+            for (int i = 0; i < n; ++i) mbar_init(&sh.bars[kind + i], count);
+        };
+        init(C::kRawFull, C::kRawStages, 1);
+        init(C::kRawEmpty, C::kRawStages, C::kTurn == kStageGroups ? 4 : kExpandWarps);
+        init(C::kScaleFull, C::kScaleStages, 32);
+        init(C::kScaleEmpty, C::kScaleStages, kEpilogueWarps);
+        init(C::kXFull, C::kXStages, 1);
+        init(C::kXEmpty, C::kXStages, kSumWarps);
+        init(C::kAFull, C::kASlots, 4);
+        init(C::kTurnDone, kDone, 1);
+        init(C::kAccEmpty, C::kSlots, kEpilogueWarps);
+        init(C::kSumFull, C::kOwnSlots, kSumWarps);
+        init(C::kSumEmpty, C::kOwnSlots, kEpilogueWarps);
+        init(C::kWindowFull, 2, 1);
+        sh.dead = 0u;
         mbar_fence_init();
         fence_async_smem();
     }
-    if (warp == 2) tmem_alloc(&s_tmem, 512);
+    if (tid == 32) {  // where the roles begin: read by each when it does, not held in registers until then
+        sh.u0 = line_at(line, blockIdx.x);
+        sh.u1 = line_at(line, blockIdx.x + 1);
+        sh.first = part_at(line, sh.u0, sh.u1, a.batch);
+    }
+    if (warp == 2) tmem_alloc(&sh.tmem, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem, tmem_a = tmem + 256;
-    volatile uint32_t* dead = &s_dead;
-    const int u0 = line_at(line, blockIdx.x, gridDim.x), u1 = line_at(line, blockIdx.x + 1, gridDim.x);
-    const int mma_cols = line.tile_cols / C::kHalves;
-    // A turn is two groups, or the last one of a part that has an odd number; a unit is a turn's MMAs into one accumulator.
-    auto turn_done = [&](uint32_t turn, auto wait) {  // all of the turn's MMAs
-        const uint32_t unit = turn * C::kHalves + C::kHalves - 1;
-        return wait(&done[unit % kDone], (unit / kDone) & 1, dead);
-    };
+    const uint32_t tmem = (uint32_t)uniform((int)sh.tmem), tmem_a = tmem + C::kACol;
+    // A turn is up to kTurn groups of a stage, each into an accumulator of its own; in tiles whose CTAs do not sum x themselves a turn
+    // after the last group of a window (four stages of a part) multiplies the window's biases.
+    auto window_ends = [&](const Part& t, int st) { return !C::kOwn && (((st - t.s0) & (kSumWindow - 1)) == kSumWindow - 1 || st + 1 == t.s1); };
     // Weight row (of the tile as the weights arrive) that tensor-memory lane r stands for: gate and up rows of one result 16 lanes apart
     auto tile_row = [](int r) { return MODE == kAffineGateUp ? (r & 16) * 4 + (r >> 5) * 16 + (r & 15) : r; };
-    // The sums of many rows of x take up to 128 registers of an epilogue thread: 128 roles + 256 epilogue + 256 expand <= 640 x 96, the launch's.
     if (warp < kEpilogueWarp) {
-    if (N >= 128) registers_down<N == 256 ? 48 : 64>();
+    registers_down<C::kFront>();
     if (warp == 0) {
-        // ── packed weights ──
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool alive = true;
-            for (int u = u0; u < u1 && alive;) {
-                const Part t = part_at(line, u, u1, a.batch);
-                for (int g = t.g0; g < t.g1; g += kStageGroups, ++it) {
-                    const uint32_t s = it % C::kRawStages, use = it / C::kRawStages;
-                    if (it == C::kRawStages) pdl_wait();
-                    if (use > 0 && !(alive = wait_alive(&raw_empty[s], (use - 1) & 1, dead))) break;
-                    mbar_arrive_expect_tx(&raw_full[s], kRawBytes);
-                    request_weights<MODE>(maps, line, t.row_tile, g, raw + s * kRawBytes, &raw_full[s]);
+        // ── packed weights, scales and biases ──
+        uint32_t requested = 0;
+        Ring<C::kRawStages> rs;
+        Ring<C::kScaleStages> ss;
+        uint32_t stage_scales = 0, stage_full = 0;
+        feed_scales<MODE>(a, line, sh.first, sh.u0, sh.u1, lane,
+            [&](uint32_t it, const Part& t, int st) {
+                if (it == C::kRawStages) pdl_wait();
+                if (!wait_warp(bar(C::kRawEmpty, rs.i), rs.phase ^ 1u, dead)) return false;
+                if (lane == 0) {
+                    arrive_expect_at(bar(C::kRawFull, rs.i), kRawBytes);
+                    request_weights<MODE>(maps, line, t.row_tile, st, raw + rs.i * kRawBytes, bar(C::kRawFull, rs.i));
                 }
-                u += t.g1 - t.g0;
-            }
-            for (uint32_t i = it > C::kRawStages ? it - C::kRawStages : 0; i < it; ++i) mbar_poll_bounded(&raw_full[i % C::kRawStages], (i / C::kRawStages) & 1);  // no copy may land after the CTA has left
-        }
+                requested = it + 1;
+                rs.next();
+                if (!wait_warp(bar(C::kScaleEmpty, ss.i), ss.phase ^ 1u, dead)) return false;
+                stage_scales = scales + ss.i * (2 * kLineRows * 8) + lane * 8;
+                stage_full = bar(C::kScaleFull, ss.i);
+                ss.next();
+                return true;
+            },
+            [&](uint32_t, int i, int which) { return stage_scales + which * (kLineRows * 8) + i * 256; }, [&](uint32_t) { return stage_full; });
+        if (lane == 0)
+#pragma unroll 1
+            for (uint32_t i = requested > C::kRawStages ? requested - C::kRawStages : 0; i < requested; ++i) mbar_poll_bounded(&sh.bars[C::kRawFull + i % C::kRawStages], (i / C::kRawStages) & 1);  // no copy may land after the CTA has left
     } else if (warp == 1) {
-        // ── activations ──
+        // ── activations, and their group sums where they were made in front ──
         if (lane == 0) {
             pdl_wait();
             const bool skip = dyn_skip(a.dyn);
-            if (skip) *dead = 2u;  // a guarded launch that is not to run: the other roles stop at their next wait
-            uint32_t it = 0;
+            if (skip) sh.dead = 2u;  // a guarded launch that is not to run: the other roles stop at their next wait
+            uint32_t it = 0, windows = 0, turn = 0;
+            Ring<C::kXStages> xs;
             bool alive = !skip;
             const uint32_t bytes = (uint32_t)line.tile_cols * kLineGroup * 2;
-            for (int u = u0; u < u1 && alive;) {
-                const Part t = part_at(line, u, u1, a.batch);
-                for (int g = t.g0; g < t.g1; g += 2, ++it) {
-                    const uint32_t s = it % C::kXStages;
-                    if (it >= C::kXStages && !(alive = turn_done(it - C::kXStages, wait_alive))) break;
-                    const int n = min(2, t.g1 - g);
-                    mbar_arrive_expect_tx(&x_full[s], bytes * n);
-                    for (int i = 0; i < n; ++i) tma_load_2d(x_tiles + (2 * s + i) * C::kXBytes, &maps.x, (g + i) * kLineGroup, t.col0, &x_full[s]);
+            const int u1 = sh.u1;
+            Part t = sh.first;
+#pragma unroll 1
+            for (int u = sh.u0; u < u1 && alive; next_part(line, t, u, u1, a.batch)) {
+#pragma unroll 1
+                for (int st = t.s0; st < t.s1 && alive; ++st) {
+                    const int n = stage_groups(line, st);
+#pragma unroll 1
+                    for (int j = 0; j < n; j += C::kTurn, ++it) {
+                        if (it >= C::kXStages) {
+                            const uint32_t last = sh.x_turns[xs.i];
+                            if (!(alive = wait_one(bar(C::kTurnDone, last % kDone), (last / kDone) & 1, dead) && (!C::kOwn || wait_one(bar(C::kXEmpty, xs.i), xs.phase ^ 1u, dead)))) break;
+                        }
+                        sh.x_turns[xs.i] = turn++;
+                        const int m = min(C::kTurn, n - j);
+                        arrive_expect_at(bar(C::kXFull, xs.i), bytes * m);
+#pragma unroll 1
+                        for (int i = 0; i < m; ++i) tma_load_2d_at(x_tiles + (C::kTurn * xs.i + i) * C::kXBytes, &maps.x, (st * kStageGroups + j + i) * kLineGroup, t.col0, bar(C::kXFull, xs.i));
+                        xs.next();
+                    }
+                    if (alive && window_ends(t, st)) {
+                        if (!(alive = wait_one(bar(C::kWindowEmpty), (windows & 1) ^ 1u, dead))) break;
+                        const int first = st - ((st - t.s0) & (kSumWindow - 1));
+                        arrive_expect_at(bar(C::kWindowFull), (uint32_t)line.tile_cols * 128);
+                        tma_load_2d_at(window, &maps.sums, first * 2 * kStageGroups, t.col0, bar(C::kWindowFull));
+                        ++windows;
+                        ++turn;
+                    }
                 }
-                u += t.g1 - t.g0;
+                u += t.s1 - t.s0;
             }
-            for (uint32_t i = it > C::kXStages ? it - C::kXStages : 0; i < it; ++i) mbar_poll_bounded(&x_full[i % C::kXStages], (i / C::kXStages) & 1);
+#pragma unroll 1
+            for (uint32_t i = it > C::kXStages ? it - C::kXStages : 0; i < it; ++i) mbar_poll_bounded(&sh.bars[C::kXFull + i % C::kXStages], (i / C::kXStages) & 1);
+            if (windows > 0) mbar_poll_bounded(&sh.bars[C::kWindowFull], (windows - 1) & 1);
         }
-    } else if (warp == 2) {
-        // ── issue ──
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(mma_cols >> 3) << 17) | ((uint32_t)(kLineRows >> 4) << 24);  // f32 += f16 x f16, K-major both
-        const uint32_t x_base = smem_u32(x_tiles);
+    } else {
+        // ── issue: two warps, each every second turn; a warp's chain from one turn to the next is longer than the MMAs ──
+        const int who = warp - 2;
+        const uint32_t shape = (1u << 4) | ((uint32_t)(line.tile_cols >> 3) << 17) | ((uint32_t)(kLineRows >> 4) << 24);  // f32 += f16 x f16, K-major both
+        const uint32_t tf32 = shape | (2u << 7) | (2u << 10);
+        const uint64_t x_desc = smem_desc_sw128(x_tiles), window_desc = smem_desc_sw128(window);
         pdl_wait();
-        uint32_t turn = 0, unit = 0;
+        Ring<C::kASlots> as;
+        Ring<C::kXStages> xs;
+        Ring<C::kSlots> slot;
+        Ring<kDone> end;
+        slot.next(who);
+        end.next(who);
+        uint32_t turn = 0, units = 0, windows = 0, last = 0;
         bool alive = true;
-        for (int u = u0; u < u1 && alive;) {
-            const Part t = part_at(line, u, u1, a.batch);
-            for (int g = t.g0; g < t.g1 && alive; g += 2, ++turn) {
-                const uint32_t as = turn % kASlots, xs = turn % C::kXStages, ap = (turn / kASlots) & 1, xp = (turn / C::kXStages) & 1;
-                const bool two = t.g1 - g > 1, b0 = peek(&x_full[xs], xp), b1 = peek(&a_full[as], ap);
-                if (!__all_sync(0xffffffffu, b0 && b1)) alive = wait_warp(&x_full[xs], xp, dead) && wait_warp(&a_full[as], ap, dead);
+        auto ready = [&](uint32_t b_full, uint32_t b_phase) {  // all three at once; what is missing is waited for
+            const uint32_t a_full = bar(C::kAFull, as.i), free = bar(C::kAccEmpty, slot.i);
+            const bool b = peek(b_full, b_phase), w = peek(a_full, as.phase), d = peek(free, slot.phase ^ 1u);
+            const bool ok = __all_sync(0xffffffffu, b && w && d) || (wait_warp(b_full, b_phase, dead) && wait_warp(a_full, as.phase, dead) && wait_warp(free, slot.phase ^ 1u, dead));
+            tc_fence_after();
+            return ok;
+        };
+        auto issued = [&] {
+            commit_elected(bar(C::kTurnDone, end.i));
+            last = end.i | end.phase << 16;
+            slot.next(2);
+            end.next(2);
+            ++units;
+        };
+        const int u1 = uniform(sh.u1);
+        Part t = uniform(sh.first);
 #pragma unroll 1
-                for (int h = 0; h < C::kHalves && alive; ++h) {
-                    const uint32_t slot = unit % C::kSlots, use = unit / C::kSlots;
-                    if (use > 0 && !(alive = wait_warp(&acc_empty[slot], (use - 1) & 1, dead))) break;
-                    tc_fence_after();
-                    const uint64_t b = smem_desc_sw128(x_base + 2 * xs * C::kXBytes + h * mma_cols * 128);
+        for (int u = uniform(sh.u0); u < u1 && alive; next_part(line, t, u, u1, a.batch)) {
 #pragma unroll 1
-                    for (int j = two ? 0 : 2; j < 4; ++j) {  // lo and lo, hi and hi: the small products first, what is cut off their sums is small too
-                        const int i = two ? j & 1 : 0, lo = two ? j < 2 : j == 2;
-                        umma_f16_group(tmem + slot * C::kMma, tmem_a + as * 128 + i * 64 + lo * 32, b + i * (C::kXBytes / 16), idesc, j > 0 && (two || j > 2) ? 1u : 0u);
+            for (int st = t.s0; st < t.s1 && alive; ++st) {
+                const int n = stage_groups(line, st);
+#pragma unroll 1
+                for (int k = 0; k < n; k += C::kTurn, ++turn, as.next(), xs.next()) {
+                    if ((int)(turn & 1) != who) continue;
+                    if (!(alive = ready(bar(C::kXFull, xs.i), xs.phase))) break;
+                    uint32_t d = tmem + slot.i * 128, at = tmem_a + as.i * (C::kTurn * 32);
+                    uint64_t b = x_desc + xs.i * (C::kTurn * C::kXBytes / 16);
+#pragma unroll 1
+                    for (int i = min(C::kTurn, n - k); i > 0; --i, d += N, at += 32, b += C::kXBytes / 16) umma_f16_group(d, at, b, shape);
+                    issued();
+                }
+                if (alive && window_ends(t, st)) {
+                    if ((int)(turn & 1) == who) {
+                        if (!(alive = ready(bar(C::kWindowFull), windows & 1))) break;
+                        const int steps = ((st - t.s0) & (kSumWindow - 1)) + 1;
+#pragma unroll 1
+                        for (int i = 0; i < steps; ++i) umma_tf32_step(tmem + slot.i * 128, tmem_a + as.i * 32 + 8 * i, window_desc + 2 * i, tf32, i > 0);
+                        commit_elected(bar(C::kWindowEmpty));
+                        issued();
                     }
-                    if (elect_one()) {
-                        umma_commit(&done[unit % kDone]);
-                        mbar_arrive(&done[unit % kDone]);  // hands the power on, which this warp has seen with a_full
-                    }
-                    __syncwarp();
-                    ++unit;
+                    ++turn;
+                    as.next();
+                    ++windows;
                 }
             }
-            u += t.g1 - t.g0;
+            u += t.s1 - t.s0;
         }
-        if (unit > 0) mbar_poll_bounded(&done[(unit - 1) % kDone], ((unit - 1) / kDone) & 1);  // the MMAs in flight read shared memory and write tensor memory
-    } else if (warp == 3) {
-        // ── scales and biases ──
-        feed_scales<MODE>(a, line, u0, u1, lane,
-            [&](uint32_t it) {
-                if (it == C::kRawStages) pdl_wait();
-                return it < C::kRawStages || wait_warp(&raw_empty[it % C::kRawStages], (it / C::kRawStages - 1) & 1, dead);
-            },
-            [&](uint32_t it, int i, int j, uint32_t sb) { scales[it % C::kRawStages][j][lane + 32 * i] = sb; },
-            [&](uint32_t it) { if (lane == 0) mbar_arrive(&scale_full[it % C::kRawStages]); });
+        // the MMAs in flight read shared memory and write tensor memory
+        if (units > 0) mbar_poll_bounded(&sh.bars[C::kTurnDone + (last & 0xffff)], last >> 16);
+        if (windows > 0) mbar_poll_bounded(&sh.bars[C::kWindowEmpty], (windows - 1) & 1);
     }
     } else if (warp < kExpandWarp) {
-        if (N >= 128) registers_up<N == 256 ? 160 : 120>();
-        // ── sums and epilogue: two sets of four warps, each half of an accumulator's columns ──
-        const int set = (warp - kEpilogueWarp) >> 2, quad = warp & 3, r = quad * 32 + lane;
-        const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
+        registers_up<C::kDrain>();
+        // ── sums and epilogue: two sets of four warps, each half of the tile's columns; a turn is 64 values of a thread, fetched at once ──
+        const int set = (warp - kEpilogueWarp) >> 2, quad = warp & 3, r = quad * 32 + lane, row = tile_row(r);
+        const int eights = line.tile_cols / 16, from = set * eights * 8;  // of a set
+        const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16) + from;
         const bool leader = tid == kEpilogueWarp * 32;
-        const int set_cols = mma_cols / 2;  // a multiple of eight
         auto all_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory"); };
-        uint32_t unit = 0, turns = 0;
+        Ring<C::kScaleStages> ss;
+        Ring<C::kSlots> slot;
+        Ring<kDone> end;
+        Ring<C::kOwnSlots> own;
         pdl_wait();
-        for (int u = u0; u < u1;) {
-            const Part t = part_at(line, u, u1, a.batch);
-            uint64_t sums[C::kSums / 2];
+        const int u1 = sh.u1;
+        Part t = sh.first;
+#pragma unroll 1
+        for (int u = sh.u0; u < u1; next_part(line, t, u, u1, a.batch)) {
+            constexpr int kSums = N / 2, kChunks = kSums / 16;  // chunks of sixteen columns of a group
+            float sums[kSums];
 #pragma unroll
-            for (int j = 0; j < C::kSums / 2; ++j) sums[j] = 0;
+            for (int j = 0; j < kSums; ++j) sums[j] = 0.f;
             bool alive = true;
-            for (int g = t.g0; g < t.g1 && alive; g += 2, ++turns) {
+            uint32_t held = 0;  // stages whose scales this window has used
+#pragma unroll 1
+            for (int st = t.s0; st < t.s1 && alive; ++st) {
+                if (!(alive = wait_warp(bar(C::kScaleFull, ss.i), ss.phase, dead))) break;
+                const uint32_t row_scales = scales + ss.i * (2 * kLineRows * 8) + row * 8;
+                const int n = stage_groups(line, st), all = n + window_ends(t, st);
+                uint2 sv = lds64(row_scales), bv = C::kOwn ? lds64(row_scales + kLineRows * 8) : make_uint2(0, 0);
+#pragma unroll 1
+                for (int k = 0; k < all; k += C::kTurn) {
+                    float s1[C::kTurn], b1[C::kTurn];
 #pragma unroll
-                for (int h = 0; h < C::kHalves; ++h, ++unit) {
-                    const uint32_t slot = unit % C::kSlots, src = lane_base + slot * C::kMma + set * set_cols;
-                    if (!(alive = wait_warp(&done[unit % kDone], (unit / kDone) & 1, dead))) break;
+                    for (int i = 0; i < C::kTurn; ++i) {
+                        const float si = __low2float(u32_as_h2(sv.x));
+                        s1[i] = C::kOwn || k < n ? si * kNibble : 1.f;
+                        b1[i] = C::kOwn ? fmaf(8.f, si, __low2float(u32_as_h2(bv.x))) : 0.f;  // the nibbles are centred
+                        sv = make_uint2(__funnelshift_r(sv.x, sv.y, 16), sv.y >> 16);
+                        bv = make_uint2(__funnelshift_r(bv.x, bv.y, 16), bv.y >> 16);
+                    }
+                    const int m = C::kOwn ? min(C::kTurn, n - k) : 1;
+                    if (!(alive = wait_warp(bar(C::kTurnDone, end.i), end.phase, dead) && (!C::kOwn || wait_warp(bar(C::kSumFull, own.i), own.phase, dead)))) break;
                     tc_fence_after();
-                    const float power = powers[turns % kPowers][r];
-                    const uint64_t power2 = pack2(power, power);
-                    // sixteen columns on their way while the sixteen before them are added, where the registers allow it
-                    constexpr int kBatches = C::kMma / 32, kAhead = N == 256 ? 0 : 1;
-                    uint32_t v[1 + kAhead][16];
-                    tmem_ld16(src, v[0]);
+                    uint32_t v[4][16];
 #pragma unroll
-                    for (int i = 0; i < kBatches; ++i) {
-                        if (i > 0 && 16 * i >= set_cols) break;
-                        const bool more = i + 1 < kBatches && 16 * (i + 1) < set_cols;
-                        tmem_wait_ld16(v[i & kAhead]);
-                        if (kAhead && more) tmem_ld16(src + 16 * (i + 1), v[(i + 1) & kAhead]);
-                        if (!more) {
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(&acc_empty[slot]);
-                        }
+                    for (int q = 0; q < 4; ++q) tmem_ld16(lane_base + slot.i * 128 + q / kChunks * N + q % kChunks * 16, v[q]);
+                    if constexpr (C::kOwn) {
+                        const uint32_t x_sums = own_sums + own.i * (C::kTurn * N * 4) + from * 4;
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            uint64_t& s = sums[h * (C::kMma / 4) + 8 * i + j];
-                            s = fma2(pack2(__uint_as_float(v[i & kAhead][2 * j]), __uint_as_float(v[i & kAhead][2 * j + 1])), power2, s);
+                        for (int q = 0; q < 4; ++q)
+                            if (q / kChunks < m) {
+                                const float b = b1[q / kChunks];
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const uint4 xs = lds128(x_sums + q / kChunks * (N * 4) + q % kChunks * 64 + 16 * j);
+                                    float* to = sums + q % kChunks * 16 + 4 * j;
+                                    to[0] = fmaf(__uint_as_float(xs.x), b, to[0]);
+                                    to[1] = fmaf(__uint_as_float(xs.y), b, to[1]);
+                                    to[2] = fmaf(__uint_as_float(xs.z), b, to[2]);
+                                    to[3] = fmaf(__uint_as_float(xs.w), b, to[3]);
+                                }
+                            }
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) tmem_wait_ld16(v[q]);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        arrive_at(bar(C::kAccEmpty, slot.i));
+                        if (C::kOwn) arrive_at(bar(C::kSumEmpty, own.i));
+                    }
+                    slot.next();
+                    end.next();
+                    own.next();
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (q / kChunks < m) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) sums[q % kChunks * 16 + j] = fmaf(__uint_as_float(v[q][j]), s1[q / kChunks], sums[q % kChunks * 16 + j]);
                         }
-                        if (!kAhead && more) tmem_ld16(src + 16 * (i + 1), v[0]);
+                }
+                if (!alive) break;
+                if (C::kOwn) {
+                    if (lane == 0) arrive_at(bar(C::kScaleEmpty, ss.i));
+                } else {
+                    ++held;
+                    if (window_ends(t, st)) {  // the expansion has read the biases of the window's stages too
+                        if (lane == 0)
+#pragma unroll 1
+                            for (uint32_t i = 0; i < held; ++i) arrive_at(bar(C::kScaleEmpty, ss.i >= i ? ss.i - i : ss.i + C::kScaleStages - i));
+                        held = 0;
                     }
                 }
+                ss.next();
             }
-            if (!alive && *dead == 0u) *dead = 1u;
-            all_sync();  // the eight warps go on together or not at all
-            if (leader) s_go = *dead == 0u ? 1u : 0u;
+            all_sync();  // the eight warps go on together or not at all: one that gave up has set the word
+            if (leader) sh.go = lds_word(dead) == 0u ? 1u : 0u;
             all_sync();
-            if (s_go == 0u) break;
-            // The sums go through scratch, a tile's alone as well: what comes then is a short loop (unrolled over the registers, its
-            // code came from beyond the instruction cache: a tile of gate and up cost 52,000 clocks).
+            if (sh.go == 0u) break;
+            // The end of a tile.  A CTA that shares it leaves its sums in scratch; the last to arrive adds them in the order of the CTAs.
             const size_t part = (size_t)line.tile_cols * kLineRows;
-            const bool shared = t.g0 != 0 || t.g1 != line.groups;
-            Sharers sh = {(int)blockIdx.x, (int)blockIdx.x, 2 * (int)blockIdx.x + 1};  // a slot that this CTA's last tile has, if it is shared
-            if (shared) sh = sharers(line, t.tile, gridDim.x);
-            float4* mine = reinterpret_cast<float4*>(a.part_scratch + (size_t)sh.slot(blockIdx.x) * part) + set * set_cols / 4 * kLineRows + r;  // [four columns][row]
-#pragma unroll
-            for (int h = 0; h < C::kHalves; ++h)
-#pragma unroll
-                for (int c0 = 0; c0 < C::kMma / 2; c0 += 4)
-                    if (c0 < set_cols) {
-                        const float2 lo = unpack2(sums[(h * (C::kMma / 2) + c0) / 2]), hi = unpack2(sums[(h * (C::kMma / 2) + c0) / 2 + 1]);
-                        __stcg(mine + (h * mma_cols + c0) / 4 * kLineRows, make_float4(lo.x, lo.y, hi.x, hi.y));
-                    }
-            bool finish = true;
-            if (shared) {
-                __threadfence();
+            constexpr int kEights = N / 16;
+            auto column = [&](int i) { return from + 8 * i; };
+            const bool together = t.s0 != 0 || t.s1 != line.stages;
+            Sharers sharing = {(int)blockIdx.x, (int)blockIdx.x, 2 * (int)blockIdx.x + 1};
+            if (together) sharing = sharers(line, t.tile);
+            float4* const mine = reinterpret_cast<float4*>(a.part_scratch + (size_t)sharing.slot(blockIdx.x) * part) + r;  // [four columns][row]
+            bool finish = true, left = false;  // left: this CTA's sums are in scratch
+            if (together) {
+                if (leader) sh.ticket = *(volatile int*)(a.part_counters + t.tile) == sharing.last - sharing.first ? 1u : 0u;
                 all_sync();
-                if (leader) s_ticket = (uint32_t)atomicAdd(a.part_counters + t.tile, 1);
+                left = sh.ticket == 0u;  // else all others have arrived: this one is the last, and its sums need not go through scratch
+                if (left) {
+#pragma unroll
+                    for (int i = 0; i < kEights; ++i)
+                        if (i < eights) {
+                            __stcg(mine + column(i) / 4 * kLineRows, make_float4(sums[8 * i], sums[8 * i + 1], sums[8 * i + 2], sums[8 * i + 3]));
+                            __stcg(mine + (column(i) / 4 + 1) * kLineRows, make_float4(sums[8 * i + 4], sums[8 * i + 5], sums[8 * i + 6], sums[8 * i + 7]));
+                        }
+                    __threadfence();
+                }
                 all_sync();
-                finish = s_ticket == (uint32_t)(sh.last - sh.first);
+                if (leader) sh.ticket = (uint32_t)atomicAdd(a.part_counters + t.tile, 1);
+                all_sync();
+                finish = sh.ticket == (uint32_t)(sharing.last - sharing.first);
                 if (finish) {
                     __threadfence();
                     if (leader) a.part_counters[t.tile] = 0;  // the next launch finds every counter at zero
                 }
             }
             if (finish) {
-                const LineRow o = line_row<MODE>(a, line, t.row_tile, tile_row(r));
+                const LineRow o = line_row<MODE>(a, line, t.row_tile, row);
                 const bool row_ok = o.row < o.rows;
                 auto write = [&](int c, float (&v)[8]) {  // eight columns of the tile from c on
                     const int n = t.live - c;
@@ -336,13 +518,11 @@ __global__ void __launch_bounds__(kThreads, 1) affine_wide_kernel(const __grid_c
                         // lanes 16 apart have gate and up of one row of the result: the gate's takes the first four columns, the up's the others
                         const bool up = r & 16;
                         __half* y = o.y + (size_t)(t.col0 + c + (up ? 4 : 0)) * o.rows + o.row;
-#pragma unroll 1
-                        for (int j = 0; j < 4; ++j, y += o.rows) {
-                            const float other = __shfl_xor_sync(0xffffffffu, up ? v[0] : v[4], 16);
-                            const __half z = swiglu_f32(up ? other : v[0], up ? v[4] : other);  // lut_matvec.metal:2228
-                            if (row_ok && j + (up ? 4 : 0) < n) *y = z;
 #pragma unroll
-                            for (int i = 0; i < 7; ++i) v[i] = v[i + 1];
+                        for (int j = 0; j < 4; ++j, y += o.rows) {
+                            const float other = __shfl_xor_sync(0xffffffffu, up ? v[j] : v[4 + j], 16);
+                            const __half z = swiglu_f32(up ? other : v[j], up ? v[4 + j] : other);  // lut_matvec.metal:2228
+                            if (row_ok && j + (up ? 4 : 0) < n) *y = z;
                         }
                     } else if (row_ok) {
                         const size_t at = (size_t)(t.col0 + c) * o.rows + o.row;
@@ -355,102 +535,198 @@ __global__ void __launch_bounds__(kThreads, 1) affine_wide_kernel(const __grid_c
                             if (j < n) o.y[at + (size_t)j * o.rows] = MODE == kAffineAdd ? __hadd(__float2half_rn(v[j]), res[j]) : __float2half_rn(v[j]);  // lut_matvec.metal:1802-1803
                     }
                 };
-                // A step: eight columns of four CTAs' sums; the next step's are on their way while these are added (one after the
-                // other a step cost 1 us, most of it latency).
-                const int chunks = set_cols / 8, rounds = (sh.last - sh.first + 4) / 4, steps = C::kHalves * chunks * rounds;
-                float4 f[4][2];
-                auto request = [&](int step) {
-                    const int c = sh.first + step % rounds * 4, i = step / rounds, col = i / chunks * mma_cols + set * set_cols + i % chunks * 8;
+                // A step: eight columns of some CTAs' sums; the next step's are on their way while these are added.  A short loop that picks its
+                // own sums from the registers by a jump: unrolled, the code would come from beyond the instruction cache.
+                constexpr int kAtOnce = 2;
+                const int rounds = (sharing.last - sharing.first + kAtOnce) / kAtOnce, steps = eights * rounds;
+                float4 f[kAtOnce][2];
+                auto request = [&](int i, int c) {
 #pragma unroll
-                    for (int z = 0; z < 4; ++z) {
-                        const float4* q = reinterpret_cast<const float4*>(a.part_scratch + (size_t)sh.slot(min(c + z, sh.last)) * part) + col / 4 * kLineRows + r;
+                    for (int z = 0; z < kAtOnce; ++z) {
+                        const float4* q = reinterpret_cast<const float4*>(a.part_scratch + (size_t)sharing.slot(min(c + z, sharing.last)) * part) + column(i) / 4 * kLineRows + r;
+                        const bool there = c + z <= sharing.last && c + z != (int)blockIdx.x;
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) f[z][j] = c + z <= sh.last ? __ldcg(q + j * kLineRows) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        for (int j = 0; j < 2; ++j) f[z][j] = there ? __ldcg(q + j * kLineRows) : make_float4(0.f, 0.f, 0.f, 0.f);
                     }
                 };
                 float v[8];
-                request(0);
+                request(0, sharing.first);
 #pragma unroll 1
-                for (int step = 0; step < steps; ++step) {
-                    if (step % rounds == 0)
+                for (int i = 0, c = sharing.first, left_steps = steps; left_steps > 0; --left_steps) {
+                    if (c == sharing.first)
 #pragma unroll
                         for (int j = 0; j < 8; ++j) v[j] = 0.f;
+                    const int me = (int)blockIdx.x - c;
+                    if (me >= 0 && me < kAtOnce) {
+                        float own_v[8];
+                        switch (i) {
+#define PICK(n)                                                    \
+    case n:                                                        \
+        if constexpr (n < kEights)                                 \
+            for (int j = 0; j < 8; ++j) own_v[j] = sums[8 * n + j];      \
+        break;
+                            PICK(0) PICK(1) PICK(2) PICK(3) PICK(4) PICK(5) PICK(6) PICK(7)
+#undef PICK
+                        }
 #pragma unroll
-                    for (int z = 0; z < 4; ++z)
+                        for (int z = 0; z < kAtOnce; ++z)
+                            if (z == me) { f[z][0] = make_float4(own_v[0], own_v[1], own_v[2], own_v[3]); f[z][1] = make_float4(own_v[4], own_v[5], own_v[6], own_v[7]); }
+                    }
+#pragma unroll
+                    for (int z = 0; z < kAtOnce; ++z)
 #pragma unroll
                         for (int j = 0; j < 2; ++j) { v[4 * j] += f[z][j].x; v[4 * j + 1] += f[z][j].y; v[4 * j + 2] += f[z][j].z; v[4 * j + 3] += f[z][j].w; }
-                    if (step + 1 < steps) request(step + 1);
-                    const int i = step / rounds, col = i / chunks * mma_cols + set * set_cols + i % chunks * 8;
-                    if (step % rounds == rounds - 1 && col < t.live) write(col, v);
+                    const int col = column(i);
+                    const bool summed = c + kAtOnce > sharing.last;
+                    if (summed) { ++i; c = sharing.first; } else c += kAtOnce;
+                    if (left_steps > 1) request(i, c);
+                    if (summed && col < t.live) write(col, v);
                 }
             }
             __syncwarp();  // the next tensor-memory load needs the whole warp
-            u += t.g1 - t.g0;
+            u += t.s1 - t.s0;
         }
-    } else {
-        if (N >= 128) registers_down<N == 256 ? 56 : 88>();
-        // ── expansion: two sets of four warps take turns ──
+    } else if (warp < kSumWarp) {
+        registers_down<C::kBehind>();
+        // ── expansion: sets of four warps take turns ──
         const int set = (warp - kExpandWarp) >> 2, quad = warp & 3, r = quad * 32 + lane, row = tile_row(r);
-        const uint32_t dst = tmem_a + ((uint32_t)(quad * 32) << 16), raw_a = smem_u32(raw);
-        uint32_t turn = 0, stage = 0;
+        const uint32_t dst = tmem_a + ((uint32_t)(quad * 32) << 16);
+        uint32_t turn = 0, minus = 0xA400A400u;  // -8 x 2^-9
+        Ring<C::kRawStages> rs;
+        Ring<C::kScaleStages> ss;
+        Ring<C::kASlots> as;
         bool alive = true;
-        for (int u = u0; u < u1 && alive;) {
-            const Part t = part_at(line, u, u1, a.batch);
-            for (int g = t.g0; g < t.g1 && alive; g += kStageGroups, ++stage) {
-                const uint32_t s = stage % C::kRawStages, ph = (stage / C::kRawStages) & 1;
-                const bool b0 = peek(&raw_full[s], ph), b1 = peek(&scale_full[s], ph);
-                if ((!__all_sync(0xffffffffu, b0) && !wait_warp(&raw_full[s], ph, dead)) || (!__all_sync(0xffffffffu, b1) && !wait_warp(&scale_full[s], ph, dead))) { alive = false; break; }
-                const uint32_t src = raw_a + s * kRawBytes + row * 128;
-                const int n = min(kStageGroups, t.g1 - g);
-                for (int k = 0; 2 * k < n; ++k, ++turn) {
-                    const uint32_t as = turn % kASlots;
-                    if ((int)as != set) continue;
-                    if (turn >= kASlots && turn < 2 * kASlots) pdl_wait();
-                    if (turn >= kASlots && !turn_done(turn - kASlots, wait_warp)) { alive = false; break; }
-                    tc_fence_after();
-                    const int last = min(n - 1, 2 * k + 1);
-                    const uint32_t top = max(top_of(__half22float2(u32_as_h2(scales[s][2 * k][row]))), top_of(__half22float2(u32_as_h2(scales[s][last][row]))));
-                    const float up = power_up(top);
-                    powers[turn % kPowers][r] = power_down(top);
+        auto slot_free = [&] {
+            if (turn >= C::kASlots && turn < C::kASlots + 2) pdl_wait();
+            if (turn >= C::kASlots) {
+                const uint32_t last = turn - C::kASlots;
+                if (!wait_warp(bar(C::kTurnDone, last % kDone), (last / kDone) & 1, dead)) return false;
+            }
+            tc_fence_after();
+            return true;
+        };
+        auto written = [&] {
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_at(bar(C::kAFull, as.i));
+        };
+        const int u1 = sh.u1;
+        Part t = sh.first;
 #pragma unroll 1
-                    for (int i = 2 * k; i <= last; ++i) {
-                        const float2 f = __half22float2(u32_as_h2(scales[s][i][row]));
-                        const uint64_t s2 = pack2(f.x * up, f.x * up), b2 = pack2(f.y * up, f.y * up);
+        for (int u = sh.u0; u < u1 && alive; next_part(line, t, u, u1, a.batch)) {
+#pragma unroll 1
+            for (int st = t.s0; st < t.s1 && alive; ++st) {
+                const int n = stage_groups(line, st);
+                const bool mine = C::kTurn < kStageGroups || (int)(turn & 1) == set;
+                if (mine && !(alive = wait_warp(bar(C::kRawFull, rs.i), rs.phase, dead) && (C::kOwn || wait_warp(bar(C::kScaleFull, ss.i), ss.phase, dead)))) break;
+                const uint32_t src = raw + rs.i * kRawBytes + row * 128, row_scales = scales + ss.i * (2 * kLineRows * 8) + row * 8;
+#pragma unroll 1
+                for (int k = 0; k < n; k += C::kTurn, ++turn, as.next()) {
+                    if ((int)(turn & 1) != set) continue;
+                    if (!C::kOwn) {
+                        bool centred;
+                        tf32_bias(lds_half(row_scales + 2 * k), lds_half(row_scales + kLineRows * 8 + 2 * k), &centred);
+                        minus = centred ? 0xA400A400u : 0u;
+                    }
+                    if (!(alive = slot_free())) break;
+                    const uint32_t to = dst + as.i * (C::kTurn * 32);
+                    const int halves = 2 * min(C::kTurn, n - k);
+#pragma unroll 1
+                    for (int i = 0; i < halves; i += 2) {  // a group
+                        const uint4 v0 = lds128(src + (((2 * k + i) ^ (row & 7)) << 4)), v1 = lds128(src + (((2 * k + i + 1) ^ (row & 7)) << 4));
+                        uint32_t pair[16], more[16];
+                        expand_nibbles(v0.x, minus, pair);
+                        expand_nibbles(v0.y, minus, pair + 4);
+                        expand_nibbles(v0.z, minus, pair + 8);
+                        expand_nibbles(v0.w, minus, pair + 12);
+                        expand_nibbles(v1.x, minus, more);
+                        expand_nibbles(v1.y, minus, more + 4);
+                        expand_nibbles(v1.z, minus, more + 8);
+                        expand_nibbles(v1.w, minus, more + 12);
+                        tmem_st16(to + i * 16, pair);
+                        tmem_st16(to + i * 16 + 16, more);
+                    }
+                    written();
+                }
+                if (!alive) break;
+                if (mine) {
+                    __syncwarp();
+                    if (lane == 0) arrive_at(bar(C::kRawEmpty, rs.i));
+                }
+                if (window_ends(t, st)) {  // biases, twice each: they meet hi and lo of the group sums
+                    if ((int)(turn & 1) == set) {
+                        if (!(alive = slot_free())) break;
+                        const uint32_t last = (st - t.s0) & (kSumWindow - 1);
+#pragma unroll 1
+                        for (uint32_t i = 0; i <= last; ++i) {
+                            const uint32_t back = last - i, at = scales + (ss.i >= back ? ss.i - back : ss.i + C::kScaleStages - back) * (2 * kLineRows * 8) + row * 8;
+                            uint32_t v[8];
+                            bool centred;
 #pragma unroll
-                        for (int p = 0; p < 2; ++p) {
-                            const uint4 v = lds128(src + (((2 * i + p) ^ (row & 7)) << 4));
-                            const uint32_t word[4] = {v.x, v.y, v.z, v.w}, to = dst + as * 128 + (i & 1) * 64 + p * 16;
-                            if constexpr (N == 256) {  // few registers
+                            for (int j = 0; j < 4; ++j) v[j] = v[4 + j] = __float_as_uint(tf32_bias(lds_half(at + 2 * j), lds_half(at + kLineRows * 8 + 2 * j), &centred));
+                            tmem_st8(dst + as.i * 32 + 8 * i, v);
+                        }
+                        written();
+                    }
+                    ++turn;
+                    as.next();
+                }
+                rs.next();
+                ss.next();
+            }
+            u += t.s1 - t.s0;
+        }
+    } else if constexpr (C::kOwn) {
+        registers_down<C::kBehind>();
+        // ── group sums of x: a thread sums the 64 columns of one row ──
+        constexpr int kRowWarps = kSumWarps / C::kTurn;  // warps that share a group's rows
+        const int i = (warp - kSumWarp) / kRowWarps, col = (warp - kSumWarp) % kRowWarps * 32 + lane;
+        Ring<C::kXStages> xs;
+        Ring<C::kOwnSlots> own;
+        bool alive = true;
+        pdl_wait();
+        const int u1 = sh.u1;
+        Part t = sh.first;
+#pragma unroll 1
+        for (int u = sh.u0; u < u1 && alive; next_part(line, t, u, u1, a.batch)) {
+#pragma unroll 1
+            for (int st = t.s0; st < t.s1 && alive; ++st) {
+                const int n = stage_groups(line, st);
+#pragma unroll 1
+                for (int k = 0; k < n; k += C::kTurn) {
+                    if (!(alive = wait_warp(bar(C::kXFull, xs.i), xs.phase, dead))) break;
+                    uint64_t sum[4] = {0, 0, 0, 0};
+                    const bool valid = k + i < n && col < line.tile_cols;
+                    if (valid) {
+                        const uint32_t src = x_tiles + (C::kTurn * xs.i + i) * C::kXBytes + col * 128;
+#pragma unroll 2
+                        for (int c = 0; c < 8; ++c) {
+                            const uint4 v = lds128(src + ((c ^ (col & 7)) << 4));
+                            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                                for (int q = 0; q < 4; q += 2) {
-                                    uint32_t hi[8], lo[8];
-                                    expand_hi_lo(word[q], s2, b2, hi, lo);
-                                    expand_hi_lo(word[q + 1], s2, b2, hi + 4, lo + 4);
-                                    tmem_st8(to + 4 * q, hi);
-                                    tmem_st8(to + 32 + 4 * q, lo);
-                                }
-                            } else {
-                                uint32_t hi[16], lo[16];
-#pragma unroll
-                                for (int q = 0; q < 4; ++q) expand_hi_lo(word[q], s2, b2, hi + 4 * q, lo + 4 * q);
-                                tmem_st16(to, hi);
-                                tmem_st16(to + 32, lo);
+                            for (int j = 0; j < 4; ++j) {
+                                const float2 f = __half22float2(u32_as_h2(w[j]));
+                                sum[j] = add2(sum[j], pack2(f.x, f.y));
                             }
                         }
                     }
-                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                    tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&a_full[as]);
+                    if (lane == 0) arrive_at(bar(C::kXEmpty, xs.i));
+                    if (!(alive = wait_warp(bar(C::kSumEmpty, own.i), own.phase ^ 1u, dead))) break;
+                    const float2 f = unpack2(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])));
+                    if (valid) sh.own_sums[own.i][i][col] = f.x + f.y;
+                    __syncwarp();
+                    if (lane == 0) arrive_at(bar(C::kSumFull, own.i));
+                    xs.next();
+                    own.next();
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&raw_empty[s]);
             }
-            u += t.g1 - t.g0;
+            u += t.s1 - t.s0;
         }
     }
     __syncthreads();
-    if (tid == 0 && a.err && *dead == 1u) atomicOr(a.err, 0x400u);
+    if (tid == 0 && a.err && lds_word(dead) == 1u) atomicOr(a.err, 0x400u);
     tc_fence_before();
     __syncthreads();
     if (warp == 2) {
@@ -459,15 +735,12 @@ __global__ void __launch_bounds__(kThreads, 1) affine_wide_kernel(const __grid_c
     }
 }
 
-template <int MODE, int N>
-cudaError_t launch_wide_t(const Launch& l, AffineArgs a, const LineMaps& maps, const Line& line, int grid) {
-    auto kern = affine_wide_kernel<MODE, N>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WideCfg<N>::kSmem);
-    if (e != cudaSuccess) return e;
+template <typename... Params, typename... Args>
+cudaError_t launch_pdl(const Launch& l, void (*kern)(Params...), dim3 grid, int threads, uint32_t smem, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = WideCfg<N>::kSmem;
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = l.stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -475,25 +748,52 @@ cudaError_t launch_wide_t(const Launch& l, AffineArgs a, const LineMaps& maps, c
     cfg.attrs = attr;
     cfg.numAttrs = l.pdl ? 1 : 0;
     prefer_max_shared(kern);
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <int MODE, int N>
+cudaError_t launch_wide_t(const Launch& l, AffineArgs a, const LineMaps& maps, const Line& line, int grid) {
+    auto kern = affine_wide_kernel<MODE, N>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WideCfg<N>::kSmem);
+    if (e != cudaSuccess) return e;
     a.dyn = dev_dyn(l);
-    return cudaLaunchKernelEx(&cfg, kern, maps, a, line);
+    return launch_pdl(l, kern, dim3(grid), WideCfg<N>::kThreads, WideCfg<N>::kSmem, maps, a, line);
 }
 
 template <int MODE>
 cudaError_t launch_wide(const Launch& l, const AffineArgs& a, const LineMaps& maps, const Line& line, int grid) {
     if (line.tile_cols <= 32) return launch_wide_t<MODE, 32>(l, a, maps, line, grid);
     if (line.tile_cols <= 64) return launch_wide_t<MODE, 64>(l, a, maps, line, grid);
-    return line.tile_cols <= 128 ? launch_wide_t<MODE, 128>(l, a, maps, line, grid) : launch_wide_t<MODE, 256>(l, a, maps, line, grid);
+    return launch_wide_t<MODE, 128>(l, a, maps, line, grid);
 }
 
 }  // namespace
 
 cudaError_t launch_affine_wide(const Launch& l, int mode, const AffineArgs& a, int group, bool* handled) {
+    // Rows of x whose group sums find room behind the shared tiles of the full scratch (40 MiB: 10,000 of 17,408 columns); more go in parts.
+    const int sm = a.sm_count > 0 ? a.sm_count : 148, stages = (a.cols / kLineGroup + kStageGroups - 1) / kStageGroups;
+    const size_t tiles = (size_t)sm * 2 * 128 * kLineRows * sizeof(float);
+    if (a.batch > 128 && a.part_scratch_bytes > tiles) {
+        const size_t rows = (a.part_scratch_bytes - tiles) / ((size_t)stages * 2 * kStageGroups * sizeof(float)) / 128 * 128;
+        if (rows >= 128 && rows < (size_t)a.batch) {
+            *handled = false;
+            for (int r0 = 0; r0 < a.batch; r0 += (int)rows) {
+                const cudaError_t e = launch_affine_wide(l, mode, affine_rows(a, r0, std::min((int)rows, a.batch - r0)), group, handled);
+                if (e != cudaSuccess || !*handled) return e;
+            }
+            return cudaSuccess;
+        }
+    }
     LineMaps maps = {};
     Line line;
+    GroupSums sums;
     int grid = 0;
-    *handled = line_plan(mode, a, group, 256, &maps, &line, &grid);
+    *handled = line_plan(mode, a, group, 128, kOwnCols, &maps, &line, &sums, &grid);
     if (!*handled) return cudaSuccess;
+    if (sums.at) {
+        const cudaError_t e = launch_pdl(l, group_sums_kernel, dim3(a.batch, std::min((line.stages + 7) / 8, 65535)), 256, 0, a.x, sums.at, a.batch, a.cols, line.stages);
+        if (e != cudaSuccess) return e;
+    }
     switch (mode) {
         case kAffinePlain: return launch_wide<kAffinePlain>(l, a, maps, line, grid);
         case kAffineAdd: return launch_wide<kAffineAdd>(l, a, maps, line, grid);

@@ -10,45 +10,73 @@ namespace smelt {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// Bounded wait on an mbarrier phase: try_wait suspends the thread in hardware for up to the hinted
-// time (a spinning warp would take issue slots from the warp that shares its scheduler), the
-// loop gives up after about a second and reports failure instead of waiting forever.
+// Waits for a phase up to 64 times; each time the thread is suspended in hardware for a while (a spinning warp would take issue slots from
+// the warps that share its scheduler).  Without the instruction's time hint: with it the compiler makes a timed loop around every
+// wait, a third of the instructions that the affine product issued.
+__device__ __forceinline__ bool mbar_tries(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
+        "mov.u32 n, 0;\n"
+        "again_%=:\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "@p bra through_%=;\n\t"
+        "add.u32 n, n, 1;\n\t"
+        "setp.lt.u32 q, n, 64;\n\t"
+        "@q bra again_%=;\n"
+        "through_%=:\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ uint64_t now_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+constexpr uint64_t kWaitNs = 1000000000ull;  // a wait gives up after a second and reports it instead of waiting forever
 __device__ __forceinline__ bool mbar_poll_bounded(uint64_t* bar, uint32_t parity) {
-    for (uint32_t i = 0; i < (1u << 20); ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
-            : "memory");
-        if (ok) return true;
-    }
+    const uint32_t at = smem_u32(bar);
+    if (mbar_tries(at, parity)) return true;
+    const uint64_t begin = now_ns();
+#pragma unroll 1
+    while (now_ns() - begin < kWaitNs)
+        if (mbar_tries(at, parity)) return true;
     return false;
 }
-// Waits for a phase; gives up after about a second, or as soon as another role has.
+// Waits for a phase; gives up after a second, or as soon as another role has.
 __device__ __forceinline__ bool wait_alive(uint64_t* bar, uint32_t parity, volatile uint32_t* dead) {
-    for (uint32_t i = 0; i < (1u << 20); ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
-            : "memory");
-        if (ok) return true;
+    const uint32_t at = smem_u32(bar);
+    if (mbar_tries(at, parity)) return true;
+    const uint64_t begin = now_ns();
+#pragma unroll 1
+    while (now_ns() - begin < kWaitNs) {
+        if (mbar_tries(at, parity)) return true;
         if (*dead) return false;
     }
     *dead = 1u;
     return false;
+}
+// A shared-memory address that stays in a register: left to itself the compiler makes it again from the CTA's number at every use.
+__device__ __forceinline__ uint32_t kept(uint32_t address) {
+    uint32_t a;
+    asm volatile("mov.u32 %0, %1;" : "=r"(a) : "r"(address));
+    return a;
 }
 // A box of a 2-D tensor map, x the inner coordinate (a multiple of 16 bytes).
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y),
                  "r"(smem_u32(bar))
                  : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_at(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void arrive_at(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void arrive_expect_at(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
