@@ -49,7 +49,7 @@ cudaError_t launch_imma_t(const Launch& l, AffineArgs a) {
     if (L.total > 226u * 1024u) return cudaErrorNotSupported;  // digit planes too large to stay resident
     a.dyn = dev_dyn(l);
     auto kern = affine_imma_kernel<MODE, DEPTH, WARPS, GPS, TG>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
+    cudaError_t e = allow_shared(kern, L.total);
     if (e != cudaSuccess) return e;
     if (NW == 1 && a.nseg <= 1) {
         a.nseg = 1;

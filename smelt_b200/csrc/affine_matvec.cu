@@ -401,7 +401,7 @@ cudaError_t launch_t(const Launch& l, AffineArgs a) {
     a.nsplit = nsplit;
     a.dyn = dev_dyn(l);
     auto kern = affine_mma_kernel<MODE, GROUP, NBT, WARPS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
+    cudaError_t e = allow_shared(kern, L.total);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((a.rows + kRows - 1) / kRows, nsplit, 1);

@@ -327,7 +327,7 @@ cudaError_t launch_stream_t(const Launch& l, AffineArgs a, int ctas_per_sm) {
     const StreamLayout L = stream_layout(NW, STAGES, a.cols, a.batch, WARPS);
     a.dyn = dev_dyn(l);
     auto kern = affine_stream_kernel<MODE, STAGES, WARPS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
+    cudaError_t e = allow_shared(kern, L.total);
     if (e != cudaSuccess) return e;
     if (NW == 1 && a.nseg <= 1) {
         a.nseg = 1;

@@ -754,7 +754,7 @@ cudaError_t launch_pdl(const Launch& l, void (*kern)(Params...), dim3 grid, int 
 template <int MODE, int N>
 cudaError_t launch_wide_t(const Launch& l, AffineArgs a, const LineMaps& maps, const Line& line, int grid) {
     auto kern = affine_wide_kernel<MODE, N>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WideCfg<N>::kSmem);
+    cudaError_t e = allow_shared(kern, WideCfg<N>::kSmem);
     if (e != cudaSuccess) return e;
     a.dyn = dev_dyn(l);
     return launch_pdl(l, kern, dim3(grid), WideCfg<N>::kThreads, WideCfg<N>::kSmem, maps, a, line);

@@ -95,7 +95,7 @@ template <int D, int NH, int NU>
 cudaError_t launch_decode_t(const Launch& l, const AttnDev& p) {
     const size_t smem = attn_smem_bytes<D, NH, NU>();
     auto kern = attn_decode_kernel<D, NH, NU>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared(kern, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.nsplits, p.a.n_kv, p.a.batch);

@@ -301,13 +301,20 @@ __device__ __forceinline__ __half gated_norm_d128_value(__half x, __half g, __ha
 // wait gives up so the host can report it instead of hanging.
 enum : uint32_t { KERR_BARRIER_TIMEOUT = 1u, KERR_FLAG_TIMEOUT = 2u };
 
+// Attributes of a kernel, set when they are first asked for and when a context has been made since (runtime.cu): set on every launch,
+// the two cost 1.5 us of a typed call's 6.5.
+cudaError_t kernel_attributes(const void* kernel, int dynamic_shared, bool max_shared);
+// Dynamic shared memory of a launch.
+template <typename Kernel>
+inline cudaError_t allow_shared(Kernel kernel, size_t bytes) {
+    return kernel_attributes(reinterpret_cast<const void*>(kernel), (int)bytes, false);
+}
 // Every kernel of a decode step asks for the same shared-memory carve-out (the largest): an SM
 // drains before it changes its L1 / shared-memory split, so kernels that prefer different
 // splits can neither overlap nor follow each other without a gap.
 template <typename Kernel>
 inline cudaError_t prefer_max_shared(Kernel kernel) {
-    return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributePreferredSharedMemoryCarveout,
-                                (int)cudaSharedmemCarveoutMaxShared);
+    return kernel_attributes(reinterpret_cast<const void*>(kernel), 0, true);
 }
 
 }  // namespace smelt

@@ -158,7 +158,7 @@ inline cudaError_t launch_chained(const Launch& l, Kernel kernel, dim3 grid, dim
     cfg.attrs = attr;
     cfg.numAttrs = l.pdl ? 1 : 0;
     if (smem > 16 * 1024) {  // the default limit is 48 KB together with the kernel's static shared memory
-        cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_shared(kernel, smem);
         if (e != cudaSuccess) return e;
     }
     prefer_max_shared(kernel);

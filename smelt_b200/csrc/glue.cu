@@ -514,11 +514,11 @@ cudaError_t launch_fp16_matvec(const Launch& l, const __half* w, const __half* x
         launch_cfg(l, cfg, attr, dim3(grid), dim3(256), smem);
         cudaError_t e;
         if (nb == 1) {
-            e = cudaFuncSetAttribute(fp16_matvec_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            e = allow_shared(fp16_matvec_kernel<1>, smem);
             prefer_max_shared(fp16_matvec_kernel<1>);
             if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fp16_matvec_kernel<1>, w, x + (size_t)b0 * cols, y + (size_t)b0 * rows, rows, cols, nb, dev_dyn(l));
         } else {
-            e = cudaFuncSetAttribute(fp16_matvec_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            e = allow_shared(fp16_matvec_kernel<8>, smem);
             prefer_max_shared(fp16_matvec_kernel<8>);
             if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, fp16_matvec_kernel<8>, w, x + (size_t)b0 * cols, y + (size_t)b0 * rows, rows, cols, nb, dev_dyn(l));
         }

@@ -282,7 +282,7 @@ cudaError_t launch_prefill_attention_ks(const Launch& l, const __half* q, const 
                                         uint32_t n_pos, uint32_t start_pos, uint32_t capacity, float scale, uint32_t window, uint32_t per_warp) {
     auto kern = attn_prefill_kernel<D, NH, KS>;
     constexpr size_t smem = prefill_attn_smem<D, NH, KS>();
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_shared(kern, smem);
     if (e != cudaSuccess) return e;
     const uint32_t step = kAttnWarps / KS * per_warp;
     cudaLaunchConfig_t cfg = {};

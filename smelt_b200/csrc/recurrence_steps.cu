@@ -402,7 +402,7 @@ cudaError_t launch_dn_fused_prefill(const Launch& l, __half* state, __half* conv
     a.conv_state = conv_state; a.conv_weight = conv_weight;
     a.head_dim = head_dim; a.heads = heads; a.qkv_dim = qkv_dim; a.conv_k = conv_k; a.seq_len = seq_len; a.head_scale = head_scale; a.eps = l2_eps;
     const size_t smem = (size_t)head_dim * (head_dim + 2) * sizeof(__half);
-    cudaError_t e = cudaFuncSetAttribute(dn_fused_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared(dn_fused_prefill_kernel, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];

@@ -1,8 +1,10 @@
 // Context, buffer slots and the typed launchers of the libsmelt_cuda C ABI.
 #include "runtime.h"
 
+#include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "affine_matvec.h"
 #include "glue.h"
@@ -37,6 +39,53 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 }  // namespace
 }  // namespace smelt
 
+// What kernel_attributes has set, by kernel: the generation of contexts it was set in (a device that was reset between two contexts has
+// forgotten it), the largest dynamic shared memory and whether the carve-out is.  A record is one word, read without a lock; only
+// setting takes one, so that a smaller size never follows a larger one of another thread.
+namespace smelt {
+namespace {
+constexpr int kKernelRecords = 1024, kRecordedDevices = 16;
+struct KernelRecord {
+    std::atomic<const void*> kernel{nullptr};
+    std::atomic<uint64_t> state[kRecordedDevices] = {};  // generation << 32 | bytes << 1 | carve-out
+};
+KernelRecord g_kernel_records[kKernelRecords];
+std::atomic<uint32_t> g_generation{1};
+std::mutex g_kernel_mutex;
+cudaError_t set_attributes(const void* kernel, int bytes, bool max_shared) {
+    if (max_shared) return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+KernelRecord* kernel_record(const void* kernel) {
+    size_t at = (reinterpret_cast<uintptr_t>(kernel) >> 4) * 0x9E3779B97F4A7C15ull >> 54;
+    for (int i = 0; i < kKernelRecords; ++i, at = (at + 1) % kKernelRecords) {
+        const void* held = g_kernel_records[at].kernel.load(std::memory_order_acquire);
+        if (held == kernel || (!held && (g_kernel_records[at].kernel.compare_exchange_strong(held, kernel) || held == kernel))) return &g_kernel_records[at];
+    }
+    return nullptr;
+}
+}  // namespace
+
+cudaError_t kernel_attributes(const void* kernel, int dynamic_shared, bool max_shared) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    KernelRecord* r = device < kRecordedDevices ? kernel_record(kernel) : nullptr;
+    if (!r) return set_attributes(kernel, dynamic_shared, max_shared);
+    auto known = [&](uint64_t s) { return (uint32_t)(s >> 32) == g_generation.load(std::memory_order_acquire) && (max_shared ? (s & 1u) != 0 : (int)((s & 0xffffffffu) >> 1) >= dynamic_shared); };
+    if (known(r->state[device].load(std::memory_order_acquire))) return cudaSuccess;
+    std::lock_guard<std::mutex> hold(g_kernel_mutex);
+    const uint32_t generation = g_generation.load(std::memory_order_acquire);
+    uint64_t s = r->state[device].load(std::memory_order_acquire);
+    if ((uint32_t)(s >> 32) != generation) s = (uint64_t)generation << 32;
+    const int bytes = (int)((s & 0xffffffffu) >> 1);
+    if (!max_shared && dynamic_shared <= bytes) return cudaSuccess;
+    e = set_attributes(kernel, dynamic_shared, max_shared);
+    if (e == cudaSuccess) r->state[device].store(max_shared ? s | 1u : (s & ~0xfffffffeull) | (uint64_t)dynamic_shared << 1, std::memory_order_release);
+    return e;
+}
+}  // namespace smelt
+
 #define CTX_OR_FAIL()                                \
     if (!ctx) return SMELT_ERR_BAD_ARGUMENT;         \
     {                                                \
@@ -65,6 +114,7 @@ smelt_status smelt_cuda_create(int device_ordinal, smelt_cuda_ctx** out_ctx) {
     if (cudaGetDeviceProperties(&prop, device_ordinal) != cudaSuccess) return SMELT_ERR_CUDA;
     if (prop.major < 10) return SMELT_ERR_UNSUPPORTED;  // kernels are built for sm_100a only
     if (cudaSetDevice(device_ordinal) != cudaSuccess) return SMELT_ERR_CUDA;
+    smelt::g_generation.fetch_add(1, std::memory_order_acq_rel);
     smelt_cuda_ctx* ctx = new (std::nothrow) smelt_cuda_ctx();
     if (!ctx) return SMELT_ERR_ALLOC;
     ctx->device = device_ordinal;

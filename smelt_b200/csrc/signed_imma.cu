@@ -346,7 +346,7 @@ cudaError_t launch_signed_imma_t(const Launch& l, const SignedArgs& a, int sm_co
     if (L.total > 226u * 1024u) return cudaSuccess;  // digit planes too large to stay resident: not handled
     *handled = true;
     auto kern = signed_imma_kernel<BITS, MODE>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
+    cudaError_t e = allow_shared(kern, L.total);
     if (e != cudaSuccess) return e;
     const int tiles = (a.rows + kTileRows - 1) / kTileRows;
     const int sm = sm_count > 0 ? sm_count : 148;

@@ -93,7 +93,7 @@ cudaError_t launch_nb(const Launch& l, const SignedArgs& a) {
     const size_t smem = (size_t)NB * a.cols * sizeof(float);
     if (smem > 200 * 1024) return cudaErrorInvalidValue;
     auto kern = signed_matvec_kernel<BITS, MODE, NB>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared(kern, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((a.rows + 7) / 8, (a.batch + NB - 1) / NB);

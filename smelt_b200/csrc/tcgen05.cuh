@@ -10,9 +10,45 @@ namespace smelt {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// Bounded wait on an mbarrier phase: try_wait suspends the thread in hardware for up to the hinted
+// time (a spinning warp would take issue slots from the warp that shares its scheduler), the
+// loop gives up after about a second and reports failure instead of waiting forever.
+__device__ __forceinline__ bool mbar_poll_bounded(uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < (1u << 20); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+// Waits for a phase; gives up after about a second, or as soon as another role has.
+__device__ __forceinline__ bool wait_alive(uint64_t* bar, uint32_t parity, volatile uint32_t* dead) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < (1u << 20); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity), "r"(1000u)
+            : "memory");
+        if (ok) return true;
+        if (*dead) return false;
+    }
+    *dead = 1u;
+    return false;
+}
 // Waits for a phase up to 64 times; each time the thread is suspended in hardware for a while (a spinning warp would take issue slots from
 // the warps that share its scheduler).  Without the instruction's time hint: with it the compiler makes a timed loop around every
-// wait, a third of the instructions that the affine product issued.
+// wait, a third of the instructions that the affine product issued (the 16-bit product, whose waits are few, is 1 % faster with it).
 __device__ __forceinline__ bool mbar_tries(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -37,28 +73,6 @@ __device__ __forceinline__ uint64_t now_ns() {
     return t;
 }
 constexpr uint64_t kWaitNs = 1000000000ull;  // a wait gives up after a second and reports it instead of waiting forever
-__device__ __forceinline__ bool mbar_poll_bounded(uint64_t* bar, uint32_t parity) {
-    const uint32_t at = smem_u32(bar);
-    if (mbar_tries(at, parity)) return true;
-    const uint64_t begin = now_ns();
-#pragma unroll 1
-    while (now_ns() - begin < kWaitNs)
-        if (mbar_tries(at, parity)) return true;
-    return false;
-}
-// Waits for a phase; gives up after a second, or as soon as another role has.
-__device__ __forceinline__ bool wait_alive(uint64_t* bar, uint32_t parity, volatile uint32_t* dead) {
-    const uint32_t at = smem_u32(bar);
-    if (mbar_tries(at, parity)) return true;
-    const uint64_t begin = now_ns();
-#pragma unroll 1
-    while (now_ns() - begin < kWaitNs) {
-        if (mbar_tries(at, parity)) return true;
-        if (*dead) return false;
-    }
-    *dead = 1u;
-    return false;
-}
 // A shared-memory address that stays in a register: left to itself the compiler makes it again from the CTA's number at every use.
 __device__ __forceinline__ uint32_t kept(uint32_t address) {
     uint32_t a;

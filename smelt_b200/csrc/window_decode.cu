@@ -251,7 +251,7 @@ template <int D, int VD, int NH>
 cudaError_t launch_t(const Launch& l, const WindowArgs& a, int head_groups, int splits) {
     auto kern = window_decode_kernel<D, VD, NH>;
     const size_t smem = decode_smem<D, VD, NH>();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_shared(kern, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(splits, a.kv_heads * head_groups);
