@@ -195,27 +195,45 @@ __device__ __forceinline__ void feed_scales(const AffineArgs& a, const Line& p, 
         bool async = (p.groups & 3) == 0;  // eight bytes at a time
 #pragma unroll
         for (int i = 0; i < 4; ++i) async = async && (reinterpret_cast<uintptr_t>(from[i]) & 7u) == 0;
+        if (!async) {  // two bytes at a time: one stage's are on their way while the one before is stored, out of L2
+#pragma unroll
+            for (int i = 0; i < 2 * kRows; ++i)
+                if (live[i >> 2] > (i >> 1 & 1) * 32)
 #pragma unroll 1
-        for (int st = t.s0; st < t.s1; ++st, ++it) {
-            if (!wait(it, t, st)) { cp_async_wait<0>(); return; }
+                    for (int g = t.s0 * kStageGroups; g < min(p.groups, t.s1 * kStageGroups); g += 16) asm volatile("prefetch.global.L2 [%0];" ::"l"(from[(i >> 2) * 2 + (i & 1)] + (i >> 1 & 1) * step + g));
+        }
+        uint2 ahead[2 * kRows];
+        auto load = [&](int st) {
             const int g = st * kStageGroups, n = stage_groups(p, st);
 #pragma unroll
             for (int i = 0; i < 2 * kRows; ++i) {
-                const uint32_t to = dst(it, i >> 1, i & 1);
                 const __half* q = from[(i >> 2) * 2 + (i & 1)] + (i >> 1 & 1) * step + g;
                 const bool ok = live[i >> 2] > (i >> 1 & 1) * 32;
-                if (async) {
-                    if (ok) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(q) : "memory");
-                } else {
-                    uint32_t h[4] = {0, 0, 0, 0};
-                    if (ok)
+                uint32_t h[4];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) h[j] = j < n ? (uint32_t)__half_as_ushort(__ldg(q + j)) : 0u;
-                    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(to), "r"(h[0] | h[1] << 16), "r"(h[2] | h[3] << 16) : "memory");
+                for (int j = 0; j < 4; ++j) h[j] = ok && j < n ? (uint32_t)__half_as_ushort(__ldg(q + j)) : 0u;
+                ahead[i] = make_uint2(h[0] | h[1] << 16, h[2] | h[3] << 16);
+            }
+        };
+        if (!async) load(t.s0);
+#pragma unroll 1
+        for (int st = t.s0; st < t.s1; ++st, ++it) {
+            if (!wait(it, t, st)) { cp_async_wait<0>(); return; }
+            const int g = st * kStageGroups;
+#pragma unroll
+            for (int i = 0; i < 2 * kRows; ++i) {
+                const uint32_t to = dst(it, i >> 1, i & 1);
+                if (!async) {
+                    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(to), "r"(ahead[i].x), "r"(ahead[i].y) : "memory");
+                } else if (live[i >> 2] > (i >> 1 & 1) * 32) {
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to), "l"(from[(i >> 2) * 2 + (i & 1)] + (i >> 1 & 1) * step + g) : "memory");
                 }
             }
             if (async) asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full(it)) : "memory");
-            else arrive_at(full(it));
+            else {
+                arrive_at(full(it));
+                if (st + 1 < t.s1) load(st + 1);
+            }
         }
         u += t.s1 - t.s0;
     }

@@ -24,6 +24,7 @@
 // tile form a thread-block cluster and are reduced through distributed shared memory in rank
 // order, so results are bit-reproducible.
 #include "affine_matvec.h"
+#include "glue.h"
 
 #include <cooperative_groups.h>
 
@@ -445,33 +446,42 @@ cudaError_t launch_group(const Launch& l, const AffineArgs& a, int group) {
     }
 }
 
-// Whether the tensor-core product (affine_wide.cu) takes a launch first.  Its expansion of the weights costs the same for any
-// number of rows, about as much as two passes of the streaming kernel with all its activations to stage.
-//   * 17 rows and more: always (gate/up 12288 x 4096, 16 rows on the streaming kernel 46.8 us, 17 rows here 57.3, 32 rows 57.7,
-//     where the streaming kernel would take four passes).
-//   * 9 to 16 rows with a residual, where the streaming kernel takes several passes over 64 K activations and more (us, passes
-//     against it): 4096 x 4096, 12 rows (48 K) 14.6 : 15.1, 16 rows 16.7 : 15.1; 2048 x 6144, 16 rows (96 K) 17.0 : 12.9; 4096 x 12288,
-//     9 rows (108 K) 32.7 : 32.9, 16 rows 51.5 : 32.9; 1024 x 12288, 9 rows 20.8 : 13.5; 5120 x 17408, 9 rows 60.2 : 50.2, 16 rows
-//     117 : 50.3.
-//   * 9 to 16 rows that the streaming kernel does not take, from 64 K activations on: gate/up 3000 x 6976, 9 rows (61 K) 49.4 on
-//     the general kernel, 12 rows (82 K) 54.9 : 38.6; 4096 x 6976, 10 rows (68 K) 27.2 : 29.8, 12 rows
-//     54.1 : 29.8.
-//   * Plain products that the streaming kernel takes stay there up to 16 rows: one launch over several tensors
-//     (affine_multi_matvec) runs on it, and gives the bits of a launch for each.
-//   * Up to eight rows never: the general kernel splits K over a cluster, and few rows of weights make no tile worth the
-//     expansion (1024 x 12288, 8 rows 9.4 : 13.4; 5120 x 17408, 8 rows 62.3 : 50.2).
+// Whether the tensor-core product (affine_wide.cu) takes a launch first (us, what would run otherwise : it).
+//   * 17 rows and more: always.  A folded norm is a launch of its own then.
+//   * 9 to 16 rows: gate/up, dual and + residual, where the streaming kernel needs two passes or more: gate/up 12288 x 4096, 9 rows
+//     38.7 : 30.0, 16 rows 46.5 : 29.2; 6144 x 2048, 9 rows 15.4 : 11.7; 4096 x 12288 + residual, 9 rows 32.7 : 17.6; 2048 x 2048, 9 rows
+//     7.5 : 7.0.  Plain products only where the streaming kernel does not take them (264 x 17408, 9 rows 28.4 : 12.7): one launch over
+//     several tensors (affine_multi_matvec) runs on it up to 16 rows, and gives the bits of a launch for each.
+//   * 6 to 8 rows, plain and + residual, that the streaming kernel does not take because their activations do not stay resident, from
+//     128 M weights x rows on: the general kernel takes about 2 + 0.08 us for a million of these, the product 8 + 0.2 for a million
+//     weights.  8 rows: 4096 x 12288 29.5 : 17.7, 2048 x 12288 18.9 : 12.2, 1024 x 17408 17.6 : 13.4, 1024 x 12288 9.4 : 11.9;
+//     6 rows: 5120 x 17408 56.9 : 26.7, 4096 x 6976 18.1 : 17.7; gate/up 3000 x 6976 21.8 : 23.8.
 bool wide_first(int mode, const AffineArgs& a, int group) {
     if (a.batch >= 17) return true;
-    if (a.batch <= 8 || a.norm_w || a.nseg > 1) return false;
-    const int passes = affine_stream_passes(mode, a, group);
-    return passes == 0 ? (size_t)a.batch * a.cols >= 65536u : passes > 1 && mode == kAffineAdd && (size_t)a.batch * a.cols >= 65536u;
+    if (a.batch <= 5 || a.nseg > 1) return false;
+    const bool streamed = affine_stream_passes(mode, a, group) != 0;
+    if (a.batch >= 9) return mode != kAffinePlain || !streamed;
+    return (mode == kAffinePlain || mode == kAffineAdd) && !streamed && (size_t)a.rows * a.cols * a.batch >= (size_t)128 << 20;
 }
 
 }  // namespace
 
 cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int group) {
     if (args.rows <= 0 || args.cols <= 0 || args.batch <= 0 || args.cols % group != 0) return cudaErrorInvalidValue;
-    if (wide_first(mode, args, group)) {  // tcgen05: the weights are expanded once per 256 rows of x
+    if (wide_first(mode, args, group)) {  // tcgen05: the weights are expanded once per 128 rows of x
+        if (args.norm_w) {  // the folded norm as a launch of its own, its rows behind everything else in scratch
+            const size_t bytes = ((size_t)args.batch * args.cols * sizeof(__half) + 255) & ~(size_t)255;
+            if (args.part_scratch && args.cols % 8 == 0 && bytes <= args.part_scratch_bytes / 4) {
+                AffineArgs s = args;
+                __half* xn = reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(args.part_scratch) + (args.part_scratch_bytes - bytes) / 256 * 256);
+                const cudaError_t e = launch_rms_norm_1pw(l, args.x, args.norm_w, xn, args.cols, args.norm_eps, args.batch);
+                if (e != cudaSuccess) return e;
+                s.x = xn;
+                s.norm_w = nullptr;
+                s.part_scratch_bytes = (args.part_scratch_bytes - bytes) / 256 * 256;
+                return launch_affine(l, mode, s, group);
+            }
+        }
         bool handled = false;
         cudaError_t e = launch_affine_wide(l, mode, args, group, &handled);
         if (handled || e != cudaSuccess) return e;

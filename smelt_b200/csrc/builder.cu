@@ -50,7 +50,7 @@ static smelt_status build_decoder_impl(smelt_cuda_ctx* ctx, const smelt_decoder_
     // bit 1: fold the norms into the projections (one QKV launch, one gate/up launch) and RoPE /
     // KV append into one launch; needs the shapes the streaming matvec kernel accepts.
     const bool fuse_tp = (d->fuse_residual & 4) != 0;  // bit 2: all-reduce and residual add in one launch over peer memory
-    const bool fuse2 = (d->fuse_residual & 2) && G == 64 && H % 1024 == 0 && qd % 16 == 0 && kvd % 16 == 0 && B <= 8 && D % 2 == 0;
+    const bool fuse2 = (d->fuse_residual & 2) && G == 64 && H % 1024 == 0 && qd % 16 == 0 && kvd % 16 == 0 && D % 2 == 0;
     const bool bt = B > 1;  // batched kernel names bind actualBatch instead of numRows
 
     if (!dry) {
