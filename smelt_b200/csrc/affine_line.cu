@@ -19,7 +19,7 @@ EncodeTiled encode_tiled() {
 }
 
 // How many CTAs take the line: either a whole number for each tile, or all SMs, whose stretches then begin and end anywhere.
-// Estimated in us.  A stage takes a CTA 0.99 us with 32 rows of x, 1.8 with 64 and 1.7 with 128 (whose group sums are made in front);
+// Estimated in us.  A stage takes a CTA 0.99 us with 32 rows of x, 1.6 with 64 and 1.65 with 128 (whose group sums are made in front);
 // a tile of k CTAs needs 1 us and 0.57, 0.85 or 2.0 for each of them more; stretches that begin anywhere 3 us and 1.3 times as much for
 // each of the CTAs that may share a tile.  Measured (us, by CTAs of a tile; 148: all SMs): 1024 x 12288, 32 rows: 4 17.3, 8 13.8, 16 15.0,
 // 148 18.5; 128 rows: 4 34.0, 6 29.9, 8 31.4, 16 43.7, 148 49.1; 4096 x 4096, 32 rows: 2 13.1, 4 10.8, 148 12.5; 128 rows: 4 23.3,
@@ -27,7 +27,7 @@ EncodeTiled encode_tiled() {
 // of whole tiles would be 3 x 16).
 int ctas_for(const Line& p, int sm, int* per_tile) {
     const long tiles = (long)p.row_tiles * p.col_tiles;
-    const double stage = p.tile_cols <= 32 ? 0.99 : p.tile_cols <= 64 ? 1.8 : 1.7, sum = p.tile_cols <= 32 ? 0.57 : p.tile_cols <= 64 ? 0.85 : 2.0;
+    const double stage = p.tile_cols <= 32 ? 0.99 : p.tile_cols <= 64 ? 1.6 : 1.65, sum = p.tile_cols <= 32 ? 0.57 : p.tile_cols <= 64 ? 0.85 : 2.0;
     *per_tile = 0;
     double least = (double)tiles * p.stages / sm * stage + 3.0 + 1.3 * sum * ((double)sm / tiles + 1.0);
     for (int k = 1; k <= p.stages && tiles * k <= sm; ++k) {

@@ -103,54 +103,24 @@ __device__ __forceinline__ void request_weights(const LineMaps& maps, const Line
     }
 }
 
-// The same by a whole warp, all of it or none: bar and dead are addresses of shared memory.
+// Waits by a whole warp, all of it or none, and by one thread: bar and dead are addresses of shared memory; the word at dead is set when a
+// wait gives up.
 __device__ __forceinline__ uint32_t lds_word(uint32_t a) {
     uint32_t v;
     asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
     return v;
 }
-__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, uint32_t dead) {
-    if (__all_sync(0xffffffffu, mbar_tries(bar, parity))) return true;
-    const uint64_t begin = now_ns();
-#pragma unroll 1
-    for (;;) {
-        if (__all_sync(0xffffffffu, mbar_tries(bar, parity))) return true;
-        const bool late = now_ns() - begin >= kWaitNs;
-        if (late) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
-        if (__any_sync(0xffffffffu, late || lds_word(dead) != 0u)) return false;
-    }
-}
-// By one thread.
 __device__ __forceinline__ bool wait_one(uint32_t bar, uint32_t parity, uint32_t dead) {
-    if (mbar_tries(bar, parity)) return true;
-    const uint64_t begin = now_ns();
-#pragma unroll 1
-    for (;;) {
-        if (mbar_tries(bar, parity)) return true;
-        if (lds_word(dead) != 0u) return false;
-        if (now_ns() - begin >= kWaitNs) break;
-    }
-    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
-    return false;
+    const bool ok = mbar_wait_short(bar, parity);
+    if (!ok) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
+    return ok;
 }
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, uint32_t dead) { return __all_sync(0xffffffffu, wait_one(bar, parity, dead)); }
 // A value that is the same in all lanes, where the compiler can see it: what follows from it stays in uniform registers.
 __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ Part uniform(const Part& t) {
     return {uniform(t.tile), uniform(t.s0), uniform(t.s1), uniform(t.row_tile), uniform(t.col_tile), uniform(t.col0), uniform(t.live)};
 }
-// Whether a phase has completed, without waiting: several are asked at once and only what is missing is waited for.
-__device__ __forceinline__ bool peek(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
     uint64_t d;
     asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
@@ -161,8 +131,6 @@ __device__ __forceinline__ float2 unpack2(uint64_t v) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
     return f;
 }
-// acc += a * b, in the accumulator's own registers
-__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
 __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     uint64_t d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));

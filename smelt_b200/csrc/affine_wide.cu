@@ -7,13 +7,15 @@
 // epilogue warps multiply what they drain by the scale and add it to fp32 registers.  The nibbles are centred (q - 8) and the bias is
 // bias + 8 scale, so that neither sum is much larger than the result.  The tensor core truncates what it adds to, here four
 // K = 16 products at a time.  Share of fp16 results that are not the correctly rounded ones, against two fp16 operands per
-// dequantised weight summed over two groups (before -> now): 4096 x 4096, 32 rows 0.12 -> 0.09 %, 512 rows 0.12 -> 0.08; gate and
-// up 12288 x 4096, 32 rows 0.20 -> 0.19, 512 rows 0.21 -> 0.15.
+// dequantised weight summed over two groups (before -> now): 4096 x 4096, 32 rows 0.12 -> 0.08 %, 512 rows 0.12 -> 0.08; gate and
+// up 12288 x 4096, 32 rows 0.20 -> 0.15, 512 rows 0.21 -> 0.15.
 //
-// bias * sum(x).  Tiles of up to 64 rows of x: four warps sum x from shared memory, the epilogue adds the products in fp32.  More
-// rows: the sums are made once in front (group_sums_kernel), as two tf32 values each, and the biases of up to sixteen groups
-// multiply them on the tensor core as one more turn; where bias + 8 scale is not exact in tf32 the group's nibbles stay as they are
-// and its bias, which is an fp16, is the operand.
+// bias * sum(x).  Tiles of up to 64 rows of x: four warps sum x from shared memory.  More: the sums are made once in front
+// (group_sums_kernel), as they would cost every CTA four warps' issue slots.  Tiles of up to 32 rows: the epilogue adds the products in fp32.
+// More: the sums are kept as two tf32 values each, and the biases of up to sixteen groups multiply them on the tensor core as one
+// more turn; where bias + 8 scale is not exact in tf32 the group's nibbles stay as they are and its bias, which is an fp16, is the operand.
+// (The epilogue's way with 64 rows: 50.2 | 31.0 | 15.2 us of the shapes below; the tensor core's with 32 rows 31.8 | 20.2 | 11.0, a turn
+// more for each of a CTA's short stretches, and a step of 32 sequences 3.88 ms instead of 3.75.)
 //
 // Mapping.  One CTA an SM takes a stretch of the launch's line of work (affine_line.cuh); a tile is 128 weight
 // rows, the MMA's M, by up to 128 rows of x, its N.  The roles, each on warps of its own, each a ring ahead of the next:
@@ -25,13 +27,14 @@
 //   * issue: two warps take turns;
 //   * sums and epilogue, eight warps: plain, + residual, SwiGLU of gate and up, dual.  A turn is 128 columns of tensor memory: four
 //     groups of 32 rows of x, two of 64, one of 128.
-// What bounds it: instruction issue (0.6 an SM quarter and clock).  What cost most on the way here: code beyond the 32 KB that the
+// What bounds it: instruction issue (0.6 an SM quarter and clock, a third of it bookkeeping of the roles) and the handing over between
+// them.  What cost most on the way here: code beyond the 32 KB that the
 // instruction cache holds (wait loops unrolled by the compiler: 122 KB), spilled registers (the shared memory leaves no first-level
 // cache: a reload is an L2 round trip), waits with a time hint (a timed loop each), shared addresses made anew at every use, packed
 // FMAs (a move each).
 // us, graph replay over distinct weights, before -> now (gate/up 12288 x 4096 x 2 | 4096 x 12288 | 4096 x 4096): 32 rows
-// 58.4 -> 31.3 | 34.4 -> 19.6 | 15.5 -> 10.8; 64 rows 63.9 -> 50.2 | 40.0 -> 31.0 | 18.3 -> 15.2; 128 rows 74.6 -> 57.1 |
-// 43.5 -> 42.0 | 22.4 -> 23.3; 512 rows 227 -> 184 | 113 -> 91 | 51.5 -> 36.0.
+// 58.4 -> 31.8 | 34.4 -> 20.2 | 15.5 -> 11.0; 64 rows 63.9 -> 44.7 | 40.0 -> 28.8 | 18.3 -> 15.2; 128 rows 74.6 -> 56.3 |
+// 43.5 -> 41.0 | 22.4 -> 23.0; 512 rows 227 -> 178 | 113 -> 89 | 51.5 -> 34.8.
 // A launch in front may take longer than a wait may (its waits on a peer are as long): every role waits for it before the first
 // wait that depends on the activations, and only what needs none of them goes ahead.
 // Every wait is bounded: on expiry the CTA sets bit 10 of the error word, its roles stop, copies and MMAs in flight are
@@ -59,7 +62,8 @@ struct Ring {
 
 template <int N>
 struct WideCfg {
-    static constexpr bool kOwn = N <= kOwnCols;
+    static constexpr bool kOwn = N <= kOwnCols;    // the CTA sums x itself
+    static constexpr bool kFolded = N <= 32;       // and the epilogue adds bias * sum in fp32: no turn for the biases
     static constexpr int kThreads = kOwn ? 768 : 640;
     // Registers of the roles in front, the epilogue, and the others; together no more than the launch's.
     static constexpr int kFront = 48, kDrain = N == 128 ? 160 : 128, kBehind = 56;
@@ -67,17 +71,17 @@ struct WideCfg {
     static constexpr int kSlots = kOwn ? 2 : 3;                           // of accumulators: 128 columns of tensor memory each
     static constexpr int kASlots = kOwn ? 256 / (32 * kTurn) : 4, kACol = kSlots * 128;
     static constexpr int kXBytes = N * kLineGroup * 2, kXStages = N == 128 ? 5 : 4, kRawStages = N == 128 ? 4 : 6;  // a stage of x is a turn's
-    static constexpr int kScaleStages = kOwn ? 8 : 12;
-    static constexpr int kWindow = kOwn ? 0 : N * 128;                    // group sums of kSumWindow stages
-    static constexpr int kOwnSlots = kOwn ? 4 : 1;                        // turns whose own group sums are kept
-    static constexpr uint32_t kSmem = kRawStages * kRawBytes + kXStages * kTurn * kXBytes + kWindow + 1024;
+    static constexpr int kScaleStages = kFolded ? 8 : 12;
+    static constexpr int kWindows = kOwn ? 2 : 1, kWindow = kFolded ? 0 : N * 128;  // group sums of kSumWindow stages
+    static constexpr int kFoldedSlots = 4;                                // turns whose sums are kept for the epilogue
+    static constexpr uint32_t kSmem = kRawStages * kRawBytes + kXStages * kTurn * kXBytes + kWindows * kWindow + 1024;
     static_assert(kSmem + 28 * 1024 <= 227u * 1024u, "shared memory");
     static_assert(kACol + kASlots * kTurn * 32 <= 512 && kTurn * N <= 128, "tensor memory");
     static_assert(kScaleStages >= 2 * kSumWindow, "the biases of a window wait for it");
     // Barriers, by the address of the first one of a kind.
     static constexpr int kRawFull = 0, kRawEmpty = kRawFull + kRawStages, kScaleFull = kRawEmpty + kRawStages, kScaleEmpty = kScaleFull + kScaleStages, kXFull = kScaleEmpty + kScaleStages,
-                         kXEmpty = kXFull + kXStages, kAFull = kXEmpty + kXStages, kTurnDone = kAFull + kASlots, kAccEmpty = kTurnDone + kDone, kSumFull = kAccEmpty + kSlots,
-                         kSumEmpty = kSumFull + kOwnSlots, kWindowFull = kSumEmpty + kOwnSlots, kWindowEmpty = kWindowFull + 1, kBarriers = kWindowEmpty + 1;
+                         kXEmpty = kXFull + kXStages, kAFull = kXEmpty + kXStages, kTurnDone = kAFull + kASlots, kAccEmpty = kTurnDone + kDone, kWindowFull = kAccEmpty + kSlots,
+                         kWindowEmpty = kWindowFull + kWindows, kSumFull = kWindowEmpty + kWindows, kSumEmpty = kSumFull + kFoldedSlots, kBarriers = kSumEmpty + kFoldedSlots;
     static_assert(128 * kFront + kEpilogueThreads * kDrain + (kThreads - 128 - kEpilogueThreads) * kBehind <= kThreads * (65536 / kThreads / 8 * 8), "registers");
 };
 
@@ -86,7 +90,7 @@ struct WideShared {
     using C = WideCfg<N>;
     uint64_t bars[C::kBarriers];
     uint2 scales[C::kScaleStages][2][kLineRows];                                    // four scales and four biases of a row
-    alignas(16) float own_sums[C::kOwnSlots][C::kOwn ? C::kTurn : 1][C::kOwn ? N : 4];  // of x by group
+    alignas(16) float folded[C::kFolded ? C::kFoldedSlots : 1][C::kTurn][C::kFolded ? N : 4];  // sums of x by group
     uint32_t x_turns[C::kXStages];                                                  // the turn that reads a stage of x
     uint32_t tmem, dead, ticket, go;
     int u0, u1;
@@ -155,11 +159,12 @@ __device__ __forceinline__ void expand_nibbles(uint32_t word, uint32_t minus, ui
 #pragma unroll
     for (int b = 0; b < 4; ++b) asm("fma.rn.f16x2 %0, %0, %1, %2;" : "+r"(pair[b]) : "r"(0x78007800u), "r"(minus));  // 2^15
 }
-__device__ __forceinline__ float lds_half(uint32_t a) {
+__device__ __forceinline__ uint32_t lds_u16(uint32_t a) {
     uint16_t h;
     asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(a));
-    return __half2float(__ushort_as_half(h));
+    return h;
 }
+__device__ __forceinline__ void sts_word(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
 __device__ __forceinline__ float tf32_of(float v) {
     uint32_t u;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(v));
@@ -200,7 +205,7 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
     __shared__ WideShared<N> sh;
     const uint32_t raw = kept((smem_u32(smem_raw) + 1023u) & ~1023u), shared = kept(smem_u32(&sh));
     const uint32_t x_tiles = raw + C::kRawStages * kRawBytes, window = x_tiles + C::kXStages * C::kTurn * C::kXBytes;
-    const uint32_t scales = shared + (uint32_t)offsetof(WideShared<N>, scales), own_sums = shared + (uint32_t)offsetof(WideShared<N>, own_sums), dead = shared + (uint32_t)offsetof(WideShared<N>, dead);
+    const uint32_t scales = shared + (uint32_t)offsetof(WideShared<N>, scales), folded = shared + (uint32_t)offsetof(WideShared<N>, folded), dead = shared + (uint32_t)offsetof(WideShared<N>, dead);
     auto bar = [&](int kind, uint32_t i = 0) { return shared + 8u * (kind + i); };
     const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
 
@@ -218,9 +223,10 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
         init(C::kAFull, C::kASlots, 4);
         init(C::kTurnDone, kDone, 1);
         init(C::kAccEmpty, C::kSlots, kEpilogueWarps);
-        init(C::kSumFull, C::kOwnSlots, kSumWarps);
-        init(C::kSumEmpty, C::kOwnSlots, kEpilogueWarps);
-        init(C::kWindowFull, 2, 1);
+        init(C::kWindowFull, C::kWindows, C::kOwn ? kSumWarps : 1);
+        init(C::kWindowEmpty, C::kWindows, 1);
+        init(C::kSumFull, C::kFoldedSlots, kSumWarps);
+        init(C::kSumEmpty, C::kFoldedSlots, kEpilogueWarps);
         sh.dead = 0u;
         mbar_fence_init();
         fence_async_smem();
@@ -235,9 +241,14 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = (uint32_t)uniform((int)sh.tmem), tmem_a = tmem + C::kACol;
-    // A turn is up to kTurn groups of a stage, each into an accumulator of its own; in tiles whose CTAs do not sum x themselves a turn
-    // after the last group of a window (four stages of a part) multiplies the window's biases.
-    auto window_ends = [&](const Part& t, int st) { return !C::kOwn && (((st - t.s0) & (kSumWindow - 1)) == kSumWindow - 1 || st + 1 == t.s1); };
+    // A turn is up to kTurn groups of a stage, each into an accumulator of its own; unless the epilogue adds the biases, one more after the
+    // last group of a window (four stages of a part) multiplies the window's.
+    // What comes after this needs the launch in front; true where a guarded launch is not to run.
+    auto started = [&] {
+        pdl_wait();
+        return dyn_skip(a.dyn);
+    };
+    auto window_ends = [&](const Part& t, int st) { return !C::kFolded && (((st - t.s0) & (kSumWindow - 1)) == kSumWindow - 1 || st + 1 == t.s1); };
     // Weight row (of the tile as the weights arrive) that tensor-memory lane r stands for: gate and up rows of one result 16 lanes apart
     auto tile_row = [](int r) { return MODE == kAffineGateUp ? (r & 16) * 4 + (r >> 5) * 16 + (r & 15) : r; };
     if (warp < kEpilogueWarp) {
@@ -250,7 +261,7 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
         uint32_t stage_scales = 0, stage_full = 0;
         feed_scales<MODE>(a, line, sh.first, sh.u0, sh.u1, lane,
             [&](uint32_t it, const Part& t, int st) {
-                if (it == C::kRawStages) pdl_wait();
+                if (it == C::kRawStages && started()) return false;
                 if (!wait_warp(bar(C::kRawEmpty, rs.i), rs.phase ^ 1u, dead)) return false;
                 if (lane == 0) {
                     arrive_expect_at(bar(C::kRawFull, rs.i), kRawBytes);
@@ -271,12 +282,9 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
     } else if (warp == 1) {
         // ── activations, and their group sums where they were made in front ──
         if (lane == 0) {
-            pdl_wait();
-            const bool skip = dyn_skip(a.dyn);
-            if (skip) sh.dead = 2u;  // a guarded launch that is not to run: the other roles stop at their next wait
             uint32_t it = 0, windows = 0, turn = 0;
             Ring<C::kXStages> xs;
-            bool alive = !skip;
+            bool alive = !started();
             const uint32_t bytes = (uint32_t)line.tile_cols * kLineGroup * 2;
             const int u1 = sh.u1;
             Part t = sh.first;
@@ -299,11 +307,13 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                         xs.next();
                     }
                     if (alive && window_ends(t, st)) {
-                        if (!(alive = wait_one(bar(C::kWindowEmpty), (windows & 1) ^ 1u, dead))) break;
-                        const int first = st - ((st - t.s0) & (kSumWindow - 1));
-                        arrive_expect_at(bar(C::kWindowFull), (uint32_t)line.tile_cols * 128);
-                        tma_load_2d_at(window, &maps.sums, first * 2 * kStageGroups, t.col0, bar(C::kWindowFull));
-                        ++windows;
+                        if (!C::kOwn) {
+                            if (!(alive = wait_one(bar(C::kWindowEmpty), (windows & 1) ^ 1u, dead))) break;
+                            const int first = st - ((st - t.s0) & (kSumWindow - 1));
+                            arrive_expect_at(bar(C::kWindowFull), (uint32_t)line.tile_cols * 128);
+                            tma_load_2d_at(window, &maps.sums, first * 2 * kStageGroups, t.col0, bar(C::kWindowFull));
+                            ++windows;
+                        }
                         ++turn;
                     }
                 }
@@ -319,19 +329,17 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
         const uint32_t shape = (1u << 4) | ((uint32_t)(line.tile_cols >> 3) << 17) | ((uint32_t)(kLineRows >> 4) << 24);  // f32 += f16 x f16, K-major both
         const uint32_t tf32 = shape | (2u << 7) | (2u << 10);
         const uint64_t x_desc = smem_desc_sw128(x_tiles), window_desc = smem_desc_sw128(window);
-        pdl_wait();
         Ring<C::kASlots> as;
         Ring<C::kXStages> xs;
         Ring<C::kSlots> slot;
         Ring<kDone> end;
+        Ring<C::kWindows> ws;
         slot.next(who);
         end.next(who);
-        uint32_t turn = 0, units = 0, windows = 0, last = 0;
-        bool alive = true;
-        auto ready = [&](uint32_t b_full, uint32_t b_phase) {  // all three at once; what is missing is waited for
-            const uint32_t a_full = bar(C::kAFull, as.i), free = bar(C::kAccEmpty, slot.i);
-            const bool b = peek(b_full, b_phase), w = peek(a_full, as.phase), d = peek(free, slot.phase ^ 1u);
-            const bool ok = __all_sync(0xffffffffu, b && w && d) || (wait_warp(b_full, b_phase, dead) && wait_warp(a_full, as.phase, dead) && wait_warp(free, slot.phase ^ 1u, dead));
+        uint32_t turn = 0, units = 0, last = 0, last_window = 2;
+        bool alive = !started();
+        auto ready = [&](uint32_t b_full, uint32_t b_phase) {
+            const bool ok = wait_warp(b_full, b_phase, dead) && wait_warp(bar(C::kAFull, as.i), as.phase, dead) && wait_warp(bar(C::kAccEmpty, slot.i), slot.phase ^ 1u, dead);
             tc_fence_after();
             return ok;
         };
@@ -361,23 +369,24 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                 }
                 if (alive && window_ends(t, st)) {
                     if ((int)(turn & 1) == who) {
-                        if (!(alive = ready(bar(C::kWindowFull), windows & 1))) break;
+                        if (!(alive = ready(bar(C::kWindowFull, ws.i), ws.phase))) break;
                         const int steps = ((st - t.s0) & (kSumWindow - 1)) + 1;
 #pragma unroll 1
-                        for (int i = 0; i < steps; ++i) umma_tf32_step(tmem + slot.i * 128, tmem_a + as.i * 32 + 8 * i, window_desc + 2 * i, tf32, i > 0);
-                        commit_elected(bar(C::kWindowEmpty));
+                        for (int i = 0; i < steps; ++i) umma_tf32_step(tmem + slot.i * 128, tmem_a + as.i * (C::kTurn * 32) + 8 * i, window_desc + ws.i * (C::kWindow / 16) + 2 * i, tf32, i > 0);
+                        commit_elected(bar(C::kWindowEmpty, ws.i));
                         issued();
                     }
+                    last_window = ws.i | ws.phase << 16;  // whichever warp issued it: a barrier's parity tells only its latest phase
                     ++turn;
                     as.next();
-                    ++windows;
+                    ws.next();
                 }
             }
             u += t.s1 - t.s0;
         }
         // the MMAs in flight read shared memory and write tensor memory
         if (units > 0) mbar_poll_bounded(&sh.bars[C::kTurnDone + (last & 0xffff)], last >> 16);
-        if (windows > 0) mbar_poll_bounded(&sh.bars[C::kWindowEmpty], (windows - 1) & 1);
+        if (last_window != 2) mbar_poll_bounded(&sh.bars[C::kWindowEmpty + (last_window & 0xffff)], last_window >> 16);
     }
     } else if (warp < kExpandWarp) {
         registers_up<C::kDrain>();
@@ -390,9 +399,8 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
         Ring<C::kScaleStages> ss;
         Ring<C::kSlots> slot;
         Ring<kDone> end;
-        Ring<C::kOwnSlots> own;
-        pdl_wait();
-        const int u1 = sh.u1;
+        Ring<C::kFoldedSlots> sum;
+        const int u1 = started() ? sh.u0 : sh.u1;
         Part t = sh.first;
 #pragma unroll 1
         for (int u = sh.u0; u < u1; next_part(line, t, u, u1, a.batch)) {
@@ -406,27 +414,27 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
             for (int st = t.s0; st < t.s1 && alive; ++st) {
                 if (!(alive = wait_warp(bar(C::kScaleFull, ss.i), ss.phase, dead))) break;
                 const uint32_t row_scales = scales + ss.i * (2 * kLineRows * 8) + row * 8;
-                const int n = stage_groups(line, st), all = n + window_ends(t, st);
-                uint2 sv = lds64(row_scales), bv = C::kOwn ? lds64(row_scales + kLineRows * 8) : make_uint2(0, 0);
+                const int n = stage_groups(line, st), groups = C::kTurn == kStageGroups ? 1 : (n + C::kTurn - 1) / C::kTurn, all = groups + window_ends(t, st);
+                uint2 sv = lds64(row_scales), bv = C::kFolded ? lds64(row_scales + kLineRows * 8) : make_uint2(0, 0);
 #pragma unroll 1
-                for (int k = 0; k < all; k += C::kTurn) {
+                for (int k = 0; k < all; ++k) {
                     float s1[C::kTurn], b1[C::kTurn];
 #pragma unroll
                     for (int i = 0; i < C::kTurn; ++i) {
                         const float si = __low2float(u32_as_h2(sv.x));
-                        s1[i] = C::kOwn || k < n ? si * kNibble : 1.f;
-                        b1[i] = C::kOwn ? fmaf(8.f, si, __low2float(u32_as_h2(bv.x))) : 0.f;  // the nibbles are centred
+                        s1[i] = C::kFolded || k < groups ? si * kNibble : 1.f;
+                        b1[i] = C::kFolded ? fmaf(8.f, si, __low2float(u32_as_h2(bv.x))) : 0.f;  // the nibbles are centred
                         sv = make_uint2(__funnelshift_r(sv.x, sv.y, 16), sv.y >> 16);
                         bv = make_uint2(__funnelshift_r(bv.x, bv.y, 16), bv.y >> 16);
                     }
-                    const int m = C::kOwn ? min(C::kTurn, n - k) : 1;
-                    if (!(alive = wait_warp(bar(C::kTurnDone, end.i), end.phase, dead) && (!C::kOwn || wait_warp(bar(C::kSumFull, own.i), own.phase, dead)))) break;
+                    const int m = k < groups ? min(C::kTurn, n - k * C::kTurn) : 1;
+                    if (!(alive = wait_warp(bar(C::kTurnDone, end.i), end.phase, dead) && (!C::kFolded || wait_warp(bar(C::kSumFull, sum.i), sum.phase, dead)))) break;
                     tc_fence_after();
                     uint32_t v[4][16];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) tmem_ld16(lane_base + slot.i * 128 + q / kChunks * N + q % kChunks * 16, v[q]);
-                    if constexpr (C::kOwn) {
-                        const uint32_t x_sums = own_sums + own.i * (C::kTurn * N * 4) + from * 4;
+                    if constexpr (C::kFolded) {
+                        const uint32_t x_sums = folded + sum.i * (C::kTurn * N * 4) + from * 4;
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
                             if (q / kChunks < m) {
@@ -448,11 +456,11 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                     __syncwarp();
                     if (lane == 0) {
                         arrive_at(bar(C::kAccEmpty, slot.i));
-                        if (C::kOwn) arrive_at(bar(C::kSumEmpty, own.i));
+                        if (C::kFolded) arrive_at(bar(C::kSumEmpty, sum.i));
                     }
                     slot.next();
                     end.next();
-                    own.next();
+                    sum.next();
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
                         if (q / kChunks < m) {
@@ -461,7 +469,7 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                         }
                 }
                 if (!alive) break;
-                if (C::kOwn) {
+                if (C::kFolded) {
                     if (lane == 0) arrive_at(bar(C::kScaleEmpty, ss.i));
                 } else {
                     ++held;
@@ -591,13 +599,13 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
         // ── expansion: sets of four warps take turns ──
         const int set = (warp - kExpandWarp) >> 2, quad = warp & 3, r = quad * 32 + lane, row = tile_row(r);
         const uint32_t dst = tmem_a + ((uint32_t)(quad * 32) << 16);
-        uint32_t turn = 0, minus = 0xA400A400u;  // -8 x 2^-9
+        uint32_t turn = 0;
         Ring<C::kRawStages> rs;
         Ring<C::kScaleStages> ss;
         Ring<C::kASlots> as;
         bool alive = true;
         auto slot_free = [&] {
-            if (turn >= C::kASlots && turn < C::kASlots + 2) pdl_wait();
+            if (turn >= C::kASlots && turn < C::kASlots + 2 && started()) return false;
             if (turn >= C::kASlots) {
                 const uint32_t last = turn - C::kASlots;
                 if (!wait_warp(bar(C::kTurnDone, last % kDone), (last / kDone) & 1, dead)) return false;
@@ -619,21 +627,31 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
             for (int st = t.s0; st < t.s1 && alive; ++st) {
                 const int n = stage_groups(line, st);
                 const bool mine = C::kTurn < kStageGroups || (int)(turn & 1) == set;
-                if (mine && !(alive = wait_warp(bar(C::kRawFull, rs.i), rs.phase, dead) && (C::kOwn || wait_warp(bar(C::kScaleFull, ss.i), ss.phase, dead)))) break;
+                if (mine && !(alive = wait_warp(bar(C::kRawFull, rs.i), rs.phase, dead) && (C::kFolded || wait_warp(bar(C::kScaleFull, ss.i), ss.phase, dead)))) break;
                 const uint32_t src = raw + rs.i * kRawBytes + row * 128, row_scales = scales + ss.i * (2 * kLineRows * 8) + row * 8;
 #pragma unroll 1
                 for (int k = 0; k < n; k += C::kTurn, ++turn, as.next()) {
                     if ((int)(turn & 1) != set) continue;
-                    if (!C::kOwn) {
-                        bool centred;
-                        tf32_bias(lds_half(row_scales + 2 * k), lds_half(row_scales + kLineRows * 8 + 2 * k), &centred);
-                        minus = centred ? 0xA400A400u : 0u;
+                    uint2 sv = make_uint2(0, 0), bv = make_uint2(0, 0);
+                    if (C::kFolded) {
+                    } else if (C::kTurn == 1) {
+                        sv = make_uint2(lds_u16(row_scales + 2 * k), 0u);
+                        bv = make_uint2(lds_u16(row_scales + kLineRows * 8 + 2 * k), 0u);
+                    } else {
+                        sv = lds64(row_scales);
+                        bv = lds64(row_scales + kLineRows * 8);
+                        if (k > 0) { sv.x = sv.y; bv.x = bv.y; }
                     }
                     if (!(alive = slot_free())) break;
                     const uint32_t to = dst + as.i * (C::kTurn * 32);
                     const int halves = 2 * min(C::kTurn, n - k);
 #pragma unroll 1
                     for (int i = 0; i < halves; i += 2) {  // a group
+                        bool centred = true;  // in fp32 every bias is exact enough
+                        if (!C::kFolded) tf32_bias(__low2float(u32_as_h2(sv.x)), __low2float(u32_as_h2(bv.x)), &centred);
+                        sv = make_uint2(__funnelshift_r(sv.x, sv.y, 16), sv.y >> 16);
+                        bv = make_uint2(__funnelshift_r(bv.x, bv.y, 16), bv.y >> 16);
+                        const uint32_t minus = centred ? 0xA400A400u : 0u;  // -8 x 2^-9
                         const uint4 v0 = lds128(src + (((2 * k + i) ^ (row & 7)) << 4)), v1 = lds128(src + (((2 * k + i + 1) ^ (row & 7)) << 4));
                         uint32_t pair[16], more[16];
                         expand_nibbles(v0.x, minus, pair);
@@ -660,12 +678,17 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                         const uint32_t last = (st - t.s0) & (kSumWindow - 1);
 #pragma unroll 1
                         for (uint32_t i = 0; i <= last; ++i) {
-                            const uint32_t back = last - i, at = scales + (ss.i >= back ? ss.i - back : ss.i + C::kScaleStages - back) * (2 * kLineRows * 8) + row * 8;
+                            const uint32_t back = last - i, stage = ss.i >= back ? ss.i - back : ss.i + C::kScaleStages - back, at = scales + stage * (2 * kLineRows * 8) + row * 8;
                             uint32_t v[8];
                             bool centred;
+                            uint2 sv = lds64(at), bv = lds64(at + kLineRows * 8);
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) v[j] = v[4 + j] = __float_as_uint(tf32_bias(lds_half(at + 2 * j), lds_half(at + kLineRows * 8 + 2 * j), &centred));
-                            tmem_st8(dst + as.i * 32 + 8 * i, v);
+                            for (int j = 0; j < 4; ++j) {
+                                v[j] = v[4 + j] = __float_as_uint(tf32_bias(__low2float(u32_as_h2(sv.x)), __low2float(u32_as_h2(bv.x)), &centred));
+                                sv = make_uint2(__funnelshift_r(sv.x, sv.y, 16), sv.y >> 16);
+                                bv = make_uint2(__funnelshift_r(bv.x, bv.y, 16), bv.y >> 16);
+                            }
+                            tmem_st8(dst + as.i * (C::kTurn * 32) + 8 * i, v);
                         }
                         written();
                     }
@@ -683,22 +706,25 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
         constexpr int kRowWarps = kSumWarps / C::kTurn;  // warps that share a group's rows
         const int i = (warp - kSumWarp) / kRowWarps, col = (warp - kSumWarp) % kRowWarps * 32 + lane;
         Ring<C::kXStages> xs;
-        Ring<C::kOwnSlots> own;
-        bool alive = true;
-        pdl_wait();
+        Ring<C::kWindows> ws;
+        Ring<C::kFoldedSlots> slot;
+        bool alive = !started();
         const int u1 = sh.u1;
         Part t = sh.first;
 #pragma unroll 1
         for (int u = sh.u0; u < u1 && alive; next_part(line, t, u, u1, a.batch)) {
 #pragma unroll 1
             for (int st = t.s0; st < t.s1 && alive; ++st) {
-                const int n = stage_groups(line, st);
+                const int n = stage_groups(line, st), at = (st - t.s0) & (kSumWindow - 1);
+                if (!C::kFolded && at == 0 && !(alive = wait_warp(bar(C::kWindowEmpty, ws.i), ws.phase ^ 1u, dead))) break;
+                // where this row's sums of the stage lie: hi of four groups and lo of four, 16 bytes each, swizzled as the MMA reads them
+                const uint32_t row_at = window + ws.i * C::kWindow + col * 128, hi_at = row_at + ((2 * at ^ (col & 7)) << 4), lo_at = row_at + (((2 * at + 1) ^ (col & 7)) << 4);
 #pragma unroll 1
                 for (int k = 0; k < n; k += C::kTurn) {
                     if (!(alive = wait_warp(bar(C::kXFull, xs.i), xs.phase, dead))) break;
-                    uint64_t sum[4] = {0, 0, 0, 0};
-                    const bool valid = k + i < n && col < line.tile_cols;
-                    if (valid) {
+                    float total = 0.f;
+                    if (k + i < n && col < line.tile_cols) {
+                        uint64_t sum[4] = {0, 0, 0, 0};
                         const uint32_t src = x_tiles + (C::kTurn * xs.i + i) * C::kXBytes + col * 128;
 #pragma unroll 2
                         for (int c = 0; c < 8; ++c) {
@@ -710,16 +736,34 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                                 sum[j] = add2(sum[j], pack2(f.x, f.y));
                             }
                         }
+                        const float2 f = unpack2(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])));
+                        total = f.x + f.y;
                     }
                     __syncwarp();
                     if (lane == 0) arrive_at(bar(C::kXEmpty, xs.i));
-                    if (!(alive = wait_warp(bar(C::kSumEmpty, own.i), own.phase ^ 1u, dead))) break;
-                    const float2 f = unpack2(add2(add2(sum[0], sum[1]), add2(sum[2], sum[3])));
-                    if (valid) sh.own_sums[own.i][i][col] = f.x + f.y;
-                    __syncwarp();
-                    if (lane == 0) arrive_at(bar(C::kSumFull, own.i));
+                    if (C::kFolded) {
+                        if (!(alive = wait_warp(bar(C::kSumEmpty, slot.i), slot.phase ^ 1u, dead))) break;
+                        sts_word(folded + slot.i * (C::kTurn * N * 4) + (i * N + col) * 4, total);
+                        __syncwarp();
+                        if (lane == 0) arrive_at(bar(C::kSumFull, slot.i));
+                        slot.next();
+                        xs.next();
+                        continue;
+                    }
+                    const float hi = tf32_of(total), lo = tf32_of(total - hi);
+                    sts_word(hi_at + 4 * (k + i), hi);
+                    sts_word(lo_at + 4 * (k + i), lo);
+                    if (C::kTurn < kStageGroups && n <= C::kTurn) {  // the groups of a short stage that no turn has
+                        sts_word(hi_at + 4 * (C::kTurn + i), 0.f);
+                        sts_word(lo_at + 4 * (C::kTurn + i), 0.f);
+                    }
                     xs.next();
-                    own.next();
+                }
+                if (alive && window_ends(t, st)) {
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0) arrive_at(bar(C::kWindowFull, ws.i));
+                    ws.next();
                 }
             }
             u += t.s1 - t.s0;

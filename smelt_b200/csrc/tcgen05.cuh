@@ -46,10 +46,11 @@ __device__ __forceinline__ bool wait_alive(uint64_t* bar, uint32_t parity, volat
     *dead = 1u;
     return false;
 }
-// Waits for a phase up to 64 times; each time the thread is suspended in hardware for a while (a spinning warp would take issue slots from
-// the warps that share its scheduler).  Without the instruction's time hint: with it the compiler makes a timed loop around every
-// wait, a third of the instructions that the affine product issued (the 16-bit product, whose waits are few, is 1 % faster with it).
-__device__ __forceinline__ bool mbar_tries(uint32_t bar, uint32_t parity) {
+// Waits for a phase; gives up after 2^23 tries, each of which suspends the thread in hardware for 0.1 us or so (a spinning warp would take
+// issue slots from the warps that share its scheduler).  As little code as that takes, for kernels whose roles compete for the
+// instruction cache: without the instruction's time hint, with which the compiler makes a timed loop around every wait (the 16-bit product, whose
+// waits are few, is 1 % faster with it), and without a look at a clock or at other roles.
+__device__ __forceinline__ bool mbar_wait_short(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
@@ -58,7 +59,7 @@ __device__ __forceinline__ bool mbar_tries(uint32_t bar, uint32_t parity) {
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "@p bra through_%=;\n\t"
         "add.u32 n, n, 1;\n\t"
-        "setp.lt.u32 q, n, 64;\n\t"
+        "setp.lt.u32 q, n, 8388608;\n\t"
         "@q bra again_%=;\n"
         "through_%=:\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
@@ -67,12 +68,6 @@ __device__ __forceinline__ bool mbar_tries(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ uint64_t now_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-constexpr uint64_t kWaitNs = 1000000000ull;  // a wait gives up after a second and reports it instead of waiting forever
 // A shared-memory address that stays in a register: left to itself the compiler makes it again from the CTA's number at every use.
 __device__ __forceinline__ uint32_t kept(uint32_t address) {
     uint32_t a;
