@@ -140,19 +140,22 @@ struct RowNormArgs {
     int group_rows, group_stride;  // rows come in groups of group_rows adjacent rows, group_stride values apart (0: all rows adjacent)
 };
 
-__global__ void __launch_bounds__(32) row_norm_kernel(const RowNormArgs a, DevDyn dyn) {
+// A row by up to eight warps, each of which stands for some of the threadgroup's simdgroups in turn; every warp then adds the simdgroups' sums in
+// the threadgroup's order.  Rows of 2048, 300 of them: 27.8 us with one warp a row, 6 with eight.
+constexpr int kRowNormWarps = 8;
+__global__ void __launch_bounds__(kRowNormWarps * 32) row_norm_kernel(const RowNormArgs a, DevDyn dyn) {
+    __shared__ float parts[32];
     pdl_trigger();
     pdl_wait();
     if (dyn_skip(dyn)) return;
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, groups = a.tgs / 32;
     const size_t off = a.group_rows ? (size_t)(blockIdx.x / a.group_rows) * a.group_stride + (size_t)(blockIdx.x % a.group_rows) * a.dim : (size_t)blockIdx.x * a.dim;
     const __half* x = a.x + off;
     auto val = [&](int i) -> float {
         if (a.pre) return __half2float(__hadd(x[i], a.pre[off + i]));
         return __half2float(x[i]);
     };
-    float total = 0.0f, mine = 0.0f;
-    for (int s = 0; s < a.tgs / 32; ++s) {
+    for (int s = warp; s < groups; s += warps) {
         const int t = 32 * s + lane;
         float p = 0.0f;
         if (a.topology == 0) {
@@ -173,21 +176,22 @@ __global__ void __launch_bounds__(32) row_norm_kernel(const RowNormArgs a, DevDy
         } else {
             for (int i = t; i < a.dim; i += a.tgs) { const float v = val(i); p = __fadd_rn(p, __fmul_rn(v, v)); }
         }
-        const float part = __shfl_sync(0xffffffffu, simd_sum_lane0(p), 0);
-        if (a.topology == 0) { if (lane == s) mine = part; }
-        else total = __fadd_rn(total, part);
+        const float part = simd_sum_lane0(p);
+        if (lane == 0) parts[s] = part;
     }
-    if (a.topology == 0) total = __shfl_sync(0xffffffffu, simd_sum_lane0(mine), 0);
+    __syncthreads();
+    float total = 0.0f;
+    if (a.topology == 0) total = __shfl_sync(0xffffffffu, simd_sum_lane0(lane < groups ? parts[lane] : 0.0f), 0);
+    else for (int s = 0; s < groups; ++s) total = __fadd_rn(total, parts[s]);
     const float rs = a.scale == 0 ? __frcp_rn(__fsqrt_rn(__fadd_rn(__fdiv_rn(total, (float)a.dim), a.eps))) : __frcp_rn(fmaxf(__fsqrt_rn(total), a.eps));
-    if (lane == 0 && a.scale_out) a.scale_out[blockIdx.x] = rs;
+    if (threadIdx.x == 0 && a.scale_out) a.scale_out[blockIdx.x] = rs;
     if (a.value == 0) {
         if (a.pre && a.y)
-            for (int i = lane; i < a.dim; i += 32) a.y[off + i] = __hadd(x[i], a.pre[off + i]);
+            for (int i = threadIdx.x; i < a.dim; i += blockDim.x) a.y[off + i] = __hadd(x[i], a.pre[off + i]);
         return;
     }
-    // in place is allowed: position i is read and written by the same lane, after the whole row was summed
-    __syncwarp();
-    for (int i = lane; i < a.dim; i += 32) {
+    // in place is allowed: position i is read and written by the same thread, after the whole row was summed
+    for (int i = threadIdx.x; i < a.dim; i += blockDim.x) {
         const float v = val(i);
         const float wv = a.w ? __half2float(a.w[i]) : 0.0f;
         __half o;
@@ -279,7 +283,7 @@ cudaError_t launch_row_norm(const Launch& l, const __half* x, const __half* pre,
     RowNormArgs a = {x, pre, w, residual, scalar, y, scale_out, dim, tgs, topology, value, scale, eps, group_rows, group_stride};
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    cfg_launch(l, cfg, attr, dim3(rows), dim3(32));
+    cfg_launch(l, cfg, attr, dim3(rows), dim3((tgs / 32 < kRowNormWarps ? tgs / 32 : kRowNormWarps) * 32));
     prefer_max_shared(row_norm_kernel);
     return cudaLaunchKernelEx(&cfg, row_norm_kernel, a, dev_dyn(l));
 }
