@@ -71,9 +71,10 @@ template <int BN, int MODE, int ACT, bool EXPERTS>
 __global__ void __launch_bounds__(kGemmThreads, 1) gemm_16bit_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const DenseGemmArgs a,
                                                                     const GemmPlan plan) {
     constexpr int kStages = gemm_stages(BN);
-    constexpr uint32_t kStageBytes = gemm_stage_bytes(BN), kTmemCols = 2 * BN < 32 ? 32 : 2 * BN;
+    constexpr bool kSums = MODE == kDenseStoreF16;  // an accumulator holds one column block, and a turn is some of them side by side
+    constexpr int kTurn = !kSums ? 1 : BN <= 64 ? 4 : BN == 128 ? 2 : 1;
+    constexpr uint32_t kStageBytes = gemm_stage_bytes(BN), kTmemCols = 2 * kTurn * BN < 32 ? 32 : 2 * kTurn * BN;
     constexpr int kChunk = BN < 32 ? BN : 32;
-    constexpr bool kSums = MODE == kDenseStoreF16;  // an accumulator holds one column block
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2];
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_16bit_kernel(const __gri
             if (!EXPERTS) pdl_wait();  // a launch in front may take longer than a wait may
             constexpr uint32_t kType = MODE == kDenseStoreF16 ? 0u : (1u << 7) | (1u << 10);  // fp16 or bf16, both operands
             constexpr uint32_t idesc = (1u << 4) | kType | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBlockRows >> 4) << 24);  // fp32 sums, K-major both
-            uint32_t it = 0, done = 0;
+            uint32_t it = 0, done = 0, turns = 0;
             bool alive = true;
             for (int u = blockIdx.x; u < units && alive; u += gridDim.x, ++done) {
                 const Unit t = unit_at(u);
@@ -170,8 +171,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_16bit_kernel(const __gri
                 tc_fence_after();
                 for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
                     const uint32_t s = it % kStages;
-                    if (kSums) {
-                        buf = it & 1; use = it >> 1;
+                    const int block = kSums ? (kb - t.kb0) % kTurn : 0;
+                    if (kSums && block == 0) {
+                        buf = turns & 1; use = turns >> 1;
                         if (use > 0 && !(alive = wait_alive(&acc_empty[buf], (use - 1) & 1, dead))) break;
                     }
                     if (!(alive = wait_alive(&full[s], (it / kStages) & 1, dead))) break;
@@ -179,9 +181,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_16bit_kernel(const __gri
                     const uint32_t w = smem_u32(smem + s * kStageBytes), x = w + kATile;
 #pragma unroll
                     for (int k = 0; k < kBlockCols / 16; ++k)
-                        umma_f16(tmem + buf * BN, smem_desc_sw128(w + k * 32), smem_desc_sw128(x + k * 32), idesc, ((!kSums && kb != t.kb0) || k != 0) ? 1u : 0u);
+                        umma_f16(tmem + (buf * kTurn + block) * BN, smem_desc_sw128(w + k * 32), smem_desc_sw128(x + k * 32), idesc, ((!kSums && kb != t.kb0) || k != 0) ? 1u : 0u);
                     umma_commit(&empty[s]);
-                    if (kSums) umma_commit(&acc_full[buf]);
+                    if (kSums && (block == kTurn - 1 || kb + 1 == t.kb1)) {
+                        umma_commit(&acc_full[buf]);
+                        ++turns;
+                    }
                 }
                 if (!kSums && alive) umma_commit(&acc_full[buf]);
             }
@@ -202,22 +207,28 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_16bit_kernel(const __gri
             if constexpr (kSums) {
 #pragma unroll
                 for (int j = 0; j < BN; ++j) sums[j] = 0.f;
-                for (int kb = t.kb0; kb < t.kb1; ++kb, ++done) {
+                for (int kb = t.kb0; kb < t.kb1; kb += kTurn, ++done) {
                     const uint32_t b = done & 1;
+                    const int n = min(kTurn, t.kb1 - kb);
                     if (!(alive = __all_sync(0xffffffffu, wait_alive(&acc_full[b], (done >> 1) & 1, dead)))) break;
                     tc_fence_after();
 #pragma unroll
                     for (int c0 = 0; c0 < BN; c0 += 16) {
-                        uint32_t v[16];
-                        tmem_ld16(lane_base + b * BN + c0, v);
-                        tmem_wait_ld16(v);
+                        uint32_t v[kTurn][16];
+#pragma unroll
+                        for (int i = 0; i < kTurn; ++i) tmem_ld16(lane_base + (b * kTurn + i) * BN + c0, v[i]);
+#pragma unroll
+                        for (int i = 0; i < kTurn; ++i) tmem_wait_ld16(v[i]);
                         if (c0 + 16 >= BN) {
                             tc_fence_before();
                             __syncwarp();
                             if (lane == 0) mbar_arrive(&acc_empty[b]);
                         }
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) sums[c0 + j] += __uint_as_float(v[j]);
+                        for (int i = 0; i < kTurn; ++i)
+                            if (i < n)
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) sums[c0 + j] += __uint_as_float(v[i][j]);
                     }
                 }
                 --done;
