@@ -116,8 +116,6 @@ __device__ __forceinline__ bool wait_one(uint32_t bar, uint32_t parity, uint32_t
     return ok;
 }
 __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, uint32_t dead) { return __all_sync(0xffffffffu, wait_one(bar, parity, dead)); }
-// A value that is the same in all lanes, where the compiler can see it: what follows from it stays in uniform registers.
-__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 __device__ __forceinline__ Part uniform(const Part& t) {
     return {uniform(t.tile), uniform(t.s0), uniform(t.s1), uniform(t.row_tile), uniform(t.col_tile), uniform(t.col0), uniform(t.live)};
 }

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_16bit_kernel(const __gri
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t s_tmem, s_dead, s_ticket, s_go;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
     const int kblocks = a.cols / kBlockCols;
 
     pdl_trigger();
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_16bit_kernel(const __gri
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = (uint32_t)uniform((int)s_tmem);
     volatile uint32_t* dead = &s_dead;
 
     int units = plan.units;
@@ -158,41 +158,40 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_16bit_kernel(const __gri
             for (uint32_t i = it > kStages ? it - kStages : 0; i < it; ++i) mbar_poll_bounded(&full[i % kStages], (i / kStages) & 1);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            if (!EXPERTS) pdl_wait();  // a launch in front may take longer than a wait may
-            constexpr uint32_t kType = MODE == kDenseStoreF16 ? 0u : (1u << 7) | (1u << 10);  // fp16 or bf16, both operands
-            constexpr uint32_t idesc = (1u << 4) | kType | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBlockRows >> 4) << 24);  // fp32 sums, K-major both
-            uint32_t it = 0, done = 0, turns = 0;
-            bool alive = true;
-            for (int u = blockIdx.x; u < units && alive; u += gridDim.x, ++done) {
-                const Unit t = unit_at(u);
-                uint32_t buf = done & 1, use = done >> 1;
-                if (!kSums && use > 0 && !(alive = wait_alive(&acc_empty[buf], (use - 1) & 1, dead))) break;
-                tc_fence_after();
-                for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
-                    const uint32_t s = it % kStages;
-                    const int block = kSums ? (kb - t.kb0) % kTurn : 0;
-                    if (kSums && block == 0) {
-                        buf = turns & 1; use = turns >> 1;
-                        if (use > 0 && !(alive = wait_alive(&acc_empty[buf], (use - 1) & 1, dead))) break;
-                    }
-                    if (!(alive = wait_alive(&full[s], (it / kStages) & 1, dead))) break;
-                    tc_fence_after();
-                    const uint32_t w = smem_u32(smem + s * kStageBytes), x = w + kATile;
-#pragma unroll
-                    for (int k = 0; k < kBlockCols / 16; ++k)
-                        umma_f16(tmem + (buf * kTurn + block) * BN, smem_desc_sw128(w + k * 32), smem_desc_sw128(x + k * 32), idesc, ((!kSums && kb != t.kb0) || k != 0) ? 1u : 0u);
-                    umma_commit(&empty[s]);
-                    if (kSums && (block == kTurn - 1 || kb + 1 == t.kb1)) {
-                        umma_commit(&acc_full[buf]);
-                        ++turns;
-                    }
+        if (!EXPERTS) pdl_wait();  // a launch in front may take longer than a wait may
+        constexpr uint32_t kType = MODE == kDenseStoreF16 ? 0u : (1u << 7) | (1u << 10);  // fp16 or bf16, both operands
+        constexpr uint32_t idesc = (1u << 4) | kType | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kBlockRows >> 4) << 24);  // fp32 sums, K-major both
+        const uint64_t w_desc = smem_desc_sw128(smem_u32(smem)), x_desc = smem_desc_sw128(smem_u32(smem) + kATile);
+        auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, wait_alive(bar, parity, dead)); };
+        uint32_t it = 0, done = 0, turns = 0, s = 0, phase = 0;  // s, phase: the stage and the parity of its use
+        bool alive = true;
+        for (int u = blockIdx.x; u < units && alive; u += gridDim.x, ++done) {
+            const Unit t = unit_at(u);
+            const int blocks = uniform(t.kb1 - t.kb0);
+            uint32_t buf = done & 1, use = done >> 1;
+            if (!kSums && use > 0 && !(alive = wait(&acc_empty[buf], (use - 1) & 1))) break;
+            tc_fence_after();
+#pragma unroll 1
+            for (int k = 0; k < blocks; ++k, ++it) {
+                const int block = kSums ? k % kTurn : 0;
+                if (kSums && block == 0) {
+                    buf = turns & 1; use = turns >> 1;
+                    if (use > 0 && !(alive = wait(&acc_empty[buf], (use - 1) & 1))) break;
                 }
-                if (!kSums && alive) umma_commit(&acc_full[buf]);
+                if (!(alive = wait(&full[s], phase))) break;
+                tc_fence_after();
+                umma_f16_block(tmem + (buf * kTurn + block) * BN, w_desc + s * (kStageBytes / 16), x_desc + s * (kStageBytes / 16), idesc, !kSums && k != 0 ? 1u : 0u);
+                commit_elected(smem_u32(&empty[s]));
+                if (kSums && (block == kTurn - 1 || k + 1 == blocks)) {
+                    commit_elected(smem_u32(&acc_full[buf]));
+                    ++turns;
+                }
+                if (++s == kStages) { s = 0; phase ^= 1u; }
             }
-            // MMAs in flight read shared memory and write tensor memory: wait for the last stage they were given
-            if (it > 0) mbar_poll_bounded(&empty[(it - 1) % kStages], ((it - 1) / kStages) & 1);
+            if (!kSums && alive) commit_elected(smem_u32(&acc_full[buf]));
         }
+        // MMAs in flight read shared memory and write tensor memory: wait for the last stage they were given
+        if (it > 0) mbar_poll_bounded(&empty[(it - 1) % kStages], ((it - 1) / kStages) & 1);
     } else {
         if (!EXPERTS) pdl_wait();
         const int quad = warp & 3, et = tid - 64;
