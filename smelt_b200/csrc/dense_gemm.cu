@@ -4,7 +4,7 @@
 // the chunk's positions its N (16 .. 256 per tile), so a tile's output is transposed on the way out:
 // tensor-memory lane r is weight row r, and a warp stores 32 adjacent rows of one position at a
 // time.  Warp 0 brings both operands with TMA (64 columns = one 128-byte swizzled row per stage,
-// rows past the matrix or the chunk read as zero); one lane of warp 1 issues the MMAs; warps 2-5
+// rows past the matrix or the chunk read as zero); warp 1 issues the MMAs; warps 2-5
 // read the accumulator of the previous tile meanwhile (two accumulators in tensor memory).  CTAs
 // are persistent, one per SM; neighbouring units share their weight tile.  A matrix with few
 // tiles splits its columns: every part leaves fp32 sums in scratch and the last one to finish
@@ -16,6 +16,9 @@
 // sums taken out of tensor memory and added in fp32 registers: the tensor core truncates each sum it adds to, and over all of K
 // that moved 1.7 % of the logits of 4096 columns to another fp16 value than the correctly rounded one; so 0.1 % are, as many as
 // of the fused multiply-adds that one sequence takes.
+// The issuing warp runs its loop as a whole and an elected lane issues a block of 64 columns as one sequence; four blocks (two of
+// 128 positions) lie side by side in tensor memory and change hands together.  151936 x 4096 (us): 16 positions 308 with one lane
+// that builds descriptors and a hand-over a block, 264 with four blocks a hand-over, 200 issued so (floor 193); 64 positions 330, 280, 212.
 //
 // Every wait is bounded: on expiry the CTA raises bit 11 of the device error word, its roles stop,
 // copies and MMAs in flight are waited for (bounded too) and the tensor memory is freed.

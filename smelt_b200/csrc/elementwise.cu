@@ -141,7 +141,7 @@ struct RowNormArgs {
 };
 
 // A row by up to eight warps, each of which stands for some of the threadgroup's simdgroups in turn; every warp then adds the simdgroups' sums in
-// the threadgroup's order.  Rows of 2048, 300 of them: 27.8 us with one warp a row, 6 with eight.
+// the threadgroup's order.  Rows of 2048, 300 of them: 27.8 us with one warp a row, 7.8 with eight (a launch alone).
 constexpr int kRowNormWarps = 8;
 __global__ void __launch_bounds__(kRowNormWarps * 32) row_norm_kernel(const RowNormArgs a, DevDyn dyn) {
     __shared__ float parts[32];

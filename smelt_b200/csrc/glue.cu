@@ -481,8 +481,8 @@ cudaError_t launch_fp16_matvec(const Launch& l, const __half* w, const __half* x
     if (cols % 8 != 0 || batch <= 0) return cudaErrorInvalidValue;
     if (std::min(batch, 8) * (size_t)cols * 2 > 200 * 1024) return cudaErrorInvalidValue;
     // Several rows: one row of weights for all of them on the tensor cores, where a warp per row spends its time on two conversions
-    // and eight FMAs per weight and row of x, once per eight rows (us: 151936 x 4096, 2 rows 391 -> 304, 8 rows 880 -> 305, 32 rows
-    // 3520 -> 308; 32768 x 2048, 2 rows 54.6 -> 37.9; 4096 x 4096, 2 rows 15.2 -> 13.5, 8 rows 39.0 -> 13.5; 128 x 4096, columns split
+    // and eight FMAs per weight and row of x, once per eight rows (us: 151936 x 4096, 2 rows 391 -> 198, 8 rows 880 -> 201, 32 rows
+    // 3520 -> 204; 32768 x 2048, 2 rows 54.6 -> 24.4; 4096 x 4096, 2 rows 15.2 -> 10.1, 8 rows 39.0 -> 10.1; 128 x 4096, columns split
     // over 16 CTAs, 2 rows 7.4 -> 7.8, 3 rows 8.7 -> 7.8, 8 rows 13.9 -> 7.8; 8 x 2048, 4 rows 5.6 -> 6.8, 8 rows 7.7 -> 6.8).  A single
     // tile of 128 rows of weights is worth it from 12288 activations on, more of them from 2048 columns, from 4096 rows with 4096
     // activations (4096 x 512, 4 rows 5.8 : 6.1, 8 rows 7.4 : 6.2; 1000 x 512, 8 rows 5.3 : 6.1) and with many rows (32768 x 64, 2 rows
