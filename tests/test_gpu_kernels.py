@@ -439,6 +439,19 @@ def test_rmsnorm_affine_gate_up_swiglu(ctx, oracle, rows, cols, batch):
     assert np.array_equal(y.download(np.uint16, (batch, rows)), y2.download(np.uint16, (batch, rows)))
 
 
+# from nine rows on the norm is a launch of its own in front of the tensor-core product
+@pytest.mark.parametrize("rows,cols,batch", [(136, 1024, 9), (200, 2048, 17), (264, 1024, 64)])
+def test_rmsnorm_affine_gate_up_swiglu_many_rows(ctx, oracle, rows, cols, batch):
+    gate, up = (synth.affine_u4(39, n, rows, cols, 64) for n in ("gate", "up"))
+    x, nw = synth.activations(39, "x", batch, cols), synth.normal_f16(39, "norm", (cols,), 0.1)
+    d = dev(ctx, *gate, *up, x, nw)
+    y = ctx.alloc(batch * rows * 2)
+    ctx.call("rmsnorm_affine_gate_up_swiglu", *d, C.c_float(1e-6), y, rows, cols, 64, batch)
+    xn, _ = _device_norm(ctx, x, nw, 1e-6)
+    ref = oracle.affine_gate_up_swiglu(*gate, *up, xn, rows, cols, 64, round_gate_up=False)
+    assert rel_err(y.download(np.float16, (batch, rows)), ref) < REL_TOL and ctx.device_error() == 0
+
+
 @pytest.mark.parametrize("position,layout", [(0, 1), (77, 1), (4095, 0), (32767, 1)])
 def test_rope_qkv_append_is_the_three_kernels(ctx, oracle, position, layout):
     nq, nkv, d, cap = 8, 2, 128, 32768
