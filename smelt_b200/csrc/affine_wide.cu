@@ -60,6 +60,35 @@ struct Ring {
     }
 };
 
+// Whether a wait of an issuing warp can be taken for one of an earlier use of its barrier: a parity tells a phase only from the one next to it, and
+// each of the two warps waits on its own turns, every second one, only.  When a warp comes to turn t it knows of a use in turn `before` if that
+// was its own, or if the accumulator of its turn in front, t - 2, was only free once that turn had been drained.  Walks tiles of rows of up to 20
+// groups from every stage on, short last stages among them.
+constexpr bool issue_waits_hold(int turn_groups, int slots, int x_stages, int a_slots, int windows, bool folded) {
+    for (int groups = 1; groups <= 20; ++groups) {
+        const int stages = (groups + kStageGroups - 1) / kStageGroups;
+        for (int first = 0; first < stages; ++first) {
+            int x_used[8] = {}, a_used[8] = {}, window_used[4] = {};  // turn + 1 of a position's latest use
+            int t = 0, x = 0, window = 0;
+            auto known = [&](int before) { return before == 0 || ((before - 1) ^ t) % 2 == 0 || before - 1 <= t - 2 - slots; };
+            for (int tile = 0; tile < 4; ++tile)
+                for (int st = tile ? 0 : first, held = 1; st < stages; ++st, ++held) {
+                    const int n = groups - st * kStageGroups < kStageGroups ? groups - st * kStageGroups : kStageGroups;
+                    for (int k = 0; k < n; k += turn_groups, ++t, ++x) {
+                        if (!known(x_used[x % x_stages]) || !known(a_used[t % a_slots])) return false;
+                        x_used[x % x_stages] = a_used[t % a_slots] = t + 1;
+                    }
+                    if (folded || (held % kSumWindow != 0 && st + 1 != stages)) continue;
+                    if (!known(window_used[window % windows]) || !known(a_used[t % a_slots])) return false;
+                    window_used[window % windows] = a_used[t % a_slots] = t + 1;
+                    ++window;
+                    ++t;
+                }
+        }
+    }
+    return true;
+}
+
 template <int N>
 struct WideCfg {
     static constexpr bool kOwn = N <= kOwnCols;    // the CTA sums x itself
@@ -72,12 +101,15 @@ struct WideCfg {
     static constexpr int kASlots = kOwn ? 256 / (32 * kTurn) : 4, kACol = kSlots * 128;
     static constexpr int kXBytes = N * kLineGroup * 2, kXStages = N == 128 ? 5 : 4, kRawStages = N == 128 ? 4 : 6;  // a stage of x is a turn's
     static constexpr int kScaleStages = kFolded ? 8 : 12;
-    static constexpr int kWindows = kOwn ? 2 : 1, kWindow = kFolded ? 0 : N * 128;  // group sums of kSumWindow stages
+    // Group sums of kSumWindow stages.  Two: with one, a window of one short last stage begins three turns after the window in front, which
+    // the other issuing warp took and this one has not seen arrive.
+    static constexpr int kWindows = 2, kWindow = kFolded ? 0 : N * 128;
     static constexpr int kFoldedSlots = 4;                                // turns whose sums are kept for the epilogue
     static constexpr uint32_t kSmem = kRawStages * kRawBytes + kXStages * kTurn * kXBytes + kWindows * kWindow + 1024;
     static_assert(kSmem + 28 * 1024 <= 227u * 1024u, "shared memory");
     static_assert(kACol + kASlots * kTurn * 32 <= 512 && kTurn * N <= 128, "tensor memory");
     static_assert(kScaleStages >= 2 * kSumWindow, "the biases of a window wait for it");
+    static_assert(issue_waits_hold(kTurn, kSlots, kXStages, kASlots, kWindows, kFolded), "an issuing warp could take a barrier's earlier use for this one");
     // Barriers, by the address of the first one of a kind.
     static constexpr int kRawFull = 0, kRawEmpty = kRawFull + kRawStages, kScaleFull = kRawEmpty + kRawStages, kScaleEmpty = kScaleFull + kScaleStages, kXFull = kScaleEmpty + kScaleStages,
                          kXEmpty = kXFull + kXStages, kAFull = kXEmpty + kXStages, kTurnDone = kAFull + kASlots, kAccEmpty = kTurnDone + kDone, kWindowFull = kAccEmpty + kSlots,
@@ -277,6 +309,7 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
         if (lane == 0) {
             uint32_t it = 0, windows = 0, turn = 0;
             Ring<C::kXStages> xs;
+            Ring<C::kWindows> ws;
             bool alive = !started();
             const uint32_t bytes = (uint32_t)line.tile_cols * kLineGroup * 2;
             const int u1 = sh.u1;
@@ -301,10 +334,11 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                     }
                     if (alive && window_ends(t, st)) {
                         if (!C::kOwn) {
-                            if (!(alive = wait_one(bar(C::kWindowEmpty), (windows & 1) ^ 1u, dead))) break;
+                            if (!(alive = wait_one(bar(C::kWindowEmpty, ws.i), ws.phase ^ 1u, dead))) break;
                             const int first = st - ((st - t.s0) & (kSumWindow - 1));
-                            arrive_expect_at(bar(C::kWindowFull), (uint32_t)line.tile_cols * 128);
-                            tma_load_2d_at(window, &maps.sums, first * 2 * kStageGroups, t.col0, bar(C::kWindowFull));
+                            arrive_expect_at(bar(C::kWindowFull, ws.i), (uint32_t)line.tile_cols * 128);
+                            tma_load_2d_at(window + ws.i * C::kWindow, &maps.sums, first * 2 * kStageGroups, t.col0, bar(C::kWindowFull, ws.i));
+                            ws.next();
                             ++windows;
                         }
                         ++turn;
@@ -314,7 +348,8 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
             }
 #pragma unroll 1
             for (uint32_t i = it > C::kXStages ? it - C::kXStages : 0; i < it; ++i) mbar_poll_bounded(&sh.bars[C::kXFull + i % C::kXStages], (i / C::kXStages) & 1);
-            if (windows > 0) mbar_poll_bounded(&sh.bars[C::kWindowFull], (windows - 1) & 1);
+#pragma unroll 1
+            for (uint32_t i = windows > C::kWindows ? windows - C::kWindows : 0; i < windows; ++i) mbar_poll_bounded(&sh.bars[C::kWindowFull + i % C::kWindows], (i / C::kWindows) & 1);
         }
     } else {
         // ── issue: two warps, each every second turn; a warp's chain from one turn to the next is longer than the MMAs ──

@@ -251,6 +251,27 @@ def test_affine_wide_one_sided_groups(ctx, rows, cols, batch):
         buf.free()
 
 
+# beyond 64 rows of x, where the last group sums of a row belong to a stage of two groups and the turns that multiply them come closest:
+# several such rows a CTA, also with nothing else in them; the bound is that of test_affine_wide_rounds_like_exact_sums
+@pytest.mark.parametrize("rows,cols,batch", [(2048, 1152, 128), (40000, 128, 65), (4104, 640, 300)])
+def test_affine_wide_short_last_stage(ctx, rows, cols, batch):
+    w, s, b = synth.affine_u4(38, "sw", rows, cols, 64)
+    x = (synth.activations(38, "sx", batch, cols).astype(np.float32) + 0.5).astype(np.float16)  # so that the group sums tell
+    d = dev(ctx, w, s, b, x)
+    y = ctx.alloc(batch * rows * 2)
+    ctx.call("affine_matvec", *d, y, rows, cols, 64, batch)
+    first = y.download(np.uint16, (batch, rows))
+    q = np.stack([w & 15, w >> 4], -1).reshape(rows, cols // 64, 64).astype(np.float64)
+    want = x.astype(np.float64) @ (q * s.astype(np.float64)[..., None] + b.astype(np.float64)[..., None]).reshape(rows, cols).T
+    assert np.mean(first.view(np.float16) != want.astype(np.float16)) < 4e-3
+    for _ in range(20):
+        ctx.call("affine_matvec", *d, y, rows, cols, 64, batch)
+        assert np.array_equal(y.download(np.uint16, (batch, rows)), first)
+    assert ctx.device_error() == 0
+    for buf in d + [y]:
+        buf.free()
+
+
 # batch 1 and 2 run on the integer-MMA kernel: every mode, row / K tails, long K, few chunks per warp
 IMMA_SHAPES = [(4096, 4096, 1), (4096, 12288, 1), (100, 128, 2), (48, 256, 1), (1000, 2048, 2), (6144, 4096, 2), (16, 8192, 1)]
 
