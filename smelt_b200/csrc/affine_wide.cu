@@ -8,7 +8,9 @@
 // bias + 8 scale, so that neither sum is much larger than the result.  The tensor core truncates what it adds to, here four
 // K = 16 products at a time.  Share of fp16 results that are not the correctly rounded ones, against two fp16 operands per
 // dequantised weight summed over two groups (before -> now): 4096 x 4096, 32 rows 0.12 -> 0.08 %, 512 rows 0.12 -> 0.08; gate and
-// up 12288 x 4096, 32 rows 0.20 -> 0.15, 512 rows 0.21 -> 0.15.
+// up 12288 x 4096, 32 rows 0.20 -> 0.15, 512 rows 0.21 -> 0.15.  Up to 32 rows the four groups of a turn are added up before they meet the
+// running sum, which rounds once for them: with two roundings a group, 5120 x 17408 had 0.16 % at 8 rows and 0.17 at 32, where the kernels
+// in front have 0.09 and 0.14; now 0.09 and 0.09 (4096 x 12288 + residual, 9 rows: 0.024, in front 0.020, now 0.008).  It costs 1 %.
 //
 // bias * sum(x).  Tiles of up to 64 rows of x: four warps sum x from shared memory.  More: the sums are made once in front
 // (group_sums_kernel), as they would cost every CTA four warps' issue slots.  Tiles of up to 32 rows: the epilogue adds the products in fp32.
@@ -461,40 +463,47 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                     uint32_t v[4][16];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) tmem_ld16(lane_base + slot.i * 128 + q / kChunks * N + q % kChunks * 16, v[q]);
-                    if constexpr (C::kFolded) {
-                        const uint32_t x_sums = folded + sum.i * (C::kTurn * N * 4) + from * 4;
-#pragma unroll
-                        for (int q = 0; q < 4; ++q)
-                            if (q / kChunks < m) {
-                                const float b = b1[q / kChunks];
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const uint4 xs = lds128(x_sums + q / kChunks * (N * 4) + q % kChunks * 64 + 16 * j);
-                                    float* to = sums + q % kChunks * 16 + 4 * j;
-                                    to[0] = fmaf(__uint_as_float(xs.x), b, to[0]);
-                                    to[1] = fmaf(__uint_as_float(xs.y), b, to[1]);
-                                    to[2] = fmaf(__uint_as_float(xs.z), b, to[2]);
-                                    to[3] = fmaf(__uint_as_float(xs.w), b, to[3]);
-                                }
-                            }
-                    }
 #pragma unroll
                     for (int q = 0; q < 4; ++q) tmem_wait_ld16(v[q]);
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) {
-                        arrive_at(bar(C::kAccEmpty, slot.i));
-                        if (C::kFolded) arrive_at(bar(C::kSumEmpty, sum.i));
-                    }
+                    if (lane == 0) arrive_at(bar(C::kAccEmpty, slot.i));
                     slot.next();
                     end.next();
-                    sum.next();
+                    if constexpr (C::kFolded) {
+                        float part[16];  // of this turn: the running sums, much larger, round once a turn and not twice a group
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (q / kChunks < m) {
+                        for (int q = 0; q < 4; ++q)
+                            if (q < m) {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j) sums[q % kChunks * 16 + j] = fmaf(__uint_as_float(v[q][j]), s1[q / kChunks], sums[q % kChunks * 16 + j]);
-                        }
+                                for (int j = 0; j < 16; ++j) part[j] = q == 0 ? __uint_as_float(v[0][j]) * s1[0] : fmaf(__uint_as_float(v[q][j]), s1[q], part[j]);
+                            }
+                        const uint32_t x_sums = folded + sum.i * (C::kTurn * N * 4) + from * 4;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (q < m) {
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    const uint4 xs = lds128(x_sums + q * (N * 4) + 16 * j);
+                                    part[4 * j] = fmaf(__uint_as_float(xs.x), b1[q], part[4 * j]);
+                                    part[4 * j + 1] = fmaf(__uint_as_float(xs.y), b1[q], part[4 * j + 1]);
+                                    part[4 * j + 2] = fmaf(__uint_as_float(xs.z), b1[q], part[4 * j + 2]);
+                                    part[4 * j + 3] = fmaf(__uint_as_float(xs.w), b1[q], part[4 * j + 3]);
+                                }
+                            }
+                        __syncwarp();
+                        if (lane == 0) arrive_at(bar(C::kSumEmpty, sum.i));
+                        sum.next();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) sums[j] += part[j];
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (q / kChunks < m) {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) sums[q % kChunks * 16 + j] = fmaf(__uint_as_float(v[q][j]), s1[q / kChunks], sums[q % kChunks * 16 + j]);
+                            }
+                    }
                 }
                 if (!alive) break;
                 if (C::kFolded) {

@@ -217,6 +217,23 @@ def test_affine_wide_rounds_like_exact_sums(ctx, rows, cols, batch):
     assert np.mean(y.download(np.float16, (batch, rows)) != want.astype(np.float16)) < 4e-3
 
 
+# As many results as before may be misrounded, whatever the rows of x: 0.1 % where fp16 operands were summed over two groups at a time and
+# the running sums in fp32 rounded once for two groups.  A fp32 sum that rounds twice for each of the 272 groups here has 0.17 %.
+@pytest.mark.parametrize("rows,cols,batch,mean", [(2048, 17408, 32, 0.0)])
+def test_affine_wide_running_sums(ctx, rows, cols, batch, mean):
+    w, s, b = synth.affine_u4_model(40, "mw", rows, cols)
+    x = (synth.activations(40, "mx", batch, cols).astype(np.float32) + mean).astype(np.float16)
+    d = dev(ctx, w, s, b, x)
+    y = ctx.alloc(batch * rows * 2)
+    ctx.call("affine_matvec", *d, y, rows, cols, 64, batch)
+    q = np.stack([w & 15, w >> 4], -1).reshape(rows, cols // 64, 64).astype(np.float64)
+    want = x.astype(np.float64) @ (q * s.astype(np.float64)[..., None] + b.astype(np.float64)[..., None]).reshape(rows, cols).T
+    # 65,000 results and more, of which the 0.1 % are known to within 12 %
+    assert np.mean(y.download(np.float16, (batch, rows)) != want.astype(np.float16)) < 1.3e-3
+    for buf in d + [y]:
+        buf.free()
+
+
 # weights beyond fp16's range, of which the nibble, the scale and the bias are not: they were never rounded to fp16
 @pytest.mark.parametrize("rows,cols,batch", [(72, 1984, 17), (136, 12288, 9), (128, 4096, 64), (264, 576, 130), (200, 512, 300)])
 def test_affine_wide_large_weights(ctx, oracle, rows, cols, batch):
