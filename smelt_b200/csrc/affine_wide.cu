@@ -4,8 +4,8 @@
 // Replaces agent_affine_qmm_fixed_batched_full and its fused gate/up form (Resources/Shaders/agent_affine_qmm.h:107-316,
 // :360-742; wrappers Resources/Shaders/lut_matvec.metal:6519-6545, :6615-6635), in their factored form: per group
 // y += scale * sum(q x) + bias * sum(x).  The tensor core multiplies the nibbles (exact in fp16) by x, one accumulator a group;
-// epilogue warps multiply what they drain by the scale and add it to fp32 registers.  The nibbles are centred (q - 8) and the bias is
-// bias + 8 scale, so that neither sum is much larger than the result.  The tensor core truncates what it adds to, here four
+// epilogue warps multiply what they drain by the scale and add it to fp32 registers.  The nibbles are centred (q - c, c = 8 up to 32 rows) and
+// the bias is bias + c scale, so that neither sum is much larger than the result.  The tensor core truncates what it adds to, here four
 // K = 16 products at a time.  Share of fp16 results that are not the correctly rounded ones, against two fp16 operands per
 // dequantised weight summed over two groups (before -> now): 4096 x 4096, 32 rows 0.12 -> 0.08 %, 512 rows 0.12 -> 0.08; gate and
 // up 12288 x 4096, 32 rows 0.20 -> 0.15, 512 rows 0.21 -> 0.15.  Up to 32 rows the four groups of a turn are added up before they meet the
@@ -15,7 +15,9 @@
 // bias * sum(x).  Tiles of up to 64 rows of x: four warps sum x from shared memory.  More: the sums are made once in front
 // (group_sums_kernel), as they would cost every CTA four warps' issue slots.  Tiles of up to 32 rows: the epilogue adds the products in fp32.
 // More: the sums are kept as two tf32 values each, and the biases of up to sixteen groups multiply them on the tensor core as one
-// more turn; where bias + 8 scale is not exact in tf32 the group's nibbles stay as they are and its bias, which is an fp16, is the operand.
+// more turn; c is chosen for each group, to the nearest eighth, so that these operands are small (tf32_bias).  With c = 8, x of mean 0.5 and biases
+// of -7.5 scales, 0.24 % of the results of 4096 columns were misrounded (before the tensor core had the biases: 0.11 %), now 0.07; it costs
+// 1 to 3 % of the time.
 // (The epilogue's way with 64 rows: 50.2 | 31.0 | 15.2 us of the shapes below; the tensor core's with 32 rows 31.8 | 20.2 | 11.0, a turn
 // more for each of a CTA's short stretches, and a step of 32 sequences 3.88 ms instead of 3.75.)
 //
@@ -167,12 +169,15 @@ __device__ __forceinline__ void tmem_st8(uint32_t t, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(t), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
 }
-// What a group's sum of x is multiplied by when its nibbles go to the tensor core as q - 8: bias + 8 scale, where a tf32 operand holds that
-// exactly (the bias of a row's group whose weights have both signs); else the bias, and the nibbles stay as they are.
-__device__ __forceinline__ float tf32_bias(float s, float b, bool* centred) {
-    const float t = fmaf(8.f, s, b);
-    *centred = (__float_as_uint(t) & 0x1FFFu) == 0u && t - 8.f * s == b;
-    return *centred ? t : b;
+// What a group's sum of x is multiplied by when its nibbles go to the tensor core as q - c: bias + c scale, with c the multiple of 1/8 that makes
+// it smallest.  The tensor core truncates the sum of these products too, over up to sixteen groups, where x has a mean that is far from
+// small beside the result.  q - c is exact in fp16 up to |c| = 240; bias + c scale, at most a sixteenth of the scale, has no more than
+// eleven bits, so that a tf32 operand holds it.  Else (a scale of zero, a bias beyond 240 scales) c is 0.  minus: -c / 512 twice.
+__device__ __forceinline__ float tf32_bias(float s, float b, uint32_t* minus) {
+    const float k = __fadd_rn(__fadd_rn(__fdividef(-8.f * b, s), 12582912.f), -12582912.f), t = fmaf(0.125f * k, s, b);  // nearest whole number
+    const bool centred = fabsf(k) <= 1920.f && (__float_as_uint(t) & 0x1FFFu) == 0u;
+    *minus = centred ? h2_as_u32(__float2half2_rn(k * (-1.f / 4096.f))) : 0u;
+    return centred ? t : b;
 }
 // Eight nibbles -> four pairs of adjacent columns: a byte that holds a nibble is an fp16 of 2^-24 of its value, brought to 2^-9 of it (and
 // centred) by one packed FMA.  (The tensor core takes the subnormals exactly too, but aligns their products by an exponent that is up to ten
@@ -684,11 +689,10 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                     const int halves = 2 * min(C::kTurn, n - k);
 #pragma unroll 1
                     for (int i = 0; i < halves; i += 2) {  // a group
-                        bool centred = true;  // in fp32 every bias is exact enough
-                        if (!C::kFolded) tf32_bias(__low2float(u32_as_h2(sv.x)), __low2float(u32_as_h2(bv.x)), &centred);
+                        uint32_t minus = 0xA400A400u;  // -8 x 2^-9: in fp32 every bias is exact enough
+                        if (!C::kFolded) tf32_bias(__low2float(u32_as_h2(sv.x)), __low2float(u32_as_h2(bv.x)), &minus);
                         sv = make_uint2(__funnelshift_r(sv.x, sv.y, 16), sv.y >> 16);
                         bv = make_uint2(__funnelshift_r(bv.x, bv.y, 16), bv.y >> 16);
-                        const uint32_t minus = centred ? 0xA400A400u : 0u;  // -8 x 2^-9
                         const uint4 v0 = lds128(src + (((2 * k + i) ^ (row & 7)) << 4)), v1 = lds128(src + (((2 * k + i + 1) ^ (row & 7)) << 4));
                         uint32_t pair[16], more[16];
                         expand_nibbles(v0.x, minus, pair);
@@ -717,11 +721,11 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                         for (uint32_t i = 0; i <= last; ++i) {
                             const uint32_t back = last - i, stage = ss.i >= back ? ss.i - back : ss.i + C::kScaleStages - back, at = scales + stage * (2 * kLineRows * 8) + row * 8;
                             uint32_t v[8];
-                            bool centred;
+                            uint32_t minus;
                             uint2 sv = lds64(at), bv = lds64(at + kLineRows * 8);
 #pragma unroll
                             for (int j = 0; j < 4; ++j) {
-                                v[j] = v[4 + j] = __float_as_uint(tf32_bias(__low2float(u32_as_h2(sv.x)), __low2float(u32_as_h2(bv.x)), &centred));
+                                v[j] = v[4 + j] = __float_as_uint(tf32_bias(__low2float(u32_as_h2(sv.x)), __low2float(u32_as_h2(bv.x)), &minus));
                                 sv = make_uint2(__funnelshift_r(sv.x, sv.y, 16), sv.y >> 16);
                                 bv = make_uint2(__funnelshift_r(bv.x, bv.y, 16), bv.y >> 16);
                             }

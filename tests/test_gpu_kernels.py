@@ -218,8 +218,9 @@ def test_affine_wide_rounds_like_exact_sums(ctx, rows, cols, batch):
 
 
 # As many results as before may be misrounded, whatever the rows of x: 0.1 % where fp16 operands were summed over two groups at a time and
-# the running sums in fp32 rounded once for two groups.  A fp32 sum that rounds twice for each of the 272 groups here has 0.17 %.
-@pytest.mark.parametrize("rows,cols,batch,mean", [(2048, 17408, 32, 0.0)])
+# the running sums in fp32 rounded once for two groups.  A fp32 sum that rounds twice for each of 272 groups has 0.17 %; and where x has a
+# mean, group sums times biases of half a scale, truncated on the tensor core over sixteen groups, have 0.24 %.
+@pytest.mark.parametrize("rows,cols,batch,mean", [(2048, 17408, 32, 0.0), (1024, 4096, 64, 0.5), (512, 4096, 128, 0.5)])
 def test_affine_wide_running_sums(ctx, rows, cols, batch, mean):
     w, s, b = synth.affine_u4_model(40, "mw", rows, cols)
     x = (synth.activations(40, "mx", batch, cols).astype(np.float32) + mean).astype(np.float16)
@@ -248,14 +249,14 @@ def test_affine_wide_large_weights(ctx, oracle, rows, cols, batch):
     assert np.all(np.isfinite(want)) and rel_err(got, want) < REL_TOL
 
 
-# groups whose weights have one sign only, of all sizes of bias: beyond 64 rows of x the centred bias of such a group is not exact in
-# tf32 and its nibbles go to the tensor core as they are; the bound is that of test_affine_wide_rounds_like_exact_sums
+# groups whose weights have one sign only, of all sizes of bias: beyond 32 rows of x the nibbles are centred by up to 128, and in one of sixty
+# groups or so not at all; the bound is that of test_affine_wide_rounds_like_exact_sums
 @pytest.mark.parametrize("rows,cols,batch", [(136, 4096, 32), (264, 4096, 64), (136, 4160, 65), (264, 4096, 128), (72, 12288, 129)])
 def test_affine_wide_one_sided_groups(ctx, rows, cols, batch):
     w, s, b = synth.affine_u4(37, "ow", rows, cols, 64)
     rng = np.random.default_rng(37)
     some = rng.random(b.shape) < 0.5
-    b[some] = (s[some].astype(np.float64) * 2.0 ** rng.uniform(-6, 7, int(some.sum())) * rng.choice([-1, 1], int(some.sum()))).astype(np.float16)
+    b[some] = (s[some].astype(np.float64) * 2.0 ** rng.uniform(-6, 8.2, int(some.sum())) * rng.choice([-1, 1], int(some.sum()))).astype(np.float16)
     x = synth.activations(37, "ox", batch, cols)
     d = dev(ctx, w, s, b, x)
     y = ctx.alloc(batch * rows * 2)
