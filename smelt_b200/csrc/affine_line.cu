@@ -25,7 +25,7 @@ EncodeTiled encode_tiled() {
 // 148 18.5; 128 rows: 4 34.0, 6 29.9, 8 31.4, 16 43.7, 148 49.1; 4096 x 4096, 32 rows: 2 13.1, 4 10.8, 148 12.5; 128 rows: 4 23.3,
 // 148 27.7; 4096 x 12288, 64 rows: 4 31.1, 148 32.1; gate/up 6144 x 2048, 32 rows: 1 12.1, 148 14.5; 512 rows: 148 63.8 (three waves
 // of whole tiles would be 3 x 16).
-int ctas_for(const Line& p, int sm, int* per_tile) {
+int ctas_for(const Line& p, int sm, int* per_tile, double* cost_us) {
     const long tiles = (long)p.row_tiles * p.col_tiles;
     const double stage = p.tile_cols <= 32 ? 0.99 : p.tile_cols <= 64 ? 1.6 : 1.65, sum = p.tile_cols <= 32 ? 0.57 : p.tile_cols <= 64 ? 0.85 : 2.0;
     *per_tile = 0;
@@ -34,7 +34,29 @@ int ctas_for(const Line& p, int sm, int* per_tile) {
         const double cost = (double)((p.stages + k - 1) / k) * stage + (k > 1 ? 1.0 + sum * k : 0.0);
         if (cost < least) { least = cost; *per_tile = k; }
     }
+    *cost_us = least + (p.tile_cols <= 32 ? 0.0 : p.tile_cols <= 64 ? 0.25 : 1.5);  // the last: group sums in front
     return (int)(*per_tile ? tiles * *per_tile : std::min((long)sm, tiles * p.stages));
+}
+
+// How many rows of x a tile has: 32, 64 or 128, whichever ctas_for's estimate says is fastest.  Narrow tiles expand the weights more often, but a small
+// matrix has few tiles, SMs idle, and a wide tile's sums take longest to put together.  us, in tiles of 32 | 64 | 128: plain 1024 x 1536, 77 rows
+// 8.2 | 10.6 | 15.0, 512 rows 9.9 | 12.8 | 17.4; gate/up 1024 x 2048, 40 rows 9.1 | 11.4, 300 rows 17.1 | 17.8 | 19.9; plain 4096 x 4096, 64 rows
+// 14.4 | 15.5, 77 rows 19.0 | 19.3 | 18.6, 128 rows 19.7 | 20.3 | 23.5; gate/up 12288 x 4096, 64 rows 55 | 45, 128 rows 99 | 78 | 57.  Of 1120 shapes (256 to 12288 rows, 512
+// to 12288 columns, 33 to 512 rows of x) the choice is 0.25 % slower than the best on average, 14 % at most.
+void choose_tile(Line* p, int batch, int max_cols, int sm) {
+    Line best = {};
+    double least = 0.0;
+    for (int cols = 32; cols <= max_cols; cols *= 2) {
+        Line q = *p;
+        const int wanted = (batch + cols - 1) / cols;
+        q.tile_cols = ((batch + wanted - 1) / wanted + 15) & ~15;
+        q.col_tiles = (batch + q.tile_cols - 1) / q.tile_cols;
+        double cost;
+        ctas_for(q, sm, &q.per_tile, &cost);
+        if (best.tile_cols == 0 || cost < least) { best = q; least = cost; }
+        if (wanted == 1) break;
+    }
+    *p = best;
 }
 
 }  // namespace
@@ -56,10 +78,6 @@ bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, int own_c
     *line = {};
     line->groups = a.cols / kLineGroup;
     line->stages = (line->groups + kStageGroups - 1) / kStageGroups;
-    const int wanted = (a.batch + max_cols - 1) / max_cols;
-    line->tile_cols = (a.batch + wanted - 1) / wanted;
-    line->tile_cols = line->tile_cols <= 128 ? (line->tile_cols + 15) & ~15 : (line->tile_cols + 31) & ~31;  // above 128 two MMAs share them
-    line->col_tiles = (a.batch + line->tile_cols - 1) / line->tile_cols;
     line->first1 = line->first2 = INT_MAX;
     for (int s = 0; s < (paired ? 2 : segs ? a.nseg : 1); ++s) {
         const uint8_t* w = segs ? a.seg[s].w : a.w[s];
@@ -72,6 +90,7 @@ bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, int own_c
         }
     }
     if (paired) line->row_tiles = (a.rows + 63) / 64;
+    choose_tile(line, a.batch, max_cols, sm);
     const long tiles = (long)line->row_tiles * line->col_tiles, units = tiles * line->stages;
     if (units >= 1l << 28 || !encode_rows(&maps->x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.x, a.batch, a.cols, line->tile_cols)) return false;
     const size_t shared = (size_t)sm * 2 * line->tile_cols * kLineRows;  // two tiles of every CTA
@@ -83,7 +102,9 @@ bool line_plan(int mode, const AffineArgs& a, int group, int max_cols, int own_c
     }
     const bool split = tiles <= 4096;  // a counter each
     line->quantum = split ? 1 : line->stages;
-    *grid = split ? ctas_for(*line, sm, &line->per_tile) : (int)std::min((long)sm, tiles);
+    double cost;
+    *grid = split ? ctas_for(*line, sm, &line->per_tile, &cost) : (int)std::min((long)sm, tiles);
+    if (!split) line->per_tile = 0;
     line->share = (int)(units / line->quantum / *grid);
     line->extra = (int)(units / line->quantum % *grid);
     return true;

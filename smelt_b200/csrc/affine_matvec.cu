@@ -468,7 +468,7 @@ bool wide_first(int mode, const AffineArgs& a, int group) {
 
 cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int group) {
     if (args.rows <= 0 || args.cols <= 0 || args.batch <= 0 || args.cols % group != 0) return cudaErrorInvalidValue;
-    if (wide_first(mode, args, group)) {  // tcgen05: the weights are expanded once per 128 rows of x
+    if (wide_first(mode, args, group)) {  // tcgen05: the weights are expanded once per tile of up to 128 rows of x
         if (args.norm_w) {  // the folded norm as a launch of its own, its rows behind everything else in scratch
             const size_t bytes = ((size_t)args.batch * args.cols * sizeof(__half) + 255) & ~(size_t)255;
             if (args.part_scratch && args.cols % 8 == 0 && bytes <= args.part_scratch_bytes / 4) {

@@ -220,7 +220,7 @@ def test_affine_wide_rounds_like_exact_sums(ctx, rows, cols, batch):
 # As many results as before may be misrounded, whatever the rows of x: 0.1 % where fp16 operands were summed over two groups at a time and
 # the running sums in fp32 rounded once for two groups.  A fp32 sum that rounds twice for each of 272 groups has 0.17 %; and where x has a
 # mean, group sums times biases of half a scale, truncated on the tensor core over sixteen groups, have 0.24 %.
-@pytest.mark.parametrize("rows,cols,batch,mean", [(2048, 17408, 32, 0.0), (1024, 4096, 64, 0.5), (512, 4096, 128, 0.5)])
+@pytest.mark.parametrize("rows,cols,batch,mean", [(2048, 17408, 32, 0.0), (12288, 2048, 64, 0.5), (12288, 2048, 128, 0.5)])
 def test_affine_wide_running_sums(ctx, rows, cols, batch, mean):
     w, s, b = synth.affine_u4_model(40, "mw", rows, cols)
     x = (synth.activations(40, "mx", batch, cols).astype(np.float32) + mean).astype(np.float16)
@@ -271,7 +271,7 @@ def test_affine_wide_one_sided_groups(ctx, rows, cols, batch):
 
 # beyond 64 rows of x, where the last group sums of a row belong to a stage of two groups and the turns that multiply them come closest:
 # several such rows a CTA, also with nothing else in them; the bound is that of test_affine_wide_rounds_like_exact_sums
-@pytest.mark.parametrize("rows,cols,batch", [(2048, 1152, 128), (40000, 128, 65), (4104, 640, 300)])
+@pytest.mark.parametrize("rows,cols,batch", [(12296, 1152, 128), (40000, 128, 257), (12296, 1152, 300)])
 def test_affine_wide_short_last_stage(ctx, rows, cols, batch):
     w, s, b = synth.affine_u4(38, "sw", rows, cols, 64)
     x = (synth.activations(38, "sx", batch, cols).astype(np.float32) + 0.5).astype(np.float16)  # so that the group sums tell
@@ -287,6 +287,39 @@ def test_affine_wide_short_last_stage(ctx, rows, cols, batch):
         assert np.array_equal(y.download(np.uint16, (batch, rows)), first)
     assert ctx.device_error() == 0
     for buf in d + [y]:
+        buf.free()
+
+
+# Matrices large enough for tiles of more than 32 rows of x (48 to 112 rows and 128 here, one tile a CTA and several), with rows and columns that
+# no tile divides and a last stage of one, two and three groups
+@pytest.mark.parametrize("rows,cols,batch", [(12296, 1152, b) for b in (33, 64, 65, 128, 130, 300)] + [(8200, 576, b) for b in (33, 64, 65, 128, 257)] +
+                         [(12296, 192, 64), (12296, 192, 128), (6152, 1984, 65), (6152, 1984, 130), (40000, 64, 300)])
+def test_affine_wide_large_matrices(ctx, rows, cols, batch):
+    a, b = (synth.affine_u4(41, n, rows, cols, 64) for n in ("la", "lb"))
+    x, res = synth.activations(41, "lx", batch, cols), synth.activations(41, "lres", batch, rows)
+    d = dev(ctx, *a, *b, x, res)
+    y0, y1 = ctx.alloc(batch * rows * 2 + 64).fill(0xFF), ctx.alloc(batch * rows * 2 + 64).fill(0xFF)
+
+    def exact(w, s, b):
+        q = np.stack([w & 15, w >> 4], -1).reshape(rows, cols // 64, 64).astype(np.float64)
+        return x.astype(np.float64) @ (q * s.astype(np.float64)[..., None] + b.astype(np.float64)[..., None]).reshape(rows, cols).T
+
+    ref_a, ref_b = exact(*a), exact(*b)
+    ctx.call("affine_matvec", *d[:3], d[6], y0, rows, cols, 64, batch)
+    assert np.mean(y0.download(np.float16, (batch, rows)) != ref_a.astype(np.float16)) < 4e-3  # test_affine_wide_rounds_like_exact_sums
+    ctx.call("affine_dual_matvec", *d[:7], y0, y1, rows, cols, 64, batch)
+    assert rel_err(y0.download(np.float16, (batch, rows)), ref_a) < REL_TOL and rel_err(y1.download(np.float16, (batch, rows)), ref_b) < REL_TOL
+    ctx.call("affine_matvec_add", *d[:3], d[6], d[7], y0, rows, cols, 64, batch)
+    assert add_rel_err(y0.download(np.float16, (batch, rows)), ref_a.astype(np.float16).astype(np.float64) + res, ref_a) < REL_TOL
+    ctx.call("affine_gate_up_swiglu", *d[:7], y1, rows, cols, 64, batch)
+    first = y1.download(np.float16, (batch, rows))
+    assert rel_err(first, ref_a / (1.0 + np.exp(-ref_a)) * ref_b) < REL_TOL
+    ctx.call("affine_gate_up_swiglu", *d[:7], y1, rows, cols, 64, batch)
+    assert np.array_equal(y1.download(np.uint16, (batch, rows)), first.view(np.uint16))  # run-to-run determinism
+    for y in (y0, y1):
+        assert np.all(y.download(np.uint8, (64,), offset=batch * rows * 2) == 0xFF)
+    assert ctx.device_error() == 0
+    for buf in d + [y0, y1]:
         buf.free()
 
 
