@@ -451,7 +451,11 @@ cudaError_t launch_group(const Launch& l, const AffineArgs& a, int group) {
 //   * 9 to 16 rows: gate/up, dual and + residual, where the streaming kernel needs two passes or more: gate/up 12288 x 4096, 9 rows
 //     38.7 : 30.0, 16 rows 46.5 : 29.2; 6144 x 2048, 9 rows 15.4 : 11.7; 4096 x 12288 + residual, 9 rows 32.7 : 17.6; 2048 x 2048, 9 rows
 //     7.5 : 7.0.  Plain products only where the streaming kernel does not take them (264 x 17408, 9 rows 28.4 : 12.7): one launch over
-//     several tensors (affine_multi_matvec) runs on it up to 16 rows, and gives the bits of a launch for each.
+//     several tensors (affine_multi_matvec) runs on it up to 16 rows, and gives the bits of a launch for each.  Not in the general kernel's one
+//     round of eight warps, 1024 to 2048 columns, where x is hardly more than the eight rows that it takes at once: plain products up to 12
+//     rows, + residual 10 (1024 x 1536 plain, 9 rows 5.7 : 6.8, 12 rows 6.8 : 6.8, + residual, 9 rows 6.5 : 7.1, 10 rows 7.0 : 7.1; 5440 x 1856
+//     plain, 12 rows 9.4 : 10.2, + residual, 10 rows 9.5 : 10.4; 1024 x 768, 9 rows 5.3 : 5.1; 1024 x 2496, 9 rows 9.0 : 7.3; dual 4096 x 1664, 9 rows 11.2 :
+//     11.0).
 //   * 6 to 8 rows, plain and + residual, that the streaming kernel does not take because their activations do not stay resident, from
 //     128 M weights x rows on: the general kernel takes about 2 + 0.08 us for a million of these, the product 8 + 0.2 for a million
 //     weights.  8 rows: 4096 x 12288 29.5 : 17.7, 2048 x 12288 18.9 : 12.2, 1024 x 17408 17.6 : 13.4, 1024 x 12288 9.4 : 11.9;
@@ -460,7 +464,8 @@ bool wide_first(int mode, const AffineArgs& a, int group) {
     if (a.batch >= 17) return true;
     if (a.batch <= 5 || a.nseg > 1) return false;
     const bool streamed = affine_stream_passes(mode, a, group) != 0;
-    if (a.batch >= 9) return mode != kAffinePlain || !streamed;
+    const bool one_round = a.cols > 768 && a.cols < 2048 && a.rows < 8192;
+    if (a.batch >= 9) return streamed ? mode != kAffinePlain : !(one_round && a.batch <= (mode == kAffinePlain ? 12 : mode == kAffineAdd ? 10 : 0));
     return (mode == kAffinePlain || mode == kAffineAdd) && !streamed && (size_t)a.rows * a.cols * a.batch >= (size_t)128 << 20;
 }
 

@@ -271,7 +271,7 @@ def test_affine_wide_one_sided_groups(ctx, rows, cols, batch):
 
 # beyond 64 rows of x, where the last group sums of a row belong to a stage of two groups and the turns that multiply them come closest:
 # several such rows a CTA, also with nothing else in them; the bound is that of test_affine_wide_rounds_like_exact_sums
-@pytest.mark.parametrize("rows,cols,batch", [(12296, 1152, 128), (40000, 128, 257), (12296, 1152, 300)])
+@pytest.mark.parametrize("rows,cols,batch", [(12296, 1152, 128), (40000, 128, 512), (12296, 1152, 300)])
 def test_affine_wide_short_last_stage(ctx, rows, cols, batch):
     w, s, b = synth.affine_u4(38, "sw", rows, cols, 64)
     x = (synth.activations(38, "sx", batch, cols).astype(np.float32) + 0.5).astype(np.float16)  # so that the group sums tell
@@ -293,7 +293,7 @@ def test_affine_wide_short_last_stage(ctx, rows, cols, batch):
 # Matrices large enough for tiles of more than 32 rows of x (48 to 112 rows and 128 here, one tile a CTA and several), with rows and columns that
 # no tile divides and a last stage of one, two and three groups
 @pytest.mark.parametrize("rows,cols,batch", [(12296, 1152, b) for b in (33, 64, 65, 128, 130, 300)] + [(8200, 576, b) for b in (33, 64, 65, 128, 257)] +
-                         [(12296, 192, 64), (12296, 192, 128), (6152, 1984, 65), (6152, 1984, 130), (40000, 64, 300)])
+                         [(12296, 192, 64), (24584, 192, 300), (6152, 1984, 65), (6152, 1984, 130), (40000, 64, 300)])
 def test_affine_wide_large_matrices(ctx, rows, cols, batch):
     a, b = (synth.affine_u4(41, n, rows, cols, 64) for n in ("la", "lb"))
     x, res = synth.activations(41, "lx", batch, cols), synth.activations(41, "lres", batch, rows)
