@@ -469,23 +469,30 @@ bool wide_first(int mode, const AffineArgs& a, int group) {
     return (mode == kAffinePlain || mode == kAffineAdd) && !streamed && (size_t)a.rows * a.cols * a.batch >= (size_t)128 << 20;
 }
 
+// The norm as a launch of its own, its rows behind everything else in scratch, and the launch that reads them; not supported where a quarter of
+// the scratch does not hold them.
+cudaError_t norm_apart(const Launch& l, const AffineArgs& a, AffineArgs* rest) {
+    const size_t bytes = ((size_t)a.batch * a.cols * sizeof(__half) + 255) & ~(size_t)255;
+    if (!a.part_scratch || bytes > a.part_scratch_bytes / 4) return cudaErrorNotSupported;
+    *rest = a;
+    rest->part_scratch_bytes = (a.part_scratch_bytes - bytes) / 256 * 256;
+    __half* xn = reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(a.part_scratch) + rest->part_scratch_bytes);
+    rest->x = xn;
+    rest->norm_w = nullptr;
+    return launch_rms_norm_1pw(l, a.x, a.norm_w, xn, a.cols, a.norm_eps, a.batch);
+}
+
 }  // namespace
 
 cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int group) {
     if (args.rows <= 0 || args.cols <= 0 || args.batch <= 0 || args.cols % group != 0) return cudaErrorInvalidValue;
     if (wide_first(mode, args, group)) {  // tcgen05: the weights are expanded once per tile of up to 128 rows of x
-        if (args.norm_w) {  // the folded norm as a launch of its own, its rows behind everything else in scratch
-            const size_t bytes = ((size_t)args.batch * args.cols * sizeof(__half) + 255) & ~(size_t)255;
-            if (args.part_scratch && args.cols % 8 == 0 && bytes <= args.part_scratch_bytes / 4) {
-                AffineArgs s = args;
-                __half* xn = reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(args.part_scratch) + (args.part_scratch_bytes - bytes) / 256 * 256);
-                const cudaError_t e = launch_rms_norm_1pw(l, args.x, args.norm_w, xn, args.cols, args.norm_eps, args.batch);
-                if (e != cudaSuccess) return e;
-                s.x = xn;
-                s.norm_w = nullptr;
-                s.part_scratch_bytes = (args.part_scratch_bytes - bytes) / 256 * 256;
-                return launch_affine(l, mode, s, group);
-            }
+        if (args.norm_w) {
+            // only the streaming kernel folds a norm: what it refuses is refused for any number of rows, not left to kernels that check less
+            if (affine_stream_passes(mode, args, group) == 0) return cudaErrorNotSupported;
+            AffineArgs s;
+            const cudaError_t e = norm_apart(l, args, &s);
+            if (e != cudaErrorNotSupported) return e != cudaSuccess ? e : launch_affine(l, mode, s, group);
         }
         bool handled = false;
         cudaError_t e = launch_affine_wide(l, mode, args, group, &handled);

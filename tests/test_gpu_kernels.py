@@ -524,6 +524,24 @@ def test_rmsnorm_affine_gate_up_swiglu_many_rows(ctx, oracle, rows, cols, batch)
     assert rel_err(y.download(np.float16, (batch, rows)), ref) < REL_TOL and ctx.device_error() == 0
 
 
+# what the folded norm is refused with, it is refused with for any number of rows: nothing is launched that reads 16 bytes at a time
+@pytest.mark.parametrize("batch", [8, 9, 17, 64])
+def test_rmsnorm_affine_gate_up_swiglu_refusals(ctx, batch):
+    rows, cols = 136, 1024
+    gate, up = (synth.affine_u4(42, n, rows, cols, 64) for n in ("gate", "up"))
+    x, nw = synth.activations(42, "x", batch, cols), synth.normal_f16(42, "norm", (cols,), 0.1)
+    d = [ctx.alloc(a.nbytes + 16) for a in (*gate, *up, x, nw)]
+    y = ctx.alloc(batch * rows * 2).fill(0xFF)
+    call = lambda p, c=cols, g=64: ctx.call_status("rmsnorm_affine_gate_up_swiglu", *p, C.c_float(1e-6), y, rows, c, g, batch)
+    p = [C.c_void_p(b.ptr) for b in d]
+    for i in range(len(p)):  # one operand at a time at a multiple of eight bytes only
+        q = list(p)
+        q[i] = C.c_void_p(d[i].ptr + 8)
+        assert call(q) == capi.UNSUPPORTED, i
+    assert call(p, 960) == capi.UNSUPPORTED and call(p, cols, 32) == capi.UNSUPPORTED
+    assert np.all(y.download(np.uint8, (batch * rows * 2,)) == 0xFF) and ctx.device_error() == 0
+
+
 @pytest.mark.parametrize("position,layout", [(0, 1), (77, 1), (4095, 0), (32767, 1)])
 def test_rope_qkv_append_is_the_three_kernels(ctx, oracle, position, layout):
     nq, nkv, d, cap = 8, 2, 128, 32768
