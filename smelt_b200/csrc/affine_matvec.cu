@@ -524,4 +524,18 @@ cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int
     }
 }
 
+cudaError_t launch_affine_apart(const Launch& l, int mode, const AffineArgs& a, int group) {
+    AffineArgs s;
+    cudaError_t e = norm_apart(l, a, &s);
+    if (e != cudaSuccess || a.nseg <= 1) return e != cudaSuccess ? e : launch_affine(l, mode, s, group);
+    s.nseg = 0;
+    s.rows = a.seg[0].rows;
+    e = launch_affine(l, kAffinePlain, s, group);
+    if (e != cudaSuccess) return e;
+    s.rows = a.seg[1].rows;
+    s.w[0] = a.seg[1].w; s.s[0] = a.seg[1].s; s.b[0] = a.seg[1].b; s.y = a.seg[1].y;
+    s.w[1] = a.seg[2].w; s.s[1] = a.seg[2].s; s.b[1] = a.seg[2].b; s.y2 = a.seg[2].y;
+    return launch_affine(l, kAffineDual, s, group);
+}
+
 }  // namespace smelt

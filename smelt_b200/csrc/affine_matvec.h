@@ -61,6 +61,9 @@ inline AffineArgs affine_rows(const AffineArgs& a, int r0, int n) {
 }
 
 cudaError_t launch_affine(const Launch& l, int mode, const AffineArgs& args, int group);
+// A folded norm and its product (one tensor, gate and up, or Q, K and V with as many rows of K as of V) as the separate launches that they stand
+// for: any alignment but that of the packed weights (16 bytes), any number of columns.
+cudaError_t launch_affine_apart(const Launch& l, int mode, const AffineArgs& args, int group);
 cudaError_t launch_affine_stream(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);
 // Tensor-core product for many rows of x (affine_wide.cu; from how many: wide_first in affine_matvec.cu).
 cudaError_t launch_affine_wide(const Launch& l, int mode, const AffineArgs& args, int group, bool* handled);

@@ -48,9 +48,9 @@ static smelt_status build_decoder_impl(smelt_cuda_ctx* ctx, const smelt_decoder_
     const bool tp = d->tp_world > 1;
     const bool fuse = (d->fuse_residual & 1) && !tp;
     // bit 1: fold the norms into the projections (one QKV launch, one gate/up launch) and RoPE /
-    // KV append into one launch; needs the shapes the streaming matvec kernel accepts.
+    // KV append into one launch; needs the shapes the streaming matvec kernel accepts, and a counter for each KV head of a sequence.
     const bool fuse_tp = (d->fuse_residual & 4) != 0;  // bit 2: all-reduce and residual add in one launch over peer memory
-    const bool fuse2 = (d->fuse_residual & 2) && G == 64 && H % 1024 == 0 && qd % 16 == 0 && kvd % 16 == 0 && D % 2 == 0;
+    const bool fuse2 = (d->fuse_residual & 2) && G == 64 && H % 1024 == 0 && qd % 16 == 0 && kvd % 16 == 0 && D % 2 == 0 && (B <= 8 || (size_t)B * d->n_kv <= 4096);
     const bool bt = B > 1;  // batched kernel names bind actualBatch instead of numRows
 
     if (!dry) {

@@ -618,6 +618,21 @@ smelt_status run_affine(Interp& in, const Pipeline& p, const smelt_dispatch_reco
     return check_cuda(ctx, launch_affine(make_launch(in, r), mode, a, p.group), p.name.c_str());
 }
 
+// A norm folded into the projections behind it.  Tables of more than eight sequences have these records whatever the image: where the fused
+// kernels do not take scales, biases or a norm off a 16-byte boundary, or that many columns, the launches that they stand for run.
+smelt_status run_normed_affine(Interp& in, const Pipeline& p, const Launch& l, int mode, const AffineArgs& a) {
+    smelt_cuda_ctx* ctx = in.ctx;
+    cudaError_t e = launch_affine(l, mode, a, p.group);
+    if (e == cudaErrorNotSupported && a.batch > 8) {
+        uintptr_t packed = 0;
+        for (int i = 0; i < (a.nseg > 1 ? a.nseg : 2); ++i) packed |= (uintptr_t)(a.nseg > 1 ? a.seg[i].w : a.w[i]);
+        if (packed & 15u) return fail(ctx, SMELT_ERR_BAD_ARGUMENT, p.name + ": packed weights must be 16-byte aligned");
+        e = launch_affine_apart(l, mode, a, p.group);
+    }
+    if (e == cudaErrorNotSupported) return fail(ctx, SMELT_ERR_UNSUPPORTED, p.name + ": shape not eligible for the fused kernel");
+    return check_cuda(ctx, e, p.name.c_str());
+}
+
 smelt_status run_signed(Interp& in, const Pipeline& p, const smelt_dispatch_record& rec, const Resolved& r) {
     smelt_cuda_ctx* ctx = in.ctx;
     // signed_quant.metal:574-583 (matvec), :662-672 (add), :625-636 (gate/up); signed_quant_precise.metal:41-50
@@ -1934,9 +1949,7 @@ smelt_status run_record(Interp& in, const smelt_dispatch_record& rec_in) {
             a.x = (const __half*)r.buf[9].ptr; a.norm_w = (const __half*)r.buf[10].ptr; a.norm_eps = as_f32(eps_bits);
             a.cols = p.cols; a.batch = (int)nb; a.err = ctx->err_dev; a.sm_count = ctx->sm_count; a.part_scratch = ctx->qmm_scratch; a.part_scratch_bytes = ctx->qmm_scratch_bytes; a.part_counters = ctx->qmm_counters;
             in.launches += 1;
-            cudaError_t e = launch_affine(l, kAffinePlain, a, p.group);
-            if (e == cudaErrorNotSupported) return fail(ctx, SMELT_ERR_UNSUPPORTED, p.name + ": shape not eligible for the fused kernel");
-            return check_cuda(ctx, e, p.name.c_str());
+            return run_normed_affine(in, p, l, kAffinePlain, a);
         }
         case PK_FUSED_NORM_GATEUP: {
             // 0-2 gate, 3-5 up, 6 x, 7 y, 9 norm weight; constants 8 rows, 10 eps, 11 batch.
@@ -1955,9 +1968,7 @@ smelt_status run_record(Interp& in, const smelt_dispatch_record& rec_in) {
             a.x = (const __half*)r.buf[6].ptr; a.y = (__half*)r.buf[7].ptr; a.norm_w = (const __half*)r.buf[9].ptr; a.norm_eps = as_f32(eps_bits);
             a.rows = (int)rows; a.cols = p.cols; a.batch = (int)nb; a.err = ctx->err_dev; a.sm_count = ctx->sm_count; a.part_scratch = ctx->qmm_scratch; a.part_scratch_bytes = ctx->qmm_scratch_bytes; a.part_counters = ctx->qmm_counters;
             in.launches += 1;
-            cudaError_t e = launch_affine(l, kAffineGateUp, a, p.group);
-            if (e == cudaErrorNotSupported) return fail(ctx, SMELT_ERR_UNSUPPORTED, p.name + ": shape not eligible for the fused kernel");
-            return check_cuda(ctx, e, p.name.c_str());
+            return run_normed_affine(in, p, l, kAffineGateUp, a);
         }
         case PK_ROPE_QKV_APPEND: {
             // 0 q (in place), 1 new K, 2 new V, 3 K cache, 4 V cache; constants 7 headDim, 8 q heads,

@@ -102,6 +102,69 @@ def test_batch_of_independent_sequences(ctx, oracle):
         assert not v["wrong"], (b, v)
 
 
+@pytest.mark.parametrize("batch", [9, 17, 33, 64])
+def test_fused_table_of_many_sequences(ctx, oracle, batch):
+    """More sequences than the streaming kernel takes at once: norms as launches of their own, products on the tensor core,
+    attention with fewer splits.  Every sequence's logits against the oracle's; eager and from the graph the same bits."""
+    cfg = package.DecoderConfig(layers=2, hidden=1024, inter=3072, n_q=8, n_kv=2, head_dim=128, vocab=2048)
+    pkg, dec = make(ctx, cfg, 9, 32, batch=batch, fuse=3)
+    ref = oracle.model_from_package(pkg, 32)
+    tokens = synth.rng_for(9, "tokens").integers(0, cfg.vocab, size=(3, batch)).astype(np.int32)
+    for pos, tok in enumerate(tokens):
+        dec.decode_step(tok, pos)
+    logits = dec.logits().copy()
+    for b in range(batch):
+        for pos in range(len(tokens)):
+            _, want = ref.decode_step(int(tokens[pos, b]), pos, want_logits=True)
+        want = want.astype(np.float32)
+        err = float(np.max(np.abs(logits[b].astype(np.float32) - want)) / np.sqrt(np.mean(want * want)))
+        assert err < 1e-2, (b, err)  # test_decode_step_matches_oracle
+    dec.reset_cache()
+    dec.build_graph()
+    for pos, tok in enumerate(tokens):
+        dec.graph_seed(tok, pos)
+        dec.graph_decode(1)
+    assert np.array_equal(dec.logits().view(np.uint16), logits.view(np.uint16)) and ctx.device_error() == 0
+
+
+@pytest.mark.parametrize("batch", [9, 17])
+def test_fused_table_of_many_sequences_takes_any_image(ctx, batch):
+    """Scales, biases and norms off a 16-byte boundary: the fused kernels refuse them, and the records run the launches that
+    they stand for, with the bits of the reference-shaped table."""
+    cfg = MID
+    pkg = package.SyntheticPackage(cfg, 8)
+    image, desc, layers = package.build_image(pkg)
+    blocks, size = [image.view(np.uint8).reshape(-1)], image.nbytes
+
+    def moved(offset, nbytes):  # a copy at a multiple of eight
+        nonlocal size
+        pad = -size % 16 + 8
+        blocks.extend([np.zeros(pad, np.uint8), blocks[0][offset:offset + nbytes]])
+        size += pad + nbytes
+        return size - nbytes
+
+    qd, kvd = cfg.n_q * cfg.head_dim, cfg.n_kv * cfg.head_dim
+    for ref in layers:
+        for name, rows in (("q", qd), ("k", kvd), ("v", kvd), ("gate", cfg.inter), ("up", cfg.inter)):
+            t, n = getattr(ref, name), rows * cfg.hidden // 64 * 2
+            t.scales, t.biases = moved(t.scales, n), moved(t.biases, n)
+        ref.input_norm, ref.post_norm = moved(ref.input_norm, cfg.hidden * 2), moved(ref.post_norm, cfg.hidden * 2)
+    image = np.concatenate(blocks)
+    tokens = synth.rng_for(8, "tokens").integers(0, cfg.vocab, size=(4, batch)).astype(np.int32)
+    logits = []
+    for fuse in (1, 3):
+        dec = package.Decoder(ctx, image, desc, layers, 32, batch, fuse_residual=fuse)
+        for pos, tok in enumerate(tokens):
+            dec.decode_step(tok, pos)
+        logits.append(dec.logits().copy())
+    assert np.all(np.isfinite(logits[0].astype(np.float32))) and np.array_equal(logits[0].view(np.uint16), logits[1].view(np.uint16))
+    layers[0].gate.packed += 8  # as of the reference-shaped records: an error, not a launch
+    dec = package.Decoder(ctx, image, desc, layers, 32, batch, fuse_residual=3)
+    with pytest.raises(capi.SmeltError) as e:
+        dec.decode_step(tokens[0], 0)
+    assert e.value.status == capi.BAD_ARGUMENT and ctx.device_error() == 0
+
+
 def test_runtime_errors(ctx):
     pkg, dec = make(ctx, SMALL, 3, 16)
     st = ctx.lib.smelt_cuda_decode_step(ctx.h, dec.table, dec.n_records, np.array([0], np.int32).ctypes.data_as(C.c_void_p), 16, None)

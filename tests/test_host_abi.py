@@ -101,6 +101,14 @@ def test_decoder_table_follows_the_reference_emitter():
     assert gate.con[0].binding_index == 8 and gate.con[0].value == 12288
 
 
+def test_fused_table_of_many_sequences_needs_a_counter_per_kv_head():
+    """The launch of RoPE, append and attention counts arrivals per (sequence, KV head), 4096 of them: beyond that a table of
+    more than eight sequences keeps the reference-shaped records."""
+    cfg = package.DecoderConfig(layers=1, hidden=2048, inter=6144, n_q=128, n_kv=128, head_dim=64, vocab=1000)
+    fused = lambda batch: any(n.startswith("smelt_") for n in _table(cfg, batch, fuse=3)[1])
+    assert fused(8) and fused(9) and fused(32) and not fused(33) and not fused(64)
+
+
 def test_decoder_table_variants():
     cfg = package.DecoderConfig(layers=1, hidden=2048, inter=6144, n_q=16, n_kv=4, head_dim=128, vocab=1000)
     _, names_b = _table(cfg, 8)
