@@ -482,6 +482,21 @@ def test_affine_multi_matvec_many_rows(ctx, oracle, rows, cols, batch):
         assert rel_err(g, ref) < REL_TOL and inf_err(g, ref) < INF_TOL
 
 
+# and with a norm, which is a launch of its own then: the bits of the norm kernel and the same launch without one
+@pytest.mark.parametrize("rows,cols,batch", [((256, 64, 64), 1024, 17), ((272, 144, 130), 2048, 33), ((2048, 512, 512), 2048, 64)])
+def test_affine_multi_matvec_many_rows_with_norm(ctx, oracle, rows, cols, batch):
+    tensors = [(*synth.affine_u4(43, f"t{i}", r, cols, 64), r) for i, r in enumerate(rows)]
+    x, nw = synth.activations(43, "x", batch, cols), synth.normal_f16(43, "norm", (cols,), 0.1)
+    st, got = _multi(ctx, tensors, x, nw, 1e-6, cols, batch)
+    assert st == 0, ctx.last_error()
+    xn, _ = _device_norm(ctx, x, nw, 1e-6)
+    st, plain = _multi(ctx, tensors, xn, None, 1e-6, cols, batch)
+    assert st == 0, ctx.last_error()
+    for (w, s, b, r), g, p in zip(tensors, got, plain):
+        ref = oracle.affine_matvec(w, s, b, xn, r, cols, 64)
+        assert rel_err(g, ref) < REL_TOL and inf_err(g, ref) < INF_TOL and np.array_equal(g.view(np.uint16), p.view(np.uint16))
+
+
 def test_affine_multi_matvec_rejects_ineligible_shapes(ctx):
     t = [(*synth.affine_u4(22, "a", 24, 1024, 64), 24), (*synth.affine_u4(22, "b", 16, 1024, 64), 16)]
     x = synth.activations(22, "x", 1, 1024)
@@ -781,7 +796,8 @@ def test_attention_many_sequences(ctx, oracle, batch, ctx_len):
 
 
 @pytest.mark.parametrize("n_q,n_kv,d,position,batch,layout", [(32, 8, 128, 0, 1, 1), (32, 8, 128, 530, 1, 1), (16, 4, 128, 4095, 2, 1),
-                                                              (8, 2, 256, 777, 1, 0), (16, 1, 64, 129, 3, 1), (4, 1, 128, 600, 1, 1), (8, 2, 128, 5000, 1, 1)])
+                                                              (8, 2, 256, 777, 1, 0), (16, 1, 64, 129, 3, 1), (4, 1, 128, 600, 1, 1), (8, 2, 128, 5000, 1, 1),
+                                                              (32, 8, 128, 300, 9, 1), (32, 8, 128, 300, 19, 1), (32, 8, 128, 129, 38, 1)])  # fewer splits
 def test_rope_attention_decode_is_the_four_kernels(ctx, oracle, n_q, n_kv, d, position, batch, layout):
     """RoPE on q, RoPE + append of K, append of V and attention in one launch: the bits of the
     four separate launches, with the new token as the last key."""
