@@ -72,6 +72,7 @@ cudaError_t launch_imma_t(const Launch& l, AffineArgs a) {
     cfg.attrs = attr;
     cfg.numAttrs = l.pdl ? 1 : 0;
     prefer_max_shared(kern);
+    l.count();
     return cudaLaunchKernelEx(&cfg, kern, a);
 }
 

@@ -426,6 +426,7 @@ cudaError_t launch_t(const Launch& l, AffineArgs a) {
     cfg.attrs = attr;
     cfg.numAttrs = na;
     prefer_max_shared(kern);
+    l.count();
     return cudaLaunchKernelEx(&cfg, kern, a);
 }
 
@@ -479,6 +480,7 @@ cudaError_t norm_apart(const Launch& l, const AffineArgs& a, AffineArgs* rest) {
     __half* xn = reinterpret_cast<__half*>(reinterpret_cast<uint8_t*>(a.part_scratch) + rest->part_scratch_bytes);
     rest->x = xn;
     rest->norm_w = nullptr;
+    l.count();
     return launch_rms_norm_1pw(l, a.x, a.norm_w, xn, a.cols, a.norm_eps, a.batch);
 }
 

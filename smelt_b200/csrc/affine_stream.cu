@@ -351,6 +351,7 @@ cudaError_t launch_stream_t(const Launch& l, AffineArgs a, int ctas_per_sm) {
     cfg.attrs = attr;
     cfg.numAttrs = l.pdl ? 1 : 0;
     prefer_max_shared(kern);
+    l.count();
     return cudaLaunchKernelEx(&cfg, kern, a);
 }
 

@@ -833,6 +833,7 @@ cudaError_t launch_pdl(const Launch& l, void (*kern)(Params...), dim3 grid, int 
     cfg.attrs = attr;
     cfg.numAttrs = l.pdl ? 1 : 0;
     prefer_max_shared(kern);
+    l.count();
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 

@@ -28,6 +28,8 @@ struct Launch {
     uint32_t arg_pos = 0;           // literal position argument of the kernel, when arg_pos_valid
     uint32_t arg_pos_valid = 0;
     bool pdl = false;               // launch with programmatic stream serialization
+    int* launches = nullptr;        // counts kernel launches where one call may take several (launch_affine); may be null
+    void count(int n = 1) const { if (launches) *launches += n; }
 };
 
 struct DevDyn {

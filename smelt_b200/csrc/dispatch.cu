@@ -614,14 +614,16 @@ smelt_status run_affine(Interp& in, const Pipeline& p, const smelt_dispatch_reco
     if (ires >= 0) { NEED_BUF(ires); NEED_BYTES(ires, (size_t)batch * rows * 2); a.residual = (const __half*)r.buf[ires].ptr; }
     a.rows = rows; a.cols = p.cols; a.batch = batch; a.err = ctx->err_dev; a.sm_count = ctx->sm_count; a.part_scratch = ctx->qmm_scratch; a.part_scratch_bytes = ctx->qmm_scratch_bytes; a.part_counters = ctx->qmm_counters;
     const int mode = p.kind == PK_AFFINE_MATVEC ? kAffinePlain : p.kind == PK_AFFINE_ADD ? kAffineAdd : p.kind == PK_AFFINE_GATEUP ? kAffineGateUp : kAffineDual;
-    in.launches += (batch + 15) / 16;
-    return check_cuda(ctx, launch_affine(make_launch(in, r), mode, a, p.group), p.name.c_str());
+    Launch l = make_launch(in, r);
+    l.launches = &in.launches;
+    return check_cuda(ctx, launch_affine(l, mode, a, p.group), p.name.c_str());
 }
 
 // A norm folded into the projections behind it.  Tables of more than eight sequences have these records whatever the image: where the fused
 // kernels do not take scales, biases or a norm off a 16-byte boundary, or that many columns, the launches that they stand for run.
-smelt_status run_normed_affine(Interp& in, const Pipeline& p, const Launch& l, int mode, const AffineArgs& a) {
+smelt_status run_normed_affine(Interp& in, const Pipeline& p, Launch l, int mode, const AffineArgs& a) {
     smelt_cuda_ctx* ctx = in.ctx;
+    l.launches = &in.launches;
     cudaError_t e = launch_affine(l, mode, a, p.group);
     if (e == cudaErrorNotSupported && a.batch > 8) {
         uintptr_t packed = 0;
@@ -1948,7 +1950,6 @@ smelt_status run_record(Interp& in, const smelt_dispatch_record& rec_in) {
             a.w[0] = a.seg[0].w; a.s[0] = a.seg[0].s; a.b[0] = a.seg[0].b; a.y = a.seg[0].y;
             a.x = (const __half*)r.buf[9].ptr; a.norm_w = (const __half*)r.buf[10].ptr; a.norm_eps = as_f32(eps_bits);
             a.cols = p.cols; a.batch = (int)nb; a.err = ctx->err_dev; a.sm_count = ctx->sm_count; a.part_scratch = ctx->qmm_scratch; a.part_scratch_bytes = ctx->qmm_scratch_bytes; a.part_counters = ctx->qmm_counters;
-            in.launches += 1;
             return run_normed_affine(in, p, l, kAffinePlain, a);
         }
         case PK_FUSED_NORM_GATEUP: {
@@ -1967,7 +1968,6 @@ smelt_status run_record(Interp& in, const smelt_dispatch_record& rec_in) {
             NEED_BYTES(6, (size_t)nb * p.cols * 2); NEED_BYTES(7, (size_t)nb * rows * 2); NEED_BYTES(9, (size_t)p.cols * 2);
             a.x = (const __half*)r.buf[6].ptr; a.y = (__half*)r.buf[7].ptr; a.norm_w = (const __half*)r.buf[9].ptr; a.norm_eps = as_f32(eps_bits);
             a.rows = (int)rows; a.cols = p.cols; a.batch = (int)nb; a.err = ctx->err_dev; a.sm_count = ctx->sm_count; a.part_scratch = ctx->qmm_scratch; a.part_scratch_bytes = ctx->qmm_scratch_bytes; a.part_counters = ctx->qmm_counters;
-            in.launches += 1;
             return run_normed_affine(in, p, l, kAffineGateUp, a);
         }
         case PK_ROPE_QKV_APPEND: {

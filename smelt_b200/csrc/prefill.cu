@@ -454,7 +454,12 @@ smelt_status smelt_cuda_prefill(smelt_cuda_ctx* ctx, const smelt_decoder_desc* d
 
     const uint8_t* W = (const uint8_t*)ws.ptr;
     const float log2_theta = log2f(d->rope_theta), scale = 1.0f / sqrtf((float)D);
-    size_t launches = 0;
+    int launches = 0;
+    auto counted = [&] {
+        Launch l = lch(ctx);
+        l.launches = &launches;
+        return l;
+    };
     auto affine = [&](int mode, const smelt_affine_ref& w0, const smelt_affine_ref* w1, const __half* x, __half* y, __half* y2, const __half* res,
                       int rows, int cols, int n) {
         AffineArgs a = {};
@@ -463,7 +468,7 @@ smelt_status smelt_cuda_prefill(smelt_cuda_ctx* ctx, const smelt_decoder_desc* d
         a.x = x; a.y = y; a.y2 = y2; a.residual = res; a.rows = rows; a.cols = cols; a.batch = n; a.nseg = 1;
         a.sm_count = ctx->sm_count; a.err = ctx->err_dev;
         a.part_scratch = ctx->qmm_scratch; a.part_scratch_bytes = ctx->qmm_scratch_bytes; a.part_counters = ctx->qmm_counters;
-        return launch_affine(lch(ctx), mode, a, G);
+        return launch_affine(counted(), mode, a, G);
     };
     // Q | K | V as one line of work, whose tiles fill the SMs better (Q 32 tiles, K and V 8 each at width 4096) and whose group sums are made
     // once; where several tensors are not taken: one launch for Q, one for K and V.  77 tokens, each launch alone
@@ -479,20 +484,21 @@ smelt_status smelt_cuda_prefill(smelt_cuda_ctx* ctx, const smelt_decoder_desc* d
             a.x = x; a.rows = qd + 2 * kvd; a.cols = H; a.batch = n; a.nseg = 3;
             a.sm_count = ctx->sm_count; a.err = ctx->err_dev;
             a.part_scratch = ctx->qmm_scratch; a.part_scratch_bytes = ctx->qmm_scratch_bytes; a.part_counters = ctx->qmm_counters;
-            const cudaError_t e = launch_affine(lch(ctx), kAffinePlain, a, G);
+            const cudaError_t e = launch_affine(counted(), kAffinePlain, a, G);
             if (e != cudaErrorNotSupported) return e;
             together = false;
         }
-        ++launches;
         const cudaError_t e = affine(kAffinePlain, w.q, nullptr, x, qb, nullptr, nullptr, qd, H, n);
         return e != cudaSuccess ? e : affine(kAffineDual, w.k, &w.v, x, kb, vb, nullptr, kvd, H, n);
     };
-#define PF(call, what)                                        \
+#define PFN(call, n, what)                                    \
     do {                                                      \
         smelt_status s_ = check_cuda(ctx, (call), what);      \
         if (s_) return s_;                                    \
-        ++launches;                                           \
+        launches += n;                                        \
     } while (0)
+#define PF(call, what) PFN(call, 1, what)
+#define PFA(call, what) PFN(call, 0, what)  // counts its launches itself
     for (int t0 = 0; t0 < n_tokens; t0 += T) {
         const int n = std::min(T, n_tokens - t0);
         const uint32_t p0 = (uint32_t)start_pos + (uint32_t)t0;
@@ -509,13 +515,13 @@ smelt_status smelt_cuda_prefill(smelt_cuda_ctx* ctx, const smelt_decoder_desc* d
             __half* kc = (__half*)ctx->slots[kKvBase + li].ptr;
             __half* vc = (__half*)ctx->slots[kKvBase + L + li].ptr;
             PF(launch_rms_norm_1pw(l, x0, (const __half*)(W + w.input_norm), xn, H, d->eps, n), "prefill: input norm");
-            PF(qkv(w, xn, n), "prefill: Q | K | V projection");
+            PFA(qkv(w, xn, n), "prefill: Q | K | V projection");
             PF(launch_rope_kv_prefill(l, qb, kb, vb, nullptr, nullptr, kc, vc, D, D, d->n_q, d->n_kv, (uint32_t)n, p0, cap, 1, log2_theta, 1, 0), "prefill: rope + kv write");
             PF(launch_attention_prefill(l, qb, kc, vc, ab, d->n_q, d->n_kv, D, (uint32_t)n, p0, cap, scale, 0, ctx->sm_count), "prefill: attention");
-            PF(affine(kAffineAdd, w.o, nullptr, ab, x1, nullptr, x0, H, qd, n), "prefill: O projection + residual");
+            PFA(affine(kAffineAdd, w.o, nullptr, ab, x1, nullptr, x0, H, qd, n), "prefill: O projection + residual");
             PF(launch_rms_norm_1pw(l, x1, (const __half*)(W + w.post_norm), xn, H, d->eps, n), "prefill: post norm");
-            PF(affine(kAffineGateUp, w.gate, &w.up, xn, hb, nullptr, nullptr, I, H, n), "prefill: gate / up + SwiGLU");
-            PF(affine(kAffineAdd, w.down, nullptr, hb, x0, nullptr, x1, H, I, n), "prefill: down projection + residual");
+            PFA(affine(kAffineGateUp, w.gate, &w.up, xn, hb, nullptr, nullptr, I, H, n), "prefill: gate / up + SwiGLU");
+            PFA(affine(kAffineAdd, w.down, nullptr, hb, x0, nullptr, x1, H, I, n), "prefill: down projection + residual");
         }
         if (t0 + n == n_tokens) {
             // the last position only: final norm, LM head, argmax (the decode table's tail)
@@ -528,7 +534,9 @@ smelt_status smelt_cuda_prefill(smelt_cuda_ctx* ctx, const smelt_decoder_desc* d
             PF(launch_argmax_reduce(l, (const uint64_t*)ctx->slots[kArgmaxScratch].ptr, (int32_t*)ctx->slots[kArgmax].ptr, parts, 1, 1), "prefill: argmax");
         }
     }
+#undef PFA
 #undef PF
+#undef PFN
     ctx->launch_count = launches;
     cudaMemcpyAsync(ctx->h_pinned + 128, ctx->slots[kArgmax].ptr, 4, cudaMemcpyDeviceToHost, ctx->stream);
     smelt_status s = check_cuda(ctx, cudaStreamSynchronize(ctx->stream), "prefill");

@@ -165,6 +165,16 @@ def test_fused_table_of_many_sequences_takes_any_image(ctx, batch):
     assert e.value.status == capi.BAD_ARGUMENT and ctx.device_error() == 0
 
 
+@pytest.mark.parametrize("batch,fuse,per_layer,once", [(8, 3, 5, 6), (9, 3, 7, 6), (17, 3, 7, 6), (17, 1, 11, 5)])
+def test_launch_count(ctx, batch, fuse, per_layer, once):
+    """What smelt_cuda_last_launch_count says of a step: norms that become launches of their own (gate / up from nine sequences on,
+    Q | K | V from seventeen) are counted, and so are two streamed passes; products that take all rows at once count once."""
+    cfg = MID
+    _, dec = make(ctx, cfg, 10, 32, batch=batch, fuse=fuse)
+    dec.decode_step(np.zeros(batch, np.int32), 0)
+    assert ctx.lib.smelt_cuda_last_launch_count(ctx.h) == cfg.layers * per_layer + once
+
+
 def test_runtime_errors(ctx):
     pkg, dec = make(ctx, SMALL, 3, 16)
     st = ctx.lib.smelt_cuda_decode_step(ctx.h, dec.table, dec.n_records, np.array([0], np.int32).ctypes.data_as(C.c_void_p), 16, None)
