@@ -110,11 +110,7 @@ __device__ __forceinline__ uint32_t lds_word(uint32_t a) {
     asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
     return v;
 }
-__device__ __forceinline__ bool wait_one(uint32_t bar, uint32_t parity, uint32_t dead) {
-    const bool ok = mbar_wait_short(bar, parity);
-    if (!ok) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(dead), "r"(1u) : "memory");
-    return ok;
-}
+__device__ __forceinline__ bool wait_one(uint32_t bar, uint32_t parity, uint32_t dead) { return wait_alive_short(bar, parity, dead); }
 __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, uint32_t dead) { return __all_sync(0xffffffffu, wait_one(bar, parity, dead)); }
 __device__ __forceinline__ Part uniform(const Part& t) {
     return {uniform(t.tile), uniform(t.s0), uniform(t.s1), uniform(t.row_tile), uniform(t.col_tile), uniform(t.col0), uniform(t.live)};

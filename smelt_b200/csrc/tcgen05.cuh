@@ -12,10 +12,11 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 // Bounded wait on an mbarrier phase: try_wait suspends the thread in hardware for up to the hinted
 // time (a spinning warp would take issue slots from the warp that shares its scheduler), the
-// loop gives up after about a second and reports failure instead of waiting forever.
+// loop gives up after about a second and reports failure instead of waiting forever: a try that fails takes
+// 4.0 us, with the hint of one as without a hint (256 to 1024 tries in a row, a warp alone or 24).
 __device__ __forceinline__ bool mbar_poll_bounded(uint64_t* bar, uint32_t parity) {
 #pragma unroll 1
-    for (uint32_t i = 0; i < (1u << 20); ++i) {
+    for (uint32_t i = 0; i < (1u << 18); ++i) {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -31,7 +32,7 @@ __device__ __forceinline__ bool mbar_poll_bounded(uint64_t* bar, uint32_t parity
 // Waits for a phase; gives up after about a second, or as soon as another role has.
 __device__ __forceinline__ bool wait_alive(uint64_t* bar, uint32_t parity, volatile uint32_t* dead) {
 #pragma unroll 1
-    for (uint32_t i = 0; i < (1u << 20); ++i) {
+    for (uint32_t i = 0; i < (1u << 18); ++i) {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -46,25 +47,30 @@ __device__ __forceinline__ bool wait_alive(uint64_t* bar, uint32_t parity, volat
     *dead = 1u;
     return false;
 }
-// Waits for a phase; gives up after 2^23 tries, each of which suspends the thread in hardware for 0.1 us or so (a spinning warp would take
-// issue slots from the warps that share its scheduler).  As little code as that takes, for kernels whose roles compete for the
-// instruction cache: without the instruction's time hint, with which the compiler makes a timed loop around every wait (the 16-bit product, whose
-// waits are few, is 1 % faster with it), and without a look at a clock or at other roles.
-__device__ __forceinline__ bool mbar_wait_short(uint32_t bar, uint32_t parity) {
+// The same with as little code as it takes, for kernels whose roles compete for the instruction cache: without the instruction's time
+// hint, with which the compiler makes a timed loop around every wait (the 16-bit product, whose waits are few, is 1 % faster with it).  2^18
+// tries are a second here too.
+// bar, dead: addresses of shared memory.
+__device__ __forceinline__ bool wait_alive_short(uint32_t bar, uint32_t parity, uint32_t dead) {
     uint32_t ok;
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\t"
-        "mov.u32 n, 0;\n"
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n, d;\n\t"
+        "mov.u32 n, 262144;\n"
         "again_%=:\n\t"
         "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
         "@p bra through_%=;\n\t"
-        "add.u32 n, n, 1;\n\t"
-        "setp.lt.u32 q, n, 8388608;\n\t"
-        "@q bra again_%=;\n"
+        "ld.volatile.shared.u32 d, [%3];\n\t"
+        "sub.u32 n, n, 1;\n\t"
+        "setp.ne.u32 q, d, 0;\n\t"
+        "@q bra through_%=;\n\t"
+        "setp.ne.u32 q, n, 0;\n\t"
+        "@q bra again_%=;\n\t"
+        "mov.u32 d, 1;\n\t"
+        "st.volatile.shared.u32 [%3], d;\n"
         "through_%=:\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "r"(dead)
         : "memory");
     return ok != 0;
 }
