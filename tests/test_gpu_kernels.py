@@ -269,6 +269,35 @@ def test_affine_wide_one_sided_groups(ctx, rows, cols, batch):
         buf.free()
 
 
+# more rows of x than have room for their group sums in scratch (10240 of 17408 columns): two launches, each with its part of x, of the
+# residual and of both outputs
+def test_affine_wide_rows_beyond_scratch(ctx):
+    rows, cols, batch = 40, 17408, 10300
+    a, b = (synth.affine_u4(44, n, rows, cols, 64) for n in ("ba", "bb"))
+    rng = synth.rng_for(44, "bx")
+    x = rng.standard_normal(size=(64, cols), dtype=np.float32).astype(np.float16)[rng.integers(0, 64, batch)]  # many rows of a few values
+    res = synth.activations(44, "bres", batch, rows)
+    d = dev(ctx, *a, *b, x, res)
+    y0, y1 = ctx.alloc(batch * rows * 2 + 64).fill(0xFF), ctx.alloc(batch * rows * 2 + 64).fill(0xFF)
+
+    def exact(w, s, b):
+        q = np.stack([w & 15, w >> 4], -1).reshape(rows, cols // 64, 64).astype(np.float64)
+        u, at = np.unique(x[:, :8].view(np.uint64)[:, 0], return_index=True)
+        out = x[at].astype(np.float64) @ (q * s.astype(np.float64)[..., None] + b.astype(np.float64)[..., None]).reshape(rows, cols).T
+        return out[np.searchsorted(u, x[:, :8].view(np.uint64)[:, 0])]
+
+    ref_a, ref_b = exact(*a), exact(*b)
+    ctx.call("affine_dual_matvec", *d[:7], y0, y1, rows, cols, 64, batch)
+    assert rel_err(y0.download(np.float16, (batch, rows)), ref_a) < REL_TOL and rel_err(y1.download(np.float16, (batch, rows)), ref_b) < REL_TOL
+    ctx.call("affine_matvec_add", *d[:3], d[6], d[7], y0, rows, cols, 64, batch)
+    assert add_rel_err(y0.download(np.float16, (batch, rows)), ref_a.astype(np.float16).astype(np.float64) + res, ref_a) < REL_TOL
+    for y in (y0, y1):
+        assert np.all(y.download(np.uint8, (64,), offset=batch * rows * 2) == 0xFF)
+    assert ctx.device_error() == 0
+    for buf in d + [y0, y1]:
+        buf.free()
+
+
 # beyond 64 rows of x, where the last group sums of a row belong to a stage of two groups and the turns that multiply them come closest:
 # several such rows a CTA, also with nothing else in them; the bound is that of test_affine_wide_rounds_like_exact_sums
 @pytest.mark.parametrize("rows,cols,batch", [(12296, 1152, 128), (40000, 128, 512), (12296, 1152, 300)])

@@ -175,6 +175,45 @@ def test_launch_count(ctx, batch, fuse, per_layer, once):
     assert ctx.lib.smelt_cuda_last_launch_count(ctx.h) == cfg.layers * per_layer + once
 
 
+def test_kernel_attributes_across_contexts_and_threads():
+    """A kernel's shared-memory limit is set when a launch first needs more and again after another context has been made: the
+    same bits from a context, from one that was made when the first was gone, and from two at once in threads of their own, whose
+    launches ask for small and large limits in different orders."""
+    import threading
+
+    shapes = [(256, 1024, 1), (136, 12288, 8), (256, 4096, 2), (264, 8192, 4), (136, 4096, 17), (72, 17408, 3)]
+    weights = [synth.affine_u4(12, f"w{i}", r, c, 64) for i, (r, c, _) in enumerate(shapes)]
+    xs = [synth.activations(12, f"x{i}", b, c) for i, (_, c, b) in enumerate(shapes)]
+
+    def run(ctx, order):
+        out = {}
+        for i in order:
+            r, c, b = shapes[i]
+            d, y = [ctx.to_device(a) for a in (*weights[i], xs[i])], ctx.alloc(b * r * 2)
+            ctx.call("affine_matvec", *d, y, r, c, 64, b)
+            out[i] = y.download(np.uint16, (b, r))
+            for buf in d + [y]:
+                buf.free()
+        return out
+
+    first = capi.Context(0)
+    want = run(first, range(len(shapes)))
+    first.close()
+    second, third, got = capi.Context(0), capi.Context(0), {}
+    threads = [threading.Thread(target=lambda c=c, o=o, k=k: got.update({k: run(c, o)})) for k, (c, o) in
+               enumerate([(second, [5, 4, 3, 2, 1, 0] * 4), (third, [0, 3, 1, 4, 2, 5] * 4)])]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in (0, 1):
+        for i in range(len(shapes)):
+            assert np.array_equal(got[k][i], want[i]), (k, i)
+    assert second.device_error() == 0 and third.device_error() == 0
+    second.close()
+    third.close()
+
+
 def test_runtime_errors(ctx):
     pkg, dec = make(ctx, SMALL, 3, 16)
     st = ctx.lib.smelt_cuda_decode_step(ctx.h, dec.table, dec.n_records, np.array([0], np.int32).ctypes.data_as(C.c_void_p), 16, None)
