@@ -17,7 +17,7 @@
 // More: the sums are kept as two tf32 values each, and the biases of up to sixteen groups multiply them on the tensor core as one
 // more turn; c is chosen for each group, to the nearest eighth, so that these operands are small (tf32_bias).  With c = 8, x of mean 0.5 and biases
 // of -7.5 scales, 0.24 % of the results of 4096 columns were misrounded (before the tensor core had the biases: 0.11 %), now 0.07; it costs
-// 1 to 3 % of the time.
+// 1 % of the time.
 // (The epilogue's way with 64 rows: 50.2 | 31.0 | 15.2 us of the shapes below; the tensor core's with 32 rows 31.8 | 20.2 | 11.0, a turn
 // more for each of a CTA's short stretches, and a step of 32 sequences 3.88 ms instead of 3.75.)
 //
@@ -174,7 +174,9 @@ __device__ __forceinline__ void tmem_st8(uint32_t t, const uint32_t (&v)[8]) {
 // small beside the result.  q - c is exact in fp16 up to |c| = 240; bias + c scale, at most a sixteenth of the scale, has no more than
 // eleven bits, so that a tf32 operand holds it.  Else (a scale of zero, a bias beyond 240 scales) c is 0.  minus: -c / 512 twice.
 __device__ __forceinline__ float tf32_bias(float s, float b, uint32_t* minus) {
-    const float k = __fadd_rn(__fadd_rn(__fdividef(-8.f * b, s), 12582912.f), -12582912.f), t = fmaf(0.125f * k, s, b);  // nearest whole number
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
+    const float k = __fadd_rn(fmaf(-8.f * b, r, 12582912.f), -12582912.f), t = fmaf(0.125f * k, s, b);  // k: to the nearest whole number
     const bool centred = fabsf(k) <= 1920.f && (__float_as_uint(t) & 0x1FFFu) == 0u;
     *minus = centred ? h2_as_u32(__float2half2_rn(k * (-1.f / 4096.f))) : 0u;
     return centred ? t : b;
