@@ -10,7 +10,7 @@
 // dequantised weight summed over two groups (before -> now): 4096 x 4096, 32 rows 0.12 -> 0.08 %, 512 rows 0.12 -> 0.08; gate and
 // up 12288 x 4096, 32 rows 0.20 -> 0.15, 512 rows 0.21 -> 0.15.  Up to 32 rows the four groups of a turn are added up before they meet the
 // running sum, which rounds once for them: with two roundings a group, 5120 x 17408 had 0.16 % at 8 rows and 0.17 at 32, where the kernels
-// in front have 0.09 and 0.14; now 0.09 and 0.09 (4096 x 12288 + residual, 9 rows: 0.024, in front 0.020, now 0.008).  It costs 1 %.
+// in front have 0.09 and 0.14; now 0.09 and 0.09 (4096 x 12288 + residual, 9 rows: 0.024, in front 0.020, now 0.008).  It costs nothing.
 //
 // bias * sum(x).  Tiles of up to 64 rows of x: four warps sum x from shared memory.  More: the sums are made once in front
 // (group_sums_kernel), as they would cost every CTA four warps' issue slots.  Tiles of up to 32 rows: the epilogue adds the products in fp32.
@@ -470,6 +470,20 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                     uint32_t v[4][16];
 #pragma unroll
                     for (int q = 0; q < 4; ++q) tmem_ld16(lane_base + slot.i * 128 + q / kChunks * N + q % kChunks * 16, v[q]);
+                    float part[C::kFolded ? 16 : 1];  // of this turn: the running sums, much larger, round once a turn and not twice a group
+                    const uint32_t x_sums = folded + sum.i * (C::kTurn * N * 4) + from * 4;
+                    auto add_biases = [&](int q) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const uint4 xs = lds128(x_sums + q * (N * 4) + 16 * j);
+                            float* to = part + 4 * j;
+                            to[0] = q == 0 ? __uint_as_float(xs.x) * b1[0] : fmaf(__uint_as_float(xs.x), b1[q], to[0]);
+                            to[1] = q == 0 ? __uint_as_float(xs.y) * b1[0] : fmaf(__uint_as_float(xs.y), b1[q], to[1]);
+                            to[2] = q == 0 ? __uint_as_float(xs.z) * b1[0] : fmaf(__uint_as_float(xs.z), b1[q], to[2]);
+                            to[3] = q == 0 ? __uint_as_float(xs.w) * b1[0] : fmaf(__uint_as_float(xs.w), b1[q], to[3]);
+                        }
+                    };
+                    if constexpr (C::kFolded) add_biases(0);  // while the accumulators are on their way: two groups ahead are slower, four spill
 #pragma unroll
                     for (int q = 0; q < 4; ++q) tmem_wait_ld16(v[q]);
                     tc_fence_before();
@@ -478,26 +492,15 @@ __global__ void __launch_bounds__(WideCfg<N>::kThreads, 1) affine_wide_kernel(co
                     slot.next();
                     end.next();
                     if constexpr (C::kFolded) {
-                        float part[16];  // of this turn: the running sums, much larger, round once a turn and not twice a group
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
                             if (q < m) {
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) part[j] = q == 0 ? __uint_as_float(v[0][j]) * s1[0] : fmaf(__uint_as_float(v[q][j]), s1[q], part[j]);
+                                for (int j = 0; j < 16; ++j) part[j] = fmaf(__uint_as_float(v[q][j]), s1[q], part[j]);
                             }
-                        const uint32_t x_sums = folded + sum.i * (C::kTurn * N * 4) + from * 4;
 #pragma unroll
-                        for (int q = 0; q < 4; ++q)
-                            if (q < m) {
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    const uint4 xs = lds128(x_sums + q * (N * 4) + 16 * j);
-                                    part[4 * j] = fmaf(__uint_as_float(xs.x), b1[q], part[4 * j]);
-                                    part[4 * j + 1] = fmaf(__uint_as_float(xs.y), b1[q], part[4 * j + 1]);
-                                    part[4 * j + 2] = fmaf(__uint_as_float(xs.z), b1[q], part[4 * j + 2]);
-                                    part[4 * j + 3] = fmaf(__uint_as_float(xs.w), b1[q], part[4 * j + 3]);
-                                }
-                            }
+                        for (int q = 1; q < 4; ++q)
+                            if (q < m) add_biases(q);
                         __syncwarp();
                         if (lane == 0) arrive_at(bar(C::kSumEmpty, sum.i));
                         sum.next();
