@@ -18,38 +18,40 @@ EncodeTiled encode_tiled() {
     return fn;
 }
 
-// How many CTAs take the line: either a whole number for each tile, or all SMs, whose stretches then begin and end anywhere.
-// Estimated in us.  A stage takes a CTA 0.99 us in tiles of 32 rows of x, 1.6 of 64 and 1.65 of 128; a tile of k CTAs needs 1 us and 0.018,
-// 0.013 or 0.016 a row of x (of 32 at least) for each of them more; stretches that begin anywhere 3 us and 1.3 times as much for each of the CTAs that may share
-// a tile; tiles of 64 rows begin 0.75 us later than those of 32, of 128, whose group sums are made in front, 2.5 us.  Where a row's groups are
-// no multiple of four, scales come two bytes at a time: 0.2 us more for a stage of tiles of 32, 0.5 beyond those that are fetched ahead, and
-// 5 us more for tiles of 128 (+ residual 3280 x 8064, 130 rows, 32 stages a CTA: 53.5 in tiles of 32; plain 4096 x 4096 and x 6976, 128
-// rows: 23.5 and 35.1 in tiles of 128).
-// Measured (us, by CTAs of a tile; 148: all SMs): 1024 x 12288, 32 rows: 4 17.3, 8 13.8, 16 15.0, 148 18.5; 128 rows: 4 34.0, 6 29.9, 8 31.4,
-// 16 43.7, 148 49.1; 4096 x 4096, 32 rows: 2 13.1, 4 10.8, 148 12.5; 128 rows: 4 23.3, 148 27.7; 4096 x 12288, 64 rows: 4 31.1, 148 32.1;
-// gate/up 6144 x 2048, 32 rows: 1 12.1, 148 14.5; 512 rows: 148 63.8 (three waves of whole tiles would be 3 x 16).
+// How many CTAs take the line: either a whole number for each tile, or all SMs, whose stretches then begin and end anywhere.  Estimated in us, for
+// tiles of up to 32 | 64 | 128 rows of x (fitted to 4,400 timings of 566 shapes, 256 to 12288 rows, 512 to 12288 columns, 33 to 512 rows of x, each
+// width both ways; off by 8 % rms):
+//   * a launch 1.7 | 1.65 | 3.0 (group sums made in front), a stage 1.0 | 1.55 | 1.6;
+//   * a tile that s CTAs share 1.5, in stretches 3.3, and 0.0175 | 0.0125 | 0.016 for each of them and row of x (of 32 at least);
+//   * the end of a tile 0.05 for each row of x;
+//   * where a row's groups are no multiple of four, scales come two bytes at a time: a launch 0.9 | 0.15 | 0 more, a stage of 128 rows 0.2, and
+//     stages beyond those that are fetched ahead 0.45 | 0.1 | 0.3.
+// Measured (us, by CTAs of a tile; 148: all SMs): 1024 x 12288, 32 rows: 4 17.3, 8 13.8, 16 15.0, 148 18.5; 4096 x 4096, 32 rows: 2 13.1, 4 10.8,
+// 148 12.5; 4096 x 12288, 64 rows: 4 31.1, 148 32.1; gate/up 6144 x 2048, 32 rows: 1 12.1, 148 14.5.
 int ctas_for(const Line& p, int sm, int* per_tile, double* cost_us) {
-    const long tiles = (long)p.row_tiles * p.col_tiles;
+    const long tiles = (long)p.row_tiles * p.col_tiles, units = tiles * p.stages, all = std::min((long)sm, units);
     const bool odd = p.groups % kStageGroups != 0;
-    struct { double stage, late, sum, begin; } const width[3] = {{odd ? 1.19 : 0.99, odd ? 0.3 : 0.0, 0.018, 0.0}, {1.6, 0.0, 0.013, 0.75}, {1.65, 0.0, 0.016, odd ? 7.5 : 2.5}};
+    struct { double begin, stage, late, sum; } const width[3] = {{odd ? 2.6 : 1.7, 1.0, odd ? 0.45 : 0.0, 0.0175}, {odd ? 1.8 : 1.65, 1.55, odd ? 0.1 : 0.0, 0.0125}, {3.0, odd ? 1.8 : 1.6, odd ? 0.3 : 0.0, 0.016}};
     const auto& w = width[p.tile_cols <= 32 ? 0 : p.tile_cols <= 64 ? 1 : 2];
-    const double sum = w.sum * std::max(p.tile_cols, 32);
-    auto stages = [&](double n) { return n * w.stage + std::max(0.0, n - 6.0) * w.late; };
+    auto cost = [&](long stages, double sharers, double tiles_each, double share) {
+        return w.begin + (double)stages * w.stage + (double)std::max(0l, stages - 6) * w.late + (sharers > 1.0 ? share + w.sum * std::max(p.tile_cols, 32) * sharers : 0.0) +
+               0.05 * p.tile_cols * tiles_each;
+    };
     *per_tile = 0;
-    double least = stages((double)tiles * p.stages / sm) + 3.0 + 1.3 * sum * ((double)sm / tiles + 1.0);
+    double least = cost((units + all - 1) / all, std::min((double)p.stages, (double)sm / tiles + 1.0), std::max(1.0, (double)tiles / sm), 3.3);
     for (int k = 1; k <= p.stages && tiles * k <= sm; ++k) {
-        const double cost = stages((p.stages + k - 1) / k) + (k > 1 ? 1.0 + sum * k : 0.0);
-        if (cost < least) { least = cost; *per_tile = k; }
+        const double c = cost((p.stages + k - 1) / k, k, 1.0, 1.5);
+        if (c < least) { least = c; *per_tile = k; }
     }
-    *cost_us = least + w.begin;
-    return (int)(*per_tile ? tiles * *per_tile : std::min((long)sm, tiles * p.stages));
+    *cost_us = least;
+    return (int)(*per_tile ? tiles * *per_tile : all);
 }
 
 // How many rows of x a tile has: 32, 64 or 128, whichever ctas_for's estimate says is fastest.  Narrow tiles expand the weights more often, but a small
 // matrix has few tiles, SMs idle, and a wide tile's sums take longest to put together.  us, in tiles of 32 | 64 | 128: plain 1024 x 1536, 77 rows
 // 8.2 | 10.6 | 15.0, 512 rows 9.9 | 12.8 | 17.4; gate/up 1024 x 2048, 40 rows 9.1 | 11.4, 300 rows 17.1 | 17.8 | 19.9; plain 4096 x 4096, 64 rows
-// 14.4 | 15.5, 77 rows 19.0 | 19.3 | 18.6, 128 rows 19.7 | 20.3 | 23.5; gate/up 12288 x 4096, 64 rows 55 | 45, 128 rows 99 | 78 | 57.  Of 1700 shapes (256 to 12288 rows, 512
-// to 12288 columns, 33 to 512 rows of x) the choice is 0.2 % slower than the best on average, 15 % at most.
+// 14.4 | 15.5, 77 rows 19.0 | 19.3 | 18.6, 128 rows 19.7 | 20.3 | 23.5; gate/up 12288 x 4096, 64 rows 55 | 45, 128 rows 99 | 78 | 57.  Of the 566 shapes the choice
+// is 0.3 % slower than the best on average, 15 % at most.
 void choose_tile(Line* p, int batch, int max_cols, int sm) {
     Line best = {};
     double least = 0.0;
