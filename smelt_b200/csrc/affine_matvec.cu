@@ -451,12 +451,15 @@ cudaError_t launch_group(const Launch& l, const AffineArgs& a, int group) {
 //   * 17 rows and more: always.  A folded norm is a launch of its own then.
 //   * 9 to 16 rows: gate/up, dual and + residual, where the streaming kernel needs two passes or more: gate/up 12288 x 4096, 9 rows
 //     38.7 : 30.0, 16 rows 46.5 : 29.2; 6144 x 2048, 9 rows 15.4 : 11.7; 4096 x 12288 + residual, 9 rows 32.7 : 17.6; 2048 x 2048, 9 rows
-//     7.5 : 7.0.  Plain products only where the streaming kernel does not take them (264 x 17408, 9 rows 28.4 : 12.7): one launch over
+//     7.5 : 7.0.  Plain products only where the streaming kernel does not take them (1024 x 2496, 9 rows 9.0 : 7.3): one launch over
 //     several tensors (affine_multi_matvec) runs on it up to 16 rows, and gives the bits of a launch for each.  Not in the general kernel's one
-//     round of eight warps, 1024 to 2048 columns, where x is hardly more than the eight rows that it takes at once: plain products up to 12
-//     rows, + residual 10 (1024 x 1536 plain, 9 rows 5.7 : 6.8, 12 rows 6.8 : 6.8, + residual, 9 rows 6.5 : 7.1, 10 rows 7.0 : 7.1; 5440 x 1856
-//     plain, 12 rows 9.4 : 10.2, + residual, 10 rows 9.5 : 10.4; 1024 x 768, 9 rows 5.3 : 5.1; 1024 x 2496, 9 rows 9.0 : 7.3; dual 4096 x 1664, 9 rows 11.2 :
-//     11.0).
+//     round of eight warps, 1024 to 2048 columns, where x is hardly more than the eight rows that it takes at once: plain products of up to
+//     10 rows of x and 2048 rows of weights.  Where a row's groups are no multiple of four, which the product likes less, up to as many rows of
+//     weights as three CTAs an SM take in one wave (7104; 6144 below 1280 columns), 11 rows of x from 4096 on.  + residual: 9 rows of x and
+//     1024 of weights, or then from 4096 on.  Plain 1024 x 1536, 9 rows 5.7 : 6.8, 10 rows 6.1 : 6.8, 11 rows 6.5 : 6.8; 4096 x 1664, 9 rows
+//     7.4 : 8.8, 11 rows 8.3 : 8.7; 6656 x 1856, 9 rows 9.0 : 10.8; 6656 x 1088, 9 rows 7.9 : 6.8; 4096 x 1536, 9 rows 8.0 : 7.7; 7168 x 1536,
+//     9 rows 13.9 : 8.3; 1024 x 960, 10 rows equal; + residual 1024 x 1536, 9 rows 6.5 : 7.1, 10 rows 7.0 : 7.1; 3072 x 1664, 9 rows 7.9 : 7.6;
+//     dual 4096 x 1664, 9 rows 11.2 : 11.0.
 //   * 6 to 8 rows, plain and + residual, that the streaming kernel does not take because their activations do not stay resident, from
 //     128 M weights x rows on: the general kernel takes about 2 + 0.08 us for a million of these, the product 8 + 0.2 for a million
 //     weights.  8 rows: 4096 x 12288 29.5 : 17.7, 2048 x 12288 18.9 : 12.2, 1024 x 17408 17.6 : 13.4, 1024 x 12288 9.4 : 11.9;
@@ -465,8 +468,13 @@ bool wide_first(int mode, const AffineArgs& a, int group) {
     if (a.batch >= 17) return true;
     if (a.batch <= 5 || a.nseg > 1) return false;
     const bool streamed = affine_stream_passes(mode, a, group) != 0;
-    const bool one_round = a.cols > 768 && a.cols < 2048 && a.rows < 8192;
-    if (a.batch >= 9) return streamed ? mode != kAffinePlain : !(one_round && a.batch <= (mode == kAffinePlain ? 12 : mode == kAffineAdd ? 10 : 0));
+    const bool odd = a.cols % 256 != 0, one_round = a.cols > 1024 && a.cols < 2048;
+    if (a.batch >= 9 && !streamed && one_round) {
+        const bool wave = odd && a.rows <= (a.cols >= 1280 ? 48 * (a.sm_count > 0 ? a.sm_count : 148) : 6144);
+        if (mode == kAffinePlain) return a.batch > (wave && a.rows >= 4096 ? 11 : 10) || (a.rows > 2048 && !wave);
+        return mode != kAffineAdd || a.batch > 9 || (a.rows > 1024 && !(wave && a.rows >= 4096));
+    }
+    if (a.batch >= 9) return mode != kAffinePlain || !streamed;
     return (mode == kAffinePlain || mode == kAffineAdd) && !streamed && (size_t)a.rows * a.cols * a.batch >= (size_t)128 << 20;
 }
 

@@ -179,7 +179,8 @@ WIDE_EDGES = [(r, c, b) for r, c in [(8, 64), (72, 192), (264, 576), (1000, 1984
 
 
 # and fewer rows whose activations do not stay resident beside the streamed weights
-@pytest.mark.parametrize("rows,cols,batch", WIDE_EDGES + [(136, 17408, 17), (24, 17408, 300), (136, 17408, 6), (136, 12288, 9), (264, 6976, 11), (72, 4096, 16)])
+@pytest.mark.parametrize("rows,cols,batch", WIDE_EDGES + [(136, 17408, 17), (24, 17408, 300), (136, 17408, 6), (136, 12288, 9), (264, 6976, 11), (72, 4096, 16),
+                                                       (264, 1600, 9), (1032, 1664, 10), (4104, 1344, 11), (264, 1856, 12)])  # 9 to 12 rows: the general kernel or the product
 def test_affine_wide_edges(ctx, oracle, rows, cols, batch):
     a, b = (synth.affine_u4(34, n, rows, cols, 64) for n in ("wa", "wb"))
     x, res = synth.activations(34, "wx", batch, cols), synth.activations(34, "wres", batch, rows)
