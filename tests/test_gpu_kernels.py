@@ -174,7 +174,7 @@ def test_affine_qmm_modes(ctx, oracle, rows, cols, batch):
 
 
 # the same product where its tiles, stages and shares of a tile end: one group, part of a stage, rows and columns that no tile
-# divides, tiles of one CTA and of several, each width of the accumulator
+# divides, tiles of one CTA and of several; matrices as small as these get tiles of 32 rows of x (wider: test_affine_wide_large_matrices)
 WIDE_EDGES = [(r, c, b) for r, c in [(8, 64), (72, 192), (264, 576), (1000, 1984), (2056, 320)] for b in (17, 64, 65, 130, 257)]
 
 
@@ -206,7 +206,7 @@ def test_affine_wide_edges(ctx, oracle, rows, cols, batch):
 # The tensor core truncates the sums it adds to, so no accumulator may hold more than a few of them: of fp32 sums of K products that
 # are rounded to nearest (relative error about 4e-7 here), 4e-7 / 2^-11 = 0.1 % lie on the other side of a rounding boundary of
 # fp16 than the exact product; four times that is allowed.
-@pytest.mark.parametrize("rows,cols,batch", [(1024, 4096, 32), (200, 12288, 64), (136, 12288, 9), (264, 4096, 130), (128, 1984, 300), (512, 12288, 300)])
+@pytest.mark.parametrize("rows,cols,batch", [(1024, 4096, 32), (200, 12288, 64), (136, 12288, 9), (264, 4096, 130), (128, 1984, 300), (512, 12288, 300), (12296, 1152, 48), (12296, 1152, 100)])
 def test_affine_wide_rounds_like_exact_sums(ctx, rows, cols, batch):
     w, s, b = synth.affine_u4(35, "rw", rows, cols, 64)
     x = synth.activations(35, "rx", batch, cols)
@@ -237,7 +237,7 @@ def test_affine_wide_running_sums(ctx, rows, cols, batch, mean):
 
 
 # weights beyond fp16's range, of which the nibble, the scale and the bias are not: they were never rounded to fp16
-@pytest.mark.parametrize("rows,cols,batch", [(72, 1984, 17), (136, 12288, 9), (128, 4096, 64), (264, 576, 130), (200, 512, 300)])
+@pytest.mark.parametrize("rows,cols,batch", [(72, 1984, 17), (136, 12288, 9), (128, 4096, 64), (264, 576, 130), (200, 512, 300), (12296, 1152, 64), (12296, 1152, 128)])
 def test_affine_wide_large_weights(ctx, oracle, rows, cols, batch):
     w, s, b = synth.affine_u4(36, "lw", rows, cols, 64)
     s[:, ::2], b[:, ::2] = 9000.0, -30000.0
@@ -250,9 +250,10 @@ def test_affine_wide_large_weights(ctx, oracle, rows, cols, batch):
     assert np.all(np.isfinite(want)) and rel_err(got, want) < REL_TOL
 
 
-# groups whose weights have one sign only, of all sizes of bias: beyond 32 rows of x the nibbles are centred by up to 128, and in one of sixty
-# groups or so not at all; the bound is that of test_affine_wide_rounds_like_exact_sums
-@pytest.mark.parametrize("rows,cols,batch", [(136, 4096, 32), (264, 4096, 64), (136, 4160, 65), (264, 4096, 128), (72, 12288, 129)])
+# groups whose weights have one sign only, of all sizes of bias: in tiles of more than 32 rows of x (the last three) the nibbles are centred by
+# up to 240, and in one of sixty groups or so not at all; the bound is that of test_affine_wide_rounds_like_exact_sums
+@pytest.mark.parametrize("rows,cols,batch", [(136, 4096, 32), (264, 4096, 64), (136, 4160, 65), (264, 4096, 128), (72, 12288, 129),
+                                             (12296, 1152, 64), (12296, 1152, 128), (6152, 1984, 300)])
 def test_affine_wide_one_sided_groups(ctx, rows, cols, batch):
     w, s, b = synth.affine_u4(37, "ow", rows, cols, 64)
     rng = np.random.default_rng(37)
