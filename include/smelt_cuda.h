@@ -629,9 +629,10 @@ SMELT_CUDA_API smelt_status smelt_cuda_affine_dual_matvec(smelt_cuda_ctx* ctx, c
  * rounding points).
  * affine_multi_matvec: rms_norm_1pw (norms.metal:9-67; skipped when norm_w_dev is NULL)
  * followed by up to three affine_matvec launches that share x (for example the Q, K and V
- * projections) in one kernel.  Needs group 64, cols a multiple of 1024, every tensor but the
- * last with rows a multiple of 16.  Nine to sixteen batch rows, and more with a norm, run as several
- * passes over the weights.  Up to sixteen rows the results are those of the separate launches bit for
+ * projections) in one kernel.  Needs group 64, cols a multiple of 1024, 16-byte aligned operands, every tensor but the
+ * last with rows a multiple of 16.  Nine to sixteen batch rows run as several
+ * passes over the weights; with more the norm is a launch of its own and the tensors are one
+ * tensor-core product.  Up to sixteen rows the results are those of the separate launches bit for
  * bit, except for three to eight rows of which x does not fit into shared memory (eight rows of 12288
  * columns), where these take another kernel; with more rows sums may be cut elsewhere along K. */
 typedef struct {
@@ -644,7 +645,8 @@ typedef struct {
 SMELT_CUDA_API smelt_status smelt_cuda_affine_multi_matvec(smelt_cuda_ctx* ctx, const smelt_affine_tensor* tensors, int n_tensors,
                                                            const void* x_dev, const void* norm_w_dev, float eps, int cols,
                                                            int group, int batch);
-/* rms_norm_1pw followed by fused_affine_gate_up_swiglu in one kernel. */
+/* rms_norm_1pw followed by fused_affine_gate_up_swiglu: up to eight batch rows in one kernel, with more a launch of the norm and
+ * one of the tensor-core product.  Needs what affine_multi_matvec needs of its operands, for any number of rows. */
 SMELT_CUDA_API smelt_status smelt_cuda_rmsnorm_affine_gate_up_swiglu(smelt_cuda_ctx* ctx, const void* gw_dev, const void* gs_dev,
                                                                      const void* gb_dev, const void* uw_dev, const void* us_dev,
                                                                      const void* ub_dev, const void* x_dev, const void* norm_w_dev,

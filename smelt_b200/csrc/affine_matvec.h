@@ -38,8 +38,9 @@ struct AffineArgs {
     AffineSeg seg[3];
     int ks, nsplit;        // filled by the launcher
     int sm_count;          // SMs of the device (0 = assume 148)
-    // Tensor-core product only: where CTAs that share a tile leave their fp32 sums
-    // (part_scratch_bytes bytes) and count their arrivals (one int per tile, 4096 of them,
+    // Tensor-core product only: where CTAs that share a tile leave their fp32 sums, behind them the group sums of x
+    // (tiles of more than 64 rows) and at the end the rows of a norm that is a launch of its own
+    // (part_scratch_bytes bytes), and where they count their arrivals (one int per tile, 4096 of them,
     // all zero between launches).  Launches that use them must not overlap on the device.
     float* part_scratch;
     size_t part_scratch_bytes;

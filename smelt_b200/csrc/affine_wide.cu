@@ -7,10 +7,10 @@
 // epilogue warps multiply what they drain by the scale and add it to fp32 registers.  The nibbles are centred (q - c, c = 8 up to 32 rows) and
 // the bias is bias + c scale, so that neither sum is much larger than the result.  The tensor core truncates what it adds to, here four
 // K = 16 products at a time.  Share of fp16 results that are not the correctly rounded ones, against two fp16 operands per
-// dequantised weight summed over two groups (before -> now): 4096 x 4096, 32 rows 0.12 -> 0.08 %, 512 rows 0.12 -> 0.08; gate and
-// up 12288 x 4096, 32 rows 0.20 -> 0.15, 512 rows 0.21 -> 0.15.  Up to 32 rows the four groups of a turn are added up before they meet the
+// dequantised weight summed over two groups (before -> now): 4096 x 4096, 32 rows 0.11 -> 0.07 %, 512 rows 0.11 -> 0.08; gate and
+// up 12288 x 4096, 32 rows 0.19 -> 0.10, 512 rows 0.19 -> 0.14.  Up to 32 rows the four groups of a turn are added up before they meet the
 // running sum, which rounds once for them: with two roundings a group, 5120 x 17408 had 0.16 % at 8 rows and 0.17 at 32, where the kernels
-// in front have 0.09 and 0.14; now 0.09 and 0.09 (4096 x 12288 + residual, 9 rows: 0.024, in front 0.020, now 0.008).  It costs nothing.
+// in front have 0.09 and 0.14; now 0.09 and 0.09 (4096 x 12288 + residual, 9 rows: 0.024, in front 0.020, now 0.009).  It costs nothing.
 //
 // bias * sum(x).  Tiles of up to 64 rows of x: four warps sum x from shared memory.  More: the sums are made once in front
 // (group_sums_kernel), as they would cost every CTA four warps' issue slots.  Tiles of up to 32 rows: the epilogue adds the products in fp32.
@@ -18,8 +18,8 @@
 // more turn; c is chosen for each group, to the nearest eighth, so that these operands are small (tf32_bias).  With c = 8, x of mean 0.5 and biases
 // of -7.5 scales, 0.24 % of the results of 4096 columns were misrounded (before the tensor core had the biases: 0.11 %), now 0.07; it costs
 // 1 % of the time.
-// (The epilogue's way with 64 rows: 50.2 | 31.0 | 15.2 us of the shapes below; the tensor core's with 32 rows 31.8 | 20.2 | 11.0, a turn
-// more for each of a CTA's short stretches, and a step of 32 sequences 3.88 ms instead of 3.75.)
+// (When that was decided: the epilogue's way with 64 rows of gate/up 12288 x 4096 50.2 us instead of 44.7; the tensor core's with 32 rows, a turn
+// more for each of a CTA's short stretches, a step of 32 sequences 3.88 ms instead of 3.75.)
 //
 // Mapping.  One CTA an SM takes a stretch of the launch's line of work (affine_line.cuh); a tile is 128 weight
 // rows, the MMA's M, by up to 128 rows of x, its N.  The roles, each on warps of its own, each a ring ahead of the next:
@@ -31,14 +31,14 @@
 //   * issue: two warps take turns;
 //   * sums and epilogue, eight warps: plain, + residual, SwiGLU of gate and up, dual.  A turn is 128 columns of tensor memory: four
 //     groups of 32 rows of x, two of 64, one of 128.
-// What bounds it: instruction issue (0.6 an SM quarter and clock, a third of it bookkeeping of the roles) and the handing over between
-// them.  What cost most on the way here: code beyond the 32 KB that the
-// instruction cache holds (wait loops unrolled by the compiler: 122 KB), spilled registers (the shared memory leaves no first-level
+// What bounds it: instruction issue (gate/up 12288 x 4096 with 32 | 64 | 512 rows: 0.60 | 0.66 | 0.72 an SM quarter and clock; the tensor pipe is
+// active 10 | 14 | 29 % of the cycles, DRAM 19 | 14 | 5) and the handing over between the roles.  What cost most on the way here: code
+// beyond what the instruction cache holds (wait loops unrolled by the compiler), spilled registers (the shared memory leaves no first-level
 // cache: a reload is an L2 round trip), waits with a time hint (a timed loop each), shared addresses made anew at every use, packed
 // FMAs (a move each).
 // us, graph replay over distinct weights, before -> now (gate/up 12288 x 4096 x 2 | 4096 x 12288 | 4096 x 4096): 32 rows
-// 58.4 -> 31.8 | 34.4 -> 20.2 | 15.5 -> 11.0; 64 rows 63.9 -> 44.7 | 40.0 -> 28.8 | 18.3 -> 15.2; 128 rows 74.6 -> 56.3 |
-// 43.5 -> 41.0 | 22.4 -> 23.0; 512 rows 227 -> 178 | 113 -> 89 | 51.5 -> 34.8.
+// 58.4 -> 30.7 | 34.5 -> 18.4 | 15.6 -> 10.7; 64 rows 63.8 -> 44.4 | 38.3 -> 27.4 | 18.4 -> 14.0; 128 rows 74.4 -> 55.9 |
+// 41.4 -> 37.3 | 22.5 -> 19.0; 512 rows 243 -> 181 | 105 -> 84 | 51.5 -> 35.1.
 // A launch in front may take longer than a wait may (its waits on a peer are as long): every role waits for it before the first
 // wait that depends on the activations, and only what needs none of them goes ahead.
 // Every wait is bounded: on expiry the CTA sets bit 10 of the error word, its roles stop, copies and MMAs in flight are

@@ -304,7 +304,7 @@ __device__ __forceinline__ __half gated_norm_d128_value(__half x, __half g, __ha
 enum : uint32_t { KERR_BARRIER_TIMEOUT = 1u, KERR_FLAG_TIMEOUT = 2u };
 
 // Attributes of a kernel, set when they are first asked for and when a context has been made since (runtime.cu): set on every launch,
-// the two cost 0.4 us of a typed call's 6.3.
+// the two cost 0.1 us of the 2.9 that the host needs for a typed call.
 cudaError_t kernel_attributes(const void* kernel, int dynamic_shared, bool max_shared);
 // Dynamic shared memory of a launch.
 template <typename Kernel>
